@@ -329,7 +329,7 @@ struct AnaArgs {
     int dim, m, n, neig, kk;       // kk: k = dim - p (IRL) or k (lansvd)
     int irl, small_side;
     double tol;
-    double *wz;                    // bidiag_scratch(dim) doubles (lane-parallel path)
+    unsigned int *ticket;          // the last CTA of the lane-parallel path (zero between launches)
 };
 
 struct SweepArgs {
@@ -352,12 +352,13 @@ struct RitzArgs {
     double *Qt;         // dim^2 : right vectors' transpose
     double *w;          // 4*(dim+1)
     int dim, m, n;
-    double *wz;         // bidiag_scratch(dim) doubles (lane-parallel path)
+    double *X;          // (dim+1)^2: X(i, :) = (Q [y_i; 0])' (lane-parallel path; leading dimension dim+1)
+    const double *sig;  // the singular values of B in decreasing order (the last analysis; null: B changed since)
     int *flag;          // set to 1 when the lane-parallel vectors are not trusted
     int k, mstart;      // the wanted vectors: indices mstart-1 .. mstart+k-2
 };
 
-// scratch of the lane-parallel bidiagonal kernels for dimension dim
+// scratch of the sweeps' rotations for dimension dim
 inline size_t bidiag_scratch(int dim) { return 8 * (size_t)(dim + 1) * (dim + 1) + 64; }
 
 // analysis: nconv_out < 0 signals that the lane-parallel path declined and

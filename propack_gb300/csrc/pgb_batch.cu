@@ -72,7 +72,7 @@ struct BCfg {
 
 // per-CTA scratch (global memory): sizes for dimension dim
 struct BScrLayout {
-    size_t P, Q, coef, tw, Mt, Xt, W, total;
+    size_t P, Q, coef, tw, Xt, W, total;
 };
 __host__ __device__ inline BScrLayout bscr_layout(int dim, int maxrows)
 {
@@ -82,8 +82,7 @@ __host__ __device__ inline BScrLayout bscr_layout(int dim, int maxrows)
     L.Q = L.P + d1 * d1;
     L.coef = L.Q + (size_t)dim * dim;
     L.tw = L.coef + (size_t)dim * 4 * d1;
-    L.Mt = L.tw + (size_t)dim * 6 * dim;
-    L.Xt = L.Mt + d1 * d1;
+    L.Xt = L.tw + (size_t)dim * 8 * dim;
     L.W = L.Xt + d1 * dim;
     L.total = L.W + (size_t)maxrows * d1;
     return L;
@@ -93,7 +92,7 @@ struct BShared {
     double red[32];
     double h[BDIM_MAX + 2];
     double d[BDIM_MAX + 2], e[BDIM_MAX + 2], sig[BDIM_MAX + 2], bnd[BDIM_MAX + 2];
-    double b2[2 * BDIM_MAX + 2];
+    double b[2 * BDIM_MAX + 2], b2[2 * BDIM_MAX + 2];  // off-diagonals of the Golub-Kahan form of R, their squares
     double cs[BDIM_MAX + 2], sn[BDIM_MAX + 2];
     double shifts[BDIM_MAX + 2];
     double scal[8];
@@ -548,44 +547,38 @@ __device__ bool b_lanbpro(BProb &P, const BCfg &c, BShared &S, float2 *xq)
 }
 
 // ------------------------------------------------------------ analysis
-// singular values of R (S.d, S.e; upper bidiagonal dim x dim) into S.sig,
-// warp multisection per value
-__device__ void b_sigmas(int dim, BShared &S)
-{
-    for (int j = threadIdx.x; j < 2 * dim - 1; j += BT) {
-        const double b = tgk_b(S.d, S.e, j);
-        S.b2[j] = b * b;
-    }
-    if (threadIdx.x == 0) tgk_bounds(S.d, S.e, dim, S.scal[0], S.scal[1]);
-    __syncthreads();
-    for (int t = (threadIdx.x >> 5) + 1; t <= dim; t += BW) {
-        const double v = warp_sigma(dim, S.b2, t, S.scal[0], S.scal[1]);
-        if ((threadIdx.x & 31) == 0) S.sig[t - 1] = v;
-    }
-    __syncthreads();
-}
-
-// dlansvd_irl.F:218-290: sigma, bounds, convergence count (IRL branch)
+// dlansvd_irl.F:218-290: sigma, bounds, convergence count (IRL branch).
+// Warp 0 forms R (rotations in S.cs, S.sn) and its scaled Golub-Kahan form;
+// then one warp per value (pgb_bidiag.cuh).  The Ritz step reads all of it.
 __device__ int b_analyse(BProb &P, const BCfg &c, BShared &S, double *scr, const BScrLayout &L)
 {
-    const int dim = c.dim, mn = P.m < P.n ? P.m : P.n;
+    const int dim = c.dim, N = 2 * dim, mn = P.m < P.n ? P.m : P.n, lane = threadIdx.x & 31;
     for (int i = threadIdx.x; i < dim; i += BT) { S.d[i] = P.alpha[i]; S.e[i] = P.beta[i]; }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double c1 = 0.0, c2 = 0.0;
-        bdqr_dev(dim == mn, dim, S.d, S.e, &c1, &c2, nullptr, 0);
-        S.scal[2] = c1;
-        S.flag = 0;
+    if (threadIdx.x < 32) {
+        warp_bdqr(dim, S.d, S.e, dim != mn, S.cs, S.sn, S.b);
+        double gersh, pivmin, sc;
+        stage_tgk(N, S.b, S.b2, gersh, pivmin, sc);
+        if (lane == 0) {
+            S.scal[0] = gersh;
+            S.scal[1] = pivmin;
+            S.scal[2] = sc;
+            S.flag = 0;
+        }
     }
     __syncthreads();
-    b_sigmas(dim, S);
-    const double c1 = S.scal[2];
-    for (int i = threadIdx.x; i < dim; i += BT) {
-        double *Dp = scr + L.tw + (size_t)i * 6 * dim, *Dm = Dp + 2 * dim;
-        const double zn = tgk_twisted(S.d, S.e, dim, S.sig[i], S.scal[1], Dp, Dm, nullptr);
-        const double b = fabs(P.rnorm * c1 * sqrt(2.0) * zn);
-        if (!(b == b) || !(S.sig[i] == S.sig[i])) S.flag = 1;
-        S.bnd[i] = b;
+    const double gersh = S.scal[0], pivmin = S.scal[1], sc = S.scal[2], c1 = S.sn[dim - 1];
+    for (int i = threadIdx.x >> 5; i < dim; i += BW) {
+        const double sig = warp_sigma(dim, S.b2, i + 1, gersh, pivmin, sc);
+        double *fn = scr + L.tw + (size_t)i * 4 * N;
+        const double zn = warp_twisted(N, S.b, S.b2, sc != 0.0 ? sig * sc : sig, sc != 0.0 ? SFMIN : pivmin,
+                                       sc != 0.0, fn, fn + N, fn + 2 * N, fn + 3 * N);
+        if (lane == 0) {
+            const double b = fabs(P.rnorm * c1 * sqrt(2.0) * zn);
+            if (!(b == b) || !(sig == sig)) S.flag = 1;
+            S.sig[i] = sig;
+            S.bnd[i] = b;
+        }
     }
     __syncthreads();
     if (S.flag) return -1;
@@ -728,85 +721,43 @@ __device__ void b_restart(BProb &P, const BCfg &c, BShared &S, double *scr, cons
 }
 
 // --------------------------------------------------------------- Ritz
-// dritzvec.F:1-199 for the leading neig triplets: dbdqr with Q', the
-// singular vectors of R by twisted factorizations, then the products.
+// dritzvec.F:1-199 for the leading neig triplets: the singular vectors that
+// the analysis' twisted factorizations left in the scratch (R, its rotations
+// and its values are still in S), then the products.
 // Returns false (single-problem driver) for values closer than 1e-9 sigma_1.
 __device__ bool b_ritz(BProb &P, const BCfg &c, BShared &S, double *scr, const BScrLayout &L)
 {
-    const int dim = c.dim, dp1 = dim + 1, neig = c.neig, mn = P.m < P.n ? P.m : P.n;
-    for (int i = threadIdx.x; i < dim; i += BT) { S.d[i] = P.alpha[i]; S.e[i] = P.beta[i]; }
+    const int dim = c.dim, N = 2 * dim, dp1 = dim + 1, neig = c.neig, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) S.flag = 0;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double cs, sn, r;
-        double *D = S.d, *E = S.e;
-        int i;
-        for (i = 1; i <= dim - 1; i++) {
-            lartg(D[i - 1], E[i - 1], cs, sn, r);
-            D[i - 1] = r;
-            E[i - 1] = sn * D[i];
-            D[i] = cs * D[i];
-            S.cs[i - 1] = cs; S.sn[i - 1] = sn;
-        }
-        int nrot = dim - 1;
-        if (dim != mn) {
-            lartg(D[dim - 1], E[dim - 1], cs, sn, r);
-            D[dim - 1] = r;
-            E[dim - 1] = 0.0;
-            S.cs[dim - 1] = cs; S.sn[dim - 1] = sn;
-            nrot = dim;
-        }
-        S.scal[3] = nrot;
-        S.flag = 0;
-    }
-    __syncthreads();
-    const int nrot = (int)S.scal[3];
-    double *Mt = scr + L.Mt;
-    for (int j = threadIdx.x; j < dp1; j += BT) {
-        double *col = Mt + (size_t)j * dp1;
-        for (int i = 0; i < dp1; i++) col[i] = 0.0;
-        if (j == 0) col[0] = 1.0;
-        else if (j - 1 < nrot) { col[j - 1] = S.sn[j - 1]; col[j] = S.cs[j - 1]; }
-        else col[j] = 1.0;
-        for (int i = (j == 0 ? 0 : j); i < nrot; i++) {
-            col[i + 1] = -S.sn[i] * col[i];
-            col[i] = S.cs[i] * col[i];
-        }
-    }
-    b_sigmas(dim, S);
-    // vectors x_q (dim) and y_q (dim) into the twisted scratch rows
-    double *tw = scr + L.tw;
-    for (int q = threadIdx.x; q < neig; q += BT) {
+    double *tw = scr + L.tw, *Xt = scr + L.Xt;
+    for (int q = threadIdx.x >> 5; q < neig; q += BW) {
         const double smax = S.sig[0];
         const double gap = fmin(q > 0 ? S.sig[q - 1] - S.sig[q] : INFINITY, q + 1 < dim ? S.sig[q] - S.sig[q + 1] : INFINITY);
-        if (!(gap > 1e-9 * smax) || !(S.sig[q] > 1e-9 * smax)) { S.flag = 1; continue; }
-        double *Dp = tw + (size_t)q * 6 * dim, *Dm = Dp + 2 * dim, *z = Dm + 2 * dim;
-        tgk_twisted(S.d, S.e, dim, S.sig[q], S.scal[1], Dp, Dm, z);
+        double *x = tw + (size_t)q * 4 * N, *t0 = x + N, *y = x + 2 * N, *z = x + 3 * N;
         double nx = 0.0, ny = 0.0;
-        for (int t = 0; t < dim; t++) { nx += z[2 * t] * z[2 * t]; ny += z[2 * t + 1] * z[2 * t + 1]; }
-        if (!(nx > 0.0) || !(ny > 0.0)) { S.flag = 1; continue; }
+        for (int t = lane; t < dim; t += 32) { nx += z[2 * t] * z[2 * t]; ny += z[2 * t + 1] * z[2 * t + 1]; }
+        nx = warp_sum(nx);
+        ny = warp_sum(ny);
+        if (!(gap > 1e-9 * smax) || !(S.sig[q] > 1e-9 * smax) || !(nx > 0.0) || !(ny > 0.0)) {
+            if (lane == 0) S.flag = 1;
+            continue;
+        }
         const double ix = 1.0 / sqrt(nx), iy = 1.0 / sqrt(ny);
-        // x_q -> Dp[0..dim), y_q -> Dm[0..dim) (the pivots are no longer needed)
-        for (int t = 0; t < dim; t++) { Dp[t] = z[2 * t] * ix; Dm[t] = z[2 * t + 1] * iy; }
+        for (int t = lane; t < dim; t += 32) { x[t] = z[2 * t] * ix; y[t] = z[2 * t + 1] * iy; }
+        __syncwarp();
+        // Xt(:, q) = Q [y_q; 0]
+        warp_apply_q(dim, S.cs, S.sn, y, 1, t0, Xt + (size_t)q * dp1, 1);
     }
     __syncthreads();
     if (S.flag) return false;
-    // Xt(l, q) = sum_t y_q(t) Mt(t, l), l < dim + 1
-    double *Xt = scr + L.Xt;
-    for (int t2 = threadIdx.x; t2 < dp1 * neig; t2 += BT) {
-        const int l = t2 % dp1, q = t2 / dp1;
-        const double *y = tw + (size_t)q * 6 * dim + 2 * dim;
-        double a = 0.0;
-        for (int t = 0; t < dim; t++) a = fma(y[t], Mt[(size_t)l * dp1 + t], a);
-        Xt[(size_t)q * dp1 + l] = a;
-    }
-    __syncthreads();
     double *W = scr + L.W;
     for (int side = 0; side < 2; side++) {
         const int rows = side == 0 ? P.m : P.n, kin = side == 0 ? dp1 : dim;
         double *A = side == 0 ? P.U : P.V;
         for (int i = threadIdx.x; i < rows; i += BT)
             for (int q = 0; q < neig; q++) {
-                const double *b = side == 0 ? Xt + (size_t)q * dp1 : tw + (size_t)q * 6 * dim;
+                const double *b = side == 0 ? Xt + (size_t)q * dp1 : tw + (size_t)q * 4 * N;
                 double a = 0.0;
                 for (int l = 0; l < kin; l++) a = fma(A[(size_t)l * rows + i], b[l], a);
                 W[(size_t)q * rows + i] = a;

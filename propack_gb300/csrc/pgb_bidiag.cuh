@@ -20,20 +20,15 @@
 //                     Dhillon 1997; the "getvec" step of MRRR): forward and
 //                     backward pivot sequences, twist index r = argmin
 //                     |gamma_r|, then z from both ends.  z = (x1, y1, x2,
-//                     y2, ...)/sqrt(2) with R x = sigma y; one lane per value.
+//                     y2, ...)/sqrt(2) with R x = sigma y; one warp per value.
 //
 // All functions are plain arithmetic on caller-provided storage, so the same
 // code serves any dimension.
 #pragma once
 #include "pgb.cuh"
+#include "pgb_scalar.cuh"
 
 namespace pgb {
-
-// b[j], j = 0..2n-2: off-diagonal of TGK; b2 = b*b
-__device__ __forceinline__ double tgk_b(const double *d, const double *e, int j)
-{
-    return (j & 1) ? e[j >> 1] : d[j >> 1];
-}
 
 // number of negative pivots of TGK - lam I (size N = 2n)
 __device__ __forceinline__ int tgk_negcount(int N, const double *b2, double lam, double pivmin)
@@ -49,17 +44,83 @@ __device__ __forceinline__ int tgk_negcount(int N, const double *b2, double lam,
     return cnt;
 }
 
+// The same count without a division in the chain: p_j = -lam p_{j-1} -
+// b2_{j-1} p_{j-2} are the leading principal minors (Wilkinson's Sturm
+// sequence; the pivots above are p_j / p_{j-1}, so a negative pivot is a sign
+// change).  One dependent FMA per step, where the pivot recurrence waits for
+// an FP64 division (~1000 cycles a step on this GPU).  The roundings of a
+// step move the b2 it uses by a few eps relative, as those of the pivot
+// recurrence do (divide by p_{j-1}), so the count is as accurate.
+// The caller scales the matrix (tgk_scale) so that |b| <= 1 and lam <= 1:
+// |p| then grows by less than 2^12 in TGK_RESCALE steps, and shrinks by no
+// more than lam^TGK_RESCALE >= 2^-640, and is brought back to exponent 0
+// after them.  A p of exactly 0 takes the sign the pivot guard would give it.
+// lam < TGK_POLY_MIN (values below 1e-12 sigma_1) keeps the pivots.
+constexpr int TGK_RESCALE = 16;
+constexpr double TGK_POLY_MIN = 9.094947017729282e-13;  // 2^-40
+
+__device__ __forceinline__ double tgk_step(double p1, double p0, double b2, double lam)
+{
+    double p2 = fma(-lam, p1, -(b2 * p0));
+    if (((unsigned)__double2hiint(p2) << 1 | (unsigned)__double2loint(p2)) == 0u)
+        p2 = p1 * -7.888609052210118e-31;  // 2^-100: far below eps lam of the scaled matrix
+    return p2;
+}
+__device__ __forceinline__ void tgk_rescale(double &p1, double &p0)
+{
+    const int e1 = (__double2hiint(p1) >> 20) & 0x7ff, e0 = (__double2hiint(p0) >> 20) & 0x7ff;
+    const int k = 1023 - max(e1, e0);
+    const double f = __hiloint2double((min(max(k, -1000), 1000) + 1023) << 20, 0);
+    p1 *= f;
+    p0 *= f;
+}
+__device__ __forceinline__ int tgk_negcount_sturm(int N, const double *b2, double lam)
+{
+    double p0 = 1.0, p1 = -lam;
+    int cnt = 1, j = 1;
+    for (; j + TGK_RESCALE <= N; j += TGK_RESCALE) {
+#pragma unroll
+        for (int q = 0; q < TGK_RESCALE; q++) {
+            const double p2 = tgk_step(p1, p0, b2[j + q - 1], lam);
+            cnt += (int)((unsigned)(__double2hiint(p2) ^ __double2hiint(p1)) >> 31);
+            p0 = p1;
+            p1 = p2;
+        }
+        tgk_rescale(p1, p0);
+    }
+    for (; j < N; j++) {
+        const double p2 = tgk_step(p1, p0, b2[j - 1], lam);
+        cnt += (int)((unsigned)(__double2hiint(p2) ^ __double2hiint(p1)) >> 31);
+        p0 = p1;
+        p1 = p2;
+    }
+    return cnt;
+}
+
+// The power of two that brings the Gershgorin bound into [1/2, 1); 0 when
+// the matrix is too small, too large or not finite to be scaled (the pivot
+// recurrence then works on the matrix as it is).
+__device__ __forceinline__ double tgk_scale(double gersh)
+{
+    const int e = (__double2hiint(gersh) >> 20) & 0x7ff;
+    return e > 1023 - 400 && e < 1023 + 400 ? __hiloint2double((2045 - e) << 20, 0) : 0.0;
+}
+
 // sigma_t (t = 1: largest) of R by warp multisection; all lanes return it.
-// hi0: an upper bound of sigma_max (Gershgorin of TGK).
-__device__ inline double warp_sigma(int n, const double *b2, int t, double hi0, double pivmin)
+// b2: the squares of the off-diagonals times sc^2 (sc = 0: unscaled), hi0 an
+// upper bound of sigma_max (Gershgorin of TGK) of the unscaled matrix.
+__device__ inline double warp_sigma(int n, const double *b2, int t, double hi0, double pivmin, double sc)
 {
     const int lane = threadIdx.x & 31, N = 2 * n;
-    double lo = 0.0, hi = hi0;
+    const double frac = (double)(lane + 1) / 33.0;
+    const double guard = sc != 0.0 ? SFMIN : pivmin;
+    double lo = 0.0, hi = sc != 0.0 ? hi0 * sc : hi0;
     for (int round = 0; round < 64; round++) {
         if (hi - lo <= 2.0 * EPS * hi) break;
-        const double p = lo + (hi - lo) * ((double)(lane + 1) / 33.0);
+        const double p = lo + (hi - lo) * frac;
         // #(sigma > p) = 2n - negcount(p) for p > 0
-        const int above = N - tgk_negcount(N, b2, p, pivmin);
+        const bool sturm = sc != 0.0 && __all_sync(0xffffffffu, p >= TGK_POLY_MIN);
+        const int above = N - (sturm ? tgk_negcount_sturm(N, b2, p) : tgk_negcount(N, b2, p, guard));
         const unsigned bal = __ballot_sync(0xffffffffu, above >= t);
         const int q = __popc(bal);  // counts are monotone: lanes 0..q-1 satisfy
         const double plo = __shfl_sync(0xffffffffu, p, q > 0 ? q - 1 : 0);
@@ -69,75 +130,236 @@ __device__ inline double warp_sigma(int n, const double *b2, int t, double hi0, 
         lo = nlo;
         hi = nhi;
     }
-    return 0.5 * (lo + hi);
+    const double s = 0.5 * (lo + hi);
+    return sc != 0.0 ? s / sc : s;
 }
 
-// Twisted factorization of TGK - lam I.  Dp/Dm: N scratch each.  When z is
-// given it receives the unit eigenvector; returns |z_N| of the unit vector.
-__device__ inline double tgk_twisted(const double *d, const double *e, int n, double lam, double pivmin, double *Dp,
-                              double *Dm, double *z)
+// Product of v over the lanes up to this one.
+__device__ __forceinline__ double warp_scan_mul(double v)
 {
-    const int N = 2 * n;
-    double D = -lam;
-    if (fabs(D) < pivmin) D = -pivmin;
-    Dp[0] = D;
-    for (int j = 1; j < N; j++) {
-        const double bj = tgk_b(d, e, j - 1);
-        D = -lam - (bj * bj) / D;
-        if (fabs(D) < pivmin) D = -pivmin;
-        Dp[j] = D;
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v *= u;
     }
-    D = -lam;
-    if (fabs(D) < pivmin) D = -pivmin;
-    Dm[N - 1] = D;
-    for (int j = N - 2; j >= 0; j--) {
-        const double bj = tgk_b(d, e, j);
-        D = -lam - (bj * bj) / D;
-        if (fabs(D) < pivmin) D = -pivmin;
-        Dm[j] = D;
+    return v;
+}
+
+// Twisted factorization of TGK - lam I by one warp: the unit eigenvector
+// goes to bd, |z_N| is returned.  b: off-diagonals, b2 their squares, both
+// scaled like lam (scaled: |b| <= 1, see above).  The forward and backward
+// minors run in lanes 0 and 1 (one dependent FMA per step); the pivots,
+// their ratios, the twist index and the products z_j from it are then formed
+// by all lanes.  fn, fd, bn, bd: N doubles of scratch each.
+__device__ inline double warp_twisted(int N, const double *b, const double *b2, double lam, double pivmin,
+                                      bool scaled, double *fn, double *fd, double *bn, double *bd)
+{
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    if (lane < 2) {
+        double *num = lane ? bn : fn, *den = lane ? bd : fd;
+        const int i0 = lane ? N - 1 : 0, st = lane ? -1 : 1;
+        if (scaled && lam >= TGK_POLY_MIN) {
+            double p0 = 1.0, p1 = -lam;
+            num[i0] = p1;
+            den[i0] = 1.0;
+            for (int j = 1; j < N; j++) {
+                const int at = i0 + st * j;
+                // forward: b2[j-1]; backward: b2[N-1-j]
+                const double p2 = tgk_step(p1, p0, b2[lane ? at : at - 1], lam);
+                num[at] = p2;
+                den[at] = p1;
+                p0 = p1;
+                p1 = p2;
+                if ((j & (TGK_RESCALE - 1)) == 0) tgk_rescale(p1, p0);
+            }
+        } else {
+            double D = -lam;
+            if (fabs(D) < pivmin) D = -pivmin;
+            num[i0] = D;
+            den[i0] = 1.0;
+            for (int j = 1; j < N; j++) {
+                const int at = i0 + st * j;
+                D = -lam - b2[lane ? at : at - 1] / D;
+                if (fabs(D) < pivmin) D = -pivmin;
+                num[at] = D;
+                den[at] = 1.0;
+            }
+        }
     }
-    // gamma_j = Dp_j + Dm_j - (T - lam I)_jj = Dp_j + Dm_j + lam
+    __syncwarp();
+    // pivots; gamma_j = Dp_j + Dm_j - (T - lam I)_jj = Dp_j + Dm_j + lam
     int r = 0;
-    double gmin = fabs(Dp[0] + Dm[0] + lam);
-    for (int j = 1; j < N; j++) {
-        const double g = fabs(Dp[j] + Dm[j] + lam);
+    double gmin = INFINITY;
+    for (int j = lane; j < N; j += 32) {
+        const double dp = fn[j] / fd[j], dm = bn[j] / bd[j];
+        fn[j] = dp;
+        bn[j] = dm;
+        const double g = fabs(dp + dm + lam);
         if (g < gmin) { gmin = g; r = j; }
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double g = __shfl_xor_sync(FULL, gmin, o);
+        const int q = __shfl_xor_sync(FULL, r, o);
+        if (g < gmin || (g == gmin && q < r)) { gmin = g; r = q; }
+    }
+    __syncwarp();
     // z_r = 1; z_j = -(b_j / Dp_j) z_{j+1} above r, -(b_{j-1} / Dm_j) z_{j-1} below
-    double nrm2 = 1.0, zN = (r == N - 1) ? 1.0 : 0.0;
-    if (z) z[r] = 1.0;
-    double zz = 1.0;
-    for (int j = r - 1; j >= 0; j--) {
-        zz = -(tgk_b(d, e, j) / Dp[j]) * zz;
-        if (z) z[j] = zz;
-        nrm2 += zz * zz;
+    double nrm2 = 0.0, carry = 1.0, zN = 1.0;
+    for (int base = r - 1; base >= 0; base -= 32) {
+        const int j = base - lane;
+        double v = j >= 0 ? -(b[j] / fn[j]) : 1.0;
+        v = warp_scan_mul(v) * carry;
+        if (j >= 0) {
+            bd[j] = v;
+            nrm2 += v * v;
+        }
+        carry = __shfl_sync(FULL, v, 31);
     }
-    zz = 1.0;
-    for (int j = r + 1; j < N; j++) {
-        zz = -(tgk_b(d, e, j - 1) / Dm[j]) * zz;
-        if (z) z[j] = zz;
-        nrm2 += zz * zz;
-        if (j == N - 1) zN = zz;
+    carry = 1.0;
+    for (int base = r + 1; base < N; base += 32) {
+        const int j = base + lane;
+        double v = j < N ? -(b[j - 1] / bn[j]) : 1.0;
+        v = warp_scan_mul(v) * carry;
+        if (j < N) {
+            bd[j] = v;
+            nrm2 += v * v;
+        }
+        carry = __shfl_sync(FULL, v, 31);
+        zN = __shfl_sync(FULL, v, min(31, N - 1 - base));
     }
+    nrm2 = warp_sum(nrm2) + 1.0;
     const double inv = 1.0 / sqrt(nrm2);
-    if (z)
-        for (int j = 0; j < N; j++) z[j] *= inv;
+    __syncwarp();
+    if (lane == 0) bd[r] = 1.0;
+    __syncwarp();
+    for (int j = lane; j < N; j += 32) bd[j] *= inv;
+    __syncwarp();
     return fabs(zN) * inv;
 }
 
-// Gershgorin bound of TGK and the pivot guard (LAPACK dstebz's pivmin)
-__device__ __forceinline__ void tgk_bounds(const double *d, const double *e, int n, double &gersh, double &pivmin)
+// dbdqr (double/dbsvd.F:87-157) of the lower bidiagonal with diagonal al
+// and subdiagonal be by one warp: R's diagonal to b[0], b[2], ..., its
+// superdiagonal to b[1], b[3], ... (the off-diagonals of TGK in order), the
+// rotations to c, s.  last: the last row is rotated too (dim != min(m, n));
+// otherwise s[n-1] = 0.  The diagonal before rotation i, dt_i, obeys
+//   1/dt_{i+1}^2 = (1 + be_i^2 / dt_i^2) / al_{i+1}^2,
+// a recurrence of positive terms with one FMA per step (each error is damped
+// by the next step's weight < 1); everything else is formed by all lanes.
+// Zeros and values whose squares leave the FP64 range take the rotations
+// one after the other (dlartg's sequence).
+__device__ inline void warp_bdqr(int n, const double *al, const double *be, bool last, double *c, double *s,
+                                 double *b)
 {
-    double g = 0.0, bmax2 = 0.0;
-    const int N = 2 * n;
-    for (int j = 0; j < N; j++) {
-        const double left = j > 0 ? fabs(tgk_b(d, e, j - 1)) : 0.0;
-        const double right = j < N - 1 ? fabs(tgk_b(d, e, j)) : 0.0;
-        g = fmax(g, left + right);
-        if (j < N - 1) bmax2 = fmax(bmax2, right * right);
+    const int lane = threadIdx.x & 31;
+    for (int i = lane; i < n; i += 32) {
+        const double g = 1.0 / (al[i] * al[i]);
+        c[i] = g;
+        s[i] = i > 0 ? be[i - 1] * be[i - 1] * g : 0.0;
     }
-    gersh = g * (1.0 + 4.0 * EPS) + SFMIN;
-    pivmin = SFMIN * fmax(1.0, bmax2);
+    __syncwarp();
+    if (lane == 0) {
+        double r = c[0];
+        b[0] = r;
+        for (int i = 1; i < n; i++) {
+            r = fma(s[i], r, c[i]);
+            b[2 * i] = r;
+        }
+    }
+    __syncwarp();
+    bool ok = true;
+    for (int i = lane; i < n; i += 32) ok = ok && b[2 * i] > 1e-280 && b[2 * i] < 1e280 && fabs(be[i]) < 1e140;
+    if (__all_sync(0xffffffffu, ok)) {
+        unsigned par = 0;  // sign of dt_i: the product of the signs of al_0 .. al_i
+        for (int i0 = 0; i0 < n; i0 += 32) {
+            const int i = i0 + lane;
+            const unsigned neg = __ballot_sync(0xffffffffu, i < n && al[i] < 0.0);
+            if (i < n) {
+                const unsigned q = (__popc(neg & (0xffffffffu >> (31 - lane))) + par) & 1u;
+                const double r = b[2 * i], bi = be[i];
+                const double dt = q ? -rsqrt(r) : rsqrt(r);
+                if (i < n - 1 || last) {
+                    const double h = sqrt(fma(bi, bi, 1.0 / r));
+                    c[i] = dt / h;
+                    s[i] = bi / h;
+                    b[2 * i] = h;
+                } else {
+                    c[i] = 1.0;
+                    s[i] = 0.0;
+                    b[2 * i] = dt;
+                }
+                if (i < n - 1) b[2 * i + 1] = s[i] * al[i + 1];
+            }
+            par += __popc(neg);
+        }
+    } else if (lane == 0) {
+        double dt = al[0], cs, sn, r;
+        for (int i = 0; i < n; i++) {
+            if (i < n - 1 || last) lartg(dt, be[i], cs, sn, r);
+            else { cs = 1.0; sn = 0.0; r = dt; }
+            c[i] = cs;
+            s[i] = sn;
+            b[2 * i] = r;
+            if (i < n - 1) {
+                b[2 * i + 1] = sn * al[i + 1];
+                dt = cs * al[i + 1];
+            }
+        }
+    }
+    __syncwarp();
+}
+
+// w = Q [y; 0] for the rotations of warp_bdqr (Q' B = [R; 0]), n + 1 entries:
+// y at y[t * sy], t < n; w to w[t * sw].  t0: n + 1 doubles of scratch.  The
+// chain is one FMA per step in lane 0.
+__device__ inline void warp_apply_q(int n, const double *c, const double *s, const double *y, int sy, double *t0,
+                                    double *w, size_t sw)
+{
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) {
+        double t = 0.0;
+        t0[n] = 0.0;
+        for (int i = n - 1; i >= 0; i--) {
+            t = fma(-s[i], t, c[i] * y[i * sy]);
+            t0[i] = t;
+        }
+        w[0] = t;
+    }
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) w[(size_t)(i + 1) * sw] = fma(c[i], t0[i + 1], s[i] * y[i * sy]);
+    __syncwarp();
+}
+
+// Gershgorin bound and pivot guard of TGK from its off-diagonals, one warp
+__device__ inline void warp_tgk_bounds(int N, const double *b, double &gersh, double &pivmin)
+{
+    const int lane = threadIdx.x & 31;
+    double g = 0.0, m2 = 0.0;
+    for (int j = lane; j < N; j += 32) {
+        const double left = j > 0 ? fabs(b[j - 1]) : 0.0, right = j < N - 1 ? fabs(b[j]) : 0.0;
+        g = fmax(g, left + right);
+        m2 = fmax(m2, right * right);
+    }
+    gersh = warp_max(g) * (1.0 + 4.0 * EPS) + SFMIN;
+    pivmin = SFMIN * fmax(1.0, warp_max(m2));
+}
+
+// The off-diagonals of TGK and their squares, scaled by the power of two of
+// the Gershgorin bound; one warp.
+__device__ inline void stage_tgk(int N, double *b, double *b2, double &gersh, double &pivmin, double &sc)
+{
+    warp_tgk_bounds(N, b, gersh, pivmin);
+    sc = tgk_scale(gersh);
+    const double f = sc != 0.0 ? sc : 1.0;
+    __syncwarp();
+    for (int j = threadIdx.x & 31; j < N - 1; j += 32) {
+        const double v = b[j] * f;
+        b[j] = v;
+        b2[j] = v * v;
+    }
+    __syncwarp();
 }
 
 }  // namespace pgb

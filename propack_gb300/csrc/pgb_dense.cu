@@ -482,117 +482,131 @@ __global__ void k_ritz_prep(RitzArgs a, int use_smem)
 
 // bidiagonal size up to which the lane-parallel kernels are used
 constexpr int PAR_DIM_MAX = 2048;
+constexpr double EPS34 = 1.0815775704056441e-12;  // EPS^(3/4)
 
-// dbdqr of B into a1 (d) / b1 (e), c1 -> bnd[dim-1], c2 -> bnd[dim]
-__global__ void k_ana_qr(AnaArgs a)
-{
-    const int dim = a.dim;
-    for (int i = threadIdx.x; i < dim; i += blockDim.x) { a.a1[i] = a.balpha[i]; a.b1[i] = a.bbeta[i]; }
-    for (int i = threadIdx.x; i <= dim; i += blockDim.x) a.bnd[i] = 0.0;
-    __syncthreads();
-    const int mn = a.m < a.n ? a.m : a.n;
-    if (threadIdx.x == 0) bdqr_dev(dim == mn, dim, a.a1, a.b1, &a.bnd[dim - 1], &a.bnd[dim], nullptr, 0);
-}
+// doubles of shared memory: al/be (reused by the factorization), b, b2 and
+// three more arrays of the Golub-Kahan size N = 2 dim; the Ritz kernel keeps
+// the rotations beside them
+static size_t ana_smem(int dim) { return sizeof(double) * 12 * (size_t)dim; }
+static size_t ritz_smem(int dim) { return sizeof(double) * 14 * (size_t)dim; }
 
-// sigma_t of the upper bidiagonal (d, e), one warp per t; sig[t-1]
-__global__ void __launch_bounds__(256) k_bisect(const double *d, const double *e, int n, double *sig)
+// The bookkeeping of k_analyse (anorm, drefinebounds, convergence count) on
+// the values w[i] and bounds w[dim + 1 + i], by one warp.  drefinebounds'
+// second loop updates bound i from the already refined bound i - 1; the warp
+// repeats it for all i at once until nothing changes, which is that loop's
+// result (the first entry is final after one pass, the next after two, ...),
+// usually after two or three passes.
+__device__ void ana_finish_warp(const AnaArgs &a, double *sm)
 {
-    extern __shared__ double b2[];
-    const int N = 2 * n;
-    for (int j = threadIdx.x; j < N - 1; j += blockDim.x) {
-        const double b = tgk_b(d, e, j);
-        b2[j] = b * b;
+    const unsigned FULL = 0xffffffffu;
+    const int dim = a.dim, lane = threadIdx.x;
+    double *th = sm, *bd = th + dim, *cur = bd + dim, *nxt = cur + dim;
+    const double rnorm = a.ctl->rnorm;
+    bool bad = false;
+    for (int i = lane; i < dim; i += 32) {
+        const double sg = __ldcg(a.w + i), bi = __ldcg(a.w + dim + 1 + i);
+        bad = bad || !(bi == bi) || !(sg == sg);
+        th[i] = sg;
+        bd[i] = fabs(rnorm * bi);
     }
-    __shared__ double gs, ps;
-    if (threadIdx.x == 0) tgk_bounds(d, e, n, gs, ps);
-    __syncthreads();
-    const int t = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5) + 1;
-    if (t > n) return;
-    const double s = warp_sigma(n, b2, t, gs, ps);
-    if ((threadIdx.x & 31) == 0) sig[t - 1] = s;
-}
-
-// bounds from the last components of the left vectors: one thread per
-// singular value, one warp per CTA (each twisted factorisation divides at
-// every step, and the FP64 pipe is the SM's); into w[dim + 1 + i]
-__global__ void k_ana_twisted(AnaArgs a)
-{
-    const int dim = a.dim, N = 2 * dim;
-    const double *sig = a.w;
-    __shared__ double gs, ps;
-    if (threadIdx.x == 0) tgk_bounds(a.a1, a.b1, dim, gs, ps);
-    __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= dim) return;
-    double *Dp = a.wz + (size_t)i * 2 * N, *Dm = Dp + N;
-    const double zn = tgk_twisted(a.a1, a.b1, dim, sig[i], ps, Dp, Dm, nullptr);
-    a.w[dim + 1 + i] = a.bnd[dim - 1] * (sqrt(2.0) * zn);
-}
-
-// the same bookkeeping as k_analyse (anorm, refinebounds, convergence
-// count) on the bounds of k_ana_twisted
-__global__ void k_ana_finish(AnaArgs a)
-{
-    const int dim = a.dim;
-    const double *sig = a.w;
-    __shared__ int bad;
-    if (threadIdx.x == 0) bad = 0;
-    __syncthreads();
-    double bi = 0.0;
-    if (threadIdx.x < dim) {
-        const int i = threadIdx.x;
-        bi = a.w[dim + 1 + i];
-        if (!(bi == bi) || !(sig[i] == sig[i])) bad = 1;
-    }
-    __syncthreads();
-    if (bad) {
-        if (threadIdx.x == 0) *a.nconv_out = -1;
+    if (__any_sync(FULL, bad)) {
+        if (lane == 0) *a.nconv_out = -1;
         return;
     }
-    if (threadIdx.x < dim) {
-        a.bnd[threadIdx.x] = bi;
-        a.a1[threadIdx.x] = sig[threadIdx.x];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double *d = a.a1, *bnd = a.bnd;
-        const int mn = a.m < a.n ? a.m : a.n;
-        const double eps34 = pow(EPS, 0.75);
-        const double epsn = (double)(a.m > a.n ? a.m : a.n) * EPS / 2.0;
-        double anorm = *a.anorm_drv;
-        if (dim > 5) anorm = d[0];
-        else anorm = fmax(anorm, d[0]);
-        *a.anorm_drv = anorm;
-        const double rnorm = a.ctl->rnorm;
-        for (int i = 0; i < dim; i++) bnd[i] = fabs(rnorm * bnd[i]);
-        int nconv = 0;
-        if (a.irl) {
-            const int neig = a.neig;
-            refinebounds_dev(mn, dim < neig ? dim : neig, d, bnd, epsn * anorm, eps34);
-            int i = 1;
-            const int lim = dim < neig ? dim : neig;
-            while (i <= lim) {
-                if (bnd[i - 1] <= a.tol * d[i - 1]) {
-                    a.sigma_out[nconv] = d[i - 1];
-                    a.bnd_out[nconv] = bnd[i - 1];
-                    nconv++;
-                    i++;
-                } else {
-                    i = a.kk + 1;
-                }
-            }
-        } else {
-            refinebounds_dev(mn, dim, d, bnd, epsn * anorm, eps34);
-            const int lim = dim < a.kk ? dim : a.kk;
-            for (int i = 0; i < lim; i++) a.bnd_out[i] = bnd[i];
-            int i = 0;
-            while (i < lim) {
-                if (bnd[i] <= a.tol * d[i]) { a.sigma_out[nconv] = d[i]; nconv++; i++; }
-                else i = a.kk;
-            }
+    __syncwarp();
+    const int mn = a.m < a.n ? a.m : a.n;
+    const double epsn = (double)(a.m > a.n ? a.m : a.n) * EPS / 2.0;
+    double anorm = *a.anorm_drv;
+    __syncwarp();
+    anorm = dim > 5 ? th[0] : fmax(anorm, th[0]);
+    if (lane == 0) *a.anorm_drv = anorm;
+    const int k = a.irl ? min(dim, a.neig) : dim;
+    const double tol = epsn * anorm;
+    if (k > 1) {
+        bool close = false;
+        for (int i = lane; i + 1 < k; i += 32) {
+            const double g = fabs(th[i] - th[i + 1]);
+            close = close || g < EPS34 * th[i] || g < EPS34 * th[i + 1];
         }
-        *a.nconv_out = nconv;
+        if (__any_sync(FULL, close)) {
+            if (lane == 0) mergebounds_dev(k, th, bd, tol, EPS34);
+            __syncwarp();
+        }
+        for (int i = lane; i < k; i += 32) cur[i] = bd[i];
+        __syncwarp();
+        for (int pass = 0; pass < k; pass++) {
+            bool moved = false;
+            for (int i = lane; i < k; i += 32) {
+                double v = bd[i];
+                if (i < k - 1 || k == mn) {
+                    double gap = INFINITY;
+                    if (i < mn - 1) gap = fabs(th[i] - th[i + 1]) - fmax(bd[i], bd[i + 1]);
+                    if (i > 0) gap = fmin(gap, fabs(th[i - 1] - th[i]) - fmax(cur[i - 1], bd[i]));
+                    if (gap > v) v = v * (v / gap);
+                }
+                moved = moved || v != cur[i];
+                nxt[i] = v;
+            }
+            __syncwarp();
+            double *t = cur;
+            cur = nxt;
+            nxt = t;
+            if (!__any_sync(FULL, moved)) break;
+        }
+        for (int i = lane; i < k; i += 32) bd[i] = cur[i];
+        __syncwarp();
     }
+    for (int i = lane; i < dim; i += 32) {
+        a.a1[i] = th[i];
+        a.bnd[i] = bd[i];
+    }
+    const int lim = min(dim, a.irl ? a.neig : a.kk);
+    int nconv = 0;
+    for (int i0 = 0; i0 < lim; i0 += 32) {
+        const int i = i0 + lane;
+        const unsigned m = __ballot_sync(FULL, i < lim && bd[i] <= a.tol * th[i]);
+        const int run = m == FULL ? 32 : __ffs(~m) - 1;
+        nconv += run;
+        if (run < 32) break;
+    }
+    for (int i = lane; i < lim; i += 32) {
+        if (i < nconv) a.sigma_out[i] = th[i];
+        if (i < nconv || !a.irl) a.bnd_out[i] = bd[i];
+    }
+    if (lane == 0) *a.nconv_out = nconv;
+}
+
+// One warp (a CTA of its own, so that its Sturm sequences have an SM's FP64
+// pipe to themselves) per singular value of R: dbdqr of B (every CTA forms
+// R for itself: ~10 us against a launch and a round trip through L2), the
+// value by multisection, and the Ritz bound from the last component of its
+// left vector by the twisted factorization; the last CTA to finish does the
+// bookkeeping.  Bound by the chain of 2 dim dependent FP64 FMAs of each
+// Sturm sequence, ~11 rounds of them.
+__global__ void __launch_bounds__(32) k_ana_values(AnaArgs a, int finish)
+{
+    extern __shared__ double sm[];
+    const int dim = a.dim, N = 2 * dim, lane = threadIdx.x;
+    double *al = sm, *be = al + dim, *b = sm + N, *b2 = b + N, *fd = b2 + N, *bn = fd + N, *bd = bn + N;
+    for (int i = lane; i < dim; i += 32) {
+        al[i] = a.balpha[i];
+        be[i] = a.bbeta[i];
+    }
+    __syncwarp();
+    warp_bdqr(dim, al, be, dim != (a.m < a.n ? a.m : a.n), fd, bn, b);
+    const double c1 = bn[dim - 1];
+    double gersh, pivmin, sc;
+    stage_tgk(N, b, b2, gersh, pivmin, sc);
+    const int t = blockIdx.x;
+    const double sig = warp_sigma(dim, b2, t + 1, gersh, pivmin, sc);
+    double zn = 0.0;
+    if (finish)
+        zn = warp_twisted(N, b, b2, sc != 0.0 ? sig * sc : sig, sc != 0.0 ? SFMIN : pivmin, sc != 0.0, al, fd, bn, bd);
+    if (lane == 0) {
+        a.w[t] = sig;
+        a.w[dim + 1 + t] = c1 * (sqrt(2.0) * zn);
+    }
+    if (finish && last_cta(a.ticket)) ana_finish_warp(a, sm);
 }
 
 // ----------------------------------------------- wavefront IRL sweeps
@@ -710,82 +724,55 @@ __global__ void __launch_bounds__(APPLY_WARPS * 32) k_irl_apply(SweepArgs a, int
 }
 
 // ----------------------------------------------- lane-parallel Ritz prep
-// dbdqr with Q' (dritzvec.F:112-114): thread 0 runs the rotation chain on
-// R, then one thread per column of Mt replays it (the same operations as
-// bdqr_dev's Q' update, column by column).
-__global__ void k_ritz_qr(RitzArgs a)
+// The wanted singular vector pairs (indices mstart-1 .. mstart+k-2 of the
+// decreasing order), one warp (CTA) each: R of dbdqr, the pair (y_i, x_i) of R
+// by the twisted factorization at the value sig[i], then Qt(i, :) = x_i' and
+// X(i, :) = (Q [y_i; 0])' by the recorded rotations (dritzvec.F:112-130; the
+// reference forms Q' and multiplies).  Values closer than 1e-9 sigma_max to
+// a neighbour are left to the QR path (flag), since single twisted vectors
+// are only accurate to eps/gap.  Bound by three chains of dim to 2 dim
+// dependent FMAs.
+__global__ void __launch_bounds__(32) k_ritz_pairs(RitzArgs a)
 {
-    const int dim = a.dim, n1 = dim + 1;
-    double *cs = a.w, *sn = a.w + n1;
-    for (int i = threadIdx.x; i < dim; i += blockDim.x) { a.D[i] = a.balpha[i]; a.E[i] = a.bbeta[i]; }
-    if (threadIdx.x == 0) *a.flag = 0;
-    __syncthreads();
-    const int mn = a.m < a.n ? a.m : a.n;
-    __shared__ int nrot_s;
-    if (threadIdx.x == 0) {
-        double c, s, r;
-        double *D = a.D, *E = a.E;
-        int i;
-        for (i = 1; i <= dim - 1; i++) {
-            lartg(D[i - 1], E[i - 1], c, s, r);
-            D[i - 1] = r;
-            E[i - 1] = s * D[i];
-            D[i] = c * D[i];
-            cs[i - 1] = c; sn[i - 1] = s;
-        }
-        int nrot = dim - 1;
-        if (dim != mn) {
-            lartg(D[dim - 1], E[dim - 1], c, s, r);
-            D[dim - 1] = r;
-            E[dim - 1] = 0.0;
-            cs[dim - 1] = c; sn[dim - 1] = s;
-            nrot = dim;
-        }
-        nrot_s = nrot;
+    extern __shared__ double sm[];
+    const int dim = a.dim, N = 2 * dim, lane = threadIdx.x;
+    const int i = a.mstart - 1 + blockIdx.x;
+    const double *sig = a.sig;
+    const double smax = sig[0], si = sig[i];
+    const double gap = fmin(i > 0 ? sig[i - 1] - si : INFINITY, i + 1 < dim ? si - sig[i + 1] : INFINITY);
+    if (!(gap > 1e-9 * smax) || !(si > 1e-9 * smax)) {
+        if (lane == 0) *a.flag = 1;
+        return;
     }
-    __syncthreads();
-    const int nrot = nrot_s;
-    // column j (0-based) of Q': created by rotation j-1 (for j >= 1), then
-    // rotated by rotations j, j+1, ..., nrot-1 on rows (i, i+1)
-    for (int j = threadIdx.x; j < n1; j += blockDim.x) {
-        double *col = a.Mt + (size_t)j * n1;
-        for (int i = 0; i < n1; i++) col[i] = 0.0;
-        if (j == 0) col[0] = 1.0;
-        else if (j - 1 < nrot) { col[j - 1] = sn[j - 1]; col[j] = cs[j - 1]; }
-        else col[j] = 1.0;
-        for (int i = (j == 0 ? 0 : j); i < nrot; i++) {
-            col[i + 1] = -sn[i] * col[i];
-            col[i] = cs[i] * col[i];
-        }
+    double *al = sm, *be = al + dim, *c = sm + N, *s = c + dim, *b = c + N, *b2 = b + N, *fd = b2 + N, *bn = fd + N,
+           *bd = bn + N;
+    for (int t = lane; t < dim; t += 32) {
+        al[t] = a.balpha[t];
+        be[t] = a.bbeta[t];
     }
-}
-
-// The wanted singular vector pairs of R (indices mstart-1 .. mstart+k-2 of
-// the decreasing order), one lane each: P(:, i) = y_i, Qt(i, :) = x_i'.
-// Values closer than 1e-9 sigma_max to a neighbour are left to the QR path
-// (flag), since single twisted vectors are only accurate to eps/gap.
-__global__ void k_ritz_vecs(RitzArgs a)
-{
-    const int dim = a.dim, N = 2 * dim;
-    const double *sig = a.w + 2 * (dim + 1);
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= a.k) return;
-    const int i = a.mstart - 1 + q;
-    const double smax = sig[0];
-    const double gap = fmin(i > 0 ? sig[i - 1] - sig[i] : INFINITY, i + 1 < dim ? sig[i] - sig[i + 1] : INFINITY);
-    double gs, ps;
-    tgk_bounds(a.D, a.E, dim, gs, ps);
-    if (!(gap > 1e-9 * smax) || !(sig[i] > 1e-9 * smax)) { *a.flag = 1; return; }
-    double *Dp = a.wz + (size_t)q * 3 * N, *Dm = Dp + N, *z = Dm + N;
-    tgk_twisted(a.D, a.E, dim, sig[i], ps, Dp, Dm, z);
+    __syncwarp();
+    warp_bdqr(dim, al, be, dim != (a.m < a.n ? a.m : a.n), c, s, b);
+    double gersh, pivmin, sc;
+    stage_tgk(N, b, b2, gersh, pivmin, sc);
+    warp_twisted(N, b, b2, sc != 0.0 ? si * sc : si, sc != 0.0 ? SFMIN : pivmin, sc != 0.0, al, fd, bn, bd);
     double nx = 0.0, ny = 0.0;
-    for (int t = 0; t < dim; t++) { nx += z[2 * t] * z[2 * t]; ny += z[2 * t + 1] * z[2 * t + 1]; }
-    if (!(nx > 0.0) || !(ny > 0.0) || !(nx < INFINITY) || !(ny < INFINITY)) { *a.flag = 1; return; }
-    const double ix = 1.0 / sqrt(nx), iy = 1.0 / sqrt(ny);
-    for (int t = 0; t < dim; t++) {
-        a.Qt[(size_t)t * dim + i] = z[2 * t] * ix;
-        a.P[(size_t)i * dim + t] = z[2 * t + 1] * iy;
+    for (int t = lane; t < dim; t += 32) {
+        nx += bd[2 * t] * bd[2 * t];
+        ny += bd[2 * t + 1] * bd[2 * t + 1];
     }
+    nx = warp_sum(nx);
+    ny = warp_sum(ny);
+    if (!(nx > 0.0) || !(ny > 0.0) || !(nx < INFINITY) || !(ny < INFINITY)) {
+        if (lane == 0) *a.flag = 1;
+        return;
+    }
+    const double ix = 1.0 / sqrt(nx), iy = 1.0 / sqrt(ny);
+    for (int t = lane; t < dim; t += 32) {
+        a.Qt[(size_t)t * dim + i] = bd[2 * t] * ix;
+        bn[t] = bd[2 * t + 1] * iy;
+    }
+    __syncwarp();
+    warp_apply_q(dim, c, s, bn, 1, fd, a.X + i, dim + 1);
 }
 
 // ------------------------------------------------------------------ GEMM
@@ -868,35 +855,16 @@ void launch_analyse_qr(const AnaArgs &a, cudaStream_t s)
     PGB_PROF(PK_ANALYSE, s, k_analyse<<<1, 32, use ? bytes : 0, s>>>(a, use));
     PGB_LAUNCHED();
 }
-static bool bisect_fits(int dim)
-{
-    return dim <= PAR_DIM_MAX && smem_for((const void *)k_bisect, sizeof(double) * 2 * (size_t)dim) != 0;
-}
-static void launch_bisect(const double *d, const double *e, int n, double *sig, cudaStream_t s)
-{
-    // one warp per CTA, so that each singular value's Sturm sequences (an
-    // FP64 division per step) have an SM's FP64 pipe to themselves
-    const int wpb = 1;
-    k_bisect<<<(n + wpb - 1) / wpb, 32 * wpb, sizeof(double) * 2 * (size_t)n, s>>>(d, e, n, sig);
-    PGB_LAUNCHED();
-}
 void launch_analyse(const AnaArgs &a, cudaStream_t s)
 {
     // the smallest triplets (which = 'S') keep the QR path: their twisted
     // vectors on the Golub-Kahan form are not reliable near sigma = 0
-    if (a.small_side || !a.wz || a.dim > 1024 || !bisect_fits(a.dim)) {
+    if (a.small_side || a.dim > 1024 || !smem_for((const void *)k_ana_values, ana_smem(a.dim))) {
         launch_analyse_qr(a, s);
         return;
     }
-    PGB_PROF(PK_ANALYSE, s, {
-        k_ana_qr<<<1, 32, 0, s>>>(a);
-        PGB_LAUNCHED();
-        launch_bisect(a.a1, a.b1, a.dim, a.w, s);
-        k_ana_twisted<<<(a.dim + 31) / 32, 32, 0, s>>>(a);
-        PGB_LAUNCHED();
-        k_ana_finish<<<1, ((a.dim + 31) / 32) * 32, 0, s>>>(a);
-        PGB_LAUNCHED();
-    });
+    PGB_PROF(PK_ANALYSE, s, k_ana_values<<<a.dim, 32, ana_smem(a.dim), s>>>(a, 1));
+    PGB_LAUNCHED();
 }
 void launch_sweeps(const SweepArgs &a, cudaStream_t s)
 {
@@ -929,12 +897,22 @@ void launch_ritz_prep_qr(const RitzArgs &a, cudaStream_t s)
 }
 bool launch_ritz_prep(const RitzArgs &a, cudaStream_t s)
 {
-    if (a.mstart != 1 || !a.wz || !a.flag || a.k < 1 || !bisect_fits(a.dim)) return false;
+    if (a.mstart != 1 || !a.flag || a.k < 1 || a.dim > PAR_DIM_MAX ||
+        !smem_for((const void *)k_ritz_pairs, ritz_smem(a.dim)))
+        return false;
+    RitzArgs r = a;
     PGB_PROF(PK_RITZ, s, {
-        k_ritz_qr<<<1, 256, 0, s>>>(a);
-        PGB_LAUNCHED();
-        launch_bisect(a.D, a.E, a.dim, a.w + 2 * (a.dim + 1), s);
-        k_ritz_vecs<<<(a.k + 31) / 32, 32, 0, s>>>(a);
+        PGB_CUDA(cudaMemsetAsync(a.flag, 0, sizeof(int), s));
+        if (!r.sig) {
+            // B changed since the last analysis: its values first
+            AnaArgs v = {};
+            v.balpha = a.balpha; v.bbeta = a.bbeta; v.w = a.w; v.dim = a.dim; v.m = a.m; v.n = a.n;
+            if (!smem_for((const void *)k_ana_values, ana_smem(a.dim))) return false;
+            k_ana_values<<<a.dim, 32, ana_smem(a.dim), s>>>(v, 0);
+            PGB_LAUNCHED();
+            r.sig = a.w;
+        }
+        k_ritz_pairs<<<a.k, 32, ritz_smem(a.dim), s>>>(r);
         PGB_LAUNCHED();
     });
     return true;

@@ -254,7 +254,8 @@ struct Ctx {
     int *nconv = nullptr;
     double *D = nullptr, *E = nullptr, *Mt = nullptr, *Pr = nullptr, *Qt = nullptr, *X = nullptr;
     double *wz = nullptr;                   // scratch of the lane-parallel bidiagonal kernels
-    int *dflag = nullptr;
+    int *dflag = nullptr;                   // Ritz path flag, ticket of the analysis
+    int sig_dim = 0;                        // dimension whose singular values a1 holds (0: B changed since)
     void *gout = nullptr;                   // GEMM output scratch (vector type)
     // FP32 (hi, lo) planes of the FP64 bases for the Gram-Schmidt passes,
     // their per-column flags and the planes of the vector being
@@ -1253,9 +1254,11 @@ static void ritz_side(Ctx &c, int side, T *A, int lda, int rows, int nc, int kk,
 }
 
 // the bidiagonal analysis; returns the number of converged values
-static int analyse(Ctx &c, const AnaArgs &a)
+static int analyse(Ctx &c, AnaArgs &a)
 {
+    a.ticket = (unsigned int *)c.dflag + 1;
     launch_analyse(a, c.s);
+    c.sig_dim = a.dim;
     g_last.nbsvd++;
     int nc = 0;
     PGB_CUDA(cudaMemcpyAsync(c.hscal, c.nconv, sizeof(int), cudaMemcpyDeviceToHost, c.s));
@@ -1278,7 +1281,8 @@ static void dev_ritzvec(Ctx &c, bool small_side, bool du, bool dv, int k, int di
     RitzArgs r;
     r.balpha = c.balpha; r.bbeta = c.bbeta; r.D = c.D; r.E = c.E; r.Mt = c.Mt; r.P = c.Pr; r.Qt = c.Qt;
     r.w = c.w; r.dim = dim; r.m = c.m; r.n = c.n;
-    r.wz = c.wz; r.flag = c.dflag;
+    r.X = c.X; r.flag = c.dflag;
+    r.sig = c.sig_dim == dim ? c.a1 : nullptr;
     r.mstart = small_side ? dim - k + 1 : 1;
     r.k = k;
     bool qr = !launch_ritz_prep(r, c.s);
@@ -1292,8 +1296,8 @@ static void dev_ritzvec(Ctx &c, bool small_side, bool du, bool dv, int k, int di
     }
     if (qr) launch_ritz_prep_qr(r, c.s);
     const int dp1 = dim + 1;
-    // X = P' Mt(1:dim, 1:dim+1)   (dim x dim+1, ld dim+1)
-    gemm<double>(dim, dp1, dim, c.Pr, dim, true, c.Mt, dp1, false, c.X, dp1, c.s);
+    // QR path: X = P' Mt(1:dim, 1:dim+1)   (dim x dim+1, ld dim+1)
+    if (qr) gemm<double>(dim, dp1, dim, c.Pr, dim, true, c.Mt, dp1, false, c.X, dp1, c.s);
     const int mstart = small_side ? dim - k + 1 : 1;
     if (du) ritz_side<T>(c, 0, (T *)c.U, c.ldu, c.m, k, dp1, c.X + (mstart - 1), dp1);
     if (dv) ritz_side<T>(c, 1, (T *)c.V, c.ldv, c.n, k, dim, c.Qt + (mstart - 1), dim);
@@ -1451,7 +1455,7 @@ static void irl_loop(Ctx &c, const IrlIn &in, double *doption, const int *ioptio
             a.balpha = c.balpha; a.bbeta = c.bbeta; a.a1 = c.a1; a.b1 = c.b1; a.bnd = c.bnd; a.w = c.w;
             a.ctl = c.ctl; a.sigma_out = c.sig_out; a.bnd_out = c.bnd_out; a.nconv_out = c.nconv;
             a.anorm_drv = c.anorm_drv; a.dim = dim; a.m = m; a.n = n; a.neig = neig0; a.kk = k;
-            a.irl = 1; a.small_side = in.small_side; a.tol = in.tol; a.wz = c.wz;
+            a.irl = 1; a.small_side = in.small_side; a.tol = in.tol;
             nconv = analyse(c, a);
         }
         if (ierr < 0) {
@@ -1474,6 +1478,7 @@ static void irl_loop(Ctx &c, const IrlIn &in, double *doption, const int *ioptio
                 sw.shifts = c.shifts; sw.w = c.w; sw.ctl = c.ctl; sw.dim = dim; sw.k = k; sw.neig = neig0;
                 sw.small_side = in.small_side; sw.min_relgap = doption[3]; sw.wz = c.wz;
                 launch_sweeps(sw, c.s);
+                c.sig_dim = 0;
             }
             {
                 Timer t(c, g_last.gemm_ms);
@@ -1728,7 +1733,7 @@ static void run_lansvd_t(const char *jobu, const char *jobv, int m, int n, int *
             a.balpha = c.balpha; a.bbeta = c.bbeta; a.a1 = c.a1; a.b1 = c.b1; a.bnd = c.bnd; a.w = c.w;
             a.ctl = c.ctl; a.sigma_out = c.sig_out; a.bnd_out = c.bnd_out; a.nconv_out = c.nconv;
             a.anorm_drv = c.anorm_drv; a.dim = j; a.m = m; a.n = n; a.neig = k; a.kk = k;
-            a.irl = 0; a.small_side = 0; a.tol = tol; a.wz = c.wz;
+            a.irl = 0; a.small_side = 0; a.tol = tol;
             neig = analyse(c, a);
         }
         if (ierr < 0) {

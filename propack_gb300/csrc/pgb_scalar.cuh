@@ -13,8 +13,11 @@ __device__ __forceinline__ void lartg(double f, double g, double &c, double &s, 
 {
     if (g == 0.0) { c = 1.0; s = 0.0; r = f; return; }
     if (f == 0.0) { c = 0.0; s = 1.0; r = g; return; }
-    // one reciprocal hypotenuse (overflow-safe) instead of hypot + 2 divides
-    const double rh = rhypot(f, g);
+    // one reciprocal hypotenuse instead of hypot + 2 divides: rsqrt of the
+    // sum of squares (a third of rhypot's dependent FP64 operations) where
+    // no square leaves the FP64 range
+    const double q = fma(f, f, g * g);
+    const double rh = q > 1e-280 && q < 1e280 ? rsqrt(q) : rhypot(f, g);
     double cc = f * rh, ss = g * rh;
     double rr = fma(f, cc, g * ss);
     if (fabs(f) > fabs(g) && cc < 0.0) { cc = -cc; ss = -ss; rr = -rr; }
@@ -77,10 +80,10 @@ __device__ inline void bdqr_dev(int ignorelast, int n, double *D, double *E, dou
 #undef QT
 }
 
-// drefinebounds (double/dbsvd.F:162-231); thread 0
-__device__ inline void refinebounds_dev(int n, int k, const double *theta, double *bound, double tol, double eps34)
+// drefinebounds' first loop (double/dbsvd.F:162-190): bounds of values that
+// agree to eps34 are merged; thread 0
+__device__ inline void mergebounds_dev(int k, const double *theta, double *bound, double tol, double eps34)
 {
-    if (k <= 1) return;
     for (int i = 1; i <= k; i++) {
         for (int l = -1; l <= 1; l += 2) {
             if ((l == 1 && i < k) || (l == -1 && i > 1)) {
@@ -93,6 +96,13 @@ __device__ inline void refinebounds_dev(int n, int k, const double *theta, doubl
             }
         }
     }
+}
+
+// drefinebounds (double/dbsvd.F:162-231); thread 0
+__device__ inline void refinebounds_dev(int n, int k, const double *theta, double *bound, double tol, double eps34)
+{
+    if (k <= 1) return;
+    mergebounds_dev(k, theta, bound, tol, eps34);
     for (int i = 1; i <= k; i++) {
         if (i < k || k == n) {
             double gap;
