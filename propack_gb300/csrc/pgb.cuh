@@ -33,6 +33,7 @@ enum ProfKind { PK_SPMV_ADJ, PK_SPMV_FWD, PK_ELR, PK_CGS_DOTS, PK_CGS_UPD, PK_TH
 extern thread_local int g_prof_on;
 void prof_mark(int kind, cudaStream_t s, bool begin);
 void prof_collect();
+void prof_add(int kind, double ms, int64_t n);
 #define PGB_PROF(kind, s, ...)                                     \
     do {                                                           \
         if (::pgb::g_prof_on) ::pgb::prof_mark((kind), (s), true); \
@@ -87,8 +88,8 @@ struct Operator {
     Csr fwd, adj, thin_r, thin_l;
     double *w = nullptr;
     double *zbuf = nullptr;      // r: the low-rank coefficients of the current product
-    double *zpart = nullptr;     // r * segs partials
-    unsigned int *zticket = nullptr;
+    double *zpart = nullptr;     // 4 * r * segs partials
+    unsigned int *zticket = nullptr;  // r counters
     int64_t id = 0;
     int device = 0;
     // 1: a complex m/2 x n/2 matrix held as its real 2x2-block form (fwd
@@ -131,23 +132,26 @@ struct LbCtl {
     int elr_need_dot;
     double elr_s_im;
     int reorth_active, reorth_iter, reorth_count;
-    int cgs_phase;          // 0: the next CGS kernel forms the projections, 1: it applies them
     double reorth_nrm0;
     int nsel;               // columns selected for reorthogonalisation
     int collapsed;          // the last reorthogonalisation zeroed the vector
     int ndot_iter;          // inner products counted per CGS pass (dreorth.F:91, :164)
     Pend pend_u, pend_v;    // deferred scaling of the newest u / v column
     int pend_u_col, pend_v_col;
-    // suspension: the device met a case the enqueued sequence cannot finish
-    int status;             // 0 running, 1 suspended, 2 finished early (invariant subspace)
-    int susp_reason;        // 1 = getu0 needed (invariant subspace test), 2 = reorth iterations
+    // suspension: the device met a case that the host has to finish
+    int status;             // 0 running, 1 suspended
+    int susp_reason;        // 1 = getu0 needed (invariant subspace test)
     int susp_side;          // 0 = V half, 1 = U half
     int susp_j;
     // statistics (double/stat.h)
     long long nopx, nreorth, ndot;
     long long cgs_cols_u, cgs_cols_v;  // basis columns streamed by Gram-Schmidt passes, per side
-    // last-CTA tickets
+    // last-CTA ticket of the flush
     unsigned int ticket;
+    // with profiling on: ns and passes of the phases SpMV A'u, SpMV Av, ELR,
+    // projections, update, low-rank prepass (tails included)
+    unsigned long long prof_ns[6];
+    int prof_n[6];
 };
 
 // Everything a Lanczos kernel needs, passed by value.
@@ -164,7 +168,6 @@ struct LbArgs {
     double *part_cols;            // (kmax+1) * nb partial CGS dots, column c at c*nb
                                   // (complex: 2 (kmax+1) * nb, re at 2c*nb, im at (2c+1)*nb)
     int nb;                 // CTAs of the vector kernels
-    int nb_spmv;            // CTAs the fused SpMV may use (>= nb; the partial-sum arrays hold it)
     int kmax;               // capacity of the column arrays
     Csr fwd, adj;           // device operator (fwd = [S|L], adj = [S'|R])
     Csr zfwd, zadj;         // a native complex operator (A, A^H; rows = 0 otherwise)
@@ -176,6 +179,22 @@ struct LbArgs {
     float2 *Up, *Vp;
     int *okU, *okV;
     float2 *xpl;
+};
+struct LbPub;
+// What the run kernel needs beside LbArgs.
+struct RunArgs {
+    unsigned *sync;         // arrivals, release word, error flag
+    LbPub *pub;
+    int j0, side0, j1, side1;  // first and last half step
+    int host_product;       // the caller's APROD already wrote the product of the (one) half step
+    int smem_tail;          // CTA 0's recurrences in dynamic shared memory from this double on (0: global)
+    int prof;
+    // low-rank prepass (r = 0: none)
+    int r;
+    Csr thin_r, thin_l;
+    const double *w;
+    double *z, *zpart;
+    unsigned *ztick;
 };
 // real scalars per element of a Lanczos vector: 1 for double and float, 2
 // for complex*16, held as double2 = (re, im).  LbArgs' ldu, ldv and the
@@ -258,6 +277,53 @@ __device__ __forceinline__ double block_sum(double v, double *sh)
     t = sh[0];
     __syncthreads();
     return t;
+}
+// CTA sums of N values with few FP64 instructions (an FP64 warp instruction
+// holds the SM's pipe for 16 clocks, so eight warps' shuffle trees cost as
+// much as a pass over the data): every thread parks its values, and warp q
+// adds value q, NT / 32 per lane and then over the lanes.  out[q] is written
+// by lane 0 of warp q (shared or global memory); the caller synchronises
+// before it reads.  buf: N * NT doubles of shared memory.
+template <int NT, int N>
+__device__ __forceinline__ void block_sums(const double (&v)[N], double *buf, double *const (&out)[N])
+{
+    static_assert(N <= NT / 32, "one warp per value");
+#pragma unroll
+    for (int q = 0; q < N; q++) buf[q * NT + threadIdx.x] = v[q];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int q = 0; q < N; q++)
+        if (w == q) {
+            double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+            for (int i = 0; i < NT / 32; i += 2) {
+                s0 += buf[q * NT + 32 * i + lane];
+                s1 += buf[q * NT + 32 * (i + 1) + lane];
+            }
+            s0 = warp_sum(s0 + s1);
+            if (lane == 0) *out[q] = s0;
+        }
+}
+// CTA maximum of non-negative values without FP64 instructions (their bits
+// order like integers); thread 0 gets the result
+template <int NT>
+__device__ __forceinline__ double block_max_pos(double v, double *sh)
+{
+    const unsigned F = 0xffffffffu;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+    const unsigned mh = __reduce_max_sync(F, hi);
+    const unsigned ml = __reduce_max_sync(F, hi == mh ? lo : 0u);
+    if (lane == 0) sh[w] = __hiloint2double((int)mh, (int)ml);
+    __syncthreads();
+    unsigned long long m = 0;
+    if (threadIdx.x == 0)
+        for (int i = 0; i < NT / 32; i++) {
+            const unsigned long long u = (unsigned long long)__double_as_longlong(sh[i]);
+            m = u > m ? u : m;
+        }
+    return __longlong_as_double((long long)m);
 }
 template <int NT>
 __device__ __forceinline__ double block_max(double v, double *sh)
@@ -380,18 +446,23 @@ bool gemm_f64_tc(int mr, int nc, int kk, const double *A, int lda, const double 
 template <typename T>
 void copy_cols(const T *src, int lds, T *dst, int ldd, int rows, int cols, cudaStream_t s);
 
-// ------------------------------------------------ Lanczos step enqueue
-void lb_set_smem_limits(int kmax);
+// ------------------------------------------------ Lanczos steps
 bool lb_planes_fit(int kmax, bool cplx);
 // Gram-Schmidt arithmetic of the FP64 form: 0 FP64 FMAs, 1 three-way
 // splits on the FP32 pipe (pgb_f3.cuh), 2 split-once planes (the default)
 enum CgsArith { CGS_FP64 = 0, CGS_F3 = 1, CGS_PLANES = 2 };
 extern thread_local int g_cgs_arith;
+size_t lb_run_scratch();
+// half steps (j0, side0) .. (j1, side1) of dlanbpro on at most `want` CTAs
 template <typename T>
-void lb_enqueue_half(const LbArgs &a, const Operator *op, int side, int j, int ielr, int ntry_spec,
-                     bool host_product, cudaStream_t s);
-template <typename T>
-void lb_enqueue_cgs_more(const LbArgs &a, int side, int j, int passes, cudaStream_t s);
+void lb_run(const LbArgs &a, RunArgs R, bool block, int want, cudaStream_t s);
+template <>
+void lb_run<double>(const LbArgs &a, RunArgs R, bool block, int want, cudaStream_t s);
+template <>
+void lb_run<float>(const LbArgs &a, RunArgs R, bool block, int want, cudaStream_t s);
+template <>
+void lb_run<double2>(const LbArgs &a, RunArgs R, bool block, int want, cudaStream_t s);
+void lb_run_fp64(const LbArgs &a, RunArgs R, int want, cudaStream_t s);
 template <typename T>
 void lb_enqueue_flush(const LbArgs &a, cudaStream_t s);
 template <typename T>

@@ -50,9 +50,6 @@ static bool trace_on()
     return on;
 }
 
-// steps enqueued between two looks at the device status word
-constexpr int LB_WINDOW = 8;
-
 // ------------------------------------------------------------ small kernels
 #define LCG_A 33952834046453ULL
 #define LCG_MASK ((1ULL << 48) - 1ULL)
@@ -242,7 +239,10 @@ struct Ctx {
     LbCtl *hctl = nullptr;  // pinned host copy
     double *balpha = nullptr, *bbeta = nullptr, *mu = nullptr, *nu = nullptr, *h = nullptr;
     double *part_sq = nullptr, *part_dot = nullptr, *part_cols = nullptr;
-    int nb_spmv = 0;  // grid bound of the fused SpMV (spmv_grid_bound)
+    int run_ctas = 0;                       // CTAs of the run kernel (run_grid)
+    char *runbuf = nullptr;                 // its barrier words and published scalars
+    double *zb = nullptr, *zpart = nullptr; // low-rank coefficients and partials of this solve
+    unsigned *ztick = nullptr;
     int *index = nullptr, *sel = nullptr;
     void *xr = nullptr, *yr = nullptr;      // max(m,n) scratch of the vector type
     double *dx = nullptr, *dy = nullptr;    // max(m,n) FP64 scratch
@@ -271,9 +271,7 @@ struct Ctx {
     propack_z16 *zparm = nullptr;
     double *hx = nullptr, *hy = nullptr;    // pinned host vectors for a host APROD
     int nb = 0;
-    int ntry_spec = 2;
-    int *hstat = nullptr;                   // pinned status words of the enqueue windows
-    cudaEvent_t wev[2] = {nullptr, nullptr};
+    int *hstat = nullptr;                   // pinned copy of the run kernel's error flag
     std::vector<void *> allocs;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, evs0 = nullptr, evs1 = nullptr;
     // the caller's page-locked U and V (set_host_out): dev_ritzvec forms
@@ -314,8 +312,6 @@ struct Ctx {
         if (hctl) cudaFreeHost(hctl);
         if (hscal) cudaFreeHost(hscal);
         if (hstat) cudaFreeHost(hstat);
-        for (cudaEvent_t e : wev)
-            if (e) cudaEventDestroy(e);
         if (hx) cudaFreeHost(hx);
         if (hy) cudaFreeHost(hy);
         if (ev0) cudaEventDestroy(ev0);
@@ -337,14 +333,13 @@ struct Ctx {
         a.index = index; a.sel = sel; a.h = h;
         a.part_sq = part_sq; a.part_dot = part_dot; a.part_cols = part_cols;
         a.nb = nb; a.kmax = kmax;
-        a.nb_spmv = std::max(nb, nb_spmv);
         if (op && op->cplx == 2) {
             // a native complex operator: its own kernels read zfwd / zadj;
             // fwd and adj carry only the vector lengths in real scalars
             a.zfwd = op->fwd; a.zadj = op->adj;
             a.fwd.rows = m * vw; a.adj.rows = n * vw; a.z = nullptr;
         } else if (op) {
-            a.fwd = op->fwd; a.adj = op->adj; a.z = op->zbuf;
+            a.fwd = op->fwd; a.adj = op->adj; a.z = zb;
         } else {
             a.fwd.rows = m * vw; a.adj.rows = n * vw; a.z = nullptr;
         }
@@ -364,25 +359,23 @@ struct Ctx {
     void put_ctl() { PGB_CUDA(cudaMemcpyAsync(ctl, hctl, sizeof(LbCtl), cudaMemcpyHostToDevice, s)); }
 };
 
-// CTAs of the vector kernels: about 2048 vector elements or 16384 nonzeros
-// each, at most the four per SM that the partial-sum arrays hold.  A small
-// problem then runs its many short kernels on a few CTAs instead of
-// launching four per SM that mostly find no work.
+// CTAs of the vector kernels: about 512 vector elements or 16384 nonzeros
+// each, at most the four per SM that the partial-sum arrays hold.
 static int vec_grid(int64_t elems, int64_t nnz)
 {
     const int64_t cap = device_info().nb;
-    const int64_t want = std::max((elems + 2047) / 2048, (nnz + 16383) / 16384);
+    const int64_t want = std::max((elems + 511) / 512, (nnz + 16383) / 16384);
     return (int)std::max<int64_t>(1, std::min(cap, want));
 }
-// CTAs the fused SpMV may use: one per 256 rows (a 32-row tile per warp),
-// at most the four per SM that the partial-sum arrays hold.  The SpMV's
-// latency chain (row bounds, indices, gathers) runs once per tile, so a
-// small matrix wants its tiles spread over warps rather than its nonzeros
-// over few CTAs.
-static int spmv_grid_bound(int64_t rows)
+// CTAs of the run kernel: one per 128 rows (half a 32-row SpMV tile per
+// warp, 64 two-element vectors of a Gram-Schmidt pass), at most what fits at once.  A
+// small problem's phases are latency chains that run once per tile, so it
+// wants its tiles spread over warps; beyond one tile per warp more CTAs only
+// make the barrier longer.
+static int run_grid(int64_t rows)
 {
     const int64_t cap = device_info().nb;
-    return (int)std::max<int64_t>(1, std::min(cap, (rows + 255) / 256));
+    return (int)std::max<int64_t>(1, std::min(cap, (rows + 127) / 128));
 }
 
 template <typename T>
@@ -423,7 +416,7 @@ static void init_ctx(Ctx &c, int m, int n, int kmax)
     PGB_CUDA(cudaMallocHost(&c.hscal, sizeof(double) * 8));
     PGB_CUDA(cudaMallocHost(&c.hstat, sizeof(int) * 2));
     c.hstat[0] = c.hstat[1] = 0;
-    for (cudaEvent_t &e : c.wev) PGB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    c.runbuf = (char *)c.dbytes(lb_run_scratch());
     const size_t d1 = kmax + 2;
     c.a1 = c.dalloc<double>(d1); c.b1 = c.dalloc<double>(d1); c.bnd = c.dalloc<double>(d1);
     c.w = c.dalloc<double>(4 * d1);
@@ -439,8 +432,9 @@ static void init_ctx(Ctx &c, int m, int n, int kmax)
     c.X = c.dalloc<double>(d1 * d1);
     // the restart/Ritz product's output: written by the GEMM before it is read
     c.gout = c.dbytes_raw(sizeof(T) * (size_t)std::max(c.ldu, c.ldv) * (kmax + 1));
-    // the partial-sum arrays above hold d.nb CTAs; the grid follows the size
+    // the partial-sum arrays above hold d.nb CTAs; the grids follow the size
     c.nb = vec_grid((int64_t)std::max(m, n) * c.vw, 0);
+    c.run_ctas = run_grid(std::max(m, n));
     constexpr bool fp64 = std::is_same<T, double>::value || std::is_same<T, double2>::value;
     if (fp64 && g_cgs_arith == CGS_PLANES && lb_planes_fit(kmax, c.vw == 2)) {
         // planes of every real scalar (complex: of re and im); written (flag
@@ -451,7 +445,6 @@ static void init_ctx(Ctx &c, int m, int n, int kmax)
         c.okU = c.dalloc<int>(kmax + 2);
         c.okV = c.dalloc<int>(kmax + 2);
     }
-    lb_set_smem_limits(kmax);
 }
 
 // ----------------------------------------------------- device utilities
@@ -615,6 +608,44 @@ struct LbResult {
     int ierr;
 };
 
+static void clear_prof(LbCtl &h)
+{
+    for (int i = 0; i < 6; i++) { h.prof_ns[i] = 0; h.prof_n[i] = 0; }
+}
+
+// Half steps (j0, side0) .. (j1, side1) on the device (one launch), then the
+// control block on the host.
+template <typename T>
+static void run_steps(Ctx &c, int j0, int side0, int j1, int side1, bool host_product)
+{
+    RunArgs R = {};
+    R.sync = (unsigned *)c.runbuf;
+    R.pub = (LbPub *)(c.runbuf + 64);
+    R.j0 = j0; R.side0 = side0; R.j1 = j1; R.side1 = side1;
+    R.host_product = host_product ? 1 : 0;
+    R.prof = g_prof_on;
+    if (c.op && c.op->r > 0 && !c.op->cplx) {
+        R.r = c.op->r;
+        R.thin_r = c.op->thin_r; R.thin_l = c.op->thin_l;
+        R.w = c.op->w;
+        R.z = c.zb; R.zpart = c.zpart; R.ztick = c.ztick;
+    }
+    lb_run<T>(c.args(), R, c.op && c.op->cplx == 1, c.run_ctas, c.s);
+    PGB_CUDA(cudaMemcpyAsync(c.hstat, R.sync + 2, sizeof(int), cudaMemcpyDeviceToHost, c.s));
+    c.get_ctl();
+    if (c.hstat[0] != 0) {
+        set_error("Lanczos run: a bounded device-side wait gave up");
+        throw WaitFailure();
+    }
+    if (g_prof_on) {
+        static const int kinds[6] = {PK_SPMV_ADJ, PK_SPMV_FWD, PK_ELR, PK_CGS_DOTS, PK_CGS_UPD, PK_THIN};
+        static const int kinds32[6] = {PK_SPMV_ADJ32, PK_SPMV_FWD32, PK_ELR, PK_CGS_DOTS32, PK_CGS_UPD32, PK_THIN};
+        for (int i = 0; i < 6; i++)
+            prof_add((sizeof(T) == 4 ? kinds32 : kinds)[i], 1e-6 * (double)c.hctl->prof_ns[i], c.hctl->prof_n[i]);
+        clear_prof(*c.hctl);
+    }
+}
+
 // Run dlanbpro (double/dlanbpro.F:1-549) from k0 to *kp on the device.
 template <typename T>
 static void dev_lanbpro(Ctx &c, int k0, int *kp, double *rnorm, double *doption, const int *ioption, int *ierr)
@@ -648,6 +679,7 @@ static void dev_lanbpro(Ctx &c, int k0, int *kp, double *rnorm, double *doption,
     h.elr_active = 0;
     h.reorth_active = 0;
     h.collapsed = 0;
+    clear_prof(h);
     double anorm;
     std::vector<double> hb(2 * (size_t)(k + 2), 0.0);
     if (k0 > 0) {
@@ -742,17 +774,16 @@ static void dev_lanbpro(Ctx &c, int k0, int *kp, double *rnorm, double *doption,
     h.ticket = 0;
     c.put_ctl();
 
-    // the step loop: enqueue everything, then look for a suspension
+    // the step loop: one launch runs until the end or a suspension
     const bool host_ap = (c.op == nullptr);
     int j = j0, side = 0;
-    bool finished = false;
+    bool finished = j0 > k;
     int rounds = 0;
     while (!finished) {
         if (++rounds > 4 * (k + 2)) {
             set_error("dlanbpro: too many suspensions");
             throw WaitFailure();
         }
-        LbArgs a = c.args();
         // the host may have written columns since the last round (start
         // vector, prologue, a suspension's fresh vector): no plane is trusted
         if (c.okU) {
@@ -760,27 +791,7 @@ static void dev_lanbpro(Ctx &c, int k0, int *kp, double *rnorm, double *doption,
             PGB_CUDA(cudaMemsetAsync(c.okV, 0, sizeof(int) * (c.kmax + 2), c.s));
         }
         if (!host_ap) {
-            // enqueue in windows of LB_WINDOW steps; before a window goes in,
-            // the status word of the window two back is read (its copy was
-            // queued behind it), so at most two windows of launches are
-            // wasted when a step suspends, and the device never runs dry
-            int wnum = 0;
-            while (j <= k) {
-                if (wnum >= 2) {
-                    PGB_CUDA(cudaEventSynchronize(c.wev[wnum & 1]));
-                    if (c.hstat[wnum & 1] != 0) break;
-                }
-                const int jend = std::min(k, j + LB_WINDOW - 1);
-                for (; j <= jend; j++) {
-                    for (; side < 2; side++) lb_enqueue_half<T>(a, c.op, side, j, h.ielr, c.ntry_spec, false, c.s);
-                    side = 0;
-                }
-                PGB_CUDA(cudaMemcpyAsync(&c.hstat[wnum & 1], &c.ctl->status, sizeof(int), cudaMemcpyDeviceToHost,
-                                         c.s));
-                PGB_CUDA(cudaEventRecord(c.wev[wnum & 1], c.s));
-                wnum++;
-            }
-            c.get_ctl();
+            run_steps<T>(c, j, side, k, 1, false);
         } else {
             // host APROD: one synchronous product per half step
             bool susp = false;
@@ -793,15 +804,13 @@ static void dev_lanbpro(Ctx &c, int k0, int *kp, double *rnorm, double *doption,
                     k_clear_pend<<<1, 1, 0, c.s>>>(c.ctl, side == 0 ? 0 : 1);
                     PGB_LAUNCHED();
                     dev_aprod<T>(c, side == 0, x, y);
-                    lb_enqueue_half<T>(a, nullptr, side, j, h.ielr, c.ntry_spec, true, c.s);
-                    c.get_ctl();
+                    run_steps<T>(c, j, side, j, side, true);
                     if (h.status != 0) susp = true;
                     if (susp) break;
                 }
                 if (susp) break;
                 side = 0;
             }
-            if (!susp) c.get_ctl();
         }
         if (h.status == 0) {
             finished = true;
@@ -812,23 +821,6 @@ static void dev_lanbpro(Ctx &c, int k0, int *kp, double *rnorm, double *doption,
         if (trace_on())
             fprintf(stderr, "[propack_gb300] lanbpro suspension: reason %d step %d side %c alpha %.3e beta %.3e anorm %.3e\n",
                     h.susp_reason, sj, ss == 0 ? 'v' : 'u', h.alpha, h.beta, h.anorm);
-        if (h.susp_reason == 2) {
-            h.status = 0;
-            c.put_ctl();
-            lb_enqueue_cgs_more<T>(c.args(), ss, sj, NTRY - c.ntry_spec, c.s);
-            c.get_ctl();
-            if (h.status != 0 && h.susp_reason == 2) {
-                set_error("reorthogonalisation did not finish within NTRY passes");
-                throw WaitFailure();
-            }
-            if (h.status == 0) {
-                // continue after the finished half step
-                if (ss == 0) { j = sj; side = 1; }
-                else { j = sj + 1; side = 0; }
-                continue;
-            }
-            // fell into an invariant-subspace suspension: handled below
-        }
         if (h.susp_reason != 1) {
             set_error("device control block reports an unknown suspension");
             throw WaitFailure();
@@ -1367,7 +1359,13 @@ static void setup_operator(Ctx &c, propack_aprod_t aprod, double *dparm, int *ip
         }
         c.op = op;
         c.nb = std::max(c.nb, vec_grid(0, std::max(op->fwd.nnz, op->adj.nnz)));
-        c.nb_spmv = spmv_grid_bound(std::max(op->fwd.rows, op->adj.rows));
+        c.run_ctas = std::max(c.run_ctas, c.nb);
+        if (op->r > 0) {
+            c.zb = c.dalloc<double>(op->r);
+            c.zpart = (double *)c.dbytes_raw(sizeof(double) * 4 * (size_t)op->r *
+                                             std::max(op->thin_r.segs, op->thin_l.segs));
+            c.ztick = c.dalloc<unsigned>(op->r);
+        }
     } else {
         c.aprod = aprod;
         c.dparm = dparm;
@@ -1399,7 +1397,7 @@ static void setup_zoperator(Ctx &c, propack_zaprod_t aprod, propack_z16 *zparm, 
         }
         c.op = op;
         c.nb = std::max(c.nb, vec_grid(0, std::max(op->fwd.nnz, op->adj.nnz)));
-        c.nb_spmv = spmv_grid_bound(std::max(op->fwd.rows, op->adj.rows));
+        c.run_ctas = std::max(c.run_ctas, c.nb);
     } else {
         c.zaprod = aprod;
         c.zparm = zparm;

@@ -28,7 +28,7 @@ void op_spmv_plain_launch(const Csr &A, const double *x, const double *z, double
 static __device__ __align__(256) double g_noalloc_scratch[PROPACK_NOALLOC_MAX_DOUBLES];
 
 // z[c] = w[c] * sum(thin row c . x), segments of NNZ_PB per CTA, partials in
-// the static scratch (the same reduction as the allocating prepass).
+// the static scratch.
 __global__ void __launch_bounds__(BS) k_thin_noalloc(Csr T, const double *__restrict__ x, const double *w, int r)
 {
     __shared__ double sred[32];

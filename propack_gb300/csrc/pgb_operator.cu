@@ -70,6 +70,12 @@ void prof_collect()
     }
     g_prof_open.clear();
 }
+// time measured on the device (the run kernel's phases)
+void prof_add(int kind, double ms, int64_t n)
+{
+    g_prof_ms[kind] += ms;
+    g_prof_cnt[kind] += n;
+}
 void prof_reset()
 {
     for (int i = 0; i < PK_N; i++) { g_prof_ms[i] = 0.0; g_prof_cnt[i] = 0; }
@@ -687,30 +693,13 @@ __global__ void k_to_float(const double *a, float *b, int64_t n)
 }
 
 // ------------------------------------------------------ application
-// z[c] = w[c] * sum(thin row c . x), split into segments of NNZ_PB.  The
-// low-rank coefficients are always formed in FP64.
+// z[c] = w[c] * sum(thin row c . x) (thin_phase).  The low-rank coefficients
+// are always formed in FP64.
 template <typename T>
-__global__ void __launch_bounds__(BS) k_thin(Csr Th, const T *__restrict__ x, const double *w, double *zpart,
-                                             double *z, unsigned int *ticket)
+__global__ void __launch_bounds__(BS) k_thin(Csr Th, const T *x, const double *w, double *zpart, double *z,
+                                             unsigned int *tick)
 {
-    __shared__ double sred[32];
-    const int nseg = Th.segs;
-    for (int t = blockIdx.x; t < Th.rows * nseg; t += gridDim.x) {
-        const int c = t / nseg, sg = t % nseg;
-        const int a = Th.ptr[c] + sg * NNZ_PB;
-        const int b = min(Th.ptr[c + 1], a + NNZ_PB);
-        double acc = 0.0;
-        for (int e = a + threadIdx.x; e < b; e += BS) acc += Th.val[e] * (double)x[Th.idx[e]];
-        acc = block_sum<BS>(acc, sred);
-        if (threadIdx.x == 0) zpart[t] = acc;
-    }
-    if (last_cta(ticket)) {
-        for (int c = threadIdx.x; c < Th.rows; c += BS) {
-            double s = 0.0;
-            for (int sg = 0; sg < nseg; sg++) s += zpart[c * nseg + sg];
-            z[c] = w[c] * s;
-        }
-    }
+    thin_phase<T>(Th, x, w, zpart, z, tick);
 }
 
 template <typename T>
@@ -756,7 +745,7 @@ void op_thin(const Operator &op, bool trans, const T *x, cudaStream_t s)
 {
     if (op.r <= 0) return;
     const Csr &Th = trans ? op.thin_l : op.thin_r;
-    const int nt = std::max(1, Th.rows * Th.segs);
+    const int nt = std::max(1, (Th.rows * Th.segs * 4 + SPMV_WARPS - 1) / SPMV_WARPS);
     k_thin<T><<<std::min(nt, device_info().nb), BS, 0, s>>>(Th, x, op.w, op.zpart, op.zbuf, op.zticket);
     PGB_LAUNCHED();
 }
@@ -1036,11 +1025,11 @@ static int create_operator(int m, int n, const int64_t *sp, const int32_t *si, c
         }
         const int segs = std::max(op->thin_r.segs, op->thin_l.segs);
         PGB_CUDA(cudaMalloc(&op->zbuf, sizeof(double) * r));
-        PGB_CUDA(cudaMalloc(&op->zpart, sizeof(double) * (size_t)r * segs));
+        PGB_CUDA(cudaMalloc(&op->zpart, sizeof(double) * 4 * (size_t)r * segs));
         PGB_CUDA(cudaMemset(op->zbuf, 0, sizeof(double) * r));
     }
-    PGB_CUDA(cudaMalloc(&op->zticket, sizeof(unsigned int)));
-    PGB_CUDA(cudaMemset(op->zticket, 0, sizeof(unsigned int)));
+    PGB_CUDA(cudaMalloc(&op->zticket, sizeof(unsigned int) * std::max(r, 1)));
+    PGB_CUDA(cudaMemset(op->zticket, 0, sizeof(unsigned int) * std::max(r, 1)));
     // FP32 copies of the values for the mixed-precision path
     for (Csr *A : {&op->fwd, &op->adj}) {
         A->valf = (float *)pool_alloc(sizeof(float) * std::max<int64_t>(A->nnz, 1), s);

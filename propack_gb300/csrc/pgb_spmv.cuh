@@ -333,6 +333,56 @@ __device__ __forceinline__ void csr_rows_chunked(const int *__restrict__ ptr, co
     }
 }
 
+// The low-rank prepass z = w .* (Th x) of a thin matrix Th (few rows, each
+// up to the length of x): a warp per segment of THIN_SEG entries, eight
+// entries of a lane in flight; the warp that completes a row (its ticket)
+// adds the row's partials in order.  zpart: rows * 4 * segs doubles, tick:
+// rows zeroed counters, left zeroed.
+constexpr int THIN_SEG = NNZ_PB / 4;
+template <typename T>
+__device__ __forceinline__ void thin_phase(const Csr &Th, const T *x, const double *w, double *zpart, double *z,
+                                           unsigned int *tick)
+{
+    const unsigned F = 0xffffffffu;
+    const int lane = threadIdx.x & 31, nwarps = gridDim.x * SPMV_WARPS;
+    const int nseg = 4 * Th.segs;
+    for (int t = blockIdx.x * SPMV_WARPS + (threadIdx.x >> 5); t < Th.rows * nseg; t += nwarps) {
+        const int c = t / nseg, sg = t % nseg;
+        const int p0 = Th.ptr[c], p1 = Th.ptr[c + 1];
+        const int used = max(1, (p1 - p0 + THIN_SEG - 1) / THIN_SEG);
+        if (sg >= used) continue;
+        const int b = min(p1, p0 + (sg + 1) * THIN_SEG);
+        double acc = 0.0;
+        int e = p0 + sg * THIN_SEG + lane;
+        for (; e + 32 * 7 < b; e += 32 * 8) {
+            int ci[8];
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) { ci[u] = Th.idx[e + 32 * u]; v[u] = Th.val[e + 32 * u]; }
+#pragma unroll
+            for (int u = 0; u < 8; u++) acc = fma(v[u], (double)x[ci[u]], acc);
+        }
+        for (; e < b; e += 32) acc = fma(Th.val[e], (double)x[Th.idx[e]], acc);
+        acc = warp_sum(acc);
+        unsigned old = 0;
+        if (lane == 0) {
+            zpart[t] = acc;
+            __threadfence();
+            old = atomicAdd(tick + c, 1u);
+        }
+        if (__shfl_sync(F, old, 0) + 1 == (unsigned)used) {
+            __threadfence();
+            double s = 0.0;
+            for (int q = lane; q < used; q += 32) s += __ldcg(zpart + (size_t)c * nseg + q);
+            s = warp_sum(s);
+            if (lane == 0) {
+                z[c] = w[c] * s;
+                tick[c] = 0u;
+            }
+        }
+    }
+}
+
 // the schedule chosen for the matrix
 template <typename VT, typename AT, typename XF, typename PF, typename EPI>
 __device__ __forceinline__ void csr_spmv(const Csr &A, const VT *__restrict__ val, XF xload, PF pre_load, EPI epi,
