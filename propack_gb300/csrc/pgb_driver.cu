@@ -210,6 +210,18 @@ __global__ void k_convert(const TS *src, TD *dst, int n)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = (TD)src[i];
 }
+// FP32 results for FP64 arrays, four elements per thread and step
+__global__ void __launch_bounds__(256) k_widen(const float *__restrict__ src, double *__restrict__ dst, size_t len)
+{
+    const size_t n4 = len / 4, st = (size_t)gridDim.x * blockDim.x;
+    const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    for (size_t i = t; i < n4; i += st) {
+        const float4 v = reinterpret_cast<const float4 *>(src)[i];
+        reinterpret_cast<double2 *>(dst)[2 * i] = make_double2(v.x, v.y);
+        reinterpret_cast<double2 *>(dst)[2 * i + 1] = make_double2(v.z, v.w);
+    }
+    if (t < len - 4 * n4) dst[4 * n4 + t] = src[4 * n4 + t];
+}
 // out[r] = sum over the first ncols columns of U (the warm start of the
 // FP64 refinement: a vector in the span of the FP32 Ritz vectors)
 template <typename T>
@@ -1151,23 +1163,37 @@ void h2d_bytes(void *dst, const void *src, size_t bytes, cudaStream_t s)
     for (size_t h = 0; h < 2 && h < np; h++) PGB_CUDA(cudaEventSynchronize(b.ev[h]));
 }
 
+// The caller's REAL arrays (the single-precision drivers): FP32 results
+// leave as they are.
+struct RealOut {
+    float *U = nullptr, *V = nullptr;  // U(:,1) is also the start vector
+    int ldu = 0, ldv = 0;
+};
+
 template <typename T>
-static void copy_out(Ctx &c, double *U, int ldu, double *V, int ldv, int ncols, bool du, bool dv)
+static void copy_out(Ctx &c, double *U, int ldu, double *V, int ldv, int ncols, bool du, bool dv,
+                     const RealOut *real = nullptr)
 {
     if (ncols <= 0) return;
     if constexpr (std::is_same<T, float>::value) {
-        // FP32 bases: widen column by column through the FP64 scratch
         for (int side = 0; side < 2; side++) {
             if (side == 0 ? !du : !dv) continue;
-            const int rows = side == 0 ? c.m : c.n;
-            double *H = side == 0 ? U : V;
-            const int ldh = side == 0 ? ldu : ldv;
-            for (int col = 0; col < ncols; col++) {
-                const T *src = side == 0 ? c.Ucol<T>(col) : c.Vcol<T>(col);
-                dev_convert<T, double>(c, src, c.dx, rows);
-                PGB_CUDA(cudaMemcpyAsync(H + (size_t)col * ldh, c.dx, sizeof(double) * rows, cudaMemcpyDeviceToHost,
-                                         c.s));
+            const int rows = side == 0 ? c.m : c.n, ld = side == 0 ? c.ldu : c.ldv;
+            const float *src = side == 0 ? c.Ucol<float>(0) : c.Vcol<float>(0);
+            if (real) {
+                d2h_columns((char *)(side == 0 ? real->U : real->V),
+                            sizeof(float) * (size_t)(side == 0 ? real->ldu : real->ldv), (const char *)src,
+                            sizeof(float) * (size_t)ld, sizeof(float) * (size_t)rows, ncols, c.s);
+                continue;
             }
+            // widened on the device, all columns in one pass (the bases' pitch: one flat array)
+            const size_t len = (size_t)ld * (ncols - 1) + rows;
+            double *wide = (double *)pool_alloc(sizeof(double) * len, c.s);
+            c.allocs.push_back(wide);
+            k_widen<<<device_info().nb, 256, 0, c.s>>>(src, wide, len);
+            PGB_LAUNCHED();
+            d2h_columns((char *)(side == 0 ? U : V), sizeof(double) * (size_t)(side == 0 ? ldu : ldv),
+                        (const char *)wide, sizeof(double) * (size_t)ld, sizeof(double) * (size_t)rows, ncols, c.s);
         }
         return;
     } else {
@@ -1541,12 +1567,26 @@ static void irl_plain(const IrlIn &in, propack_aprod_t aprod, double *dparm, pro
     add_ctx_counters(c);
 }
 
+// the FP32 form's start vector from the caller's REAL or DOUBLE array
+static void load_start32(Ctx &c, const double *U, const RealOut *real)
+{
+    if (real) {
+        PGB_CUDA(cudaMemcpyAsync(c.U, real->U, sizeof(float) * c.m, cudaMemcpyHostToDevice, c.s));
+        PGB_CUDA(cudaEventRecord(c.evs0, c.s));
+    } else {
+        PGB_CUDA(cudaMemcpyAsync(c.dx, U, sizeof(double) * c.m, cudaMemcpyHostToDevice, c.s));
+        PGB_CUDA(cudaEventRecord(c.evs0, c.s));
+        dev_convert<double, float>(c, c.dx, c.Ucol<float>(0), c.m);
+    }
+}
+
 static void run_irl(const char *which, const char *jobu, const char *jobv, int m, int n, int dim, int p, int *neig,
                     int maxiter, propack_aprod_t aprod, double *U, int ldu, double *sigma, double *bnd, double *V,
-                    int ldv, double tolin, double *doption, const int *ioption, int *info, double *dparm, int *iparm)
+                    int ldv, double tolin, double *doption, const int *ioption, int *info, double *dparm, int *iparm,
+                    const RealOut *real = nullptr)
 {
-    if (m <= 0 || n <= 0 || dim <= 0 || p < 0 || *neig < 0 || ldu < m || ldv < n || !aprod || !U || !V || !sigma ||
-        !bnd || !doption || !ioption) {
+    if (m <= 0 || n <= 0 || dim <= 0 || p < 0 || *neig < 0 || ldu < m || ldv < n || !aprod || (!real && (!U || !V)) ||
+        !sigma || !bnd || !doption || !ioption) {
         set_error("dlansvd_irl_: invalid argument");
         throw ArgFailure();
     }
@@ -1576,9 +1616,7 @@ static void run_irl(const char *which, const char *jobu, const char *jobv, int m
         init_ctx<float>(c, m, n, in.dim);
         setup_operator(c, aprod, dparm, iparm);
         PGB_CUDA(cudaEventRecord(c.ev0, c.s));
-        PGB_CUDA(cudaMemcpyAsync(c.dx, U, sizeof(double) * m, cudaMemcpyHostToDevice, c.s));
-        PGB_CUDA(cudaEventRecord(c.evs0, c.s));
-        dev_convert<double, float>(c, c.dx, c.Ucol<float>(0), m);
+        load_start32(c, U, real);
         double dop32[4] = {doption[0], doption[1], doption[2], doption[3]};
         if (dop32[0] >= 0) dop32[0] = std::max(dop32[0], std::sqrt(EPS32));
         if (dop32[1] >= 0) dop32[1] = std::max(dop32[1], std::pow(EPS32, 0.75));
@@ -1586,7 +1624,7 @@ static void run_irl(const char *which, const char *jobu, const char *jobv, int m
         in32.tol = std::min(1.0, std::max(16.0 * EPS32, tolin));
         irl_loop<float>(c, in32, dop32, ioption, out);
         PGB_CUDA(cudaEventRecord(c.evs1, c.s));
-        copy_out<float>(c, U, ldu, V, ldv, out.nconv, in.du, in.dv);
+        copy_out<float>(c, U, ldu, V, ldv, out.nconv, in.du, in.dv, real);
         PGB_CUDA(cudaEventRecord(c.ev1, c.s));
         c.sync();
         float ms = 0;
@@ -1673,12 +1711,13 @@ template <typename T>
 static void run_lansvd_t(const char *jobu, const char *jobv, int m, int n, int *kp, int kmax, propack_aprod_t aprod,
                        double *U, int ldu, double *sigma, double *bnd, double *V, int ldv, double tolin,
                        double *doption, const int *ioption, int *info, double *dparm, int *iparm,
-                       propack_zaprod_t zaprod = nullptr, propack_z16 *zparm = nullptr)
+                       propack_zaprod_t zaprod = nullptr, propack_z16 *zparm = nullptr,
+                       const RealOut *real = nullptr)
 {
     const int k = *kp;
     constexpr bool cplx = VecW<T>::w == 2;
     if (m <= 0 || n <= 0 || k <= 0 || kmax <= 0 || ldu < m || ldv < n || !(cplx ? (void *)zaprod : (void *)aprod) ||
-        !U || !V || !sigma || !bnd || !doption || !ioption) {
+        (!real && (!U || !V)) || !sigma || !bnd || !doption || !ioption) {
         set_error(cplx ? "zlansvd_: invalid argument" : "dlansvd_: invalid argument");
         throw ArgFailure();
     }
@@ -1700,10 +1739,11 @@ static void run_lansvd_t(const char *jobu, const char *jobv, int m, int n, int *
     if constexpr (cplx) {
         PGB_CUDA(cudaMemcpyAsync(c.U, U, sizeof(T) * m, cudaMemcpyHostToDevice, c.s));
         PGB_CUDA(cudaEventRecord(c.evs0, c.s));
+    } else if constexpr (f32) {
+        load_start32(c, U, real);
     } else {
-        PGB_CUDA(cudaMemcpyAsync(c.dx, U, sizeof(double) * m, cudaMemcpyHostToDevice, c.s));
+        PGB_CUDA(cudaMemcpyAsync(c.U, U, sizeof(double) * m, cudaMemcpyHostToDevice, c.s));
         PGB_CUDA(cudaEventRecord(c.evs0, c.s));
-        dev_convert<double, T>(c, c.dx, c.Ucol<T>(0), m);
     }
     double rnorm = dev_nrm2<T>(c, c.Ucol<T>(0), m);
     int ierr = 0;
@@ -1764,7 +1804,7 @@ static void run_lansvd_t(const char *jobu, const char *jobv, int m, int n, int *
         dev_ritzvec<T>(c, false, du, dv, neig, jold);
     }
     PGB_CUDA(cudaEventRecord(c.evs1, c.s));
-    copy_out<T>(c, U, ldu, V, ldv, neig, du, dv);
+    copy_out<T>(c, U, ldu, V, ldv, neig, du, dv, real);
     doption[2] = dop[2];
     PGB_CUDA(cudaEventRecord(c.ev1, c.s));
     c.sync();
@@ -1783,11 +1823,12 @@ static void run_lansvd_t(const char *jobu, const char *jobv, int m, int n, int *
 // dlansvd (double/dlansvd.F:131-291); FP32 vectors when the precision is 2
 static void run_lansvd(const char *jobu, const char *jobv, int m, int n, int *kp, int kmax, propack_aprod_t aprod,
                        double *U, int ldu, double *sigma, double *bnd, double *V, int ldv, double tolin,
-                       double *doption, const int *ioption, int *info, double *dparm, int *iparm)
+                       double *doption, const int *ioption, int *info, double *dparm, int *iparm,
+                       const RealOut *real = nullptr)
 {
     if (g_precision == 2)
         run_lansvd_t<float>(jobu, jobv, m, n, kp, kmax, aprod, U, ldu, sigma, bnd, V, ldv, tolin, doption, ioption,
-                            info, dparm, iparm);
+                            info, dparm, iparm, nullptr, nullptr, real);
     else
         run_lansvd_t<double>(jobu, jobv, m, n, kp, kmax, aprod, U, ldu, sigma, bnd, V, ldv, tolin, doption,
                              ioption, info, dparm, iparm);
@@ -1975,8 +2016,9 @@ extern "C" void zlansvd_(const char *jobu, const char *jobv, const int *m, const
 // ---------------------------------------------- single-precision drivers
 // SLANSVD / SLANSVD_IRL (single/slansvd.F:1-3, single/slansvd_irl.F:1-3):
 // the same argument lists with REAL arrays and a REAL APROD.  They run the
-// FP32 form (FP32 vectors, SpMV and Gram-Schmidt, FP64 scalars) and widen /
-// narrow at the boundary.  A user APROD is reached through a trampoline that
+// FP32 form (FP32 vectors, SpMV and Gram-Schmidt, FP64 scalars); the start
+// vector and the Ritz vectors cross the boundary in FP32 (which = 'S', which
+// runs in FP64, widens and narrows).  A user APROD is reached through a trampoline that
 // narrows the FP64 vectors of the host path to the caller's REAL arrays.
 struct SAprod {
     propack_saprod_t f = nullptr;
@@ -1998,22 +2040,30 @@ static void saprod_trampoline(const char *transa, const int *m, const int *n, co
     for (int i = 0; i < nout; i++) y[i] = g_saprod.yf[i];
 }
 
-// widened copies of the caller's REAL arrays for the FP64-interfaced drivers
+// FP64 scalars and, where the solve runs in FP64 (which = 'S'), widened
+// copies of the caller's REAL arrays
 struct SArgs {
     std::vector<double> U, V, sig, bnd, opt;
     propack_aprod_t ap = nullptr;
+    RealOut real;
+    bool wide = false;
 };
 static void s_prepare(SArgs &w, propack_saprod_t aprod, int m, int n, int ncols_u, int ncols_v, int ldu, int ldv,
-                      const float *U, int nsig, const float *soption, int nopt, float *sparm)
+                      float *U, float *V, int nsig, const float *soption, int nopt, float *sparm)
 {
-    w.U.assign((size_t)m * ncols_u, 0.0);
-    for (int i = 0; i < m; i++) w.U[i] = U[i];  // U(:,1), the start vector
-    w.V.assign((size_t)n * ncols_v, 0.0);
+    if (w.wide) {
+        w.U.assign((size_t)m * ncols_u, 0.0);
+        for (int i = 0; i < m; i++) w.U[i] = U[i];  // U(:,1), the start vector
+        w.V.assign((size_t)n * ncols_v, 0.0);
+    }
+    w.real.U = U;
+    w.real.V = V;
+    w.real.ldu = ldu;
+    w.real.ldv = ldv;
     w.sig.assign(std::max(nsig, 1), 0.0);
     w.bnd.assign(std::max(nsig, 1), 0.0);
     w.opt.assign(4, 0.0);
     for (int i = 0; i < nopt; i++) w.opt[i] = soption[i];
-    (void)ldu; (void)ldv;
     if (aprod == propack_gpu_csr_saprod_) {
         w.ap = propack_gpu_csr_aprod_;
     } else {
@@ -2025,7 +2075,7 @@ static void s_prepare(SArgs &w, propack_saprod_t aprod, int m, int n, int ncols_
 static void s_finish(const SArgs &w, int m, int n, int ncols, bool du, bool dv, float *U, int ldu, float *V, int ldv,
                      float *sigma, float *bnd, int nsig, float *soption, int nopt)
 {
-    for (int c = 0; c < ncols; c++) {
+    for (int c = 0; w.wide && c < ncols; c++) {
         if (du)
             for (int i = 0; i < m; i++) U[(size_t)c * ldu + i] = (float)w.U[(size_t)c * m + i];
         if (dv)
@@ -2054,10 +2104,12 @@ extern "C" void slansvd_irl_(const char *which, const char *jobu, const char *jo
         check_work("slansvd_irl_", true, *m, *n, *dim, lwork, liwork, nullptr, false);
         SArgs w;
         const int k0 = *neig;
-        s_prepare(w, aprod, *m, *n, *dim + 1, *dim, *ldu, *ldv, U, k0, soption, 4, sparm);
+        w.wide = which && (which[0] == 's' || which[0] == 'S');
+        s_prepare(w, aprod, *m, *n, *dim + 1, *dim, *ldu, *ldv, U, V, k0, soption, 4, sparm);
         g_precision = 2;
         run_irl(which, jobu, jobv, *m, *n, *dim, *p, neig, *maxiter, w.ap, w.U.data(), *m, w.sig.data(),
-                w.bnd.data(), w.V.data(), *n, (double)*tolin, w.opt.data(), ioption, info, nullptr, iparm);
+                w.bnd.data(), w.V.data(), *n, (double)*tolin, w.opt.data(), ioption, info, nullptr, iparm,
+                w.wide ? nullptr : &w.real);
         g_precision = saved;
         s_finish(w, *m, *n, std::min(*neig, k0), yes(jobu), yes(jobv), U, *ldu, V, *ldv, sigma, bnd,
                  std::min(*neig, k0), soption, 4);
@@ -2091,10 +2143,10 @@ extern "C" void slansvd_(const char *jobu, const char *jobv, const int *m, const
         check_work("slansvd_", false, *m, *n, *kmax, lwork, liwork, nullptr, false);
         SArgs w;
         const int k0 = *k;
-        s_prepare(w, aprod, *m, *n, *kmax + 1, *kmax, *ldu, *ldv, U, k0, soption, 3, sparm);
+        s_prepare(w, aprod, *m, *n, *kmax + 1, *kmax, *ldu, *ldv, U, V, k0, soption, 3, sparm);
         g_precision = 2;
         run_lansvd(jobu, jobv, *m, *n, k, *kmax, w.ap, w.U.data(), *m, w.sig.data(), w.bnd.data(), w.V.data(), *n,
-                   (double)*tolin, w.opt.data(), ioption, info, nullptr, iparm);
+                   (double)*tolin, w.opt.data(), ioption, info, nullptr, iparm, &w.real);
         g_precision = saved;
         // dlansvd returns bounds for the first k values even when fewer converged
         s_finish(w, *m, *n, std::min(*k, k0), yes(jobu), yes(jobv), U, *ldu, V, *ldv, sigma, bnd, k0, soption, 3);
