@@ -34,6 +34,7 @@
 
 #include "../../include/propack_gb300.h"
 #include "pgb.cuh"
+#include "pgb_spmv.cuh"
 #include "pgb_tc.cuh"
 
 namespace pgb {
@@ -51,7 +52,7 @@ struct Mlp {
     bf16 *W1b = nullptr, *W2b = nullptr, *W2Tb = nullptr, *w3b = nullptr;
     int64_t step = 0;
     int cap = 0;
-    int64_t ucap = 0;
+    int64_t ucap = 0, omcap = 0;
     float *F = nullptr, *out = nullptr, *gout = nullptr, *D1 = nullptr;
     bf16 *H1 = nullptr, *H2 = nullptr, *D2 = nullptr;
     double *Y = nullptr, *om = nullptr, *U = nullptr, *red = nullptr, *coef = nullptr;
@@ -69,49 +70,160 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long z)
     z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
     return z ^ (z >> 31);
 }
-// Omega(j, c): standard normal from two counter-based uniforms (Box-Muller)
-__global__ void k_mlp_omega(int n, int col, unsigned long long seed, double *x)
+// Omega(j, c): standard normal from two counter-based uniforms (Box-Muller),
+// row-major n x MLP_SK, so that one entry of A meets its 16 numbers in one
+// 128-byte line.  Bound by the FP64 pipe (log, sqrt and cospi of every
+// element; 105 us of it at n = 50,000).
+__global__ void k_mlp_omega(int n, unsigned long long seed, double *om)
 {
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < (long long)n * MLP_SK;
+         t += (long long)gridDim.x * blockDim.x) {
+        const int j = (int)(t / MLP_SK), col = (int)(t % MLP_SK);
         const unsigned long long a = mix64(seed ^ mix64(((unsigned long long)col << 40) ^ (unsigned long long)j));
         const unsigned long long b = mix64(a);
         const double u1 = ((double)(a >> 11) + 0.5) * (1.0 / 9007199254740992.0);
         const double u2 = (double)(b >> 11) * (1.0 / 9007199254740992.0);
-        x[j] = sqrt(-2.0 * log(u1)) * cospi(2.0 * u2);
+        om[t] = sqrt(-2.0 * log(u1)) * cospi(2.0 * u2);
     }
 }
 
-// sum over rows of ||y_i||^2 (Y column-major m x 16): partials per CTA
-__global__ void __launch_bounds__(256) k_mlp_sumsq(int m, const double *Y, double *part)
+// sum over entries e0 .. e1 of val[e] X[idx[e]][c] by a half warp (lane c of
+// 16); columns from n0 on read the rows of Z
+constexpr int SK_UNROLL = 4;
+__device__ __forceinline__ double sketch_sum(const int *__restrict__ idx, const double *__restrict__ val, int e0,
+                                             int e1, int step, int n0, const double *X, const double *Z, int c)
 {
-    __shared__ double red[32];
-    double s = 0.0;
-    for (int i = blockIdx.x * 256 + threadIdx.x; i < m; i += gridDim.x * 256)
-        for (int c = 0; c < MLP_SK; c++) {
-            const double y = Y[(size_t)c * m + i];
-            s = fma(y, y, s);
-        }
-    s = block_sum<256>(s, red);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
+    double acc = 0.0;
+    int e = e0;
+    for (; e + (SK_UNROLL - 1) * step < e1; e += SK_UNROLL * step) {
+        int ci[SK_UNROLL];
+        double v[SK_UNROLL], x[SK_UNROLL];
+#pragma unroll
+        for (int u = 0; u < SK_UNROLL; u++) { ci[u] = idx[e + u * step]; v[u] = val[e + u * step]; }
+#pragma unroll
+        for (int u = 0; u < SK_UNROLL; u++)
+            x[u] = ci[u] < n0 ? X[(size_t)ci[u] * MLP_SK + c] : Z[(size_t)(ci[u] - n0) * MLP_SK + c];
+#pragma unroll
+        for (int u = 0; u < SK_UNROLL; u++) acc = fma(v[u], x[u], acc);
+    }
+    for (; e < e1; e += step) {
+        const int ci = idx[e];
+        acc = fma(val[e], ci < n0 ? X[(size_t)ci * MLP_SK + c] : Z[(size_t)(ci - n0) * MLP_SK + c], acc);
+    }
+    return acc;
 }
 
-__global__ void k_mlp_features(int m, const int *rowptr, const double *Y, const double *part, int nparts, float *F)
+// Z = diag(w) R' Omega (r x MLP_SK): a warp per segment of THIN_SEG entries of
+// a row of Th = R' (its halves take alternate entries); the warp that
+// completes a row adds its partials in order.  zpart: rows * 4 segs * MLP_SK,
+// tick: rows zeroed counters, left zeroed.
+__global__ void __launch_bounds__(256) k_mlp_thin(Csr Th, const double *om, const double *w, double *zpart,
+                                                  double *Z, unsigned int *tick)
 {
-    __shared__ double rho;
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int b = 0; b < nparts; b++) s += part[b];
-        rho = sqrt(s / (double)m);
-        if (!(rho > 0.0)) rho = 1.0;
+    const unsigned F = 0xffffffffu;
+    const int lane = threadIdx.x & 31, h = lane >> 4, c = lane & 15;
+    const int nseg = 4 * Th.segs, nw = gridDim.x * 8;
+    for (int t = blockIdx.x * 8 + (threadIdx.x >> 5); t < Th.rows * nseg; t += nw) {
+        const int row = t / nseg, sg = t % nseg;
+        const int p0 = Th.ptr[row], p1 = Th.ptr[row + 1];
+        const int used = max(1, (p1 - p0 + THIN_SEG - 1) / THIN_SEG);
+        if (sg >= used) continue;
+        const int e0 = p0 + sg * THIN_SEG;
+        double acc = sketch_sum(Th.idx, Th.val, e0 + h, min(p1, e0 + THIN_SEG), 2, INT_MAX, om, nullptr, c);
+        acc += __shfl_xor_sync(F, acc, 16);
+        if (h == 0) zpart[(size_t)t * MLP_SK + c] = acc;
+        __threadfence();
+        __syncwarp();
+        unsigned old = 0;
+        if (lane == 0) old = atomicAdd(tick + row, 1u);
+        if (__shfl_sync(F, old, 0) + 1 == (unsigned)used) {
+            __threadfence();
+            double s = 0.0;
+            for (int q = h; q < used; q += 2) s += __ldcg(zpart + ((size_t)row * nseg + q) * MLP_SK + c);
+            s += __shfl_xor_sync(F, s, 16);
+            if (h == 0) Z[(size_t)row * MLP_SK + c] = w[row] * s;
+            if (lane == 0) tick[row] = 0u;
+        }
+    }
+}
+
+// Y = A Omega (row-major m x MLP_SK) in one pass over A, a half warp per row
+// and column c per lane, and the CTAs' partial sums of ||y_i||^2.  As sixteen
+// products by one column each it read A sixteen times behind 48 launches (830
+// us at 200,000 x 50,000 with 14 entries per row, 500 us at a quarter of it).
+// Bound by the FP64 pipe: one FMA per entry and column.
+// Rows longer than SK_LONG wait in a list for the whole CTA (its half warps
+// take every 16th entry), so that no half warp walks one alone; rows are dealt
+// round-robin, so that few long rows reach all CTAs.
+constexpr int SK_LONG = 256, SK_LIST = 64;
+__global__ void __launch_bounds__(256) k_mlp_sketch(Csr A, const double *om, const double *Z, double *Y,
+                                                    double *part)
+{
+    __shared__ double buf[256];
+    __shared__ int list[SK_LIST], nlist;
+    const int c = threadIdx.x & 15, hw = threadIdx.x >> 4;
+    if (threadIdx.x == 0) nlist = 0;
+    __syncthreads();
+    double sq = 0.0;
+    for (long long rr = blockIdx.x + (long long)gridDim.x * hw; rr < A.rows; rr += (long long)gridDim.x * 16) {
+        const int r = (int)rr, e0 = A.ptr[r], e1 = A.ptr[r + 1];
+        if (e1 - e0 > SK_LONG) {
+            int at = 0;
+            if (c == 0) at = atomicAdd(&nlist, 1);
+            at = __shfl_sync(0xffffu << (threadIdx.x & 16), at, 0, 16);
+            if (at < SK_LIST) {
+                if (c == 0) list[at] = r;
+                continue;
+            }
+        }
+        const double y = sketch_sum(A.idx, A.val, e0, e1, 1, A.ncol0, om, Z, c);
+        Y[(size_t)r * MLP_SK + c] = y;
+        sq = fma(y, y, sq);
     }
     __syncthreads();
+    const int nl = min(nlist, SK_LIST);
+    for (int q = 0; q < nl; q++) {
+        const int r = list[q];
+        buf[threadIdx.x] = sketch_sum(A.idx, A.val, A.ptr[r] + hw, A.ptr[r + 1], 16, A.ncol0, om, Z, c);
+        __syncthreads();
+        if (hw == 0) {
+            double y = 0.0;
+            for (int i = 0; i < 16; i++) y += buf[16 * i + c];
+            Y[(size_t)r * MLP_SK + c] = y;
+            sq = fma(y, y, sq);
+        }
+        __syncthreads();
+    }
+    block_sums<256, 1>({sq}, buf, {part + blockIdx.x});
+}
+
+__global__ void __launch_bounds__(256) k_mlp_features(int m, const int *rowptr, const double *Y, const double *part,
+                                                      int nparts, float *F)
+{
+    __shared__ double buf[256], tot, irho;
+    double s = 0.0;
+    for (int b = threadIdx.x; b < nparts; b += 256) s += part[b];
+    block_sums<256, 1>({s}, buf, {&tot});
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double rho = sqrt(tot / (double)m);
+        if (!(rho > 0.0)) rho = 1.0;
+        irho = 1.0 / rho;
+    }
+    __syncthreads();
+    const double ir = irho;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
         float *f = F + (size_t)i * MLP_IN;
+        const double2 *y2 = reinterpret_cast<const double2 *>(Y + (size_t)i * MLP_SK);
         double nn = 0.0;
-        for (int c = 0; c < MLP_SK; c++) {
-            const double y = Y[(size_t)c * m + i] / rho;
-            nn = fma(y, y, nn);
-            f[2 + c] = (float)(2.0 * y);
+#pragma unroll
+        for (int c = 0; c < MLP_SK / 2; c++) {
+            const double2 v = y2[c];
+            const double a = v.x * ir, b = v.y * ir;
+            nn = fma(a, a, nn);
+            nn = fma(b, b, nn);
+            f[2 + 2 * c] = (float)(2.0 * a);
+            f[3 + 2 * c] = (float)(2.0 * b);
         }
         f[0] = (float)(log1p((double)(rowptr[i + 1] - rowptr[i])) / 4.0);
         f[1] = (float)sqrt(nn);
@@ -542,6 +654,7 @@ static void mlp_reserve(Mlp &M, int m, int k)
 }
 
 constexpr int MLP_GRID = 1024;         // CTAs of the row-parallel reductions
+constexpr int MLP_RED_GRID = 4096;     // partials that the reduction scratch holds at least
 constexpr int MLP_DW2_CHUNKS = 64;     // row chunks of dW2
 
 static void mlp_cast(Mlp &M)
@@ -555,16 +668,37 @@ static void mlp_features(Mlp &M, const Operator &op, unsigned long long seed)
 {
     const int m = op.m, n = op.n;
     mlp_reserve(M, m, 1);
-    if (!M.om) PGB_CUDA(cudaMalloc(&M.om, sizeof(double) * (size_t)std::max(n, 1)));
-    for (int c = 0; c < MLP_SK; c++) {
-        k_mlp_omega<<<std::min(4096, (n + 255) / 256), 256, 0, M.s>>>(n, c, seed, M.om);
-        PGB_LAUNCHED();
-        op_apply<double>(op, false, M.om, M.Y + (size_t)c * m, M.s);
+    const int64_t nom = (int64_t)std::max(n, 1) * MLP_SK;
+    if (nom > M.omcap) {
+        if (M.om) PGB_CUDA(cudaFree(M.om));
+        M.om = nullptr;
+        M.omcap = 0;
+        PGB_CUDA(cudaMalloc(&M.om, sizeof(double) * (size_t)nom));
+        M.omcap = nom;
     }
-    k_mlp_sumsq<<<MLP_GRID, 256, 0, M.s>>>(m, M.Y, M.red);
+    const int full = 8 * device_info().sms;  // CTAs of 256 threads that fit at once
+    k_mlp_omega<<<std::min<int64_t>(full, (nom + 255) / 256), 256, 0, M.s>>>(n, seed, M.om);
     PGB_LAUNCHED();
-    k_mlp_features<<<std::min(4096, (m + 255) / 256), 256, 0, M.s>>>(m, op.fwd.ptr, M.Y, M.red, MLP_GRID, M.F);
+    double *Z = nullptr, *zpart = nullptr;
+    unsigned *tick = nullptr;
+    if (op.r > 0) {
+        const int nt = op.thin_r.rows * 4 * op.thin_r.segs;
+        Z = (double *)pool_alloc(sizeof(double) * MLP_SK * (size_t)op.r, M.s);
+        zpart = (double *)pool_alloc(sizeof(double) * MLP_SK * (size_t)nt, M.s);
+        tick = (unsigned *)pool_alloc(sizeof(unsigned) * (size_t)op.r, M.s);
+        PGB_CUDA(cudaMemsetAsync(tick, 0, sizeof(unsigned) * (size_t)op.r, M.s));
+        k_mlp_thin<<<std::max(1, std::min(full, (nt + 7) / 8)), 256, 0, M.s>>>(op.thin_r, M.om, op.w, zpart, Z, tick);
+        PGB_LAUNCHED();
+    }
+    const int64_t want = std::max<int64_t>((m + 15) / 16, std::min<int64_t>(m, op.fwd.nnz / 4096));
+    const int g = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(full, MLP_RED_GRID), want));
+    k_mlp_sketch<<<g, 256, 0, M.s>>>(op.fwd, M.om, Z, M.Y, M.red);
     PGB_LAUNCHED();
+    k_mlp_features<<<std::max(1, std::min(full, (m + 255) / 256)), 256, 0, M.s>>>(m, op.fwd.ptr, M.Y, M.red, g, M.F);
+    PGB_LAUNCHED();
+    pool_free(Z, M.s);
+    pool_free(zpart, M.s);
+    pool_free(tick, M.s);
 }
 
 static size_t mm_smem() { return sizeof(unsigned short) * MLP_H * W2S; }
@@ -657,6 +791,10 @@ static Operator *mlp_operator(int64_t op_handle)
     Operator *op = lookup_operator(op_handle);
     if (!op) {
         set_error("no live operator handle");
+        throw ArgFailure();
+    }
+    if (op->cplx == 2) {
+        set_error("the learned start takes real operators");
         throw ArgFailure();
     }
     return op;
