@@ -1131,7 +1131,7 @@ static void d2h_columns(char *dst, size_t dpitch, const char *src, size_t spitch
 }
 
 // bytes from host src to device dst on stream s: straight when src is
-// pinned (or small); otherwise through the bounce buffer, each 64 MB piece
+// pinned (or small); otherwise through the bounce buffer, each piece
 // copied into a half by the host pool while the other half's copy to the
 // device runs.  Returns when the buffer is free again (its last copies
 // done); the device copies are ordered on s.
@@ -1145,9 +1145,12 @@ void h2d_bytes(void *dst, const void *src, size_t bytes, cudaStream_t s)
     BounceLease lease;
     Bounce &b = lease.b;
     HostPool &pool = HostPool::get();
-    const size_t np = (bytes + BOUNCE_BYTES - 1) / BOUNCE_BYTES;
+    // eight pieces at least (of 4 MB and more), so that the first copies to
+    // the device start early
+    const size_t piece = std::min(BOUNCE_BYTES, std::max((size_t)4 << 20, (bytes / 8 + 4095) / 4096 * 4096));
+    const size_t np = (bytes + piece - 1) / piece;
     for (size_t i = 0; i < np; i++) {
-        const size_t off = i * BOUNCE_BYTES, len = std::min(BOUNCE_BYTES, bytes - off);
+        const size_t off = i * piece, len = std::min(piece, bytes - off);
         char *half = b.buf + (i & 1) * BOUNCE_BYTES;
         if (i >= 2) PGB_CUDA(cudaEventSynchronize(b.ev[i & 1]));  // piece i-2 has left this half
         const int parts = (int)std::min<size_t>((size_t)pool.threads() * 2, std::max<size_t>(1, len >> 20));

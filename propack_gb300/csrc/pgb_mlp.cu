@@ -44,6 +44,7 @@ constexpr int OW1 = 0, OB1 = OW1 + MLP_H * MLP_IN, OW2 = OB1 + MLP_H, OB2 = OW2 
               OW3 = OB2 + MLP_H, OB3 = OW3 + MLP_H, MLP_NP = OB3 + 1;
 constexpr int W2S = MLP_H + 8;  // padded row stride of the BF16 W2 copies in shared memory
 constexpr double MLP_EPS = 1e-4;
+constexpr int MLP_LOSS_AT = 4095;  // the loss in the coefficient array (k <= 4000)
 
 typedef __nv_bfloat16 bf16;
 
@@ -59,7 +60,8 @@ struct Mlp {
     float *part = nullptr;  // per-CTA partial sums of the reductions
     int *err = nullptr;     // set by the tensor-core kernel when a bounded wait runs out
     int device = 0;
-    cudaStream_t s = nullptr;
+    cudaStream_t s = nullptr, s2 = nullptr;  // s2: uploads of U
+    cudaEvent_t ev = nullptr;
 };
 
 // ------------------------------------------------------------- helpers
@@ -230,20 +232,47 @@ __global__ void __launch_bounds__(256) k_mlp_features(int m, const int *rowptr, 
     }
 }
 
-// h1 = relu(W1 f + b1) as BF16, row-major m x 256; one thread per (row, unit)
-__global__ void __launch_bounds__(MLP_H) k_mlp_l1(int m, const float *F, const bf16 *W1b, const float *b1, bf16 *H1)
+// h1 = relu(W1 f + b1) as BF16, row-major m x 256: a thread holds the weights
+// of two units and takes every other row of a 32-row tile of features in
+// shared memory (five 16-byte broadcasts and 36 FMAs a row); as one row
+// per CTA at a time it waited on a global load per 18 FMAs (186 us at 200,000
+// rows).
+constexpr int L1_TR = 32, L1_FS = 20;  // rows per tile, padded row of features
+__global__ void __launch_bounds__(256) k_mlp_l1(int m, const float *F, const bf16 *W1b, const float *b1, bf16 *H1)
 {
-    __shared__ float w[MLP_H * MLP_IN];
-    for (int t = threadIdx.x; t < MLP_H * MLP_IN; t += MLP_H) w[t] = __bfloat162float(W1b[t]);
-    __syncthreads();
-    const int j = threadIdx.x;
-    const float bj = b1[j];
-    for (int i = blockIdx.x; i < m; i += gridDim.x) {
-        const float *f = F + (size_t)i * MLP_IN;
-        float z = bj;
+    __shared__ __align__(16) float f[L1_TR * L1_FS];
+    const int u = threadIdx.x & 127, g = threadIdx.x >> 7;
+    float w0[MLP_IN], w1[MLP_IN];
 #pragma unroll
-        for (int q = 0; q < MLP_IN; q++) z = fmaf(w[j * MLP_IN + q], f[q], z);
-        H1[(size_t)i * MLP_H + j] = __float2bfloat16_rn(fmaxf(z, 0.f));
+    for (int q = 0; q < MLP_IN; q++) {
+        w0[q] = __bfloat162float(W1b[(2 * u) * MLP_IN + q]);
+        w1[q] = __bfloat162float(W1b[(2 * u + 1) * MLP_IN + q]);
+    }
+    const float c0 = b1[2 * u], c1 = b1[2 * u + 1];
+    for (long long i0 = (long long)blockIdx.x * L1_TR; i0 < m; i0 += (long long)gridDim.x * L1_TR) {
+        const int nr = (int)min((long long)L1_TR, m - i0);
+        for (int t = threadIdx.x; t < nr * MLP_IN; t += 256)
+            f[(t / MLP_IN) * L1_FS + t % MLP_IN] = F[i0 * MLP_IN + t];
+        __syncthreads();
+        for (int r = g; r < nr; r += 2) {
+            float fv[L1_FS];
+#pragma unroll
+            for (int q = 0; q < L1_FS / 4; q++) {
+                const float4 v = *reinterpret_cast<const float4 *>(f + r * L1_FS + 4 * q);
+                fv[4 * q] = v.x; fv[4 * q + 1] = v.y; fv[4 * q + 2] = v.z; fv[4 * q + 3] = v.w;
+            }
+            float z0 = c0, z1 = c1;
+#pragma unroll
+            for (int q = 0; q < MLP_IN; q++) {
+                z0 = fmaf(w0[q], fv[q], z0);
+                z1 = fmaf(w1[q], fv[q], z1);
+            }
+            __nv_bfloat162 h;
+            h.x = __float2bfloat16_rn(fmaxf(z0, 0.f));
+            h.y = __float2bfloat16_rn(fmaxf(z1, 0.f));
+            *reinterpret_cast<__nv_bfloat162 *>(H1 + (i0 + r) * MLP_H + 2 * u) = h;
+        }
+        __syncthreads();
     }
 }
 
@@ -334,6 +363,7 @@ constexpr int TM_SMEM = TM_KSTEPS * (TM_ATILE + TM_BTILE) + 128;
 constexpr uint32_t TM_IDESC = tc_idesc_bf16(TM_BM, TM_N);
 constexpr unsigned TM_TMEM_COLS = TM_N;
 constexpr long TM_WAIT_LIMIT = 1L << 22;
+constexpr int TM_PRE = TM_BM * (MLP_H / 8) / 256;  // 16-byte pieces of a tile per thread
 static_assert(TM_SMEM <= 227 * 1024, "shared memory");
 
 template <int MODE>
@@ -371,14 +401,27 @@ __global__ void __launch_bounds__(256, 1) k_mlp_mm_tc(int m, const bf16 *X, cons
     const uint32_t tmem = *tslot;
     int it = 0;
     bool bad = false;
+    // a tile of X in registers (rows past m read as zeros): the next tile's
+    // loads are in flight while this tile's MMAs and epilogue run
+    uint4 pre[TM_PRE];
+    auto fetch = [&](int tile) {
+#pragma unroll
+        for (int i = 0; i < TM_PRE; i++) {
+            const int q = tid + 256 * i;
+            const int r = (q >> 1) & (TM_BM - 1), kc = ((q >> 8) << 1) | (q & 1);
+            const long long row = (long long)tile * TM_BM + r;
+            pre[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (row < m) pre[i] = *reinterpret_cast<const uint4 *>(X + row * MLP_H + kc * 8);
+        }
+    };
+    if ((int)blockIdx.x < ntiles) fetch(blockIdx.x);
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, it++) {
         const int row0 = t * TM_BM;
-        // the tile of X (rows past m read as zeros)
-        for (int q = tid; q < TM_BM * (MLP_H / 8); q += blockDim.x) {
+#pragma unroll
+        for (int i = 0; i < TM_PRE; i++) {
+            const int q = tid + 256 * i;
             const int r = (q >> 1) & (TM_BM - 1), kc = ((q >> 8) << 1) | (q & 1);
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (row0 + r < m) v = *reinterpret_cast<const uint4 *>(X + (size_t)(row0 + r) * MLP_H + kc * 8);
-            tc_st16(a_s + (kc >> 1) * TM_ATILE + (r >> 3) * 256 + (kc & 1) * 128 + (r & 7) * 16, v);
+            tc_st16(a_s + (kc >> 1) * TM_ATILE + (r >> 3) * 256 + (kc & 1) * 128 + (r & 7) * 16, pre[i]);
         }
         tc_fence_proxy();
         __syncthreads();
@@ -389,6 +432,7 @@ __global__ void __launch_bounds__(256, 1) k_mlp_mm_tc(int m, const bf16 *X, cons
                 tc_mma(tmem, tc_desc(a_s + ks * TM_ATILE), tc_desc(b_s + ks * TM_BTILE), TM_IDESC, ks > 0 ? 1u : 0u);
             tc_commit(bar_s);
         }
+        if (t + (int)gridDim.x < ntiles) fetch(t + gridDim.x);
         const bool ok = tc_bar_wait(bar_s, (unsigned)(it & 1), TM_WAIT_LIMIT);
         if (__syncthreads_or(!ok)) {
             bad = true;
@@ -460,18 +504,69 @@ __global__ void k_mlp_l3(int m, const bf16 *H2, const bf16 *w3b, const float *b3
     }
 }
 
-// partials of c = U' u0 (k values) and ||u0||^2: part[b * (k+1) + j]
-__global__ void __launch_bounds__(256) k_mlp_proj(int m, int k, const double *U, const float *out, double *part)
+// partials of c = U' u0 (k values) and ||u0||^2 (column k): a warp per column
+// and row segment, part[seg * (k+1) + j].  A block reduction per column had
+// cost more than the columns (131 us for the 51 MB of 200,000 x 32).
+__global__ void __launch_bounds__(256) k_mlp_proj(int m, int k, int nseg, const double *U, const float *out,
+                                                  double *part)
 {
-    __shared__ double red[32];
-    for (int j = 0; j <= k; j++) {
-        double s = 0.0;
-        for (int i = blockIdx.x * 256 + threadIdx.x; i < m; i += gridDim.x * 256) {
-            const double o = out[i];
-            s = fma(j < k ? U[(size_t)j * m + i] : o, o, s);
+    const int lane = threadIdx.x & 31, nw = gridDim.x * 8;
+    const int len = (m + nseg - 1) / nseg;
+    for (int t = blockIdx.x * 8 + (threadIdx.x >> 5); t < (k + 1) * nseg; t += nw) {
+        const int j = t % (k + 1), sg = t / (k + 1);
+        const long long i0 = (long long)sg * len, i1 = min((long long)m, i0 + len);
+        const double *u = U + (size_t)min(j, k - 1) * m;
+        double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+        long long i = i0 + lane;
+        for (; i + 96 < i1; i += 128) {
+            const double o0 = out[i], o1 = out[i + 32], o2 = out[i + 64], o3 = out[i + 96];
+            s0 = fma(j < k ? u[i] : o0, o0, s0);
+            s1 = fma(j < k ? u[i + 32] : o1, o1, s1);
+            s2 = fma(j < k ? u[i + 64] : o2, o2, s2);
+            s3 = fma(j < k ? u[i + 96] : o3, o3, s3);
         }
-        s = block_sum<256>(s, red);
-        if (threadIdx.x == 0) part[(size_t)blockIdx.x * (k + 1) + j] = s;
+        for (; i < i1; i += 32) {
+            const double o = out[i];
+            s0 = fma(j < k ? u[i] : o, o, s0);
+        }
+        const double s = warp_sum((s0 + s1) + (s2 + s3));
+        if (lane == 0) part[t] = s;
+    }
+}
+
+// c, the loss and the coefficients of dL/du0 from the partials; one CTA.
+// L = log ||u0||^2 - (1/k) sum_j log(c_j^2 + eps), eps = MLP_EPS ||u0||^2 / k:
+// coef_j multiplies U_j, coef_k multiplies u0.
+__global__ void __launch_bounds__(256) k_mlp_coef(int k, int nseg, const double *part, double *coef, double *loss)
+{
+    __shared__ double buf[512], tot[2], nrm;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // column k first: the others need eps
+    if (w == 0) {
+        double s = 0.0;
+        for (int q = lane; q < nseg; q += 32) s += part[(size_t)q * (k + 1) + k];
+        s = warp_sum(s);
+        if (lane == 0) nrm = fmax(s, 1e-300);
+    }
+    __syncthreads();
+    const double nrm2 = nrm, eps = MLP_EPS * nrm2 / k;
+    double lg = 0.0, rec = 0.0;
+    for (int j = w; j < k; j += 8) {
+        double s = 0.0;
+        for (int q = lane; q < nseg; q += 32) s += part[(size_t)q * (k + 1) + j];
+        s = warp_sum(s);
+        if (lane == 0) {
+            const double d = s * s + eps;
+            coef[j] = -2.0 * s / (d * k);
+            lg += log(d);
+            rec += (MLP_EPS / k) / d;
+        }
+    }
+    block_sums<256, 2>({lg, rec}, buf, {tot, tot + 1});
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        coef[k] = 2.0 / nrm2 - 2.0 * tot[1] / k;
+        *loss = log(nrm2) - tot[0] / k;
     }
 }
 
@@ -485,109 +580,214 @@ __global__ void k_mlp_gout(int m, int k, const double *U, const double *coef, co
     }
 }
 
-// layer 3 backward: partials of dw3 (256) and db3, and D2 = bf16(g w3 [h2 > 0])
-__global__ void __launch_bounds__(MLP_H) k_mlp_b3(int m, const float *g, const bf16 *H2, const bf16 *w3b, bf16 *D2,
-                                                  float *part)
+// layer 3 backward: D2 = bf16(g w3 [h2 > 0]) and partials of dw3, db2 (the
+// column sums of D2) and db3: a thread takes two units of every other row of
+// the CTA, four rows in flight.  part[b * B3_N]: dw3, db2, db3.
+constexpr int B3_N = 2 * MLP_H + 1, B3_UNROLL = 4;
+__global__ void __launch_bounds__(256) k_mlp_b3(int m, const float *g, const bf16 *H2, const bf16 *w3b, bf16 *D2,
+                                                float *part)
 {
-    const int j = threadIdx.x;
-    const float w = __bfloat162float(w3b[j]);
-    float dw = 0.f, db = 0.f;
-    for (int i = blockIdx.x; i < m; i += gridDim.x) {
-        const float gi = g[i];
-        const float h = __bfloat162float(H2[(size_t)i * MLP_H + j]);
-        dw = fmaf(gi, h, dw);
+    __shared__ float red[128][5];
+    const int u = threadIdx.x & 127, gr = threadIdx.x >> 7;
+    const float w0 = __bfloat162float(w3b[2 * u]), w1 = __bfloat162float(w3b[2 * u + 1]);
+    float a0 = 0.f, a1 = 0.f, d0 = 0.f, d1 = 0.f, db = 0.f;
+    const long long st = 2LL * gridDim.x;
+    auto one = [&](long long i, float gi, __nv_bfloat162 h) {
+        const float h0 = __bfloat162float(h.x), h1 = __bfloat162float(h.y);
+        a0 = fmaf(gi, h0, a0);
+        a1 = fmaf(gi, h1, a1);
+        __nv_bfloat162 d;
+        d.x = __float2bfloat16_rn(h0 > 0.f ? gi * w0 : 0.f);
+        d.y = __float2bfloat16_rn(h1 > 0.f ? gi * w1 : 0.f);
+        d0 += __bfloat162float(d.x);
+        d1 += __bfloat162float(d.y);
         db += gi;
-        D2[(size_t)i * MLP_H + j] = __float2bfloat16_rn(h > 0.f ? gi * w : 0.f);
+        *reinterpret_cast<__nv_bfloat162 *>(D2 + i * MLP_H + 2 * u) = d;
+    };
+    long long i = 2LL * blockIdx.x + gr;
+    for (; i + (B3_UNROLL - 1) * st < m; i += B3_UNROLL * st) {
+        float gi[B3_UNROLL];
+        __nv_bfloat162 h[B3_UNROLL];
+#pragma unroll
+        for (int q = 0; q < B3_UNROLL; q++) {
+            gi[q] = g[i + q * st];
+            h[q] = *reinterpret_cast<const __nv_bfloat162 *>(H2 + (i + q * st) * MLP_H + 2 * u);
+        }
+#pragma unroll
+        for (int q = 0; q < B3_UNROLL; q++) one(i + q * st, gi[q], h[q]);
     }
-    part[(size_t)blockIdx.x * (MLP_H + 1) + j] = dw;
-    if (j == 0) part[(size_t)blockIdx.x * (MLP_H + 1) + MLP_H] = db;
+    for (; i < m; i += st) one(i, g[i], *reinterpret_cast<const __nv_bfloat162 *>(H2 + i * MLP_H + 2 * u));
+    if (gr == 1) { red[u][0] = a0; red[u][1] = a1; red[u][2] = d0; red[u][3] = d1; red[u][4] = db; }
+    __syncthreads();
+    if (gr == 0) {
+        float *P = part + (size_t)blockIdx.x * B3_N;
+        P[2 * u] = a0 + red[u][0];
+        P[2 * u + 1] = a1 + red[u][1];
+        P[MLP_H + 2 * u] = d0 + red[u][2];
+        P[MLP_H + 2 * u + 1] = d1 + red[u][3];
+        if (u == 0) P[2 * MLP_H] = db + red[u][4];
+    }
 }
 
-// dW2 = D2' H1 (256 x 256, summed over rows) and db2 = sum D2: CTA (tile,
-// chunk) owns a 64 x 64 block of dW2 over one row chunk; partials per chunk
-constexpr int DW_TR = 32;
-__global__ void __launch_bounds__(256) k_mlp_dw2(int m, int chunk, const bf16 *D2, const bf16 *H1, float *part)
+// dW2 = D2' H1 (256 x 256, summed over rows) on the tensor cores: CTA (tile,
+// chunk) owns a 128 x 128 block over one row chunk, its eight warps 64 x 32
+// each (mma.sync m16n8k16, BF16 products, FP32 accumulation).  Both operands
+// are row-major with the rows as K, so ldmatrix.trans hands the fragments out;
+// stages of 32 rows arrive by cp.async, three in flight.  The accumulators are
+// added into a second set every DW_FLUSH rows, so that no sum passes through
+// more than a few MMAs of the unit's own rounding.  Partials per chunk.  On
+// FP32 FMAs the product had taken 1075 us at 200,000 rows.
+constexpr int DW_TR = 32, DW_LD = 128 + 8, DW_STAGES = 3, DW_FLUSH = 64;
+constexpr int DW_SMEM = DW_STAGES * 2 * DW_TR * DW_LD * 2;
+__global__ void __launch_bounds__(256, 1) k_mlp_dw2(int m, int chunk, const bf16 *D2, const bf16 *H1, float *part)
 {
-    __shared__ float dt[DW_TR][64 + 1], ht[DW_TR][64 + 1];
-    const int tj = blockIdx.x / 4, tl = blockIdx.x % 4;  // 64-row block of j (D2 col), of l (H1 col)
-    const int i0 = blockIdx.y * chunk, i1 = min(m, i0 + chunk);
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    float acc[4][4] = {};
-    float dbs = 0.f;
-    for (int ib = i0; ib < i1; ib += DW_TR) {
-        for (int t = threadIdx.x; t < DW_TR * 64; t += 256) {
-            const int r = t / 64, c = t % 64, i = ib + r;
-            dt[r][c] = i < i1 ? __bfloat162float(D2[(size_t)i * MLP_H + tj * 64 + c]) : 0.f;
-            ht[r][c] = i < i1 ? __bfloat162float(H1[(size_t)i * MLP_H + tl * 64 + c]) : 0.f;
+    extern __shared__ __align__(16) unsigned short dws[];
+    const int tj = (blockIdx.x >> 1) * 128, tl = (blockIdx.x & 1) * 128;
+    const long long i0 = (long long)blockIdx.y * chunk, i1 = min((long long)m, i0 + chunk);
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int wj = (w & 1) * 64, wl = (w >> 1) * 32;
+    const uint32_t base = tc_smem(dws);
+    const int nst = i1 > i0 ? (int)((i1 - i0 + DW_TR - 1) / DW_TR) : 0;
+    // stage s: D2 rows [DW_TR][DW_LD], then H1 rows; rows past i1 are zeros
+    auto issue = [&](int s) {
+        if (s < nst) {
+            const uint32_t st = base + (uint32_t)(s % DW_STAGES) * (2 * DW_TR * DW_LD * 2);
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const int t = tid + 256 * q;  // 2 operands x 32 rows x 16 pieces
+                const int op = t >> 9, r = (t >> 4) & 31, c = t & 15;
+                const long long i = i0 + (long long)s * DW_TR + r;
+                const bf16 *src = (op ? H1 : D2) + (i < i1 ? i : i0) * MLP_H + (op ? tl : tj) + c * 8;
+                const uint32_t dst = st + (uint32_t)(op * DW_TR * DW_LD + r * DW_LD + c * 8) * 2;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(i < i1 ? 16 : 0)
+                             : "memory");
+            }
         }
-        __syncthreads();
-#pragma unroll 4
-        for (int r = 0; r < DW_TR; r++) {
-            float dv[4], hv[4];
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float acc[4][4][4], tot[4][4][4];
 #pragma unroll
-            for (int q = 0; q < 4; q++) { dv[q] = dt[r][ty + 16 * q]; hv[q] = ht[r][tx + 16 * q]; }
+    for (int a = 0; a < 4; a++)
 #pragma unroll
-            for (int p = 0; p < 4; p++)
+        for (int b = 0; b < 4; b++)
 #pragma unroll
-                for (int q = 0; q < 4; q++) acc[p][q] = fmaf(dv[p], hv[q], acc[p][q]);
+            for (int q = 0; q < 4; q++) acc[a][b][q] = tot[a][b][q] = 0.f;
+    auto flush = [&]() {
+#pragma unroll
+        for (int a = 0; a < 4; a++)
+#pragma unroll
+            for (int b = 0; b < 4; b++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    tot[a][b][q] += acc[a][b][q];
+                    acc[a][b][q] = 0.f;
+                }
+    };
+    auto ldm = [](uint32_t (&v)[4], uint32_t at) {
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                     : "r"(at)
+                     : "memory");
+    };
+    const int mt = lane >> 3, mr = lane & 7;
+    for (int s = 0; s < DW_STAGES - 1; s++) issue(s);
+    for (int s = 0; s < nst; s++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(DW_STAGES - 2) : "memory");
+        __syncthreads();  // stage s has arrived, stage s - 1 has been read by all
+        issue(s + DW_STAGES - 1);
+        const uint32_t st = base + (uint32_t)(s % DW_STAGES) * (2 * DW_TR * DW_LD * 2), sh = st + DW_TR * DW_LD * 2;
+#pragma unroll
+        for (int k0 = 0; k0 < DW_TR; k0 += 16) {
+            uint32_t bf[2][4];
+#pragma unroll
+            for (int b = 0; b < 2; b++)
+                ldm(bf[b], sh + (uint32_t)((k0 + (mt & 1) * 8 + mr) * DW_LD + wl + 16 * b + (mt >> 1) * 8) * 2);
+#pragma unroll
+            for (int a = 0; a < 4; a++) {
+                uint32_t af[4];
+                ldm(af, st + (uint32_t)((k0 + (mt >> 1) * 8 + mr) * DW_LD + wj + 16 * a + (mt & 1) * 8) * 2);
+#pragma unroll
+                for (int b = 0; b < 4; b++) mma16816(acc[a][b], af, bf[b >> 1][2 * (b & 1)], bf[b >> 1][2 * (b & 1) + 1]);
+            }
         }
-        if (tl == 0 && threadIdx.x < 64)
-            for (int r = 0; r < DW_TR; r++) dbs += dt[r][threadIdx.x];
-        __syncthreads();
+        if ((s + 1) % (DW_FLUSH / DW_TR) == 0) flush();
     }
-    float *P = part + (size_t)blockIdx.y * (MLP_H * MLP_H + MLP_H);
+    flush();
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    float *P = part + (size_t)blockIdx.y * (MLP_H * MLP_H);
+    const int gid = lane >> 2, tig = lane & 3;
 #pragma unroll
-    for (int p = 0; p < 4; p++)
+    for (int a = 0; a < 4; a++)
 #pragma unroll
-        for (int q = 0; q < 4; q++) P[(size_t)(tj * 64 + ty + 16 * p) * MLP_H + tl * 64 + tx + 16 * q] = acc[p][q];
-    if (tl == 0 && threadIdx.x < 64) P[MLP_H * MLP_H + tj * 64 + threadIdx.x] = dbs;
+        for (int b = 0; b < 4; b++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int j = tj + wj + 16 * a + gid + 8 * h, l = tl + wl + 8 * b + 2 * tig;
+                *reinterpret_cast<float2 *>(P + (size_t)j * MLP_H + l) =
+                    make_float2(tot[a][b][2 * h], tot[a][b][2 * h + 1]);
+            }
 }
 
-// dW1 = D1' F (256 x 18) and db1 = sum D1: partials per CTA, thread = unit
+// dW1 = D1' F (256 x 18) and db1 = sum D1: thread = unit, tiles of 32 rows of
+// features in shared memory, eight rows of D1 in flight; partials per CTA
 __global__ void __launch_bounds__(MLP_H) k_mlp_dw1(int m, const float *D1, const float *F, float *part)
 {
+    __shared__ __align__(16) float f[L1_TR * L1_FS];
     const int j = threadIdx.x;
     float acc[MLP_IN + 1] = {};
-    for (int i = blockIdx.x; i < m; i += gridDim.x) {
-        const float d = D1[(size_t)i * MLP_H + j];
-        const float *f = F + (size_t)i * MLP_IN;
+    for (long long i0 = (long long)blockIdx.x * L1_TR; i0 < m; i0 += (long long)gridDim.x * L1_TR) {
+        const int nr = (int)min((long long)L1_TR, m - i0);
+        for (int t = threadIdx.x; t < L1_TR * L1_FS; t += MLP_H) {
+            const int r = t / L1_FS, q = t % L1_FS;
+            f[t] = r < nr && q < MLP_IN ? F[(i0 + r) * MLP_IN + q] : 0.f;
+        }
+        __syncthreads();
+        for (int r0 = 0; r0 < nr; r0 += 8) {
+            float d[8];
 #pragma unroll
-        for (int q = 0; q < MLP_IN; q++) acc[q] = fmaf(d, f[q], acc[q]);
-        acc[MLP_IN] += d;
+            for (int q = 0; q < 8; q++) d[q] = r0 + q < nr ? D1[(i0 + r0 + q) * MLP_H + j] : 0.f;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                float fv[L1_FS];
+#pragma unroll
+                for (int c = 0; c < L1_FS / 4; c++) {
+                    const float4 v = *reinterpret_cast<const float4 *>(f + (r0 + q) * L1_FS + 4 * c);
+                    fv[4 * c] = v.x; fv[4 * c + 1] = v.y; fv[4 * c + 2] = v.z; fv[4 * c + 3] = v.w;
+                }
+#pragma unroll
+                for (int c = 0; c < MLP_IN; c++) acc[c] = fmaf(d[q], fv[c], acc[c]);
+                acc[MLP_IN] += d[q];
+            }
+        }
+        __syncthreads();
     }
     float *P = part + (size_t)blockIdx.x * (MLP_H * (MLP_IN + 1));
 #pragma unroll
     for (int q = 0; q <= MLP_IN; q++) P[(size_t)q * MLP_H + j] = acc[q];
 }
 
-// fixed-order sums of the partials into the flat gradient
-__global__ void k_mlp_sum_b3(int nb, const float *part, float *g)
+// fixed-order sums of nb rows of n partials into the flat gradient: a CTA per
+// 32 columns, eight row groups.  KIND 0: dw3, db2, db3; 1: dW2; 2: dW1, db1.
+template <int KIND>
+__global__ void __launch_bounds__(256) k_mlp_sum(int nb, int n, const float *part, float *g)
 {
-    const int j = threadIdx.x;  // 0..256
-    if (j > MLP_H) return;
+    __shared__ float red[8][33];
+    const int c = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int t = blockIdx.x * 32 + c;
     float s = 0.f;
-    for (int b = 0; b < nb; b++) s += part[(size_t)b * (MLP_H + 1) + j];
-    if (j < MLP_H) g[OW3 + j] = s;
-    else g[OB3] = s;
-}
-__global__ void k_mlp_sum_dw2(int nchunk, const float *part, float *g)
-{
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= MLP_H * MLP_H + MLP_H) return;
-    float s = 0.f;
-    for (int b = 0; b < nchunk; b++) s += part[(size_t)b * (MLP_H * MLP_H + MLP_H) + t];
-    if (t < MLP_H * MLP_H) g[OW2 + t] = s;
-    else g[OB2 + (t - MLP_H * MLP_H)] = s;
-}
-__global__ void k_mlp_sum_dw1(int nb, const float *part, float *g)
-{
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;  // q * 256 + j
-    if (t >= MLP_H * (MLP_IN + 1)) return;
-    float s = 0.f;
-    for (int b = 0; b < nb; b++) s += part[(size_t)b * (MLP_H * (MLP_IN + 1)) + t];
-    const int q = t / MLP_H, j = t % MLP_H;
-    if (q < MLP_IN) g[OW1 + j * MLP_IN + q] = s;
-    else g[OB1 + j] = s;
+    if (t < n)
+#pragma unroll 4
+        for (int b = w; b < nb; b += 8) s += part[(size_t)b * n + t];
+    red[w][c] = s;
+    __syncthreads();
+    if (w != 0 || t >= n) return;
+    for (int q = 1; q < 8; q++) s += red[q][c];
+    if (KIND == 0) g[t < MLP_H ? OW3 + t : t < 2 * MLP_H ? OB2 + t - MLP_H : OB3] = s;
+    else if (KIND == 1) g[OW2 + t] = s;
+    else {
+        const int q = t / MLP_H, j = t % MLP_H;
+        g[q < MLP_IN ? OW1 + j * MLP_IN + q : OB1 + j] = s;
+    }
 }
 
 // Adam (Kingma & Ba 2015) on the FP32 master copy
@@ -653,9 +853,10 @@ static void mlp_reserve(Mlp &M, int m, int k)
     }
 }
 
-constexpr int MLP_GRID = 1024;         // CTAs of the row-parallel reductions
+constexpr int MLP_GRID = 608;          // CTAs of the row-parallel reductions at most
+constexpr int MLP_SEGS = 64;           // row segments of the projections
 constexpr int MLP_RED_GRID = 4096;     // partials that the reduction scratch holds at least
-constexpr int MLP_DW2_CHUNKS = 64;     // row chunks of dW2
+constexpr int MLP_DW2_CHUNKS = 38;     // row chunks of dW2 at most (four blocks each: one CTA per SM)
 
 static void mlp_cast(Mlp &M)
 {
@@ -734,56 +935,57 @@ static void mlp_check(Mlp &M)
 
 static void mlp_forward(Mlp &M, int m)
 {
-    k_mlp_l1<<<std::min(8192, m), MLP_H, 0, M.s>>>(m, M.F, M.W1b, M.p + OB1, M.H1);
+    const int g = std::max(1, std::min(4 * device_info().sms, (m + L1_TR - 1) / L1_TR));
+    k_mlp_l1<<<g, 256, 0, M.s>>>(m, M.F, M.W1b, M.p + OB1, M.H1);
     PGB_LAUNCHED();
     mlp_mm<0>(M, m, M.H1, M.W2b, M.p + OB2, nullptr, M.H2, nullptr);
     k_mlp_l3<<<std::min(4096, (m + 7) / 8), 256, 0, M.s>>>(m, M.H2, M.w3b, M.p + OB3, M.out);
     PGB_LAUNCHED();
 }
 
-// loss and flat gradient for the matrix whose features sit in M.F and whose
-// leading left singular vectors (m x k, column-major) sit in M.U
-static double mlp_backward(Mlp &M, int m, int k)
+// flat gradient (M.g) and loss (device, M.coef[4095]) for the matrix whose
+// features sit in M.F and whose leading left singular vectors (m x k,
+// column-major) sit in M.U
+static void mlp_backward(Mlp &M, int m, int k)
 {
-    k_mlp_proj<<<MLP_GRID, 256, 0, M.s>>>(m, k, M.U, M.out, M.red);
+    const int sms = device_info().sms;
+    k_mlp_proj<<<std::min(8 * sms, ((k + 1) * MLP_SEGS + 7) / 8), 256, 0, M.s>>>(m, k, MLP_SEGS, M.U, M.out, M.red);
     PGB_LAUNCHED();
-    std::vector<double> part((size_t)MLP_GRID * (k + 1));
-    PGB_CUDA(cudaMemcpyAsync(part.data(), M.red, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, M.s));
-    PGB_CUDA(cudaStreamSynchronize(M.s));
-    std::vector<double> c(k + 1, 0.0);
-    for (int b = 0; b < MLP_GRID; b++)
-        for (int j = 0; j <= k; j++) c[j] += part[(size_t)b * (k + 1) + j];
-    const double nrm2 = std::max(c[k], 1e-300);
-    const double eps = MLP_EPS * nrm2 / k;
-    double loss = std::log(nrm2);
-    std::vector<double> coef(k + 1);
-    for (int j = 0; j < k; j++) {
-        loss -= std::log(c[j] * c[j] + eps) / k;
-        coef[j] = -2.0 * c[j] / ((c[j] * c[j] + eps) * k);
-    }
-    // d/du0 of log ||u0||^2 plus the eps ||u0||^2 terms
-    double s = 0.0;
-    for (int j = 0; j < k; j++) s += (MLP_EPS / k) / (c[j] * c[j] + eps);
-    coef[k] = 2.0 / nrm2 - 2.0 * s / k;
-    PGB_CUDA(cudaMemcpyAsync(M.coef, coef.data(), sizeof(double) * (k + 1), cudaMemcpyHostToDevice, M.s));
+    k_mlp_coef<<<1, 256, 0, M.s>>>(k, MLP_SEGS, M.red, M.coef, M.coef + MLP_LOSS_AT);
+    PGB_LAUNCHED();
     k_mlp_gout<<<std::min(4096, (m + 255) / 256), 256, 0, M.s>>>(m, k, M.U, M.coef, M.out, M.gout);
     PGB_LAUNCHED();
     float *pf = reinterpret_cast<float *>(M.red);
-    k_mlp_b3<<<MLP_GRID, MLP_H, 0, M.s>>>(m, M.gout, M.H2, M.w3b, M.D2, pf);
+    const int gb = std::max(1, std::min(std::min(MLP_GRID, 4 * sms), (m + 15) / 16));
+    k_mlp_b3<<<gb, 256, 0, M.s>>>(m, M.gout, M.H2, M.w3b, M.D2, pf);
     PGB_LAUNCHED();
-    k_mlp_sum_b3<<<1, 288, 0, M.s>>>(MLP_GRID, pf, M.g);
+    k_mlp_sum<0><<<(B3_N + 31) / 32, 256, 0, M.s>>>(gb, B3_N, pf, M.g);
     PGB_LAUNCHED();
-    const int chunk = (m + MLP_DW2_CHUNKS - 1) / MLP_DW2_CHUNKS;
-    k_mlp_dw2<<<dim3(16, MLP_DW2_CHUNKS), 256, 0, M.s>>>(m, chunk, M.D2, M.H1, M.part);
+    // whole stages per chunk, at least a flush interval
+    const int nch = std::max(1, std::min(MLP_DW2_CHUNKS, (m + DW_FLUSH - 1) / DW_FLUSH));
+    const int chunk = ((m + nch - 1) / nch + DW_TR - 1) / DW_TR * DW_TR;
+    k_mlp_dw2<<<dim3(4, nch), 256, DW_SMEM, M.s>>>(m, chunk, M.D2, M.H1, M.part);
     PGB_LAUNCHED();
-    k_mlp_sum_dw2<<<(MLP_H * MLP_H + MLP_H + 255) / 256, 256, 0, M.s>>>(MLP_DW2_CHUNKS, M.part, M.g);
+    k_mlp_sum<1><<<MLP_H * MLP_H / 32, 256, 0, M.s>>>(nch, MLP_H * MLP_H, M.part, M.g);
     PGB_LAUNCHED();
     mlp_mm<1>(M, m, M.D2, M.W2Tb, nullptr, M.H1, nullptr, M.D1);
-    k_mlp_dw1<<<MLP_GRID, MLP_H, 0, M.s>>>(m, M.D1, M.F, pf);
+    const int g1 = std::max(1, std::min(std::min(MLP_GRID, 4 * sms), (m + L1_TR - 1) / L1_TR));
+    k_mlp_dw1<<<g1, MLP_H, 0, M.s>>>(m, M.D1, M.F, pf);
     PGB_LAUNCHED();
-    k_mlp_sum_dw1<<<(MLP_H * (MLP_IN + 1) + 255) / 256, 256, 0, M.s>>>(MLP_GRID, pf, M.g);
+    k_mlp_sum<2><<<MLP_H * (MLP_IN + 1) / 32, 256, 0, M.s>>>(g1, MLP_H * (MLP_IN + 1), pf, M.g);
     PGB_LAUNCHED();
-    return loss;
+}
+
+// U (host, leading dimension ldu) to M.U on the copy stream, while the
+// features and the forward pass run; M.s waits for it
+static void mlp_upload(Mlp &M, const double *U, int ldu, int m, int k)
+{
+    if (ldu == m) h2d_bytes(M.U, U, sizeof(double) * (size_t)m * k, M.s2);
+    else
+        PGB_CUDA(cudaMemcpy2DAsync(M.U, sizeof(double) * m, U, sizeof(double) * ldu, sizeof(double) * m, k,
+                                   cudaMemcpyHostToDevice, M.s2));
+    PGB_CUDA(cudaEventRecord(M.ev, M.s2));
+    PGB_CUDA(cudaStreamWaitEvent(M.s, M.ev, 0));
 }
 
 static Operator *mlp_operator(int64_t op_handle)
@@ -823,6 +1025,8 @@ extern "C" int propack_mlp_create(uint64_t seed, int64_t *handle)
         Mlp *M = new Mlp();
         PGB_CUDA(cudaGetDevice(&M->device));
         PGB_CUDA(cudaStreamCreateWithFlags(&M->s, cudaStreamNonBlocking));
+        PGB_CUDA(cudaStreamCreateWithFlags(&M->s2, cudaStreamNonBlocking));
+        PGB_CUDA(cudaEventCreateWithFlags(&M->ev, cudaEventDisableTiming));
         // He-style initialisation, drawn on the host (small)
         std::vector<float> p(MLP_NP, 0.f);
         unsigned long long st = seed * 0x9E3779B97F4A7C15ull + 12345ull;
@@ -850,12 +1054,13 @@ extern "C" int propack_mlp_create(uint64_t seed, int64_t *handle)
         PGB_CUDA(cudaMalloc(&M->W2Tb, sizeof(bf16) * MLP_H * MLP_H));
         PGB_CUDA(cudaMalloc(&M->w3b, sizeof(bf16) * MLP_H));
         const size_t red = std::max<size_t>((size_t)MLP_GRID * (MLP_H * (MLP_IN + 1)) * sizeof(float),
-                                            (size_t)MLP_GRID * 4096 * sizeof(double));
+                                            (size_t)MLP_SEGS * 4096 * sizeof(double));
         PGB_CUDA(cudaMalloc(&M->red, red));
         PGB_CUDA(cudaMalloc(&M->coef, sizeof(double) * 4096));
-        PGB_CUDA(cudaMalloc(&M->part, sizeof(float) * (size_t)MLP_DW2_CHUNKS * (MLP_H * MLP_H + MLP_H)));
+        PGB_CUDA(cudaMalloc(&M->part, sizeof(float) * (size_t)MLP_DW2_CHUNKS * (MLP_H * MLP_H)));
         PGB_CUDA(cudaFuncSetAttribute(k_mlp_mm<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mm_smem()));
         PGB_CUDA(cudaFuncSetAttribute(k_mlp_mm<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mm_smem()));
+        PGB_CUDA(cudaFuncSetAttribute(k_mlp_dw2, cudaFuncAttributeMaxDynamicSharedMemorySize, DW_SMEM));
         PGB_CUDA(cudaFuncSetAttribute(k_mlp_mm_tc<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, TM_SMEM));
         PGB_CUDA(cudaFuncSetAttribute(k_mlp_mm_tc<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TM_SMEM));
         PGB_CUDA(cudaMalloc(&M->err, sizeof(int)));
@@ -885,6 +1090,8 @@ extern "C" int propack_mlp_destroy(int64_t handle)
                     (void *)M->red, (void *)M->coef, (void *)M->part, (void *)M->err})
         if (q) cudaFree(q);
     cudaStreamDestroy(M->s);
+    cudaStreamDestroy(M->s2);
+    cudaEventDestroy(M->ev);
     delete M;
     return 0;
 }
@@ -954,14 +1161,15 @@ extern "C" int propack_mlp_grad(int64_t handle, int64_t op_handle, uint64_t seed
         if (!U || ldu < m || k < 1 || k > 4000) { set_error("propack_mlp_grad: invalid U"); throw ArgFailure(); }
         mlp_features(*M, *op, seed);
         mlp_reserve(*M, m, k);
-        PGB_CUDA(cudaMemcpy2DAsync(M->U, sizeof(double) * m, U, sizeof(double) * ldu, sizeof(double) * m, k,
-                                   cudaMemcpyHostToDevice, M->s));
         mlp_forward(*M, m);
-        const double L = mlp_backward(*M, m, k);
-        if (loss) *loss = L;
+        mlp_upload(*M, U, ldu, m, k);
+        mlp_backward(*M, m, k);
+        double L = 0.0;
+        PGB_CUDA(cudaMemcpyAsync(&L, M->coef + MLP_LOSS_AT, sizeof(double), cudaMemcpyDeviceToHost, M->s));
         if (grad) PGB_CUDA(cudaMemcpyAsync(grad, M->g, sizeof(float) * MLP_NP, cudaMemcpyDeviceToHost, M->s));
         PGB_CUDA(cudaStreamSynchronize(M->s));
         mlp_check(*M);
+        if (loss) *loss = L;
     })
 }
 
@@ -977,11 +1185,11 @@ extern "C" int propack_mlp_train_step(int64_t handle, int64_t op_handle, uint64_
         if (!U || ldu < m || k < 1 || k > 4000) { set_error("propack_mlp_train_step: invalid U"); throw ArgFailure(); }
         mlp_features(*M, *op, seed);
         mlp_reserve(*M, m, k);
-        PGB_CUDA(cudaMemcpy2DAsync(M->U, sizeof(double) * m, U, sizeof(double) * ldu, sizeof(double) * m, k,
-                                   cudaMemcpyHostToDevice, M->s));
         mlp_forward(*M, m);
-        const double L = mlp_backward(*M, m, k);
-        if (loss) *loss = L;
+        mlp_upload(*M, U, ldu, m, k);
+        mlp_backward(*M, m, k);
+        double L = 0.0;
+        PGB_CUDA(cudaMemcpyAsync(&L, M->coef + MLP_LOSS_AT, sizeof(double), cudaMemcpyDeviceToHost, M->s));
         M->step++;
         const float c1 = 1.f - std::pow(0.9f, (float)M->step), c2 = 1.f - std::pow(0.999f, (float)M->step);
         k_mlp_adam<<<(MLP_NP + 255) / 256, 256, 0, M->s>>>(M->p, M->g, M->m1, M->m2, (float)lr, c1, c2);
@@ -989,5 +1197,6 @@ extern "C" int propack_mlp_train_step(int64_t handle, int64_t op_handle, uint64_
         mlp_cast(*M);
         PGB_CUDA(cudaStreamSynchronize(M->s));
         mlp_check(*M);
+        if (loss) *loss = L;
     })
 }
