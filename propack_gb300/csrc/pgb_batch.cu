@@ -92,6 +92,7 @@ struct BShared {
     double red[32];
     double h[BDIM_MAX + 2];
     double d[BDIM_MAX + 2], e[BDIM_MAX + 2], sig[BDIM_MAX + 2], bnd[BDIM_MAX + 2];
+    float b2f[2 * BDIM_MAX + 2];
     double b[2 * BDIM_MAX + 2], b2[2 * BDIM_MAX + 2];  // off-diagonals of the Golub-Kahan form of R, their squares
     double cs[BDIM_MAX + 2], sn[BDIM_MAX + 2];
     double shifts[BDIM_MAX + 2];
@@ -558,7 +559,7 @@ __device__ int b_analyse(BProb &P, const BCfg &c, BShared &S, double *scr, const
     if (threadIdx.x < 32) {
         warp_bdqr(dim, S.d, S.e, dim != mn, S.cs, S.sn, S.b);
         double gersh, pivmin, sc;
-        stage_tgk(N, S.b, S.b2, gersh, pivmin, sc);
+        stage_tgk(N, S.b, S.b2, S.b2f, gersh, pivmin, sc);
         if (lane == 0) {
             S.scal[0] = gersh;
             S.scal[1] = pivmin;
@@ -569,7 +570,7 @@ __device__ int b_analyse(BProb &P, const BCfg &c, BShared &S, double *scr, const
     __syncthreads();
     const double gersh = S.scal[0], pivmin = S.scal[1], sc = S.scal[2], c1 = S.sn[dim - 1];
     for (int i = threadIdx.x >> 5; i < dim; i += BW) {
-        const double sig = warp_sigma(dim, S.b2, i + 1, gersh, pivmin, sc);
+        const double sig = warp_sigma(dim, S.b2, S.b2f, i + 1, gersh, pivmin, sc);
         double *fn = scr + L.tw + (size_t)i * 4 * N;
         const double zn = warp_twisted(N, S.b, S.b2, sc != 0.0 ? sig * sc : sig, sc != 0.0 ? SFMIN : pivmin,
                                        sc != 0.0, fn, fn + N, fn + 2 * N, fn + 3 * N);

@@ -47,24 +47,23 @@ __device__ __forceinline__ int tgk_negcount(int N, const double *b2, double lam,
 // The same count without a division in the chain: p_j = -lam p_{j-1} -
 // b2_{j-1} p_{j-2} are the leading principal minors (Wilkinson's Sturm
 // sequence; the pivots above are p_j / p_{j-1}, so a negative pivot is a sign
-// change).  One dependent FMA per step, where the pivot recurrence waits for
-// an FP64 division (~1000 cycles a step on this GPU).  The roundings of a
-// step move the b2 it uses by a few eps relative, as those of the pivot
-// recurrence do (divide by p_{j-1}), so the count is as accurate.
+// change).  Two FP64 instructions per step (128 cycles: one warp gets one per
+// 64 on this GPU), where the pivot recurrence waited for a division (~1000).
+// The roundings of a step move the b2 it uses by a few eps relative, as those
+// of the pivot recurrence do (divide by p_{j-1}), so the count is as accurate.
 // The caller scales the matrix (tgk_scale) so that |b| <= 1 and lam <= 1:
 // |p| then grows by less than 2^12 in TGK_RESCALE steps, and shrinks by no
 // more than lam^TGK_RESCALE >= 2^-640, and is brought back to exponent 0
-// after them.  A p of exactly 0 takes the sign the pivot guard would give it.
-// lam < TGK_POLY_MIN (values below 1e-12 sigma_1) keeps the pivots.
+// after them.  A p of exactly 0 takes the sign opposite to its predecessor's
+// (the pivot guard's); two in a row (an exact eigenvalue of a decoupled
+// leading block) leave no sign to count, and the caller falls back on the
+// pivots.  lam < TGK_POLY_MIN (values below 1e-12 sigma_1) keeps the pivots.
 constexpr int TGK_RESCALE = 16;
 constexpr double TGK_POLY_MIN = 9.094947017729282e-13;  // 2^-40
 
-__device__ __forceinline__ double tgk_step(double p1, double p0, double b2, double lam)
+__device__ __forceinline__ bool tgk_is_zero(double p)
 {
-    double p2 = fma(-lam, p1, -(b2 * p0));
-    if (((unsigned)__double2hiint(p2) << 1 | (unsigned)__double2loint(p2)) == 0u)
-        p2 = p1 * -7.888609052210118e-31;  // 2^-100: far below eps lam of the scaled matrix
-    return p2;
+    return ((unsigned)__double2hiint(p) << 1 | (unsigned)__double2loint(p)) == 0u;
 }
 __device__ __forceinline__ void tgk_rescale(double &p1, double &p0)
 {
@@ -74,25 +73,49 @@ __device__ __forceinline__ void tgk_rescale(double &p1, double &p0)
     p1 *= f;
     p0 *= f;
 }
+// the count, or -1 when two successive minors vanish
 __device__ __forceinline__ int tgk_negcount_sturm(int N, const double *b2, double lam)
 {
     double p0 = 1.0, p1 = -lam;
     int cnt = 1, j = 1;
+    int sg = -1;  // sign word of p1
+    auto step = [&](double b) {
+        const double p2 = fma(-lam, p1, -(b * p0));
+        const int s2 = tgk_is_zero(p2) ? ~sg : __double2hiint(p2);
+        cnt += (int)((unsigned)(s2 ^ sg) >> 31);
+        sg = s2;
+        p0 = p1;
+        p1 = p2;
+    };
     for (; j + TGK_RESCALE <= N; j += TGK_RESCALE) {
 #pragma unroll
-        for (int q = 0; q < TGK_RESCALE; q++) {
-            const double p2 = tgk_step(p1, p0, b2[j + q - 1], lam);
-            cnt += (int)((unsigned)(__double2hiint(p2) ^ __double2hiint(p1)) >> 31);
+        for (int q = 0; q < TGK_RESCALE; q++) step(b2[j + q - 1]);
+        tgk_rescale(p1, p0);
+    }
+    for (; j < N; j++) step(b2[j - 1]);
+    return tgk_is_zero(p1) && tgk_is_zero(p0) ? -1 : cnt;
+}
+// the count in FP32 (b2 rounded to FP32, lam >= TGK_F32_MIN): exact for a
+// matrix whose entries moved by a few 2^-24 relative, so the values it locates
+// are right to about 4 N 2^-24; at a tenth of the FP64 count's time
+constexpr float TGK_F32_MIN = 0.000244140625f;  // 2^-12: lam^8 stays far from underflow
+__device__ __forceinline__ int tgk_negcount_f32(int N, const float *b2, float lam)
+{
+    float p0 = 1.f, p1 = -lam;
+    int cnt = 1, j = 1;
+    while (j < N) {
+        const int je = min(N, j + 8);
+        for (; j < je; j++) {
+            float p2 = fmaf(-lam, p1, -(b2[j - 1] * p0));
+            if (p2 == 0.f) p2 = p1 * -1.f;  // any value of the guard's sign
+            cnt += (int)((unsigned)(__float_as_int(p2) ^ __float_as_int(p1)) >> 31);
             p0 = p1;
             p1 = p2;
         }
-        tgk_rescale(p1, p0);
-    }
-    for (; j < N; j++) {
-        const double p2 = tgk_step(p1, p0, b2[j - 1], lam);
-        cnt += (int)((unsigned)(__double2hiint(p2) ^ __double2hiint(p1)) >> 31);
-        p0 = p1;
-        p1 = p2;
+        const int k = 127 - max((__float_as_int(p1) >> 23) & 0xff, (__float_as_int(p0) >> 23) & 0xff);
+        const float f = __int_as_float((min(max(k, -120), 120) + 127) << 23);
+        p1 *= f;
+        p0 *= f;
     }
     return cnt;
 }
@@ -107,24 +130,56 @@ __device__ __forceinline__ double tgk_scale(double gersh)
 }
 
 // sigma_t (t = 1: largest) of R by warp multisection; all lanes return it.
-// b2: the squares of the off-diagonals times sc^2 (sc = 0: unscaled), hi0 an
-// upper bound of sigma_max (Gershgorin of TGK) of the unscaled matrix.
-__device__ inline double warp_sigma(int n, const double *b2, int t, double hi0, double pivmin, double sc)
+// b2: the squares of the off-diagonals times sc^2 (sc = 0: unscaled), b2f the
+// same in FP32 (scaled only), hi0 an upper bound of sigma_max (Gershgorin of
+// TGK) of the unscaled matrix.  Three rounds of FP32 counts find a bracket of
+// ~2^-13, which one round of FP64 counts at its widened ends confirms (or the
+// search starts from [0, hi0]); FP64 rounds finish, 5 bits each.
+__device__ inline double warp_sigma(int n, const double *b2, const float *b2f, int t, double hi0, double pivmin,
+                                    double sc)
 {
+    const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, N = 2 * n;
-    const double frac = (double)(lane + 1) / 33.0;
     const double guard = sc != 0.0 ? SFMIN : pivmin;
+    // #(sigma > p) = 2n - negcount(p) for p > 0
+    auto above = [&](double p) {
+        int c = -1;
+        if (sc != 0.0 && __all_sync(FULL, p >= TGK_POLY_MIN)) c = tgk_negcount_sturm(N, b2, p);
+        if (__any_sync(FULL, c < 0)) c = tgk_negcount(N, b2, p, guard);
+        return N - c;
+    };
     double lo = 0.0, hi = sc != 0.0 ? hi0 * sc : hi0;
+    if (sc != 0.0) {
+        float fl = 0.f, fh = (float)hi;
+        for (int round = 0; round < 3; round++) {
+            const float p = fl + (fh - fl) * ((float)(lane + 1) / 33.f);
+            if (!__all_sync(FULL, p >= TGK_F32_MIN)) break;
+            const unsigned bal = __ballot_sync(FULL, N - tgk_negcount_f32(N, b2f, p) >= t);
+            const int q = __popc(bal);
+            const float plo = __shfl_sync(FULL, p, q > 0 ? q - 1 : 0), phi = __shfl_sync(FULL, p, q < 32 ? q : 31);
+            if (q > 0) fl = plo;
+            if (q < 32) fh = phi;
+        }
+        if (fl > 0.f) {
+            const double w = 4.0 * N * 5.9604644775390625e-08;
+            const double a = (double)fl * (1.0 - w), z = fmin((double)fh * (1.0 + w), hi);
+            const double p = a + (z - a) * ((double)lane / 31.0);
+            const unsigned bal = __ballot_sync(FULL, above(p) >= t);
+            const int q = __popc(bal);
+            if (q > 0 && q < 32) {
+                lo = __shfl_sync(FULL, p, q - 1);
+                hi = __shfl_sync(FULL, p, q);
+            }
+        }
+    }
+    const double frac = (double)(lane + 1) / 33.0;
     for (int round = 0; round < 64; round++) {
         if (hi - lo <= 2.0 * EPS * hi) break;
         const double p = lo + (hi - lo) * frac;
-        // #(sigma > p) = 2n - negcount(p) for p > 0
-        const bool sturm = sc != 0.0 && __all_sync(0xffffffffu, p >= TGK_POLY_MIN);
-        const int above = N - (sturm ? tgk_negcount_sturm(N, b2, p) : tgk_negcount(N, b2, p, guard));
-        const unsigned bal = __ballot_sync(0xffffffffu, above >= t);
+        const unsigned bal = __ballot_sync(FULL, above(p) >= t);
         const int q = __popc(bal);  // counts are monotone: lanes 0..q-1 satisfy
-        const double plo = __shfl_sync(0xffffffffu, p, q > 0 ? q - 1 : 0);
-        const double phi = __shfl_sync(0xffffffffu, p, q < 32 ? q : 31);
+        const double plo = __shfl_sync(FULL, p, q > 0 ? q - 1 : 0);
+        const double phi = __shfl_sync(FULL, p, q < 32 ? q : 31);
         const double nlo = q > 0 ? plo : lo, nhi = q < 32 ? phi : hi;
         if (nlo == lo && nhi == hi) break;  // no representable progress
         lo = nlo;
@@ -167,7 +222,8 @@ __device__ inline double warp_twisted(int N, const double *b, const double *b2, 
             for (int j = 1; j < N; j++) {
                 const int at = i0 + st * j;
                 // forward: b2[j-1]; backward: b2[N-1-j]
-                const double p2 = tgk_step(p1, p0, b2[lane ? at : at - 1], lam);
+                double p2 = fma(-lam, p1, -(b2[lane ? at : at - 1] * p0));
+                if (tgk_is_zero(p2)) p2 = p1 * -7.888609052210118e-31;  // 2^-100: far below eps lam
                 num[at] = p2;
                 den[at] = p1;
                 p0 = p1;
@@ -346,9 +402,9 @@ __device__ inline void warp_tgk_bounds(int N, const double *b, double &gersh, do
     pivmin = SFMIN * fmax(1.0, warp_max(m2));
 }
 
-// The off-diagonals of TGK and their squares, scaled by the power of two of
-// the Gershgorin bound; one warp.
-__device__ inline void stage_tgk(int N, double *b, double *b2, double &gersh, double &pivmin, double &sc)
+// The off-diagonals of TGK and their squares (b2f: in FP32), scaled by the
+// power of two of the Gershgorin bound; one warp.
+__device__ inline void stage_tgk(int N, double *b, double *b2, float *b2f, double &gersh, double &pivmin, double &sc)
 {
     warp_tgk_bounds(N, b, gersh, pivmin);
     sc = tgk_scale(gersh);
@@ -358,6 +414,7 @@ __device__ inline void stage_tgk(int N, double *b, double *b2, double &gersh, do
         const double v = b[j] * f;
         b[j] = v;
         b2[j] = v * v;
+        if (b2f) b2f[j] = (float)(v * v);
     }
     __syncwarp();
 }

@@ -485,9 +485,9 @@ constexpr int PAR_DIM_MAX = 2048;
 constexpr double EPS34 = 1.0815775704056441e-12;  // EPS^(3/4)
 
 // doubles of shared memory: al/be (reused by the factorization), b, b2 and
-// three more arrays of the Golub-Kahan size N = 2 dim; the Ritz kernel keeps
-// the rotations beside them
-static size_t ana_smem(int dim) { return sizeof(double) * 12 * (size_t)dim; }
+// three more arrays of the Golub-Kahan size N = 2 dim, b2 in FP32 (values) or
+// the rotations (vectors)
+static size_t ana_smem(int dim) { return sizeof(double) * 13 * (size_t)dim; }
 static size_t ritz_smem(int dim) { return sizeof(double) * 14 * (size_t)dim; }
 
 // The bookkeeping of k_analyse (anorm, drefinebounds, convergence count) on
@@ -581,13 +581,14 @@ __device__ void ana_finish_warp(const AnaArgs &a, double *sm)
 // R for itself: ~10 us against a launch and a round trip through L2), the
 // value by multisection, and the Ritz bound from the last component of its
 // left vector by the twisted factorization; the last CTA to finish does the
-// bookkeeping.  Bound by the chain of 2 dim dependent FP64 FMAs of each
-// Sturm sequence, ~11 rounds of them.
+// bookkeeping.  Bound by the FP64 instructions of the Sturm sequences: 4 dim
+// per round at 64 cycles each, ~8 rounds.
 __global__ void __launch_bounds__(32) k_ana_values(AnaArgs a, int finish)
 {
     extern __shared__ double sm[];
     const int dim = a.dim, N = 2 * dim, lane = threadIdx.x;
     double *al = sm, *be = al + dim, *b = sm + N, *b2 = b + N, *fd = b2 + N, *bn = fd + N, *bd = bn + N;
+    float *b2f = reinterpret_cast<float *>(bd + N);
     for (int i = lane; i < dim; i += 32) {
         al[i] = a.balpha[i];
         be[i] = a.bbeta[i];
@@ -596,9 +597,9 @@ __global__ void __launch_bounds__(32) k_ana_values(AnaArgs a, int finish)
     warp_bdqr(dim, al, be, dim != (a.m < a.n ? a.m : a.n), fd, bn, b);
     const double c1 = bn[dim - 1];
     double gersh, pivmin, sc;
-    stage_tgk(N, b, b2, gersh, pivmin, sc);
+    stage_tgk(N, b, b2, b2f, gersh, pivmin, sc);
     const int t = blockIdx.x;
-    const double sig = warp_sigma(dim, b2, t + 1, gersh, pivmin, sc);
+    const double sig = warp_sigma(dim, b2, b2f, t + 1, gersh, pivmin, sc);
     double zn = 0.0;
     if (finish)
         zn = warp_twisted(N, b, b2, sc != 0.0 ? sig * sc : sig, sc != 0.0 ? SFMIN : pivmin, sc != 0.0, al, fd, bn, bd);
@@ -753,7 +754,7 @@ __global__ void __launch_bounds__(32) k_ritz_pairs(RitzArgs a)
     __syncwarp();
     warp_bdqr(dim, al, be, dim != (a.m < a.n ? a.m : a.n), c, s, b);
     double gersh, pivmin, sc;
-    stage_tgk(N, b, b2, gersh, pivmin, sc);
+    stage_tgk(N, b, b2, nullptr, gersh, pivmin, sc);
     warp_twisted(N, b, b2, sc != 0.0 ? si * sc : si, sc != 0.0 ? SFMIN : pivmin, sc != 0.0, al, fd, bn, bd);
     double nx = 0.0, ny = 0.0;
     for (int t = lane; t < dim; t += 32) {
