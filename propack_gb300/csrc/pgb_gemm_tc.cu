@@ -913,7 +913,10 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_oz_umma_ws(int mr, int nc, in
                 const int orow = row0 + L + lane;
 #pragma unroll
                 for (int ph = 0; ph < 2; ph++) {
-                    const int cb = hc * 16 + ph * 8;
+                    // eight columns per warp group and round, so that the
+                    // groups share a tile with few columns evenly
+                    const int cb = ph * 32 + hc * 8;
+                    if (col0 + cb >= nc) break;
                     uint32_t v[OZ_S][8];
 #pragma unroll
                     for (int gg = 0; gg < OZ_S; gg++)
