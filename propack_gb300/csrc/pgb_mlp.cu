@@ -115,23 +115,25 @@ __device__ __forceinline__ double sketch_sum(const int *__restrict__ idx, const 
     return acc;
 }
 
-// Z = diag(w) R' Omega (r x MLP_SK): a warp per segment of THIN_SEG entries of
-// a row of Th = R' (its halves take alternate entries); the warp that
-// completes a row adds its partials in order.  zpart: rows * 4 segs * MLP_SK,
-// tick: rows zeroed counters, left zeroed.
-__global__ void __launch_bounds__(256) k_mlp_thin(Csr Th, const double *om, const double *w, double *zpart,
-                                                  double *Z, unsigned int *tick)
+// Z = diag(w) R' Omega (r x MLP_SK): a warp per segment of `seg` entries of a
+// row of Th = R' (its halves take alternate entries); the warp that
+// completes a row adds its partials in order.  zpart: rows * nseg * MLP_SK,
+// tick: rows zeroed counters, left zeroed.  seg is as short as it takes to
+// give every resident warp a segment (64 at least, 512 at most): a segment's
+// entries are a chain of gathers.
+__global__ void __launch_bounds__(256) k_mlp_thin(Csr Th, const double *om, const double *w, int seg, int nseg,
+                                                  double *zpart, double *Z, unsigned int *tick)
 {
     const unsigned F = 0xffffffffu;
     const int lane = threadIdx.x & 31, h = lane >> 4, c = lane & 15;
-    const int nseg = 4 * Th.segs, nw = gridDim.x * 8;
+    const int nw = gridDim.x * 8;
     for (int t = blockIdx.x * 8 + (threadIdx.x >> 5); t < Th.rows * nseg; t += nw) {
         const int row = t / nseg, sg = t % nseg;
         const int p0 = Th.ptr[row], p1 = Th.ptr[row + 1];
-        const int used = max(1, (p1 - p0 + THIN_SEG - 1) / THIN_SEG);
+        const int used = max(1, (p1 - p0 + seg - 1) / seg);
         if (sg >= used) continue;
-        const int e0 = p0 + sg * THIN_SEG;
-        double acc = sketch_sum(Th.idx, Th.val, e0 + h, min(p1, e0 + THIN_SEG), 2, INT_MAX, om, nullptr, c);
+        const int e0 = p0 + sg * seg;
+        double acc = sketch_sum(Th.idx, Th.val, e0 + h, min(p1, e0 + seg), 2, INT_MAX, om, nullptr, c);
         acc += __shfl_xor_sync(F, acc, 16);
         if (h == 0) zpart[(size_t)t * MLP_SK + c] = acc;
         __threadfence();
@@ -140,8 +142,14 @@ __global__ void __launch_bounds__(256) k_mlp_thin(Csr Th, const double *om, cons
         if (lane == 0) old = atomicAdd(tick + row, 1u);
         if (__shfl_sync(F, old, 0) + 1 == (unsigned)used) {
             __threadfence();
-            double s = 0.0;
-            for (int q = h; q < used; q += 2) s += __ldcg(zpart + ((size_t)row * nseg + q) * MLP_SK + c);
+            double s0 = 0.0, s1 = 0.0;
+            int q = h;
+            for (; q + 2 < used; q += 4) {
+                s0 += __ldcg(zpart + ((size_t)row * nseg + q) * MLP_SK + c);
+                s1 += __ldcg(zpart + ((size_t)row * nseg + q + 2) * MLP_SK + c);
+            }
+            if (q < used) s0 += __ldcg(zpart + ((size_t)row * nseg + q) * MLP_SK + c);
+            double s = s0 + s1;
             s += __shfl_xor_sync(F, s, 16);
             if (h == 0) Z[(size_t)row * MLP_SK + c] = w[row] * s;
             if (lane == 0) tick[row] = 0u;
@@ -883,12 +891,16 @@ static void mlp_features(Mlp &M, const Operator &op, unsigned long long seed)
     double *Z = nullptr, *zpart = nullptr;
     unsigned *tick = nullptr;
     if (op.r > 0) {
-        const int nt = op.thin_r.rows * 4 * op.thin_r.segs;
+        const int64_t mx = (int64_t)op.thin_r.segs * NNZ_PB;  // bounds the longest row
+        int64_t seg = (mx * op.thin_r.rows / (8 * (int64_t)full) + 31) / 32 * 32;
+        seg = std::max<int64_t>(64, std::min<int64_t>(THIN_SEG, seg));
+        const int nseg = (int)((mx + seg - 1) / seg), nt = op.thin_r.rows * nseg;
         Z = (double *)pool_alloc(sizeof(double) * MLP_SK * (size_t)op.r, M.s);
         zpart = (double *)pool_alloc(sizeof(double) * MLP_SK * (size_t)nt, M.s);
         tick = (unsigned *)pool_alloc(sizeof(unsigned) * (size_t)op.r, M.s);
         PGB_CUDA(cudaMemsetAsync(tick, 0, sizeof(unsigned) * (size_t)op.r, M.s));
-        k_mlp_thin<<<std::max(1, std::min(full, (nt + 7) / 8)), 256, 0, M.s>>>(op.thin_r, M.om, op.w, zpart, Z, tick);
+        k_mlp_thin<<<std::max(1, std::min(full, (nt + 7) / 8)), 256, 0, M.s>>>(op.thin_r, M.om, op.w, (int)seg, nseg,
+                                                                                         zpart, Z, tick);
         PGB_LAUNCHED();
     }
     const int64_t want = std::max<int64_t>((m + 15) / 16, std::min<int64_t>(m, op.fwd.nnz / 4096));
