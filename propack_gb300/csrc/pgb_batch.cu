@@ -8,7 +8,11 @@
 // and the Gram-Schmidt passes read the bases as FP32 (hi, lo) planes, split
 // once per final column (pgb_planes.cuh; propack_batch_set_arith).
 //
-// Execution: one CTA owns one problem at a time.  A persistent grid pulls
+// Execution: a cluster of 1, 2, 4 or 8 CTAs owns one problem at a time, each
+// CTA a contiguous range of its rows and of its columns (batch_cluster picks
+// the size for the batch).  Norms and projections are exchanged through
+// distributed shared memory, every CTA runs the scalar logic and the small
+// bidiagonal algebra on the same numbers.  A persistent grid pulls
 // problems from a work queue ordered by decreasing cost (an atomic ticket)
 // and runs up to BATCH_CYCLES_PER_LAUNCH restart cycles of each active problem:
 //   Lanczos extension k0 -> dim (both SpMVs, ELR, CGS) ... dlanbpro.F
@@ -88,8 +92,13 @@ __host__ __device__ inline BScrLayout bscr_layout(int dim, int maxrows)
     return L;
 }
 
+constexpr int BCS_MAX = 8;  // CTAs per problem at most
 struct BShared {
     double red[32];
+    double xch[2][BDIM_MAX + 2];  // this CTA's partial sums, read by its peers (two buffers in turn)
+    int par;                      // buffer of the next exchange
+    int ncl, rank;                // CTAs of the cluster, this one's place
+    int pidx;
     double h[BDIM_MAX + 2];
     double d[BDIM_MAX + 2], e[BDIM_MAX + 2], sig[BDIM_MAX + 2], bnd[BDIM_MAX + 2];
     float b2f[2 * BDIM_MAX + 2];
@@ -101,86 +110,169 @@ struct BShared {
     int flag, xe;
 };
 
-// ------------------------------------------------------ CTA vector helpers
-__device__ __forceinline__ double cta_sum(double v, BShared &S) { return block_sum<BT>(v, S.red); }
+// ---------------------------------------------------------- the cluster
+__device__ __forceinline__ void cl_init(BShared &S)
+{
+    if (threadIdx.x == 0) {
+        unsigned n, r;
+        asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
+        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+        S.ncl = (int)n;
+        S.rank = (int)r;
+        S.par = 0;
+    }
+    __syncthreads();
+}
+// every thread of the problem's CTAs; global and shared writes before it are
+// seen after it
+__device__ __forceinline__ void csync(const BShared &S)
+{
+    if (S.ncl == 1) {
+        __syncthreads();
+    } else {
+        __threadfence();
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        __threadfence();  // the peers' global writes: nothing older in this SM's L1
+    }
+}
+__device__ __forceinline__ double peer_f64(const double *p, int rank)
+{
+    uint32_t at = (uint32_t)__cvta_generic_to_shared(p), ra;
+    double v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(at), "r"(rank));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(ra) : "memory");
+    return v;
+}
+// the sum over the problem's CTAs of v (the CTA's own value in thread 0), in
+// rank order; all threads get it
+__device__ double cl_sum(double v, BShared &S)
+{
+    const int par = S.par;
+    if (threadIdx.x == 0) S.xch[par][0] = v;
+    csync(S);
+    double t = 0.0;
+    for (int r = 0; r < S.ncl; r++) t += S.ncl == 1 ? S.xch[par][0] : peer_f64(&S.xch[par][0], r);
+    __syncthreads();
+    if (threadIdx.x == 0) S.par = par ^ 1;
+    __syncthreads();
+    return t;
+}
+// this CTA's share of [0, len)
+struct Own {
+    int a, b;
+};
+__device__ __forceinline__ Own own_of(int len, const BShared &S)
+{
+    const int per = (len + S.ncl - 1) / S.ncl;
+    Own o;
+    o.a = min(len, S.rank * per);
+    o.b = min(len, o.a + per);
+    return o;
+}
 
+// ------------------------------------------------------ CTA vector helpers
+// The loops over a vector run over the CTA's own elements, always with the
+// same thread for an element; sums go over the cluster.
+__device__ __forceinline__ double cta_sum(double v, BShared &S)
+{
+    v = block_sum<BT>(v, S.red);
+    return S.ncl == 1 ? v : cl_sum(v, S);
+}
 __device__ double cta_nrm2(const double *x, int n, BShared &S)
 {
+    const Own o = own_of(n, S);
     double a = 0.0;
-    for (int i = threadIdx.x; i < n; i += BT) a = fma(x[i], x[i], a);
+    for (int i = o.a + threadIdx.x; i < o.b; i += BT) a = fma(x[i], x[i], a);
     return sqrt(cta_sum(a, S));
 }
 __device__ double cta_dot(const double *x, const double *y, int n, BShared &S)
 {
+    const Own o = own_of(n, S);
     double a = 0.0;
-    for (int i = threadIdx.x; i < n; i += BT) a = fma(x[i], y[i], a);
+    for (int i = o.a + threadIdx.x; i < o.b; i += BT) a = fma(x[i], y[i], a);
     return cta_sum(a, S);
 }
-__device__ void cta_axpy(int n, double a, const double *x, double *y)
+__device__ void cta_axpy(int n, double a, const double *x, double *y, const BShared &S)
 {
-    for (int i = threadIdx.x; i < n; i += BT) y[i] = fma(a, x[i], y[i]);
+    const Own o = own_of(n, S);
+    for (int i = o.a + threadIdx.x; i < o.b; i += BT) y[i] = fma(a, x[i], y[i]);
     __syncthreads();
 }
 // dsafescal (dsafescal.F:4-55)
-__device__ void cta_safescal(int n, double a, double *x)
+__device__ void cta_safescal(int n, double a, double *x, const BShared &S)
 {
+    const Own o = own_of(n, S);
     if (fabs(a) >= SFMIN) {
         const double r = 1.0 / a;
-        for (int i = threadIdx.x; i < n; i += BT) x[i] *= r;
+        for (int i = o.a + threadIdx.x; i < o.b; i += BT) x[i] *= r;
     } else {
-        for (int i = threadIdx.x; i < n; i += BT) x[i] /= a;
+        for (int i = o.a + threadIdx.x; i < o.b; i += BT) x[i] /= a;
     }
     __syncthreads();
 }
-// y = A x (A: rows x *, CSR with FP32 values) with g lanes per row (the row
-// split, g a power of two <= 32): a group of g lanes takes a row, each lane
-// every g-th nonzero with four (index, value) pairs and four gathers in
-// flight, then the group adds its partial sums by a shuffle tree.  g = 1 is
+// an FP32 value widened with integer operations: the conversion instruction
+// runs on the FP64 pipe (64 cycles a warp), and the products below would
+// spend as much of that pipe on it as on their FMAs
+__device__ __forceinline__ double b_widen(float f)
+{
+    const unsigned u = __float_as_uint(f), e = (u >> 23) & 0xffu;
+    if (e - 1u < 0xfeu)  // normal
+        return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))), (int)(u << 29));
+    if ((u << 1) == 0u) return __hiloint2double((int)u, 0);
+    return (double)f;  // subnormal, infinite, NaN
+}
+// y = A x on the CTA's own rows of A (CSR with FP32 values) with g lanes per
+// row (the row split, g a power of two <= 32): a group of g lanes takes a row,
+// each lane every g-th nonzero with four (index, value) pairs and four gathers
+// in flight, then the group adds its partial sums by a shuffle tree.  g = 1 is
 // one thread per row.  The autotuner picks g per problem class: long rows
 // and few of them favour wide groups, many short rows g = 1.
 __device__ void cta_spmv(const int *ptr, const int *idx, const float *val, int rows, const double *x, double *y,
-                         int g)
+                         int g, const BShared &S)
 {
     const int grp = threadIdx.x / g, lig = threadIdx.x % g, ngrp = BT / g;
-    for (int r0 = 0; r0 < rows; r0 += ngrp) {
+    const Own o = own_of(rows, S);
+    for (int r0 = o.a; r0 < o.b; r0 += ngrp) {
         const int r = r0 + grp;
         double s = 0.0;
-        if (r < rows) {
+        if (r < o.b) {
             const int e1 = ptr[r + 1];
             int e = ptr[r] + lig;
             for (; e + 3 * g < e1; e += 4 * g) {
                 const int c0 = idx[e], c1 = idx[e + g], c2 = idx[e + 2 * g], c3 = idx[e + 3 * g];
                 const float v0 = val[e], v1 = val[e + g], v2 = val[e + 2 * g], v3 = val[e + 3 * g];
                 const double x0 = x[c0], x1 = x[c1], x2 = x[c2], x3 = x[c3];
-                s = fma((double)v0, x0, s);
-                s = fma((double)v1, x1, s);
-                s = fma((double)v2, x2, s);
-                s = fma((double)v3, x3, s);
+                s = fma(b_widen(v0), x0, s);
+                s = fma(b_widen(v1), x1, s);
+                s = fma(b_widen(v2), x2, s);
+                s = fma(b_widen(v3), x3, s);
             }
-            for (; e < e1; e += g) s = fma((double)val[e], x[idx[e]], s);
+            for (; e < e1; e += g) s = fma(b_widen(val[e]), x[idx[e]], s);
         }
         // every lane of a warp takes part (rows past the end add zeros)
-        for (int o = g >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, g);
-        if (r < rows && lig == 0) y[r] = s;
+        for (int q = g >> 1; q > 0; q >>= 1) s += __shfl_xor_sync(0xffffffffu, s, q, g);
+        if (r < o.b && lig == 0) y[r] = s;
     }
     __syncthreads();
 }
 // dreorth with iterated CGS (dreorth.F:106-210): x against the first ncols
 // columns of W (leading dimension ld); *nrm is ||x|| on entry and exit
-// projections h = W(:, 0:ncols)' x into S.h: each warp takes dc adjacent
-// columns at a time and reads each x element once for all of them (the
-// autotuner's choice of dc; every column's sum is formed in the same order
-// whatever dc is, so the choice does not change the result)
+// projections W(:, 0:ncols)' x over the CTA's own rows into S.xch[S.par]: each
+// warp takes dc adjacent columns at a time and reads each x element once for
+// all of them (the autotuner's choice of dc; every column's sum is formed in
+// the same order whatever dc is, so the choice does not change the result)
 template <int DC>
 __device__ void cta_proj(const double *W, int ld, int ncols, const double *x, int len, BShared &S)
 {
+    const Own o = own_of(len, S);
     const int lane = threadIdx.x & 31;
+    double *h = S.xch[S.par];
     for (int c0 = (threadIdx.x >> 5) * DC; c0 < ncols; c0 += BW * DC) {
         const int nc = min(DC, ncols - c0);
         double s[DC];
 #pragma unroll
         for (int u = 0; u < DC; u++) s[u] = 0.0;
-        for (int i = lane; i < len; i += 32) {
+        for (int i = o.a + lane; i < o.b; i += 32) {
             const double xi = x[i];
 #pragma unroll
             for (int u = 0; u < DC; u++)
@@ -189,7 +281,7 @@ __device__ void cta_proj(const double *W, int ld, int ncols, const double *x, in
 #pragma unroll
         for (int u = 0; u < DC; u++) {
             const double t = warp_sum(s[u]);
-            if (lane == 0 && u < nc) S.h[c0 + u] = t;
+            if (lane == 0 && u < nc) h[c0 + u] = t;
         }
     }
 }
@@ -199,17 +291,32 @@ __device__ void cta_proj_dc(const double *W, int ld, int ncols, const double *x,
     else if (dc == 2) cta_proj<2>(W, ld, ncols, x, len, S);
     else cta_proj<1>(W, ld, ncols, x, len, S);
 }
+// S.h[0 .. ncols) = the sum over the CTAs of their S.xch[S.par]
+__device__ void cl_gather_h(int ncols, BShared &S)
+{
+    csync(S);
+    const int par = S.par;
+    for (int c = threadIdx.x; c < ncols; c += BT) {
+        double t = 0.0;
+        for (int r = 0; r < S.ncl; r++) t += S.ncl == 1 ? S.xch[par][c] : peer_f64(&S.xch[par][c], r);
+        S.h[c] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) S.par = par ^ 1;
+    __syncthreads();
+}
 
 __device__ void cta_reorth(const double *W, int ld, int ncols, double *x, int len, double *nrm, BShared &S, int &count,
                            int dc)
 {
     if (ncols <= 0) return;
+    const Own o = own_of(len, S);
     double nrm0 = *nrm;
     for (int it = 0; it < NTRY; it++) {
         cta_proj_dc(W, ld, ncols, x, len, S, dc);
-        __syncthreads();
+        cl_gather_h(ncols, S);
         double a = 0.0;
-        for (int i = threadIdx.x; i < len; i += BT) {
+        for (int i = o.a + threadIdx.x; i < o.b; i += BT) {
             double v = x[i];
             int c = 0;
             for (; c + 3 < ncols; c += 4) {
@@ -232,7 +339,7 @@ __device__ void cta_reorth(const double *W, int ld, int ncols, double *x, int le
         }
         nrm0 = s;
     }
-    for (int i = threadIdx.x; i < len; i += BT) x[i] = 0.0;
+    for (int i = o.a + threadIdx.x; i < o.b; i += BT) x[i] = 0.0;
     __syncthreads();
     *nrm = 0.0;
     count++;
@@ -248,22 +355,24 @@ __device__ void cta_reorth(const double *W, int ld, int ncols, double *x, int le
 // matvecs against 4299 ms and 581,632 with the FP64 routines above, which
 // stay the default.
 
-__device__ void cta_split_col(const double *w, float2 *wp, int len)
+__device__ void cta_split_col(const double *w, float2 *wp, int len, const BShared &S)
 {
-    for (int i = threadIdx.x; i < len; i += BT) wp[i] = pl_split(w[i]);
+    const Own o = own_of(len, S);
+    for (int i = o.a + threadIdx.x; i < o.b; i += BT) wp[i] = pl_split(w[i]);
 }
 
 // y = A x with x given by its planes: each product val * (hi + lo) with the
 // FP32 value exact, summed as a compensated pair, the row split g as in
 // cta_spmv; y in FP64
 __device__ void cta_spmv_pl(const int *ptr, const int *idx, const float *val, int rows, const float2 *xp, double *y,
-                            int g)
+                            int g, const BShared &S)
 {
     const int grp = threadIdx.x / g, lig = threadIdx.x % g, ngrp = BT / g;
-    for (int r0 = 0; r0 < rows; r0 += ngrp) {
+    const Own o = own_of(rows, S);
+    for (int r0 = o.a; r0 < o.b; r0 += ngrp) {
         const int r = r0 + grp;
         PlAcc acc;
-        if (r < rows) {
+        if (r < o.b) {
             const int e1 = ptr[r + 1];
             int e = ptr[r] + lig;
             for (; e + 3 * g < e1; e += 4 * g) {
@@ -280,24 +389,27 @@ __device__ void cta_spmv_pl(const int *ptr, const int *idx, const float *val, in
                 acc.add(val[e], 0.f, xv.x, xv.y);
             }
         }
-        for (int o = g >> 1; o > 0; o >>= 1)
-            pl_pair_add(acc.s, acc.c, __shfl_xor_sync(0xffffffffu, acc.s, o, g),
-                        __shfl_xor_sync(0xffffffffu, acc.c, o, g));
-        if (r < rows && lig == 0) y[r] = acc.value_int();
+        for (int q = g >> 1; q > 0; q >>= 1)
+            pl_pair_add(acc.s, acc.c, __shfl_xor_sync(0xffffffffu, acc.s, q, g),
+                        __shfl_xor_sync(0xffffffffu, acc.c, q, g));
+        if (r < o.b && lig == 0) y[r] = acc.value_int();
     }
     __syncthreads();
 }
 
-// projections S.h = Wp(:, 0:ncols)' xq * back from the planes, dc adjacent
+// projections Wp(:, 0:ncols)' xq * back from the planes over the CTA's own
+// rows into S.xch[S.par], dc adjacent
 // columns per warp (every column's sum in the same order whatever dc is)
 template <int DC>
 __device__ void cta_proj_pl(const float2 *Wp, int ld, int ncols, const float2 *xq, int len, double back, BShared &S)
 {
+    const Own o = own_of(len, S);
     const int lane = threadIdx.x & 31;
+    double *h = S.xch[S.par];
     for (int c0 = (threadIdx.x >> 5) * DC; c0 < ncols; c0 += BW * DC) {
         const int nc = min(DC, ncols - c0);
         PlAcc acc[DC];
-        for (int i = lane; i < len; i += 32) {
+        for (int i = o.a + lane; i < o.b; i += 32) {
             const float2 xv = xq[i];
 #pragma unroll
             for (int u = 0; u < DC; u++)
@@ -309,7 +421,7 @@ __device__ void cta_proj_pl(const float2 *Wp, int ld, int ncols, const float2 *x
 #pragma unroll
         for (int u = 0; u < DC; u++) {
             const double t = warp_sum(acc[u].value_int());
-            if (lane == 0 && u < nc) S.h[c0 + u] = t * back;
+            if (lane == 0 && u < nc) h[c0 + u] = t * back;
         }
     }
 }
@@ -321,18 +433,19 @@ __device__ void cta_proj_pl_dc(const float2 *Wp, int ld, int ncols, const float2
     else cta_proj_pl<1>(Wp, ld, ncols, xq, len, back, S);
 }
 
-// x (len) as planes in xq, scaled by 2^-xs for the CTA's largest exponent
+// the CTA's own part of x as planes in xq, scaled by 2^-xs for its largest exponent
 // (|x 2^-xs| < 2); returns 2^xs
 __device__ double cta_xplanes(const double *x, int len, float2 *xq, BShared &S)
 {
+    const Own o = own_of(len, S);
     if (threadIdx.x == 0) S.xe = 0;
     __syncthreads();
     int e = 0;
-    for (int i = threadIdx.x; i < len; i += BT) e = max(e, f3_expo(x[i]));
+    for (int i = o.a + threadIdx.x; i < o.b; i += BT) e = max(e, f3_expo(x[i]));
     if (e) atomicMax(&S.xe, e);
     __syncthreads();
     const int xs = S.xe == 0 ? 0 : S.xe - 1023;
-    for (int i = threadIdx.x; i < len; i += BT) xq[i] = pl_xsplit(x[i], xs);
+    for (int i = o.a + threadIdx.x; i < o.b; i += BT) xq[i] = pl_xsplit(x[i], xs);
     __syncthreads();
     return f3_pow2(xs);
 }
@@ -343,11 +456,12 @@ __device__ void cta_reorth_pl(const float2 *Wp, int ld, int ncols, double *x, in
                               int &count, int dc, float2 *xq)
 {
     if (ncols <= 0) return;
+    const Own o = own_of(len, S);
     double nrm0 = *nrm;
     for (int it = 0; it < NTRY; it++) {
         const double back = cta_xplanes(x, len, xq, S);
         cta_proj_pl_dc(Wp, ld, ncols, xq, len, back, S, dc);
-        __syncthreads();
+        cl_gather_h(ncols, S);
         // h as planes, scaled by the power of two of its largest entry
         if (threadIdx.x == 0) S.xe = 0;
         __syncthreads();
@@ -360,7 +474,7 @@ __device__ void cta_reorth_pl(const float2 *Wp, int ld, int ncols, double *x, in
         __syncthreads();
         const double hback = f3_pow2(hs);
         double a = 0.0;
-        for (int i = threadIdx.x; i < len; i += BT) {
+        for (int i = o.a + threadIdx.x; i < o.b; i += BT) {
             PlAcc sm;
             for (int c = 0; c < ncols; c++) {
                 const float2 wv = Wp[(size_t)c * ld + i];
@@ -380,7 +494,7 @@ __device__ void cta_reorth_pl(const float2 *Wp, int ld, int ncols, double *x, in
         }
         nrm0 = s;
     }
-    for (int i = threadIdx.x; i < len; i += BT) x[i] = 0.0;
+    for (int i = o.a + threadIdx.x; i < o.b; i += BT) x[i] = 0.0;
     __syncthreads();
     *nrm = 0.0;
     count++;
@@ -404,8 +518,8 @@ __device__ bool b_lanbpro(BProb &P, const BCfg &c, BShared &S, float2 *xq)
     if (k0 == 0) {
         beta = P.rnorm;
         alpha = 0.0;
-        cta_safescal(m, beta, U);
-        if (PL) cta_split_col(U, Up, m);
+        cta_safescal(m, beta, U, S);
+        if (PL) cta_split_col(U, Up, m, S);
         __syncthreads();
         j0 = 1;
     } else {
@@ -414,18 +528,19 @@ __device__ bool b_lanbpro(BProb &P, const BCfg &c, BShared &S, float2 *xq)
         // the restart rewrote U(:, 0:k0) and V(:, 0:k0): their planes
         if (PL)
             for (int q = 0; q < k0; q++) {
-                cta_split_col(U + (size_t)q * m, Up + (size_t)q * m, m);
-                cta_split_col(V + (size_t)q * n, Vp + (size_t)q * n, n);
+                cta_split_col(U + (size_t)q * m, Up + (size_t)q * m, m, S);
+                cta_split_col(V + (size_t)q * n, Vp + (size_t)q * n, n, S);
             }
         __syncthreads();
         double *uk = U + (size_t)k0 * m;
-        for (int i = threadIdx.x; i < m; i += BT) uk[i] *= P.rnorm;
+        const Own o = own_of(m, S);
+        for (int i = o.a + threadIdx.x; i < o.b; i += BT) uk[i] *= P.rnorm;
         __syncthreads();
         double r = P.rnorm;
         if (PL) cta_reorth_pl(Up, m, k0, uk, m, &r, S, nre, P.dc, xq);
         else cta_reorth(U, m, k0, uk, m, &r, S, nre, P.dc);
-        cta_safescal(m, r, uk);
-        if (PL) cta_split_col(uk, Up + (size_t)k0 * m, m);
+        cta_safescal(m, r, uk, S);
+        if (PL) cta_split_col(uk, Up + (size_t)k0 * m, m, S);
         __syncthreads();
         beta = r;
         if (threadIdx.x == 0) bb[k0 - 1] = beta;
@@ -450,19 +565,20 @@ __device__ bool b_lanbpro(BProb &P, const BCfg &c, BShared &S, float2 *xq)
     for (int j = j0; j <= dim; j++) {
         double *vj = V + (size_t)(j - 1) * n, *uj = U + (size_t)(j - 1) * m, *uj1 = U + (size_t)j * m;
         // alpha_j v_j = A' u_j - beta_j v_{j-1}
-        if (PL) cta_spmv_pl(P.tptr, P.tidx, P.tval, n, Up + (size_t)(j - 1) * m, vj, P.g);
-        else cta_spmv(P.tptr, P.tidx, P.tval, n, uj, vj, P.g);
+        csync(S);  // the other CTAs' parts of u_j
+        if (PL) cta_spmv_pl(P.tptr, P.tidx, P.tval, n, Up + (size_t)(j - 1) * m, vj, P.g, S);
+        else cta_spmv(P.tptr, P.tidx, P.tval, n, uj, vj, P.g, S);
         nopx++;
         if (j == 1) {
             alpha = cta_nrm2(vj, n, S);
             anorm = fmax(anorm, FUDGE * alpha);
         } else {
-            cta_axpy(n, -beta, vj - n, vj);
+            cta_axpy(n, -beta, vj - n, vj, S);
             alpha = cta_nrm2(vj, n, S);
             if (c.ielr > 0 && alpha < KAPPA * beta) {
                 for (int i = 1; i <= c.ielr; i++) {
                     s = cta_dot(vj - n, vj, n, S);
-                    cta_axpy(n, -s, vj - n, vj);
+                    cta_axpy(n, -s, vj - n, vj, S);
                     if (beta != 0.0) {
                         beta = beta + s;
                         if (threadIdx.x == 0) bb[j - 2] = beta;
@@ -490,21 +606,22 @@ __device__ bool b_lanbpro(BProb &P, const BCfg &c, BShared &S, float2 *xq)
         }
         if (alpha < anorm * epsn && j < dim) { ok = false; break; }
         if (threadIdx.x == 0) ba[j - 1] = alpha;
-        if (alpha != 0.0) cta_safescal(n, alpha, vj);
+        if (alpha != 0.0) cta_safescal(n, alpha, vj, S);
         if (PL) {
-            cta_split_col(vj, Vp + (size_t)(j - 1) * n, n);
+            cta_split_col(vj, Vp + (size_t)(j - 1) * n, n, S);
             __syncthreads();
         }
         // beta_{j+1} u_{j+1} = A v_j - alpha_j u_j
-        if (PL) cta_spmv_pl(P.ptr, P.idx, P.val, m, Vp + (size_t)(j - 1) * n, uj1, P.g);
-        else cta_spmv(P.ptr, P.idx, P.val, m, vj, uj1, P.g);
+        csync(S);  // the other CTAs' parts of v_j
+        if (PL) cta_spmv_pl(P.ptr, P.idx, P.val, m, Vp + (size_t)(j - 1) * n, uj1, P.g, S);
+        else cta_spmv(P.ptr, P.idx, P.val, m, vj, uj1, P.g, S);
         nopx++;
-        cta_axpy(m, -alpha, uj, uj1);
+        cta_axpy(m, -alpha, uj, uj1, S);
         beta = cta_nrm2(uj1, m, S);
         if (c.ielr > 0 && beta < KAPPA * alpha) {
             for (int i = 1; i <= c.ielr; i++) {
                 s = cta_dot(uj, uj1, m, S);
-                cta_axpy(m, -s, uj, uj1);
+                cta_axpy(m, -s, uj, uj1, S);
                 if (alpha != 0.0) {
                     alpha = alpha + s;
                     if (threadIdx.x == 0) ba[j - 1] = alpha;
@@ -530,20 +647,21 @@ __device__ bool b_lanbpro(BProb &P, const BCfg &c, BShared &S, float2 *xq)
         }
         if (beta < anorm * epsn && j < dim) { ok = false; break; }
         if (threadIdx.x == 0) bb[j - 1] = beta;
-        if (beta != 0.0) cta_safescal(m, beta, uj1);
+        if (beta != 0.0) cta_safescal(m, beta, uj1, S);
         if (PL) {
-            cta_split_col(uj1, Up + (size_t)j * m, m);
+            cta_split_col(uj1, Up + (size_t)j * m, m, S);
             __syncthreads();
         }
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    // every CTA has read what rank 0 rewrites
+    csync(S);
+    if (threadIdx.x == 0 && S.rank == 0) {
         P.rnorm = beta;
         P.anorm = anorm;
         P.nopx += nopx;
         P.nreorth += nre;
     }
-    __syncthreads();
+    csync(S);
     return ok;
 }
 
@@ -582,14 +700,17 @@ __device__ int b_analyse(BProb &P, const BCfg &c, BShared &S, double *scr, const
         }
     }
     __syncthreads();
-    if (S.flag) return -1;
+    if (S.flag) {
+        csync(S);
+        return -1;
+    }
     if (threadIdx.x == 0) {
         const double eps34 = pow(EPS, 0.75);
         const double epsn = (double)(P.m > P.n ? P.m : P.n) * EPS / 2.0;
         double anorm = P.anorm;
         if (dim > 5) anorm = S.sig[0];
         else anorm = fmax(anorm, S.sig[0]);
-        P.anorm = anorm;
+        S.scal[3] = anorm;
         const int lim = dim < c.neig ? dim : c.neig;
         refinebounds_dev(mn, lim, S.sig, S.bnd, epsn * anorm, eps34);
         int nconv = 0, i = 1;
@@ -597,10 +718,16 @@ __device__ int b_analyse(BProb &P, const BCfg &c, BShared &S, double *scr, const
             if (S.bnd[i - 1] <= c.tol * S.sig[i - 1]) { nconv++; i++; }
             else i = c.k + 1;
         }
+        S.scal[4] = nconv;
+    }
+    // every CTA has read alpha, beta, rnorm and anorm
+    csync(S);
+    const int nconv = (int)S.scal[4];
+    if (threadIdx.x == 0 && S.rank == 0) {
+        P.anorm = S.scal[3];
         P.nconv = nconv;
     }
-    __syncthreads();
-    return P.nconv;
+    return nconv;
 }
 
 // ------------------------------------------------------------- restart
@@ -695,30 +822,32 @@ __device__ void b_restart(BProb &P, const BCfg &c, BShared &S, double *scr, cons
             }
         }
     }
-    for (int i = threadIdx.x; i < dim; i += BT) { P.alpha[i] = D[i]; P.beta[i] = E[i]; }
-    __syncthreads();
-    // restart products through the W scratch (rows x (k+1))
+    csync(S);  // every CTA has read the old alpha, beta
+    if (S.rank == 0)
+        for (int i = threadIdx.x; i < dim; i += BT) { P.alpha[i] = D[i]; P.beta[i] = E[i]; }
+    // restart products through the W scratch (rows x (k+1)), on the CTA's own rows
     double *W = scr + L.W;
     for (int side = 0; side < 2; side++) {
         const int rows = side == 0 ? P.m : P.n, kin = side == 0 ? dp1 : dim, kout = side == 0 ? k + 1 : k;
         double *A = side == 0 ? P.U : P.V;
         const double *B = side == 0 ? Pm : Qm;
         const int ldb = side == 0 ? dp1 : dim;
-        for (int i = threadIdx.x; i < rows; i += BT)
+        const Own o = own_of(rows, S);
+        for (int i = o.a + threadIdx.x; i < o.b; i += BT)
             for (int cc = 0; cc < kout; cc++) {
                 double a = 0.0;
                 for (int l = 0; l < kin; l++) a = fma(A[(size_t)l * rows + i], B[(size_t)cc * ldb + l], a);
                 W[(size_t)cc * rows + i] = a;
             }
-        __syncthreads();
-        for (size_t t = threadIdx.x; t < (size_t)rows * kout; t += BT) A[t] = W[t];
+        for (int cc = 0; cc < kout; cc++)
+            for (int i = o.a + threadIdx.x; i < o.b; i += BT) A[(size_t)cc * rows + i] = W[(size_t)cc * rows + i];
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && S.rank == 0) {
         P.rnorm = E[k - 1];
         P.k0 = k;
     }
-    __syncthreads();
+    csync(S);
 }
 
 // --------------------------------------------------------------- Ritz
@@ -756,18 +885,20 @@ __device__ bool b_ritz(BProb &P, const BCfg &c, BShared &S, double *scr, const B
     for (int side = 0; side < 2; side++) {
         const int rows = side == 0 ? P.m : P.n, kin = side == 0 ? dp1 : dim;
         double *A = side == 0 ? P.U : P.V;
-        for (int i = threadIdx.x; i < rows; i += BT)
+        const Own o = own_of(rows, S);
+        for (int i = o.a + threadIdx.x; i < o.b; i += BT)
             for (int q = 0; q < neig; q++) {
                 const double *b = side == 0 ? Xt + (size_t)q * dp1 : tw + (size_t)q * 4 * N;
                 double a = 0.0;
                 for (int l = 0; l < kin; l++) a = fma(A[(size_t)l * rows + i], b[l], a);
                 W[(size_t)q * rows + i] = a;
             }
-        __syncthreads();
-        for (size_t t = threadIdx.x; t < (size_t)rows * neig; t += BT) A[t] = W[t];
+        for (int q = 0; q < neig; q++)
+            for (int i = o.a + threadIdx.x; i < o.b; i += BT) A[(size_t)q * rows + i] = W[(size_t)q * rows + i];
         __syncthreads();
     }
-    for (int q = threadIdx.x; q < neig; q += BT) { P.sig[q] = S.sig[q]; P.bnd[q] = S.bnd[q]; }
+    if (S.rank == 0)
+        for (int q = threadIdx.x; q < neig; q += BT) { P.sig[q] = S.sig[q]; P.bnd[q] = S.bnd[q]; }
     __syncthreads();
     return true;
 }
@@ -779,13 +910,19 @@ __global__ void __launch_bounds__(BT, 2) k_batch_cycle(BProb *probs, const int *
                                                     int cycles_per_launch)
 {
     __shared__ BShared S;
-    __shared__ int pidx;
+    cl_init(S);
     const BScrLayout L = bscr_layout(c.dim, 0);
     double *scr = scratch + (size_t)blockIdx.x * scr_stride;
     while (true) {
-        if (threadIdx.x == 0) pidx = atomicAdd(ticket, 1);
-        __syncthreads();
-        const int qi = pidx;
+        if (threadIdx.x == 0 && S.rank == 0) S.pidx = atomicAdd(ticket, 1);
+        csync(S);
+        if (threadIdx.x == 0 && S.rank != 0) {
+            uint32_t at = (uint32_t)__cvta_generic_to_shared(&S.pidx), ra;
+            asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(ra) : "r"(at));
+            asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(S.pidx) : "r"(ra) : "memory");
+        }
+        csync(S);  // rank 0 takes its next ticket only when all have read this one
+        const int qi = S.pidx;
         if (qi >= nprob) break;
         BProb &P = probs[order[qi]];
         // up to cycles_per_launch restart cycles of this problem, then it is
@@ -793,29 +930,32 @@ __global__ void __launch_bounds__(BT, 2) k_batch_cycle(BProb *probs, const int *
         for (int rep = 0; rep < cycles_per_launch && P.status == BS_ACTIVE; rep++) {
             bool ok = b_lanbpro<PL>(P, c, S, reinterpret_cast<float2 *>(scr + L.W));
             int nconv = ok ? b_analyse(P, c, S, scr, L) : -1;
+            int status = BS_ACTIVE, iter = P.iter;
+            bool values = false, bounds = false;
             if (nconv < 0) {
-                if (threadIdx.x == 0) P.status = BS_FALLBACK;
+                status = BS_FALLBACK;
             } else if (nconv >= c.neig) {
-                // the bounds of the converged values are the ones reported
-                for (int q = threadIdx.x; q < c.neig; q += BT) P.bnd[q] = S.bnd[q];
-                if (!b_ritz(P, c, S, scr, L)) {
-                    if (threadIdx.x == 0) P.status = BS_FALLBACK;
-                } else if (threadIdx.x == 0) {
-                    P.status = BS_CONVERGED;
-                }
+                status = b_ritz(P, c, S, scr, L) ? BS_CONVERGED : BS_FALLBACK;
+                bounds = true;  // those of the converged values are the ones reported
             } else {
                 b_restart(P, c, S, scr, L);
-                if (threadIdx.x == 0) {
-                    P.iter++;
-                    if (P.iter >= c.maxiter) {
-                        P.status = BS_MAXITER;
-                        for (int q = 0; q < c.neig; q++) { P.sig[q] = S.sig[q]; P.bnd[q] = S.bnd[q]; }
-                    }
+                if (++iter >= c.maxiter) {
+                    status = BS_MAXITER;
+                    values = true;
                 }
             }
-            __syncthreads();
+            csync(S);  // every CTA has read status and iter
+            if (threadIdx.x == 0 && S.rank == 0) {
+                P.iter = iter;
+                P.status = status;
+                for (int q = 0; q < c.neig && (values || bounds); q++) {
+                    if (values) P.sig[q] = S.sig[q];
+                    P.bnd[q] = S.bnd[q];
+                }
+            }
+            csync(S);
         }
-        if (threadIdx.x == 0 && P.status == BS_ACTIVE) atomicAdd(active, 1);
+        if (threadIdx.x == 0 && S.rank == 0 && P.status == BS_ACTIVE) atomicAdd(active, 1);
         __syncthreads();
     }
 }
@@ -831,17 +971,18 @@ __global__ void __launch_bounds__(BT) k_batch_probe(const BProb *probs, const in
                                                     int ncols)
 {
     __shared__ BShared S;
+    cl_init(S);
     for (int q = blockIdx.x; q < ns; q += gridDim.x) {
         const BProb &P = probs[sample[q]];
         if (PL) {
-            cta_spmv_pl(P.tptr, P.tidx, P.tval, P.n, P.Up, P.V, g);
-            cta_spmv_pl(P.ptr, P.idx, P.val, P.m, P.Vp, P.U + P.m, g);
+            cta_spmv_pl(P.tptr, P.tidx, P.tval, P.n, P.Up, P.V, g, S);
+            cta_spmv_pl(P.ptr, P.idx, P.val, P.m, P.Vp, P.U + P.m, g, S);
             cta_proj_pl_dc(P.Up, P.m, ncols, P.Up + (size_t)ncols * P.m, P.m, 1.0, S, dc);
             __syncthreads();
             cta_proj_pl_dc(P.Vp, P.n, ncols, P.Vp + (size_t)ncols * P.n, P.n, 1.0, S, dc);
         } else {
-            cta_spmv(P.tptr, P.tidx, P.tval, P.n, P.U, P.V, g);
-            cta_spmv(P.ptr, P.idx, P.val, P.m, P.V, P.U + P.m, g);
+            cta_spmv(P.tptr, P.tidx, P.tval, P.n, P.U, P.V, g, S);
+            cta_spmv(P.ptr, P.idx, P.val, P.m, P.V, P.U + P.m, g, S);
             cta_proj_dc(P.U, P.m, ncols, P.U + (size_t)ncols * P.m, P.m, S, dc);
             __syncthreads();
             cta_proj_dc(P.V, P.n, ncols, P.V + (size_t)ncols * P.n, P.n, S, dc);
@@ -854,6 +995,7 @@ __global__ void __launch_bounds__(BT) k_batch_probe(const BProb *probs, const in
 __global__ void __launch_bounds__(BT) k_batch_start(BProb *probs, int nprob)
 {
     __shared__ BShared S;
+    cl_init(S);
     for (int p = blockIdx.x; p < nprob; p += gridDim.x) {
         BProb &P = probs[p];
         const double r = cta_nrm2(P.U, P.m, S);
@@ -868,6 +1010,29 @@ __global__ void __launch_bounds__(BT) k_batch_start(BProb *probs, int nprob)
             P.status = r > 0.0 ? BS_ACTIVE : BS_FALLBACK;
         }
         __syncthreads();
+    }
+}
+
+// U(:,1) of every problem from the concatenated start vectors, and the wanted
+// columns of every problem (contiguous, leading dimension = rows) into one
+// array: one copy over the host link each way instead of one per problem
+__global__ void __launch_bounds__(BT) k_batch_unpack(const BProb *probs, const int *moff, int nprob, const double *u0)
+{
+    for (int p = blockIdx.x; p < nprob; p += gridDim.x) {
+        const BProb &P = probs[p];
+        for (int i = threadIdx.x; i < P.m; i += BT) P.U[i] = u0[moff[p] + i];
+    }
+}
+template <int SIDE>
+__global__ void __launch_bounds__(BT) k_batch_pack(const BProb *probs, const int *off, int nprob, int neig, double *out)
+{
+    for (int q = blockIdx.x; q < nprob * neig; q += gridDim.x) {
+        const BProb &P = probs[q / neig];
+        const int rows = SIDE == 0 ? P.m : P.n, c = q % neig;
+        if (P.status != BS_CONVERGED) continue;
+        const double *a = (SIDE == 0 ? P.U : P.V) + (size_t)c * rows;
+        double *o = out + (size_t)off[q / neig] * neig + (size_t)c * rows;
+        for (int i = threadIdx.x; i < rows; i += BT) o[i] = a[i];
     }
 }
 
@@ -938,6 +1103,26 @@ static std::mutex g_batch_mu;
 static std::map<int64_t, Batch *> g_batches;
 static int64_t g_batch_next = 1;
 static thread_local propack_batch_stats_t g_batch_stats;
+
+// CTAs per problem: the smallest of 1, 2, 4, 8 with which the costliest
+// problem takes no longer than the whole batch's work spread over the SMs, so
+// that neither a few large problems (192 of the batched workload: 229 ms with
+// one CTA each, the largest alone ~200 ms) nor the barriers of clusters that
+// are not needed set the time; a problem under CLUSTER_MIN per CTA stays whole
+// (its phases are shorter than the barriers).
+constexpr double CLUSTER_MIN = 40000.0;  // cost (nonzeros + 8 (m + n)) per CTA
+static int batch_cluster(const Batch &B)
+{
+    double total = 0.0, most = 0.0;
+    for (int p = 0; p < B.nprob; p++) {
+        const double c = (double)(B.zoff[p + 1] - B.zoff[p]) + 8.0 * (B.m[p] + B.n[p]);
+        total += c;
+        most = std::max(most, c);
+    }
+    int cs = 1;
+    while (cs < BCS_MAX && most / cs > total / device_info().sms && most / (2 * cs) >= CLUSTER_MIN) cs *= 2;
+    return cs;
+}
 
 // Time every candidate (row split g, projection tile dc) on a sample of each
 // size class and keep the fastest; the defaults (1, 1) stay unless a
@@ -1162,7 +1347,7 @@ extern "C" int propack_batch_solve(int64_t handle, int dim, int neig, int maxite
         int *dorder = nullptr, *dticket = nullptr, *dactive = nullptr, *hactive = nullptr;
         std::vector<void *> allocs;
         auto alloc = [&](void **p, size_t bytes) {
-            PGB_CUDA(cudaMalloc(p, std::max<size_t>(bytes, 16)));
+            *p = pool_alloc(std::max<size_t>(bytes, 16), s);
             allocs.push_back(*p);
         };
         alloc((void **)&dU, sizeof(double) * (size_t)B->total_m * d1);
@@ -1182,10 +1367,32 @@ extern "C" int propack_batch_solve(int64_t handle, int dim, int neig, int maxite
         alloc((void **)&dticket, sizeof(int));
         alloc((void **)&dactive, sizeof(int));
         PGB_CUDA(cudaMallocHost(&hactive, sizeof(int)));
+        const auto kernel = pl ? k_batch_cycle<true> : k_batch_cycle<false>;
         int occ = 0;
-        PGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, pl ? k_batch_cycle<true> : k_batch_cycle<false>,
-                                                               BT, 0));
-        const int grid = std::max(1, std::min(np, std::max(1, occ) * device_info().sms));
+        PGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, BT, 0));
+        const int ctas = std::max(1, occ) * device_info().sms;
+        int cs = batch_cluster(*B);
+        cudaLaunchConfig_t lc = {};
+        cudaLaunchAttribute la[1];
+        la[0].id = cudaLaunchAttributeClusterDimension;
+        la[0].val.clusterDim.y = la[0].val.clusterDim.z = 1;
+        lc.blockDim = dim3(BT);
+        lc.stream = s;
+        lc.attrs = la;
+        lc.numAttrs = 1;
+        int clusters = 0;
+        for (;; cs /= 2) {
+            la[0].val.clusterDim.x = cs;
+            lc.gridDim = dim3((unsigned)(ctas / cs * cs));
+            if (cs == 1) clusters = ctas;
+            else if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &lc) != cudaSuccess) {
+                cudaGetLastError();
+                clusters = 0;
+            }
+            if (clusters > 0) break;
+        }
+        const int grid = cs * std::max(1, std::min(np, clusters));
+        lc.gridDim = dim3((unsigned)grid);
         const BScrLayout L = bscr_layout(dim, maxrows);
         const size_t stride = (L.total + 31) / 32 * 32;
         alloc((void **)&scratch, sizeof(double) * stride * grid);
@@ -1228,9 +1435,9 @@ extern "C" int propack_batch_solve(int64_t handle, int dim, int neig, int maxite
             if (pl) {
                 PGB_CUDA(cudaMemsetAsync(dUp, 0, sizeof(float2) * (size_t)B->total_m * d1, s));
                 PGB_CUDA(cudaMemsetAsync(dVp, 0, sizeof(float2) * (size_t)B->total_n * dim, s));
-                batch_tune<true>(B, dprob, grid, dim, s);
+                batch_tune<true>(B, dprob, ctas, dim, s);
             } else {
-                batch_tune<false>(B, dprob, grid, dim, s);
+                batch_tune<false>(B, dprob, ctas, dim, s);
             }
             g_batch_stats.tune_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0)
                                         .count();
@@ -1244,12 +1451,14 @@ extern "C" int propack_batch_solve(int64_t handle, int dim, int neig, int maxite
         PGB_CUDA(cudaMemcpyAsync(dorder, B->order.data(), sizeof(int) * np, cudaMemcpyHostToDevice, s));
         PGB_CUDA(cudaMemsetAsync(dab, 0, sizeof(double) * (size_t)np * 2 * (d1 + 1), s));
         PGB_CUDA(cudaEventRecord(e0, s));
-        // start vectors: U(:,1) of problem p = u0[moff[p] .. moff[p+1])
-        mo = 0;
-        for (int p = 0; p < np; p++) {
-            PGB_CUDA(cudaMemcpyAsync(hp[p].U, u0 + mo, sizeof(double) * B->m[p], cudaMemcpyHostToDevice, s));
-            mo += B->m[p];
-        }
+        // start vectors: U(:,1) of problem p = u0[moff[p] .. moff[p+1]); the
+        // staging array also takes the packed results
+        double *stage = nullptr;
+        const size_t nstage = std::max<size_t>((size_t)B->total_m, (size_t)std::max(B->total_m, B->total_n) * neig);
+        alloc((void **)&stage, sizeof(double) * nstage);
+        h2d_bytes(stage, u0, sizeof(double) * (size_t)B->total_m, s);
+        k_batch_unpack<<<std::min(np, 4096), BT, 0, s>>>(dprob, B->d_moff, np, stage);
+        PGB_LAUNCHED();
         k_batch_start<<<std::min(np, 4096), BT, 0, s>>>(dprob, np);
         PGB_LAUNCHED();
         BCfg cfg;
@@ -1266,12 +1475,8 @@ extern "C" int propack_batch_solve(int64_t handle, int dim, int neig, int maxite
         PGB_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
         PGB_CUDA(cudaMemsetAsync(dticket, 0, sizeof(int), s));
         PGB_CUDA(cudaMemsetAsync(dactive, 0, sizeof(int), s));
-        if (pl)
-            k_batch_cycle<true><<<grid, BT, 0, s>>>(dprob, dorder, np, cfg, scratch, stride, dticket, dactive,
-                                                    BATCH_CYCLES_PER_LAUNCH);
-        else
-            k_batch_cycle<false><<<grid, BT, 0, s>>>(dprob, dorder, np, cfg, scratch, stride, dticket, dactive,
-                                                     BATCH_CYCLES_PER_LAUNCH);
+        PGB_CUDA(cudaLaunchKernelEx(&lc, kernel, dprob, (const int *)dorder, np, cfg, scratch, stride, dticket, dactive,
+                                    (int)BATCH_CYCLES_PER_LAUNCH));
         PGB_CUDA(cudaMemcpyAsync(hactive, dactive, sizeof(int), cudaMemcpyDeviceToHost, s));
         PGB_CUDA(cudaStreamEndCapture(s, &graph));
         PGB_CUDA(cudaGraphInstantiate(&exec, graph, 0));
@@ -1288,8 +1493,6 @@ extern "C" int propack_batch_solve(int64_t handle, int dim, int neig, int maxite
         std::vector<double> hsb((size_t)np * 2 * neig);
         PGB_CUDA(cudaMemcpyAsync(hsb.data(), dsb, sizeof(double) * hsb.size(), cudaMemcpyDeviceToHost, s));
         PGB_CUDA(cudaStreamSynchronize(s));
-        mo = 0;
-        no = 0;
         for (int p = 0; p < np; p++) {
             const BProb &P = hp[p];
             for (int q = 0; q < neig; q++) {
@@ -1297,22 +1500,35 @@ extern "C" int propack_batch_solve(int64_t handle, int dim, int neig, int maxite
                 bnd[(size_t)p * neig + q] = hsb[(size_t)p * 2 * neig + neig + q];
             }
             info[p] = P.status == BS_CONVERGED ? 0 : (P.status == BS_MAXITER ? -1 : 1);
-            if (P.status == BS_CONVERGED) {
-                if (U)
-                    PGB_CUDA(cudaMemcpyAsync(U + mo * neig, P.U, sizeof(double) * (size_t)P.m * neig,
-                                             cudaMemcpyDeviceToHost, s));
-                if (V)
-                    PGB_CUDA(cudaMemcpyAsync(V + no * neig, P.V, sizeof(double) * (size_t)P.n * neig,
-                                             cudaMemcpyDeviceToHost, s));
-            }
             g_batch_stats.nopx += P.nopx;
             g_batch_stats.nreorth += P.nreorth;
             g_batch_stats.converged += P.status == BS_CONVERGED;
             g_batch_stats.fallback += P.status == BS_FALLBACK;
-            mo += P.m;
-            no += P.n;
         }
-        PGB_CUDA(cudaStreamSynchronize(s));
+        for (int side = 0; side < 2; side++) {
+            double *out = side == 0 ? U : V;
+            if (!out) continue;
+            const int *off = side == 0 ? B->d_moff : B->d_noff;
+            const int g = std::min(np * neig, 8 * device_info().sms);
+            if (side == 0) k_batch_pack<0><<<g, BT, 0, s>>>(dprob, off, np, neig, stage);
+            else k_batch_pack<1><<<g, BT, 0, s>>>(dprob, off, np, neig, stage);
+            PGB_LAUNCHED();
+            // a problem that did not converge leaves its part of the caller's array alone
+            int64_t p0 = 0, at = 0;
+            const std::vector<int> &len = side == 0 ? B->m : B->n;
+            int64_t run = 0;
+            for (int p = 0; p <= np; p++) {
+                const bool take = p < np && hp[p].status == BS_CONVERGED;
+                if (take) run += len[p];
+                if (!take && run > 0) {
+                    d2h_bytes(out + p0 * neig, stage + p0 * neig, sizeof(double) * (size_t)run * neig, s);
+                    run = 0;
+                }
+                if (p < np) at += len[p];
+                if (!take) p0 = at;
+            }
+            PGB_CUDA(cudaStreamSynchronize(s));
+        }
         float ms = 0.f;
         cudaEventElapsedTime(&ms, e0, e1);
         g_batch_stats.device_ms = ms;
@@ -1323,7 +1539,8 @@ extern "C" int propack_batch_solve(int64_t handle, int dim, int neig, int maxite
         cudaGraphDestroy(graph);
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        for (void *q : allocs) cudaFree(q);
+        for (void *q : allocs) pool_free(q, s);
+        PGB_CUDA(cudaStreamSynchronize(s));
         cudaFreeHost(hactive);
         cudaStreamDestroy(s);
     })

@@ -1130,6 +1130,13 @@ static void d2h_columns(char *dst, size_t dpitch, const char *src, size_t spitch
     }
 }
 
+void d2h_bytes(void *dst, const void *src, size_t bytes, cudaStream_t s)
+{
+    if (bytes == 0) return;
+    if (bytes < ((size_t)4 << 20)) PGB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
+    else d2h_columns((char *)dst, bytes, (const char *)src, bytes, bytes, 1, s);
+}
+
 // bytes from host src to device dst on stream s: straight when src is
 // pinned (or small); otherwise through the bounce buffer, each piece
 // copied into a half by the host pool while the other half's copy to the
