@@ -443,6 +443,10 @@ void gemm(int mr, int nc, int kk, const T *A, int lda, bool ta, const double *B,
 // when the shape is outside its range (then the caller uses the FP64 kernel)
 bool gemm_f64_tc(int mr, int nc, int kk, const double *A, int lda, const double *B, int ldb, bool tb, double *C,
                  int ldc, cudaStream_t s);
+// whether a bounded wait of this thread's products gave up since the last
+// question (then with the error set); asked once their stream has been
+// synchronised
+bool gemm_failed();
 template <typename T>
 void copy_cols(const T *src, int lds, T *dst, int ldd, int rows, int cols, cudaStream_t s);
 
@@ -484,6 +488,7 @@ const Dev &device_info();
 // for mapping GBs of device memory each time; propack_release_memory()
 // gives it back.
 cudaMemPool_t lib_pool();
+void release_host_kits();       // idle streams, events and pinned words of the drivers
 void release_bounce_buffers();  // the idle pinned bounce buffers of pageable result copies
 // host -> device copy on s; pageable sources go through the bounce buffers
 void h2d_bytes(void *dst, const void *src, size_t bytes, cudaStream_t s);

@@ -16,6 +16,7 @@
 #include <cstring>
 #include <condition_variable>
 #include <functional>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <type_traits>
@@ -242,13 +243,93 @@ __global__ void k_sum_cols(const T *U, size_t ldu, int m, int ncols, double *out
 constexpr int RITZ_CHUNK_ROWS = 1 << 19;
 constexpr int RITZ_MAX_CHUNKS = 8;
 
+// What a driver call needs on the host side: two streams, events, pinned
+// words.  Creating and destroying them took a quarter of a small solve, so
+// they are kept in a free list (KITS_KEPT per process; a call takes one of its
+// device for its duration, so concurrent calls have one each) and destroyed by
+// propack_release_memory().
+struct HostKit {
+    int device = -1;
+    cudaStream_t s = nullptr, s2 = nullptr;
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr, evs0 = nullptr, evs1 = nullptr, ev_s2 = nullptr;
+    cudaEvent_t ev_chunk[2][RITZ_MAX_CHUNKS] = {};
+    std::vector<cudaEvent_t> timers;
+    char *pin = nullptr;
+    size_t pin_bytes = 0;
+    ~HostKit()
+    {
+        for (cudaEvent_t e : {ev0, ev1, evs0, evs1, ev_s2})
+            if (e) cudaEventDestroy(e);
+        for (auto &side : ev_chunk)
+            for (cudaEvent_t e : side)
+                if (e) cudaEventDestroy(e);
+        for (cudaEvent_t e : timers) cudaEventDestroy(e);
+        if (s2) cudaStreamDestroy(s2);
+        if (s) cudaStreamDestroy(s);
+        if (pin) cudaFreeHost(pin);
+    }
+};
+constexpr size_t KITS_KEPT = 8;
+static std::mutex g_kit_mu;
+static std::vector<HostKit *> g_kits;
+static HostKit *take_kit(int device, size_t pin_bytes)
+{
+    HostKit *k = nullptr;
+    {
+        std::lock_guard<std::mutex> lk(g_kit_mu);
+        for (size_t i = 0; i < g_kits.size(); i++)
+            if (g_kits[i]->device == device) {
+                k = g_kits[i];
+                g_kits.erase(g_kits.begin() + i);
+                break;
+            }
+    }
+    std::unique_ptr<HostKit> own(k ? k : new HostKit());
+    if (!k) {
+        own->device = device;
+        PGB_CUDA(cudaStreamCreateWithFlags(&own->s, cudaStreamNonBlocking));
+        PGB_CUDA(cudaStreamCreateWithFlags(&own->s2, cudaStreamNonBlocking));
+        for (cudaEvent_t *e : {&own->ev0, &own->ev1, &own->evs0, &own->evs1}) PGB_CUDA(cudaEventCreate(e));
+        PGB_CUDA(cudaEventCreateWithFlags(&own->ev_s2, cudaEventDisableTiming));
+    }
+    if (own->pin_bytes < pin_bytes) {
+        if (own->pin) PGB_CUDA(cudaFreeHost(own->pin));
+        own->pin = nullptr;
+        own->pin_bytes = 0;
+        PGB_CUDA(cudaMallocHost(&own->pin, pin_bytes));
+        own->pin_bytes = pin_bytes;
+    }
+    return own.release();
+}
+static void give_kit(HostKit *k, bool good)
+{
+    if (!k) return;
+    if (good) {
+        std::lock_guard<std::mutex> lk(g_kit_mu);
+        if (g_kits.size() < KITS_KEPT) {
+            g_kits.push_back(k);
+            return;
+        }
+    }
+    delete k;
+}
+void release_host_kits()
+{
+    std::lock_guard<std::mutex> lk(g_kit_mu);
+    for (HostKit *k : g_kits) delete k;
+    g_kits.clear();
+}
+
 struct Ctx {
     int m = 0, n = 0, kmax = 0, ldu = 0, ldv = 0, es = 8;
     int vw = 1;                             // real scalars per vector element (2: complex*16)
-    cudaStream_t s = nullptr;
+    HostKit *kit = nullptr;
+    cudaStream_t s = nullptr;               // the kit's
     void *U = nullptr, *V = nullptr;        // Lanczos vectors (double or float)
     LbCtl *ctl = nullptr;
-    LbCtl *hctl = nullptr;  // pinned host copy
+    LbCtl *hctl = nullptr;                  // pinned host copy, current whenever the host reads it
+    double *hB = nullptr;                   // pinned copies of balpha, then bbeta (get_ctl)
+    double *hsig = nullptr;                 // pinned: sigma_out, then bnd_out (analyse)
     double *balpha = nullptr, *bbeta = nullptr, *mu = nullptr, *nu = nullptr, *h = nullptr;
     double *part_sq = nullptr, *part_dot = nullptr, *part_cols = nullptr;
     int run_ctas = 0;                       // CTAs of the run kernel (run_grid)
@@ -268,7 +349,7 @@ struct Ctx {
     double *wz = nullptr;                   // scratch of the lane-parallel bidiagonal kernels
     int *dflag = nullptr;                   // Ritz path flag, ticket of the analysis
     int sig_dim = 0;                        // dimension whose singular values a1 holds (0: B changed since)
-    void *gout = nullptr;                   // GEMM output scratch (vector type)
+    void *gout = nullptr;                   // GEMM output (vector type); changes places with the longer basis
     // FP32 (hi, lo) planes of the FP64 bases for the Gram-Schmidt passes,
     // their per-column flags and the planes of the vector being
     // reorthogonalised (null: the FP64 or three-way-split kernels)
@@ -283,18 +364,19 @@ struct Ctx {
     propack_z16 *zparm = nullptr;
     double *hx = nullptr, *hy = nullptr;    // pinned host vectors for a host APROD
     int nb = 0;
-    int *hstat = nullptr;                   // pinned copy of the run kernel's error flag
+    int *hstat = nullptr;                   // pinned: the run kernel's error flag, nconv
     std::vector<void *> allocs;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr, evs0 = nullptr, evs1 = nullptr;
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr, evs0 = nullptr, evs1 = nullptr;  // the kit's
+    // phase timers still to be read: event pairs of the kit and their sums
+    std::vector<std::pair<size_t, double *>> pending;
+    size_t ntimer = 0;
     // the caller's page-locked U and V (set_host_out): dev_ritzvec forms
     // the Ritz vectors in row chunks and copies each finished chunk there on
     // s2 while the next chunks are formed on s; done[side] = columns copied
     char *hout[2] = {nullptr, nullptr};
     size_t hpitch[2] = {0, 0};
     int done[2] = {0, 0};
-    cudaStream_t s2 = nullptr;
-    cudaEvent_t ev_chunk[2][RITZ_MAX_CHUNKS] = {};
-    cudaEvent_t ev_s2 = nullptr;
+    bool copying = false;                   // copies are in flight on the kit's s2
 
     // zero-filled device memory from the library's pool
     void *dbytes(size_t bytes)
@@ -316,26 +398,25 @@ struct Ctx {
     T *dalloc(size_t count) { return (T *)dbytes(sizeof(T) * count); }
     ~Ctx()
     {
-        if (s2) cudaStreamSynchronize(s2);  // copies of Ritz chunks read pool memory
-        if (s) {
-            for (void *p : allocs) pool_free(p, s);
-            cudaStreamSynchronize(s);
-        }
-        if (hctl) cudaFreeHost(hctl);
-        if (hscal) cudaFreeHost(hscal);
-        if (hstat) cudaFreeHost(hstat);
+        if (!kit) return;
+        bool good = cudaStreamSynchronize(kit->s2) == cudaSuccess;  // copies of Ritz chunks read pool memory
+        for (void *p : allocs) pool_free(p, s);
+        good = cudaStreamSynchronize(s) == cudaSuccess && good;
+        gemm_failed();  // a call that threw leaves no flag behind for the next
         if (hx) cudaFreeHost(hx);
         if (hy) cudaFreeHost(hy);
-        if (ev0) cudaEventDestroy(ev0);
-        if (ev1) cudaEventDestroy(ev1);
-        if (evs0) cudaEventDestroy(evs0);
-        if (evs1) cudaEventDestroy(evs1);
-        for (auto &side : ev_chunk)
-            for (cudaEvent_t e : side)
-                if (e) cudaEventDestroy(e);
-        if (ev_s2) cudaEventDestroy(ev_s2);
-        if (s2) cudaStreamDestroy(s2);
-        if (s) cudaStreamDestroy(s);
+        give_kit(kit, good);
+    }
+    // the sums of the phase timers recorded so far (their events must be done)
+    void read_timers()
+    {
+        for (auto &t : pending) {
+            float ms = 0;
+            cudaEventElapsedTime(&ms, kit->timers[t.first], kit->timers[t.first + 1]);
+            *t.second += ms;
+        }
+        pending.clear();
+        ntimer = 0;
     }
     LbArgs args() const
     {
@@ -363,9 +444,11 @@ struct Ctx {
     template <typename T>
     T *Vcol(int c) const { return (T *)V + (size_t)c * ldv; }
     void sync() { PGB_CUDA(cudaStreamSynchronize(s)); }
+    // the control block and B
     void get_ctl()
     {
         PGB_CUDA(cudaMemcpyAsync(hctl, ctl, sizeof(LbCtl), cudaMemcpyDeviceToHost, s));
+        PGB_CUDA(cudaMemcpyAsync(hB, balpha, sizeof(double) * 2 * (kmax + 2), cudaMemcpyDeviceToHost, s));
         sync();
     }
     void put_ctl() { PGB_CUDA(cudaMemcpyAsync(ctl, hctl, sizeof(LbCtl), cudaMemcpyHostToDevice, s)); }
@@ -399,82 +482,89 @@ static void init_ctx(Ctx &c, int m, int n, int kmax)
     c.ldu = (m + 31) / 32 * 32;
     c.ldv = (n + 31) / 32 * 32;
     c.nb = d.nb;
-    PGB_CUDA(cudaStreamCreateWithFlags(&c.s, cudaStreamNonBlocking));
-    PGB_CUDA(cudaEventCreate(&c.ev0));
-    PGB_CUDA(cudaEventCreate(&c.ev1));
-    PGB_CUDA(cudaEventCreate(&c.evs0));
-    PGB_CUDA(cudaEventCreate(&c.evs1));
-    c.U = c.dalloc<T>((size_t)c.ldu * (kmax + 1));
-    c.V = c.dalloc<T>((size_t)c.ldv * (kmax + 1));
-    c.ctl = c.dalloc<LbCtl>(1);
-    PGB_CUDA(cudaMallocHost(&c.hctl, sizeof(LbCtl)));
-    memset(c.hctl, 0, sizeof(LbCtl));
-    c.balpha = c.dalloc<double>(kmax + 2);
-    c.bbeta = c.dalloc<double>(kmax + 2);
-    c.mu = c.dalloc<double>(kmax + 2);
-    c.nu = c.dalloc<double>(kmax + 2);
-    c.h = c.dalloc<double>((size_t)(kmax + 2) * c.vw);
-    c.part_sq = c.dalloc<double>(c.nb);
-    c.part_dot = c.dalloc<double>(c.nb);
-    c.part_cols = c.dalloc<double>((size_t)c.nb * (kmax + 2) * c.vw);
-    c.index = c.dalloc<int>(2 * (size_t)kmax + 8);
-    c.sel = c.dalloc<int>(kmax + 2);
-    const int mn = std::max(m, n);
-    c.xr = c.dalloc<T>(mn);
-    c.yr = c.dalloc<T>(mn);
-    c.dx = c.dalloc<double>(mn);
-    c.dy = c.dalloc<double>(mn);
-    c.scal = c.dalloc<double>(8);
-    PGB_CUDA(cudaMallocHost(&c.hscal, sizeof(double) * 8));
-    PGB_CUDA(cudaMallocHost(&c.hstat, sizeof(int) * 2));
-    c.hstat[0] = c.hstat[1] = 0;
-    c.runbuf = (char *)c.dbytes(lb_run_scratch());
     const size_t d1 = kmax + 2;
-    c.a1 = c.dalloc<double>(d1); c.b1 = c.dalloc<double>(d1); c.bnd = c.dalloc<double>(d1);
-    c.w = c.dalloc<double>(4 * d1);
-    c.wz = c.dalloc<double>(bidiag_scratch(kmax));
-    c.dflag = c.dalloc<int>(4);
-    c.P = c.dalloc<double>(d1 * d1); c.Q = c.dalloc<double>(d1 * d1);
-    c.shifts = c.dalloc<double>(d1);
-    c.sig_out = c.dalloc<double>(d1); c.bnd_out = c.dalloc<double>(d1);
-    c.anorm_drv = c.dalloc<double>(1);
-    c.nconv = c.dalloc<int>(1);
-    c.D = c.dalloc<double>(d1); c.E = c.dalloc<double>(d1);
-    c.Mt = c.dalloc<double>(d1 * d1); c.Pr = c.dalloc<double>(d1 * d1); c.Qt = c.dalloc<double>(d1 * d1);
-    c.X = c.dalloc<double>(d1 * d1);
-    // the restart/Ritz product's output: written by the GEMM before it is read
+    // pinned: control block, scalars, flag, B, sigma and bounds
+    const size_t octl = (sizeof(LbCtl) + 63) / 64 * 64;
+    c.kit = take_kit(d.device, octl + 128 + sizeof(double) * 4 * d1);
+    c.s = c.kit->s;
+    c.ev0 = c.kit->ev0; c.ev1 = c.kit->ev1; c.evs0 = c.kit->evs0; c.evs1 = c.kit->evs1;
+    c.hctl = (LbCtl *)c.kit->pin;
+    memset((void *)c.hctl, 0, sizeof(LbCtl));
+    c.hscal = (double *)(c.kit->pin + octl);
+    c.hstat = (int *)(c.kit->pin + octl + 64);
+    c.hstat[0] = 0;
+    c.hB = (double *)(c.kit->pin + octl + 128);
+    c.hsig = c.hB + 2 * d1;
+    // vectors: always written before they are read
+    const int mn = std::max(m, n);
+    c.U = c.dbytes_raw(sizeof(T) * (size_t)c.ldu * (kmax + 1));
+    c.V = c.dbytes_raw(sizeof(T) * (size_t)c.ldv * (kmax + 1));
     c.gout = c.dbytes_raw(sizeof(T) * (size_t)std::max(c.ldu, c.ldv) * (kmax + 1));
+    c.xr = c.dbytes_raw(sizeof(T) * (size_t)mn);
+    c.yr = c.dbytes_raw(sizeof(T) * (size_t)mn);
+    c.dx = (double *)c.dbytes_raw(sizeof(double) * (size_t)mn);
+    c.dy = (double *)c.dbytes_raw(sizeof(double) * (size_t)mn);
+    // the small arrays: one zeroed block
+    std::vector<std::pair<void **, size_t>> small;
+    auto want = [&](auto *&p, size_t count) { small.push_back({(void **)&p, sizeof(*p) * count}); };
+    want(c.ctl, 1);
+    want(c.balpha, 2 * d1);  // bbeta follows (get_ctl copies both)
+    want(c.mu, d1);
+    want(c.nu, d1);
+    want(c.h, d1 * c.vw);
+    want(c.part_sq, c.nb);
+    want(c.part_dot, c.nb);
+    want(c.part_cols, (size_t)c.nb * d1 * c.vw);
+    want(c.index, 2 * (size_t)kmax + 8);
+    want(c.sel, d1);
+    want(c.scal, 8);
+    want(c.a1, d1);
+    want(c.b1, d1);
+    want(c.bnd, d1);
+    want(c.w, 4 * d1);
+    want(c.wz, bidiag_scratch(kmax));
+    want(c.dflag, 4);
+    want(c.P, d1 * d1);
+    want(c.Q, d1 * d1);
+    want(c.shifts, d1);
+    want(c.sig_out, 2 * d1);  // bnd_out follows (analyse copies both)
+    want(c.nconv, 2);
+    want(c.anorm_drv, 1);
+    want(c.D, d1);
+    want(c.E, d1);
+    want(c.Mt, d1 * d1);
+    want(c.Pr, d1 * d1);
+    want(c.Qt, d1 * d1);
+    want(c.X, d1 * d1);
+    want(c.runbuf, lb_run_scratch());
+    constexpr bool fp64 = std::is_same<T, double>::value || std::is_same<T, double2>::value;
+    const bool planes = fp64 && g_cgs_arith == CGS_PLANES && lb_planes_fit(kmax, c.vw == 2);
+    if (planes) {
+        want(c.okU, d1);
+        want(c.okV, d1);
+    }
+    size_t total = 0;
+    for (auto &r : small) total += (r.second + 255) / 256 * 256;
+    char *base = (char *)c.dbytes(total);
+    for (auto &r : small) {
+        *r.first = base;
+        base += (r.second + 255) / 256 * 256;
+    }
+    c.bbeta = c.balpha + d1;
+    c.bnd_out = c.sig_out + d1;
     // the partial-sum arrays above hold d.nb CTAs; the grids follow the size
     c.nb = vec_grid((int64_t)std::max(m, n) * c.vw, 0);
     c.run_ctas = run_grid(std::max(m, n));
-    constexpr bool fp64 = std::is_same<T, double>::value || std::is_same<T, double2>::value;
-    if (fp64 && g_cgs_arith == CGS_PLANES && lb_planes_fit(kmax, c.vw == 2)) {
+    if (planes) {
         // planes of every real scalar (complex: of re and im); written (flag
         // set) before any kernel reads them
         c.Up = (float2 *)c.dbytes_raw(sizeof(float2) * (size_t)c.ldu * c.vw * (kmax + 1));
         c.Vp = (float2 *)c.dbytes_raw(sizeof(float2) * (size_t)c.ldv * c.vw * (kmax + 1));
-        c.xpl = c.dalloc<float2>((size_t)mn * c.vw);
-        c.okU = c.dalloc<int>(kmax + 2);
-        c.okV = c.dalloc<int>(kmax + 2);
+        c.xpl = (float2 *)c.dbytes_raw(sizeof(float2) * (size_t)mn * c.vw);
     }
 }
 
 // ----------------------------------------------------- device utilities
-template <typename T>
-static double dev_nrm2(Ctx &c, const T *x, int n)
-{
-    if constexpr (VecW<T>::w == 2) {
-        return dev_nrm2<double>(c, (const double *)x, 2 * n);
-    } else {
-        k_sumsq_part<T><<<c.nb, BS, 0, c.s>>>(x, n, c.part_sq);
-        PGB_LAUNCHED();
-        k_sum_final<<<1, BS, 0, c.s>>>(c.part_sq, c.nb, c.scal);
-        PGB_LAUNCHED();
-        PGB_CUDA(cudaMemcpyAsync(c.hscal, c.scal, sizeof(double), cudaMemcpyDeviceToHost, c.s));
-        c.sync();
-        return std::sqrt(c.hscal[0]);
-    }
-}
 template <typename T>
 static void dev_scale(Ctx &c, T *x, int n, int mode, double val)
 {
@@ -498,6 +588,29 @@ static void dev_convert(Ctx &c, const TS *src, TD *dst, int n)
 {
     k_convert<TS, TD><<<c.nb, 256, 0, c.s>>>(src, dst, n);
     PGB_LAUNCHED();
+}
+
+// ||x|| into the scalar slot `at`, on the device
+template <typename T>
+static void dev_nrm2_async(Ctx &c, const T *x, int n, int at)
+{
+    if constexpr (VecW<T>::w == 2) {
+        dev_nrm2_async<double>(c, (const double *)x, 2 * n, at);
+    } else {
+        k_sumsq_part<T><<<c.nb, BS, 0, c.s>>>(x, n, c.part_sq);
+        PGB_LAUNCHED();
+        k_sum_final<<<1, BS, 0, c.s>>>(c.part_sq, c.nb, c.scal + at);
+        PGB_LAUNCHED();
+    }
+}
+
+template <typename T>
+static double dev_nrm2(Ctx &c, const T *x, int n)
+{
+    dev_nrm2_async<T>(c, x, n, 0);
+    PGB_CUDA(cudaMemcpyAsync(c.hscal, c.scal, sizeof(double), cudaMemcpyDeviceToHost, c.s));
+    c.sync();
+    return std::sqrt(c.hscal[0]);
 }
 
 // y = op(A) x on device vectors, through the device operator or the
@@ -592,10 +705,14 @@ static int dev_getu0(Ctx &c, bool trans, int j, int ntry, T *u0, double *u0norm,
         k_rng_pm1<E><<<std::max(1, std::min(c.nb, (nch + 255) / 256)), 256, 0, c.s>>>((E *)xr, nval, seed,
                                                                                       (long long)itry * nval);
         PGB_LAUNCHED();
-        const double nrm = dev_nrm2<T>(c, xr, rsize);
+        dev_nrm2_async<T>(c, xr, rsize, 0);
         dev_aprod<T>(c, trans, xr, u0);
         g_last.nopx++;
-        *u0norm = dev_nrm2<T>(c, u0, usize);
+        dev_nrm2_async<T>(c, u0, usize, 1);
+        PGB_CUDA(cudaMemcpyAsync(c.hscal, c.scal, 2 * sizeof(double), cudaMemcpyDeviceToHost, c.s));
+        c.sync();
+        const double nrm = std::sqrt(c.hscal[0]);
+        *u0norm = std::sqrt(c.hscal[1]);
         *anormest = *u0norm / nrm;
         // dgetu0.F:30 has a REAL literal, zgetu0.F:30 a DOUBLE one
         if (j >= 1) dev_reorth_full<T>(c, W, ld, usize, j, u0, u0norm, VecW<T>::w == 2 ? KAPPA : KAPPA_GETU0);
@@ -664,10 +781,9 @@ static void dev_lanbpro(Ctx &c, int k0, int *kp, double *rnorm, double *doption,
 {
     const int m = c.m, n = c.n;
     int k = *kp;
+    // the host's copies of the control block (counters) and of B are current:
+    // every launch that changes them is followed by get_ctl
     LbCtl &h = *c.hctl;
-    // the device holds the authoritative control block between calls;
-    // refresh the host copy (counters, pending scales)
-    c.get_ctl();
     const int mn = std::max(m, n);
     h.m = m; h.n = n; h.k = k; h.ldu = c.ldu * c.vw; h.ldv = c.ldv * c.vw;
     h.icgs = ioption[0]; h.ielr = ioption[1];
@@ -693,13 +809,7 @@ static void dev_lanbpro(Ctx &c, int k0, int *kp, double *rnorm, double *doption,
     h.collapsed = 0;
     clear_prof(h);
     double anorm;
-    std::vector<double> hb(2 * (size_t)(k + 2), 0.0);
-    if (k0 > 0) {
-        PGB_CUDA(cudaMemcpyAsync(hb.data(), c.balpha, sizeof(double) * k0, cudaMemcpyDeviceToHost, c.s));
-        PGB_CUDA(cudaMemcpyAsync(hb.data() + k + 2, c.bbeta, sizeof(double) * k0, cudaMemcpyDeviceToHost, c.s));
-        c.sync();
-    }
-    double *ba = hb.data(), *bb = hb.data() + k + 2;
+    double *ba = c.hB, *bb = c.hB + c.kmax + 2;
     if (doption[2] > 0) {
         anorm = doption[2];
     } else if (k0 > 0) {
@@ -902,9 +1012,10 @@ static void dev_lanbpro(Ctx &c, int k0, int *kp, double *rnorm, double *doption,
             continue;
         }
     }
-    // apply the deferred scaling of the newest columns
+    // apply the deferred scaling of the newest columns (the kernel clears it)
     lb_enqueue_flush<T>(c.args(), c.s);
-    c.get_ctl();
+    h.pend_u.mode = 0;
+    h.pend_v.mode = 0;
     *kp = k;
     *rnorm = h.rnorm;
     *ierr = h.ierr;
@@ -1214,9 +1325,9 @@ static void copy_out(Ctx &c, double *U, int ldu, double *V, int ldv, int ncols, 
         d2h_columns((char *)U, sizeof(T) * ldu, (const char *)c.U, sizeof(T) * c.ldu, sizeof(T) * c.m, ncols, c.s);
     if (dv && c.done[1] < ncols)
         d2h_columns((char *)V, sizeof(T) * ldv, (const char *)c.V, sizeof(T) * c.ldv, sizeof(T) * c.n, ncols, c.s);
-    if (c.s2) {
-        PGB_CUDA(cudaEventRecord(c.ev_s2, c.s2));
-        PGB_CUDA(cudaStreamWaitEvent(c.s, c.ev_s2, 0));
+    if (c.copying) {
+        PGB_CUDA(cudaEventRecord(c.kit->ev_s2, c.kit->s2));
+        PGB_CUDA(cudaStreamWaitEvent(c.s, c.kit->ev_s2, 0));
     }
     }
 }
@@ -1230,54 +1341,78 @@ static void set_host_out(Ctx &c, double *U, int ldu, double *V, int ldv, bool du
     if (dv && host_pinned(V)) { c.hout[1] = (char *)V; c.hpitch[1] = sizeof(T) * (size_t)ldv; }
 }
 
-// A(:,0:nc) <- A(:,0:kk) op(B)   (dgemm_ovwr_left) on rows r0:r1
-// (complex A times the real B: the real GEMM on the (re, im) rows,
-// zdgemm_ovwr_left of complex16/zgemm_ovwr.F).  Row i of the product
-// reads only row i of A, so a row range can be overwritten once its own
-// product is formed.
+// rows r0:r1 of G(:,0:nc) = A(:,0:kk) op(B), A and G with the basis' leading
+// dimension (complex A times the real B: the real GEMM on the (re, im) rows,
+// zdgemm_ovwr_left of complex16/zgemm_ovwr.F)
 template <typename T>
-static void ovwr_left(Ctx &c, T *A, int lda, int rows, int nc, int kk, const double *B, int ldb, bool tb, int r0 = 0,
-                      int r1 = -1)
+static void basis_product(Ctx &c, const T *A, T *G, int lda, int r0, int r1, int nc, int kk, const double *B, int ldb,
+                          bool tb)
 {
-    if (r1 < 0) r1 = rows;
-    const int nr = r1 - r0;
-    if constexpr (VecW<T>::w == 2) {
-        const double *Ar = (const double *)A + 2 * (size_t)r0;
-        double *Gr = (double *)c.gout + 2 * (size_t)r0;
-        gemm<double>(2 * nr, nc, kk, Ar, 2 * lda, false, B, ldb, tb, Gr, 2 * lda, c.s);
-        copy_cols<double>(Gr, 2 * lda, (double *)A + 2 * (size_t)r0, 2 * lda, 2 * nr, nc, c.s);
-    } else {
-        gemm<T>(nr, nc, kk, A + r0, lda, false, B, ldb, tb, (T *)c.gout + r0, lda, c.s);
-        copy_cols<T>((T *)c.gout + r0, lda, A + r0, lda, nr, nc, c.s);
-    }
+    if constexpr (VecW<T>::w == 2)
+        gemm<double>(2 * (r1 - r0), nc, kk, (const double *)(A + r0), 2 * lda, false, B, ldb, tb, (double *)(G + r0),
+                     2 * lda, c.s);
+    else
+        gemm<T>(r1 - r0, nc, kk, A + r0, lda, false, B, ldb, tb, G + r0, lda, c.s);
+}
+
+// Where the product of a side ends up.  gout has the longer side's leading
+// dimension, so that side's basis and gout change places (the basis' other
+// columns are rewritten before they are read); a shorter side's product is
+// copied back, row range by row range: row i of it reads only row i.
+static bool swaps(const Ctx &c, int side) { return (side == 0 ? c.ldu : c.ldv) == std::max(c.ldu, c.ldv); }
+
+// U(:,0:nc) <- U(:,0:kk) op(B) (side 1: V; dgemm_ovwr_left)
+template <typename T>
+static void ovwr_left(Ctx &c, int side, int nc, int kk, const double *B, int ldb, bool tb, int r0 = 0, int r1 = -1)
+{
+    void *&W = side == 0 ? c.U : c.V;
+    const int ld = side == 0 ? c.ldu : c.ldv;
+    if (r1 < 0) r1 = side == 0 ? c.m : c.n;
+    T *A = (T *)W, *G = (T *)c.gout;
+    basis_product<T>(c, A, G, ld, r0, r1, nc, kk, B, ldb, tb);
+    if (swaps(c, side))
+        std::swap(W, c.gout);
+    else if constexpr (VecW<T>::w == 2)
+        copy_cols<double>((double *)(G + r0), 2 * ld, (double *)(A + r0), 2 * ld, 2 * (r1 - r0), nc, c.s);
+    else
+        copy_cols<T>(G + r0, ld, A + r0, ld, r1 - r0, nc, c.s);
 }
 
 // the Ritz product of one side; with a page-locked host array (FP64 and
 // complex*16 bases) in row chunks, each copied to the host on s2 as soon as
 // it is formed
 template <typename T>
-static void ritz_side(Ctx &c, int side, T *A, int lda, int rows, int nc, int kk, const double *B, int ldb)
+static void ritz_side(Ctx &c, int side, int nc, int kk, const double *B, int ldb)
 {
+    void *&W = side == 0 ? c.U : c.V;
+    const int rows = side == 0 ? c.m : c.n, ld = side == 0 ? c.ldu : c.ldv;
     if (sizeof(T) < 8 || !c.hout[side] || rows < 2 * RITZ_CHUNK_ROWS) {
-        ovwr_left<T>(c, A, lda, rows, nc, kk, B, ldb, true);
+        ovwr_left<T>(c, side, nc, kk, B, ldb, true);
         return;
     }
     const int nch = std::min(RITZ_MAX_CHUNKS, (rows + RITZ_CHUNK_ROWS - 1) / RITZ_CHUNK_ROWS);
     const int per = ((rows + nch - 1) / nch + 127) / 128 * 128;
-    if (!c.s2) PGB_CUDA(cudaStreamCreateWithFlags(&c.s2, cudaStreamNonBlocking));
-    if (!c.ev_s2) PGB_CUDA(cudaEventCreateWithFlags(&c.ev_s2, cudaEventDisableTiming));
+    const bool sw = swaps(c, side);
+    const T *P = (const T *)(sw ? c.gout : W);  // where the product lies
     for (int i = 0; i < nch; i++) {
         const int r0 = i * per, r1 = std::min(rows, r0 + per);
         if (r0 >= r1) break;
-        ovwr_left<T>(c, A, lda, rows, nc, kk, B, ldb, true, r0, r1);
-        cudaEvent_t &e = c.ev_chunk[side][i];
+        if (sw)
+            basis_product<T>(c, (const T *)W, (T *)c.gout, ld, r0, r1, nc, kk, B, ldb, true);
+        else
+            ovwr_left<T>(c, side, nc, kk, B, ldb, true, r0, r1);
+        cudaEvent_t &e = c.kit->ev_chunk[side][i];
         if (!e) PGB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         PGB_CUDA(cudaEventRecord(e, c.s));
-        PGB_CUDA(cudaStreamWaitEvent(c.s2, e, 0));
-        PGB_CUDA(cudaMemcpy2DAsync(c.hout[side] + sizeof(T) * (size_t)r0, c.hpitch[side], A + r0,
-                                   sizeof(T) * (size_t)lda, sizeof(T) * (size_t)(r1 - r0), nc,
-                                   cudaMemcpyDeviceToHost, c.s2));
+        PGB_CUDA(cudaStreamWaitEvent(c.kit->s2, e, 0));
+        PGB_CUDA(cudaMemcpy2DAsync(c.hout[side] + sizeof(T) * (size_t)r0, c.hpitch[side], P + r0,
+                                   sizeof(T) * (size_t)ld, sizeof(T) * (size_t)(r1 - r0), nc,
+                                   cudaMemcpyDeviceToHost, c.kit->s2));
+        c.copying = true;
     }
+    // (the other side's product then goes to this side's old basis, which no
+    // copy reads)
+    if (sw) std::swap(W, c.gout);
     c.done[side] = nc;
 }
 
@@ -1288,16 +1423,19 @@ static int analyse(Ctx &c, AnaArgs &a)
     launch_analyse(a, c.s);
     c.sig_dim = a.dim;
     g_last.nbsvd++;
-    int nc = 0;
-    PGB_CUDA(cudaMemcpyAsync(c.hscal, c.nconv, sizeof(int), cudaMemcpyDeviceToHost, c.s));
-    c.sync();
-    memcpy(&nc, c.hscal, sizeof(int));
+    // the number of converged values, and the values and bounds themselves
+    auto fetch = [&]() {
+        const size_t d1 = c.kmax + 2;
+        PGB_CUDA(cudaMemcpyAsync(c.hstat + 1, c.nconv, sizeof(int), cudaMemcpyDeviceToHost, c.s));
+        PGB_CUDA(cudaMemcpyAsync(c.hsig, c.sig_out, sizeof(double) * 2 * d1, cudaMemcpyDeviceToHost, c.s));
+        c.sync();
+        return c.hstat[1];
+    };
+    int nc = fetch();
     if (nc < 0) {
         if (trace_on()) fprintf(stderr, "[propack_gb300] analysis: lane-parallel path declined, QR path\n");
         launch_analyse_qr(a, c.s);
-        PGB_CUDA(cudaMemcpyAsync(c.hscal, c.nconv, sizeof(int), cudaMemcpyDeviceToHost, c.s));
-        c.sync();
-        memcpy(&nc, c.hscal, sizeof(int));
+        nc = fetch();
     }
     return nc;
 }
@@ -1327,35 +1465,44 @@ static void dev_ritzvec(Ctx &c, bool small_side, bool du, bool dv, int k, int di
     // QR path: X = P' Mt(1:dim, 1:dim+1)   (dim x dim+1, ld dim+1)
     if (qr) gemm<double>(dim, dp1, dim, c.Pr, dim, true, c.Mt, dp1, false, c.X, dp1, c.s);
     const int mstart = small_side ? dim - k + 1 : 1;
-    if (du) ritz_side<T>(c, 0, (T *)c.U, c.ldu, c.m, k, dp1, c.X + (mstart - 1), dp1);
-    if (dv) ritz_side<T>(c, 1, (T *)c.V, c.ldv, c.n, k, dim, c.Qt + (mstart - 1), dim);
+    if (du) ritz_side<T>(c, 0, k, dp1, c.X + (mstart - 1), dp1);
+    if (dv) ritz_side<T>(c, 1, k, dim, c.Qt + (mstart - 1), dim);
 }
 
+// device time of a scope into acc, read at the end of the call (read_timers):
+// waiting for each scope's end would leave the GPU idle between the phases
+constexpr size_t TIMER_EVENTS = 256;
 struct Timer {
     Ctx &c;
     double &acc;
-    cudaEvent_t a, b;
+    size_t at;
     Timer(Ctx &cc, double &ac) : c(cc), acc(ac)
     {
-        cudaEventCreate(&a);
-        cudaEventCreate(&b);
-        cudaEventRecord(a, c.s);
+        if (c.ntimer + 2 > TIMER_EVENTS) {
+            cudaStreamSynchronize(c.s);
+            c.read_timers();
+        }
+        at = c.ntimer;
+        c.ntimer += 2;
+        while (c.kit->timers.size() < c.ntimer) {
+            cudaEvent_t e = nullptr;
+            PGB_CUDA(cudaEventCreate(&e));
+            c.kit->timers.push_back(e);
+        }
+        cudaEventRecord(c.kit->timers[at], c.s);
     }
     ~Timer()
     {
-        cudaEventRecord(b, c.s);
-        cudaEventSynchronize(b);
-        float ms = 0;
-        cudaEventElapsedTime(&ms, a, b);
-        acc += ms;
-        cudaEventDestroy(a);
-        cudaEventDestroy(b);
+        cudaEventRecord(c.kit->timers[at + 1], c.s);
+        c.pending.push_back({at, &acc});
     }
 };
 
+// after the call's last wait: the timers, the products' flag, the counters
 static void add_ctx_counters(Ctx &c)
 {
-    c.get_ctl();
+    c.read_timers();
+    if (gemm_failed()) throw WaitFailure();
     g_last.nopx += c.hctl->nopx;
     g_last.nreorth += c.hctl->nreorth;
     g_last.ndot += c.hctl->ndot;
@@ -1516,8 +1663,8 @@ static void irl_loop(Ctx &c, const IrlIn &in, double *doption, const int *ioptio
             }
             {
                 Timer t(c, g_last.gemm_ms);
-                ovwr_left<T>(c, (T *)c.U, c.ldu, m, k + 1, dim + 1, c.P, dim + 1, false);
-                ovwr_left<T>(c, (T *)c.V, c.ldv, n, k, dim, c.Q, dim, false);
+                ovwr_left<T>(c, 0, k + 1, dim + 1, c.P, dim + 1, false);
+                ovwr_left<T>(c, 1, k, dim, c.Q, dim, false);
             }
             // rnorm = beta_k after the sweeps (written into the control block)
             c.get_ctl();
@@ -1526,13 +1673,13 @@ static void irl_loop(Ctx &c, const IrlIn &in, double *doption, const int *ioptio
         }
         iter++;
     }
+    // (the analysis brought them; none when no cycle ran)
     out.sigma.assign(std::max(nconv, 1), 0.0);
     out.bnd.assign(std::max(nconv, 1), 0.0);
-    PGB_CUDA(cudaMemcpyAsync(out.sigma.data(), c.sig_out, sizeof(double) * std::max(nconv, 1), cudaMemcpyDeviceToHost,
-                             c.s));
-    PGB_CUDA(cudaMemcpyAsync(out.bnd.data(), c.bnd_out, sizeof(double) * std::max(nconv, 1), cudaMemcpyDeviceToHost,
-                             c.s));
-    c.sync();
+    for (int i = 0; i < nconv; i++) {
+        out.sigma[i] = c.hsig[i];
+        out.bnd[i] = c.hsig[c.kmax + 2 + i];
+    }
     if ((nconv >= neig0 || out.info > 0) && (in.du || in.dv)) {
         Timer t(c, g_last.gemm_ms);
         dev_ritzvec<T>(c, in.small_side, in.du, in.dv, nconv, dim);
@@ -1562,7 +1709,7 @@ static void irl_plain(const IrlIn &in, propack_aprod_t aprod, double *dparm, pro
     else setup_operator(c, aprod, dparm, iparm);
     set_host_out<T>(c, U, ldu, V, ldv, in.du, in.dv);
     PGB_CUDA(cudaEventRecord(c.ev0, c.s));
-    PGB_CUDA(cudaMemcpyAsync(c.U, U, sizeof(T) * in.m, cudaMemcpyHostToDevice, c.s));
+    h2d_bytes(c.U, U, sizeof(T) * (size_t)in.m, c.s);
     PGB_CUDA(cudaEventRecord(c.evs0, c.s));
     irl_loop<T>(c, in, doption, ioption, out);
     PGB_CUDA(cudaEventRecord(c.evs1, c.s));
@@ -1581,10 +1728,10 @@ static void irl_plain(const IrlIn &in, propack_aprod_t aprod, double *dparm, pro
 static void load_start32(Ctx &c, const double *U, const RealOut *real)
 {
     if (real) {
-        PGB_CUDA(cudaMemcpyAsync(c.U, real->U, sizeof(float) * c.m, cudaMemcpyHostToDevice, c.s));
+        h2d_bytes(c.U, real->U, sizeof(float) * (size_t)c.m, c.s);
         PGB_CUDA(cudaEventRecord(c.evs0, c.s));
     } else {
-        PGB_CUDA(cudaMemcpyAsync(c.dx, U, sizeof(double) * c.m, cudaMemcpyHostToDevice, c.s));
+        h2d_bytes(c.dx, U, sizeof(double) * (size_t)c.m, c.s);
         PGB_CUDA(cudaEventRecord(c.evs0, c.s));
         dev_convert<double, float>(c, c.dx, c.Ucol<float>(0), c.m);
     }
@@ -1654,7 +1801,7 @@ static void run_irl(const char *which, const char *jobu, const char *jobv, int m
         init_ctx<float>(c32, m, n, in.dim);
         setup_operator(c32, aprod, dparm, iparm);
         PGB_CUDA(cudaEventRecord(c32.ev0, c32.s));
-        PGB_CUDA(cudaMemcpyAsync(c32.dx, U, sizeof(double) * m, cudaMemcpyHostToDevice, c32.s));
+        h2d_bytes(c32.dx, U, sizeof(double) * (size_t)m, c32.s);
         PGB_CUDA(cudaEventRecord(c32.evs0, c32.s));
         dev_convert<double, float>(c32, c32.dx, c32.Ucol<float>(0), m);
         double dop32[4] = {doption[0], doption[1], doption[2], doption[3]};
@@ -1668,10 +1815,10 @@ static void run_irl(const char *which, const char *jobu, const char *jobv, int m
         in32.stall_limit = 8;
         IrlOut out32;
         irl_loop<float>(c32, in32, dop32, ioption, out32);
-        add_ctx_counters(c32);
-        const int64_t nopx32 = g_last.nopx;
         PGB_CUDA(cudaEventRecord(c32.evs1, c32.s));
         c32.sync();
+        add_ctx_counters(c32);
+        const int64_t nopx32 = g_last.nopx;
         float ms32 = 0;
         cudaEventElapsedTime(&ms32, c32.evs0, c32.evs1);
         // FP64 refinement: the FP64 IRL with the caller's dim and shifts,
@@ -1747,12 +1894,12 @@ static void run_lansvd_t(const char *jobu, const char *jobv, int m, int n, int *
     if constexpr (sizeof(T) >= 8) set_host_out<T>(c, U, ldu, V, ldv, yes(jobu), yes(jobv));
     PGB_CUDA(cudaEventRecord(c.ev0, c.s));
     if constexpr (cplx) {
-        PGB_CUDA(cudaMemcpyAsync(c.U, U, sizeof(T) * m, cudaMemcpyHostToDevice, c.s));
+        h2d_bytes(c.U, U, sizeof(T) * (size_t)m, c.s);
         PGB_CUDA(cudaEventRecord(c.evs0, c.s));
     } else if constexpr (f32) {
         load_start32(c, U, real);
     } else {
-        PGB_CUDA(cudaMemcpyAsync(c.U, U, sizeof(double) * m, cudaMemcpyHostToDevice, c.s));
+        h2d_bytes(c.U, U, sizeof(double) * (size_t)m, c.s);
         PGB_CUDA(cudaEventRecord(c.evs0, c.s));
     }
     double rnorm = dev_nrm2<T>(c, c.Ucol<T>(0), m);
@@ -1768,7 +1915,6 @@ static void run_lansvd_t(const char *jobu, const char *jobv, int m, int n, int *
     *info = 0;
     int neig = 0, jold = 0;
     int j = std::min(k + std::max(8, k) + 1, lanmax);
-    std::vector<double> hs(lanmax + 2), hb(lanmax + 2);
     while (neig < k) {
         {
             Timer t(c, g_last.lanczos_ms);
@@ -1803,11 +1949,8 @@ static void run_lansvd_t(const char *jobu, const char *jobv, int m, int n, int *
         j = std::min(j + dj, lanmax);
     }
     const int lim = std::min(j, k);
-    PGB_CUDA(cudaMemcpyAsync(hs.data(), c.sig_out, sizeof(double) * std::max(neig, 1), cudaMemcpyDeviceToHost, c.s));
-    PGB_CUDA(cudaMemcpyAsync(hb.data(), c.bnd_out, sizeof(double) * std::max(lim, 1), cudaMemcpyDeviceToHost, c.s));
-    c.sync();
-    for (int i = 0; i < neig; i++) sigma[i] = hs[i];
-    for (int i = 0; i < lim; i++) bnd[i] = hb[i];
+    for (int i = 0; i < neig; i++) sigma[i] = c.hsig[i];
+    for (int i = 0; i < lim; i++) bnd[i] = c.hsig[c.kmax + 2 + i];
     const bool du = yes(jobu), dv = yes(jobv);
     if ((neig >= k || *info > 0) && (du || dv)) {
         Timer t(c, g_last.gemm_ms);

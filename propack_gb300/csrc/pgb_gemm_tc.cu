@@ -949,8 +949,10 @@ __global__ void __launch_bounds__(WS_THREADS, 1) k_oz_umma_ws(int mr, int nc, in
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(UM_TMEM_COLS) : "memory");
 }
 
-// scratch for the digits of B (grown on demand, per host thread)
+// scratch for the digits of B (grown on demand, per host thread); `used` is
+// the last product's end: one on another stream waits for it
 struct OzScratch {
+    cudaEvent_t used = nullptr;
     unsigned short *bd = nullptr;
     int *fe = nullptr;
     int *err = nullptr;
@@ -963,8 +965,10 @@ struct OzScratch {
         if (fe) cudaFree(fe);
         if (err) cudaFree(err);
         if (herr) cudaFreeHost(herr);
+        if (used) cudaEventDestroy(used);
     }
 };
+static thread_local OzScratch t_oz;
 
 // need: digit elements of B; nfe: column exponents
 static void oz_scratch(OzScratch &sc, size_t need, int nfe)
@@ -987,8 +991,20 @@ static void oz_scratch(OzScratch &sc, size_t need, int nfe)
     }
     if (!sc.err) {
         PGB_CUDA(cudaMalloc(&sc.err, sizeof(int)));
+        PGB_CUDA(cudaMemset(sc.err, 0, sizeof(int)));
         PGB_CUDA(cudaMallocHost(&sc.herr, sizeof(int)));
+        *sc.herr = 0;
+        PGB_CUDA(cudaEventCreateWithFlags(&sc.used, cudaEventDisableTiming));
     }
+}
+
+bool gemm_failed()
+{
+    if (!t_oz.herr || *t_oz.herr == 0) return false;
+    *t_oz.herr = 0;
+    cudaMemset(t_oz.err, 0, sizeof(int));
+    set_error("tensor-core GEMM: an mbarrier wait ran out");
+    return true;
 }
 
 // impl 0: mma.sync kernel; impl 1: tcgen05 kernel; impl 2: tcgen05,
@@ -996,18 +1012,18 @@ static void oz_scratch(OzScratch &sc, size_t need, int nfe)
 static void oz_gemm_launch(int impl, int mr, int nc, int kk, const double *A, int lda, const double *B, int ldb,
                            bool tb, double *C, int ldc, cudaStream_t s)
 {
-    static thread_local OzScratch sc;
+    OzScratch &sc = t_oz;
     if (impl == 1 || impl == 2) {
         const int ntc = (nc + UM_BN - 1) / UM_BN;
         const int nstage = (kk + UM_KC - 1) / UM_KC;
         oz_scratch(sc, (size_t)ntc * nstage * UM_BSTAGE / 2, ntc * UM_BN);
+        PGB_CUDA(cudaStreamWaitEvent(s, sc.used, 0));
         static thread_local int attr = -1;
         if (attr != 1) {
             PGB_CUDA(cudaFuncSetAttribute(k_oz_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, UM_SMEM));
             PGB_CUDA(cudaFuncSetAttribute(k_oz_umma_ws, cudaFuncAttributeMaxDynamicSharedMemorySize, UM_SMEM));
             attr = 1;
         }
-        PGB_CUDA(cudaMemsetAsync(sc.err, 0, sizeof(int), s));
         PGB_PROF(PK_GEMM, s, {
             k_oz_bimg<<<(ntc * UM_BN + 127) / 128, 128, 0, s>>>(kk, nc, B, ldb, tb ? 1 : 0, ntc, nstage, sc.bd, sc.fe);
             PGB_LAUNCHED();
@@ -1020,17 +1036,16 @@ static void oz_gemm_launch(int impl, int mr, int nc, int kk, const double *A, in
                 k_oz_umma<<<grid, UM_THREADS, UM_SMEM, s>>>(mr, nc, kk, A, lda, sc.bd, sc.fe, nstage, C, ldc, sc.err);
             PGB_LAUNCHED();
         });
+        // read by gemm_failed after the caller's next wait (a wait here would
+        // leave the GPU idle between the products)
         PGB_CUDA(cudaMemcpyAsync(sc.herr, sc.err, sizeof(int), cudaMemcpyDeviceToHost, s));
-        PGB_CUDA(cudaStreamSynchronize(s));
-        if (*sc.herr) {
-            set_error("tensor-core GEMM: an mbarrier wait ran out");
-            throw WaitFailure();
-        }
+        PGB_CUDA(cudaEventRecord(sc.used, s));
         return;
     }
     const int Kp = (kk + 15) / 16 * 16;
     const int ncp = (nc + OZ_BN - 1) / OZ_BN * OZ_BN;
     oz_scratch(sc, (size_t)OZ_S * ncp * Kp, ncp);
+    PGB_CUDA(cudaStreamWaitEvent(s, sc.used, 0));
     const size_t smem = sizeof(unsigned short) * OZ_S * OZ_BN * (size_t)(Kp + 8);
     static thread_local size_t smem_set = 0;
     if (smem > 48 * 1024 && smem_set < smem) {
@@ -1044,6 +1059,7 @@ static void oz_gemm_launch(int impl, int mr, int nc, int kk, const double *A, in
         k_oz_gemm<<<grid, OZ_WARPS * 32, smem, s>>>(mr, nc, kk, A, lda, sc.bd, sc.fe, Kp, ncp, C, ldc);
         PGB_LAUNCHED();
     });
+    PGB_CUDA(cudaEventRecord(sc.used, s));
 }
 
 // the tcgen05 kernel of the library's restart and Ritz products
@@ -1082,6 +1098,7 @@ extern "C" int propack_gemm_f64_tc(int impl, int mr, int nc, int kk, const doubl
     try {
         oz_gemm_launch(impl, mr, nc, kk, A, lda, B, ldb, tb != 0, C, ldc, 0);
         PGB_CUDA(cudaStreamSynchronize(0));
+        if (gemm_failed()) throw WaitFailure();
     } catch (const CudaFailure &) {
         return PROPACK_ERR_CUDA;
     } catch (const WaitFailure &) {

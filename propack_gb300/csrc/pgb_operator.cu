@@ -1345,6 +1345,7 @@ extern "C" int propack_release_memory(void)
         PGB_CUDA(cudaDeviceSynchronize());
         PGB_CUDA(cudaMemPoolTrimTo(lib_pool(), 0));
         release_bounce_buffers();
+        release_host_kits();
     } catch (const CudaFailure &) {
         return PROPACK_ERR_CUDA;
     }
