@@ -831,30 +831,16 @@ __device__ __forceinline__ void dots_f32(const LbArgs &a, int j, int L, double *
         for (int u = 0; u < DOT_COLS; u++) Wq[u] = Wv + (size_t)ssel[cb + (u < nc ? u : 0)] * ldq;
         Acc<float> acc[DOT_COLS];
         int v = v0 + lane;
-        for (; v + 32 < v1; v += 64) {
-            float4 w0[DOT_COLS], w1[DOT_COLS];
+#pragma unroll 1
+        for (; v < v1; v += 32) {  // one vector of each column in flight: see dots_pl
+            float4 w0[DOT_COLS];
 #pragma unroll
-            for (int u = 0; u < DOT_COLS; u++) {
-                w0[u] = __ldcs(Wq[u] + v);
-                w1[u] = __ldcs(Wq[u] + v + 32);
-            }
-            const float4 x0 = xv[v], x1 = xv[v + 32];
+            for (int u = 0; u < DOT_COLS; u++) w0[u] = __ldcs(Wq[u] + v);
+            const float4 x0 = xv[v];
 #pragma unroll
             for (int u = 0; u < DOT_COLS; u++)
 #pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    acc[u].add_prod(Vec16<float>::get(w0[u], q), Vec16<float>::get(x0, q));
-                    acc[u].add_prod(Vec16<float>::get(w1[u], q), Vec16<float>::get(x1, q));
-                }
-        }
-        if (v < v1) {
-            const float4 x0 = xv[v];
-#pragma unroll
-            for (int u = 0; u < DOT_COLS; u++) {
-                const float4 w0 = __ldcs(Wq[u] + v);
-#pragma unroll
-                for (int q = 0; q < 4; q++) acc[u].add_prod(Vec16<float>::get(w0, q), Vec16<float>::get(x0, q));
-            }
+                for (int q = 0; q < 4; q++) acc[u].add_prod(Vec16<float>::get(w0[u], q), Vec16<float>::get(x0, q));
         }
         if (r0 < len) {
             const float xr = x[r0];
@@ -1162,31 +1148,23 @@ __device__ __forceinline__ void dots_pl(const LbArgs &a, int j, int L, double *w
             Wq[u] = reinterpret_cast<const float4 *>(Wp) + (size_t)ssel[cb + (u < nc ? u : 0)] * ldq;
         PlAcc acc[DOT_COLS];
         int v = v0 + lane;
-        // the planes stream through once (evict-first), so that the x
-        // planes, read again by every group, stay in L2
-        for (; v + 32 < v1; v += 64) {
-            float4 w0[DOT_COLS], w1[DOT_COLS];
+        // The planes stream through once (evict-first), so that the x
+        // planes, read again by every group, stay in L2.  One vector of each
+        // column in flight per lane: a second one lets the warps' streams
+        // thrash each other (1000003 x 250007, 120 columns: 141 us a pass
+        // with two, 106 with one; 4M rows, 75 columns: 548 and 506), and
+        // eight columns at a time or slices interleaved over the CTA's warps do
+        // the same (146 and 151; 626 and 606).
+#pragma unroll 1
+        for (; v < v1; v += 32) {
+            float4 w0[DOT_COLS];
 #pragma unroll
-            for (int u = 0; u < DOT_COLS; u++) {
-                w0[u] = __ldcs(Wq[u] + v);
-                w1[u] = __ldcs(Wq[u] + v + 32);
-            }
-            const float4 x0 = xq[v], x1 = xq[v + 32];
+            for (int u = 0; u < DOT_COLS; u++) w0[u] = __ldcs(Wq[u] + v);
+            const float4 x0 = xq[v];
 #pragma unroll
             for (int u = 0; u < DOT_COLS; u++) {
                 acc[u].add(w0[u].x, w0[u].y, x0.x, x0.y);
                 acc[u].add(w0[u].z, w0[u].w, x0.z, x0.w);
-                acc[u].add(w1[u].x, w1[u].y, x1.x, x1.y);
-                acc[u].add(w1[u].z, w1[u].w, x1.z, x1.w);
-            }
-        }
-        if (v < v1) {
-            const float4 x0 = xq[v];
-#pragma unroll
-            for (int u = 0; u < DOT_COLS; u++) {
-                const float4 w0 = __ldcs(Wq[u] + v);
-                acc[u].add(w0.x, w0.y, x0.x, x0.y);
-                acc[u].add(w0.z, w0.w, x0.z, x0.w);
             }
         }
         if (tail_row) {
