@@ -6,10 +6,12 @@ namespace pgb {
 // Gram-Schmidt arithmetic of the FP64 form (propack_set_cgs_arith)
 thread_local int g_cgs_arith = CGS_PLANES;
 
-// the planes are used when the driver allocated them (FP64 form, kmax small
-// enough for the projections' per-warp partials in shared memory; complex
-// vectors keep twice the partials)
-bool lb_planes_fit(int kmax, bool cplx) { return (cplx ? zpl_smem(kmax) : pl_smem(kmax)) <= PL_SMEM_MAX; }
+// the planes are used when the driver allocated them (FP64 form, kmax up to
+// some 2800; complex vectors 1500)
+bool lb_planes_fit(int kmax, bool cplx)
+{
+    return (size_t)((cplx ? 2 : 1) * sizeof(double) * PL_WARPS + 2 * sizeof(int)) * (kmax + 1) <= PL_SMEM_MAX;
+}
 
 // device words of the barrier, the published scalars
 size_t lb_run_scratch() { return 64 + sizeof(LbPub); }

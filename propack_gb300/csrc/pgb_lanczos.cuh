@@ -620,7 +620,7 @@ __device__ __forceinline__ LbPub publish(const LbCtl &c)
 // one; 2: either, by the matrix (Csr::short_rows).
 template <typename T, int SHORT>
 struct SpmvShared {
-    SpmvStage<T, T> st[SHORT == 1 ? 1 : SPMV_WARPS];
+    std::conditional_t<SHORT == 1, int, SpmvStage<T, T>[SPMV_WARPS]> st;
     ChunkStage<T> cst[SHORT == 0 ? 1 : SPMV_WARPS];
 };
 
@@ -665,9 +665,10 @@ __device__ __forceinline__ void spmv_phase(const LbArgs &a, int j, int host_prod
     auto pre = [&](int r) -> double { return has_prev ? (double)prev[r] : 0.0; };
     if (!host_product) {
         auto xl = [&](int c) -> T { return c < n0 ? x[c] : (T)z[c - n0]; };
-        if (SHORT == 1 || (SHORT == 2 && A.short_rows))
+        if (SHORT == 1 || A.short_rows)
             csr_rows_chunked<T, T>(A.ptr, A.tbase, A.cidx, chunk_vals<T>(A), A.rows, xl, pre, epi, sh.cst, tb0, tb1);
-        else csr_rows_staged<T, T>(A.ptr, A.idx, csr_vals<T>(A), A.blk, A.nblk, xl, pre, epi, sh.st);
+        else if constexpr (SHORT != 1)
+            csr_rows_staged<T, T>(A.ptr, A.idx, csr_vals<T>(A), A.blk, A.nblk, xl, pre, epi, sh.st);
     } else {
         for (int r = blockIdx.x * BS + threadIdx.x; r < A.rows; r += gridDim.x * BS) epi(r, (double)out[r], pre(r));
     }
@@ -730,6 +731,9 @@ struct Vec16<double> {
 // vector it loads serves four columns (ten 16-byte loads in flight per
 // lane).  The last CTA also takes the rows past the last whole vector.
 constexpr int DOT_COLS = 4;
+// columns whose per-slice partials lie in shared memory at a time: what a CTA
+// takes of it comes out of the L1 that holds the SpMV's gathers in flight
+constexpr int WPART_COLS = 64;
 template <int SIDE>
 __device__ __forceinline__ void dots_f64(const LbArgs &a, int j, int L)
 {
@@ -805,8 +809,7 @@ __device__ __forceinline__ int dot_slices(int chunk)
 template <int SIDE>
 __device__ __forceinline__ void dots_f32(const LbArgs &a, int j, int L, double *wpart)
 {
-    const int K1 = a.kmax + 1;
-    int *ssel = reinterpret_cast<int *>(wpart + (size_t)(BS / 32) * K1);
+    int *ssel = reinterpret_cast<int *>(wpart + BS / 32 * WPART_COLS);
     for (int c = threadIdx.x; c < L; c += BS) ssel[c] = a.sel[c];
     __syncthreads();
     const int len = SIDE == 0 ? a.adj.rows : a.fwd.rows;
@@ -824,44 +827,48 @@ __device__ __forceinline__ void dots_f32(const LbArgs &a, int j, int L, double *
     const int v0 = min(cb1, cb0 + ws * sl), v1 = min(cb1, v0 + sl);
     // the rows past the last whole vector: the last slice's warps of the last CTA
     const int r0 = blockIdx.x == gridDim.x - 1 && ws == rs - 1 ? nvec * 4 + lane : len;
-    for (int cb = wg * DOT_COLS; cb < L; cb += cgs * DOT_COLS) {
-        const int nc = min(DOT_COLS, L - cb);
-        const float4 *Wq[DOT_COLS];
+    for (int b0 = 0; b0 < L; b0 += WPART_COLS) {
+        const int b1 = min(L, b0 + WPART_COLS);
+        for (int cb = b0 + wg * DOT_COLS; cb < b1; cb += cgs * DOT_COLS) {
+            const int nc = min(DOT_COLS, b1 - cb);
+            const float4 *Wq[DOT_COLS];
 #pragma unroll
-        for (int u = 0; u < DOT_COLS; u++) Wq[u] = Wv + (size_t)ssel[cb + (u < nc ? u : 0)] * ldq;
-        Acc<float> acc[DOT_COLS];
-        int v = v0 + lane;
+            for (int u = 0; u < DOT_COLS; u++) Wq[u] = Wv + (size_t)ssel[cb + (u < nc ? u : 0)] * ldq;
+            Acc<float> acc[DOT_COLS];
+            int v = v0 + lane;
 #pragma unroll 1
-        for (; v < v1; v += 32) {  // one vector of each column in flight: see dots_pl
-            float4 w0[DOT_COLS];
+            for (; v < v1; v += 32) {  // one vector of each column in flight: see dots_pl
+                float4 w0[DOT_COLS];
 #pragma unroll
-            for (int u = 0; u < DOT_COLS; u++) w0[u] = __ldcs(Wq[u] + v);
-            const float4 x0 = xv[v];
+                for (int u = 0; u < DOT_COLS; u++) w0[u] = __ldcs(Wq[u] + v);
+                const float4 x0 = xv[v];
 #pragma unroll
-            for (int u = 0; u < DOT_COLS; u++)
+                for (int u = 0; u < DOT_COLS; u++)
 #pragma unroll
-                for (int q = 0; q < 4; q++) acc[u].add_prod(Vec16<float>::get(w0[u], q), Vec16<float>::get(x0, q));
+                    for (int q = 0; q < 4; q++) acc[u].add_prod(Vec16<float>::get(w0[u], q), Vec16<float>::get(x0, q));
+            }
+            if (r0 < len) {
+                const float xr = x[r0];
+#pragma unroll
+                for (int u = 0; u < DOT_COLS; u++)
+                    if (u < nc) acc[u].add_prod(W[(size_t)ssel[cb + u] * (4 * ldq) + r0], xr);
+            }
+            PlAcc p[DOT_COLS];
+#pragma unroll
+            for (int u = 0; u < DOT_COLS; u++) {
+                p[u].s = acc[u].s;
+                p[u].c = acc[u].c;
+            }
+            const PlAcc tot = pl_warp_sum4(p);
+            if ((lane & 7) == 0 && (lane >> 3) < nc) wpart[ws * WPART_COLS + cb - b0 + (lane >> 3)] = tot.value();
         }
-        if (r0 < len) {
-            const float xr = x[r0];
-#pragma unroll
-            for (int u = 0; u < DOT_COLS; u++)
-                if (u < nc) acc[u].add_prod(W[(size_t)ssel[cb + u] * (4 * ldq) + r0], xr);
+        __syncthreads();
+        for (int c = threadIdx.x; c < b1 - b0; c += BS) {
+            double sum = 0.0;
+            for (int ww = 0; ww < rs; ww++) sum += wpart[ww * WPART_COLS + c];
+            a.part_cols[(size_t)(b0 + c) * a.nb + blockIdx.x] = sum;
         }
-        PlAcc p[DOT_COLS];
-#pragma unroll
-        for (int u = 0; u < DOT_COLS; u++) {
-            p[u].s = acc[u].s;
-            p[u].c = acc[u].c;
-        }
-        const PlAcc tot = pl_warp_sum4(p);
-        if ((lane & 7) == 0 && (lane >> 3) < nc) wpart[(size_t)ws * K1 + cb + (lane >> 3)] = tot.value();
-    }
-    __syncthreads();
-    for (int c = threadIdx.x; c < L; c += BS) {
-        double sum = 0.0;
-        for (int ww = 0; ww < rs; ww++) sum += wpart[(size_t)ww * K1 + c];
-        a.part_cols[(size_t)c * a.nb + blockIdx.x] = sum;
+        __syncthreads();
     }
 }
 
@@ -1073,15 +1080,14 @@ __device__ __forceinline__ void upd_f3(const LbArgs &a, int j, int L, double *dy
 // per group), then added over the warps in a fixed order, then over the
 // CTAs by the last CTA.  The grid is one wave at the kernel's occupancy (<= nb CTAs).
 constexpr int PL_WARPS = BS / 32;
-constexpr size_t PL_SMEM_MAX = 200 * 1024;  // per-warp partials + selection of the projections
+constexpr size_t PL_SMEM_MAX = 200 * 1024;  // bounds the dimension of the plane form (lb_planes_fit)
 constexpr int PL_SPLIT_UNROLL = 4;          // FP64 loads in flight per lane when a column is split
 template <int SIDE>
 __device__ __forceinline__ void dots_pl(const LbArgs &a, int j, int L, double *wpart)
 {
-    // wpart: [PL_WARPS][kmax + 1] per-slice partial projections | sel[kmax + 1] | fresh[kmax + 1]
-    const int K1 = a.kmax + 1;
-    int *ssel = reinterpret_cast<int *>(wpart + (size_t)PL_WARPS * K1);
-    int *sfresh = ssel + K1;
+    // wpart: [PL_WARPS][WPART_COLS] per-slice partial projections | sel[kmax + 1] | fresh[kmax + 1]
+    int *ssel = reinterpret_cast<int *>(wpart + PL_WARPS * WPART_COLS);
+    int *sfresh = ssel + a.kmax + 1;
     int *ok = SIDE == 0 ? a.okV : a.okU;
     for (int c = threadIdx.x; c < L; c += BS) {
         const int col = a.sel[c];
@@ -1140,50 +1146,54 @@ __device__ __forceinline__ void dots_pl(const LbArgs &a, int j, int L, double *w
         for (; v < v1; v += 32) Wq[v] = pl_split2(Wd[v]);
         if (tail_row) Wp[(size_t)col * ld + len - 1] = pl_split(W[(size_t)col * ld + len - 1]);
     }
-    for (int cb = wg * DOT_COLS; cb < L; cb += cgs * DOT_COLS) {
-        const int nc = min(DOT_COLS, L - cb);
-        const float4 *Wq[DOT_COLS];
+    for (int b0 = 0; b0 < L; b0 += WPART_COLS) {
+        const int b1 = min(L, b0 + WPART_COLS);
+        for (int cb = b0 + wg * DOT_COLS; cb < b1; cb += cgs * DOT_COLS) {
+            const int nc = min(DOT_COLS, b1 - cb);
+            const float4 *Wq[DOT_COLS];
 #pragma unroll
-        for (int u = 0; u < DOT_COLS; u++)
-            Wq[u] = reinterpret_cast<const float4 *>(Wp) + (size_t)ssel[cb + (u < nc ? u : 0)] * ldq;
-        PlAcc acc[DOT_COLS];
-        int v = v0 + lane;
-        // The planes stream through once (evict-first), so that the x
-        // planes, read again by every group, stay in L2.  One vector of each
-        // column in flight per lane: a second one lets the warps' streams
-        // thrash each other (1000003 x 250007, 120 columns: 141 us a pass
-        // with two, 106 with one; 4M rows, 75 columns: 548 and 506), and
-        // eight columns at a time or slices interleaved over the CTA's warps do
-        // the same (146 and 151; 626 and 606).
+            for (int u = 0; u < DOT_COLS; u++)
+                Wq[u] = reinterpret_cast<const float4 *>(Wp) + (size_t)ssel[cb + (u < nc ? u : 0)] * ldq;
+            PlAcc acc[DOT_COLS];
+            int v = v0 + lane;
+            // The planes stream through once (evict-first), so that the x
+            // planes, read again by every group, stay in L2.  One vector of each
+            // column in flight per lane: a second one lets the warps' streams
+            // thrash each other (1000003 x 250007, 120 columns: 141 us a pass
+            // with two, 106 with one; 4M rows, 75 columns: 548 and 506), and
+            // eight columns at a time or slices interleaved over the CTA's warps do
+            // the same (146 and 151; 626 and 606).
 #pragma unroll 1
-        for (; v < v1; v += 32) {
-            float4 w0[DOT_COLS];
+            for (; v < v1; v += 32) {
+                float4 w0[DOT_COLS];
 #pragma unroll
-            for (int u = 0; u < DOT_COLS; u++) w0[u] = __ldcs(Wq[u] + v);
-            const float4 x0 = xq[v];
+                for (int u = 0; u < DOT_COLS; u++) w0[u] = __ldcs(Wq[u] + v);
+                const float4 x0 = xq[v];
 #pragma unroll
-            for (int u = 0; u < DOT_COLS; u++) {
-                acc[u].add(w0[u].x, w0[u].y, x0.x, x0.y);
-                acc[u].add(w0[u].z, w0[u].w, x0.z, x0.w);
+                for (int u = 0; u < DOT_COLS; u++) {
+                    acc[u].add(w0[u].x, w0[u].y, x0.x, x0.y);
+                    acc[u].add(w0[u].z, w0[u].w, x0.z, x0.w);
+                }
             }
-        }
-        if (tail_row) {
+            if (tail_row) {
 #pragma unroll
-            for (int u = 0; u < DOT_COLS; u++) {
-                if (u >= nc) break;
-                const float2 wr = Wp[(size_t)ssel[cb + u] * ld + len - 1];
-                acc[u].add(wr.x, wr.y, xr.x, xr.y);
+                for (int u = 0; u < DOT_COLS; u++) {
+                    if (u >= nc) break;
+                    const float2 wr = Wp[(size_t)ssel[cb + u] * ld + len - 1];
+                    acc[u].add(wr.x, wr.y, xr.x, xr.y);
+                }
             }
+            static_assert(DOT_COLS == 4, "pl_warp_sum4 sums four columns");
+            const PlAcc tot = pl_warp_sum4(acc);
+            if ((lane & 7) == 0 && (lane >> 3) < nc) wpart[ws * WPART_COLS + cb - b0 + (lane >> 3)] = tot.value() * back;
         }
-        static_assert(DOT_COLS == 4, "pl_warp_sum4 sums four columns");
-        const PlAcc tot = pl_warp_sum4(acc);
-        if ((lane & 7) == 0 && (lane >> 3) < nc) wpart[(size_t)ws * K1 + cb + (lane >> 3)] = tot.value() * back;
-    }
-    __syncthreads();
-    for (int c = threadIdx.x; c < L; c += BS) {
-        double s = 0.0;
-        for (int ww = 0; ww < rs; ww++) s += wpart[(size_t)ww * K1 + c];
-        a.part_cols[(size_t)c * a.nb + blockIdx.x] = s;
+        __syncthreads();
+        for (int c = threadIdx.x; c < b1 - b0; c += BS) {
+            double s = 0.0;
+            for (int ww = 0; ww < rs; ww++) s += wpart[ww * WPART_COLS + c];
+            a.part_cols[(size_t)(b0 + c) * a.nb + blockIdx.x] = s;
+        }
+        __syncthreads();
     }
 }
 
@@ -1486,10 +1496,9 @@ constexpr int ZPL_COLS = 2;
 template <int SIDE>
 __device__ __forceinline__ void zdots_pl(const LbArgs &a, int j, int L, double *wpart)
 {
-    // wpart: [PL_WARPS][2 (kmax + 1)] per-slice partials | sel[kmax + 1] | fresh[kmax + 1]
-    const int K1 = a.kmax + 1, K2 = 2 * K1;
-    int *ssel = reinterpret_cast<int *>(wpart + (size_t)PL_WARPS * K2);
-    int *sfresh = ssel + K1;
+    // wpart: [PL_WARPS][2 WPART_COLS] per-slice partials | sel[kmax + 1] | fresh[kmax + 1]
+    int *ssel = reinterpret_cast<int *>(wpart + PL_WARPS * 2 * WPART_COLS);
+    int *sfresh = ssel + a.kmax + 1;
     int *ok = SIDE == 0 ? a.okV : a.okU;
     for (int c = threadIdx.x; c < L; c += BS) {
         const int col = a.sel[c];
@@ -1547,43 +1556,47 @@ __device__ __forceinline__ void zdots_pl(const LbArgs &a, int j, int L, double *
         im.add(wv.x, wv.y, xq4.z, xq4.w);
         im.add(wv.z, wv.w, -xq4.x, -xq4.y);
     };
-    for (int cb = wg * ZPL_COLS; cb < L; cb += cgs * ZPL_COLS) {
-        const int nc = min(ZPL_COLS, L - cb);
-        const float4 *Wq[ZPL_COLS];
+    for (int b0 = 0; b0 < L; b0 += WPART_COLS) {
+        const int b1 = min(L, b0 + WPART_COLS);
+        for (int cb = b0 + wg * ZPL_COLS; cb < b1; cb += cgs * ZPL_COLS) {
+            const int nc = min(ZPL_COLS, b1 - cb);
+            const float4 *Wq[ZPL_COLS];
 #pragma unroll
-        for (int u = 0; u < ZPL_COLS; u++)
-            Wq[u] = reinterpret_cast<const float4 *>(Wp) + (size_t)ssel[cb + (u < nc ? u : 0)] * ldq;
-        PlAcc acc[2 * ZPL_COLS];  // re, im of column cb, then of column cb + 1
-        int v = v0 + lane;
-        for (; v + 32 < v1; v += 64) {
-            float4 w0[ZPL_COLS], w1[ZPL_COLS];
+            for (int u = 0; u < ZPL_COLS; u++)
+                Wq[u] = reinterpret_cast<const float4 *>(Wp) + (size_t)ssel[cb + (u < nc ? u : 0)] * ldq;
+            PlAcc acc[2 * ZPL_COLS];  // re, im of column cb, then of column cb + 1
+            int v = v0 + lane;
+            for (; v + 32 < v1; v += 64) {
+                float4 w0[ZPL_COLS], w1[ZPL_COLS];
 #pragma unroll
-            for (int u = 0; u < ZPL_COLS; u++) {
-                w0[u] = __ldcs(Wq[u] + v);
-                w1[u] = __ldcs(Wq[u] + v + 32);
+                for (int u = 0; u < ZPL_COLS; u++) {
+                    w0[u] = __ldcs(Wq[u] + v);
+                    w1[u] = __ldcs(Wq[u] + v + 32);
+                }
+                const float4 x0 = xq[v], x1 = xq[v + 32];
+#pragma unroll
+                for (int u = 0; u < ZPL_COLS; u++) {
+                    zacc(acc[2 * u], acc[2 * u + 1], w0[u], x0);
+                    zacc(acc[2 * u], acc[2 * u + 1], w1[u], x1);
+                }
             }
-            const float4 x0 = xq[v], x1 = xq[v + 32];
+            if (v < v1) {
+                const float4 x0 = xq[v];
 #pragma unroll
-            for (int u = 0; u < ZPL_COLS; u++) {
-                zacc(acc[2 * u], acc[2 * u + 1], w0[u], x0);
-                zacc(acc[2 * u], acc[2 * u + 1], w1[u], x1);
+                for (int u = 0; u < ZPL_COLS; u++) zacc(acc[2 * u], acc[2 * u + 1], __ldcs(Wq[u] + v), x0);
             }
+            static_assert(2 * ZPL_COLS == 4, "pl_warp_sum4 sums four accumulators");
+            const PlAcc tot = pl_warp_sum4(acc);
+            const int q = lane >> 3;  // accumulator q: column cb + q / 2, part q % 2
+            if ((lane & 7) == 0 && (q >> 1) < nc) wpart[(ws * WPART_COLS + cb - b0) * 2 + q] = tot.value() * back;
         }
-        if (v < v1) {
-            const float4 x0 = xq[v];
-#pragma unroll
-            for (int u = 0; u < ZPL_COLS; u++) zacc(acc[2 * u], acc[2 * u + 1], __ldcs(Wq[u] + v), x0);
+        __syncthreads();
+        for (int c = threadIdx.x; c < 2 * (b1 - b0); c += BS) {
+            double s = 0.0;
+            for (int ww = 0; ww < rs; ww++) s += wpart[ww * 2 * WPART_COLS + c];
+            a.part_cols[(size_t)(2 * b0 + c) * a.nb + blockIdx.x] = s;
         }
-        static_assert(2 * ZPL_COLS == 4, "pl_warp_sum4 sums four accumulators");
-        const PlAcc tot = pl_warp_sum4(acc);
-        const int q = lane >> 3;  // accumulator q: column cb + q / 2, part q % 2
-        if ((lane & 7) == 0 && (q >> 1) < nc) wpart[(size_t)ws * K2 + 2 * cb + q] = tot.value() * back;
-    }
-    __syncthreads();
-    for (int c = threadIdx.x; c < 2 * L; c += BS) {
-        double s = 0.0;
-        for (int ww = 0; ww < rs; ww++) s += wpart[(size_t)ww * K2 + c];
-        a.part_cols[(size_t)c * a.nb + blockIdx.x] = s;
+        __syncthreads();
     }
 }
 
@@ -1946,9 +1959,12 @@ __global__ void __launch_bounds__(BS, run_minb<T, SHORT>()) k_lb_run(const __gri
 }
 
 // ------------------------------------------------------------ host side
-inline size_t pl_smem(int kmax) { return (sizeof(double) * PL_WARPS + 2 * sizeof(int)) * (size_t)(kmax + 1); }
+inline size_t pl_smem(int kmax)
+{
+    return sizeof(double) * PL_WARPS * WPART_COLS + 2 * sizeof(int) * (size_t)(kmax + 1);
+}
 // the complex projections keep (re, im) partials per warp
-inline size_t zpl_smem(int kmax) { return (2 * sizeof(double) * PL_WARPS + 2 * sizeof(int)) * (size_t)(kmax + 1); }
+inline size_t zpl_smem(int kmax) { return pl_smem(kmax) + sizeof(double) * PL_WARPS * WPART_COLS; }
 // h (as two double slots per column at most) and the selection
 inline size_t upd_smem(int kmax) { return (2 * sizeof(double) + sizeof(int)) * (size_t)(kmax + 1) + 16; }
 

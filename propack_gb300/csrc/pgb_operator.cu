@@ -709,35 +709,48 @@ __device__ __forceinline__ const double *plain_vals<double>(const Csr &A) { retu
 template <>
 __device__ __forceinline__ const float *plain_vals<float>(const Csr &A) { return A.valf; }
 
-// y = A x (A = fwd or adj) with x already carrying z for the tail columns
-template <typename T>
-__global__ void __launch_bounds__(BS) k_spmv_plain(Csr A, const T *__restrict__ x, const double *__restrict__ z,
-                                                   T *__restrict__ y)
+// y = A x (A = fwd or adj) with x already carrying z for the tail columns.
+// SHORT: the chunked schedule, compiled by itself: the staged one's shared
+// memory would come out of the L1 that holds the gathers in flight.
+template <typename T, bool SHORT>
+__global__ void __launch_bounds__(BS, SHORT ? 4 : 1) k_spmv_plain(Csr A, const T *__restrict__ x,
+                                                                  const double *__restrict__ z, T *__restrict__ y)
 {
-    __shared__ SpmvStage<T, T> st[SPMV_WARPS];
-    __shared__ ChunkStage<T> cst[SPMV_WARPS];
     const int n0 = A.ncol0;
     auto xl = [&](int c) -> T { return c < n0 ? __ldg(x + c) : (T)z[c - n0]; };
     auto pre = [&](int r) -> double { return 0.0; };
     auto epi = [&](int r, double acc, double) { y[r] = (T)acc; };
-    csr_spmv<T, T>(A, plain_vals<T>(A), xl, pre, epi, st, cst);
+    if constexpr (SHORT) {
+        __shared__ ChunkStage<T> cst[SPMV_WARPS];
+        csr_rows_piped<T, T>(A.ptr, A.tbase, A.cidx, chunk_vals<T>(A), A.rows, xl, pre, epi, cst);
+    } else {
+        __shared__ SpmvStage<T, T> st[SPMV_WARPS];
+        csr_rows_staged<T, T>(A.ptr, A.idx, plain_vals<T>(A), A.blk, A.nblk, xl, pre, epi, st);
+    }
 }
 
 // one wave of CTAs at the kernel's occupancy
 // (cached per host thread for the current device; recomputed when the
 // thread moves to another device)
-template <typename T>
-static int spmv_plain_grid()
+template <typename T, bool SHORT>
+static void spmv_plain(const Csr &A, const T *x, const double *z, T *y, cudaStream_t s)
 {
     static thread_local int g = 0, dev = -1;
     const Dev &d = device_info();
     if (g == 0 || dev != d.device) {
         int per = 0;
-        PGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_spmv_plain<T>, BS, 0));
+        PGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_spmv_plain<T, SHORT>, BS, 0));
         g = std::max(1, per) * d.sms;
         dev = d.device;
     }
-    return g;
+    k_spmv_plain<T, SHORT><<<g, BS, 0, s>>>(A, x, z, y);
+    PGB_LAUNCHED();
+}
+template <typename T>
+static void spmv_plain(const Csr &A, const T *x, const double *z, T *y, cudaStream_t s)
+{
+    if (A.short_rows) spmv_plain<T, true>(A, x, z, y, s);
+    else spmv_plain<T, false>(A, x, z, y, s);
 }
 
 template <typename T>
@@ -753,8 +766,7 @@ void op_thin(const Operator &op, bool trans, const T *x, cudaStream_t s)
 // y = A x with a caller-supplied z (the low-rank coefficients); no scratch
 void op_spmv_plain_launch(const Csr &A, const double *x, const double *z, double *y, cudaStream_t s)
 {
-    k_spmv_plain<double><<<spmv_plain_grid<double>(), BS, 0, s>>>(A, x, z, y);
-    PGB_LAUNCHED();
+    spmv_plain<double>(A, x, z, y, s);
 }
 
 // ------------------------------------------------- schedule selection
@@ -830,8 +842,7 @@ void op_apply(const Operator &op, bool trans, const T *x, T *y, cudaStream_t s)
 {
     op_thin<T>(op, trans, x, s);
     const Csr &A = trans ? op.adj : op.fwd;
-    k_spmv_plain<T><<<spmv_plain_grid<T>(), BS, 0, s>>>(A, x, op.zbuf, y);
-    PGB_LAUNCHED();
+    spmv_plain<T>(A, x, op.zbuf, y, s);
 }
 // y = A x for one side of a native complex operator (chunked schedule,
 // complex accumulation)

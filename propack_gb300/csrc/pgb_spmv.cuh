@@ -21,12 +21,20 @@
 //   length of its longest row, which matters on a GPU whose FP64 pipe
 //   retires two lanes per clock.  A row that ends inside a run is summed
 //   by that lane alone, in CSR order; a row spread over several runs adds
-//   the runs' partial sums in lane order.
+//   the runs' partial sums in lane order, or, FP64 and where a row of the
+//   tile lies in more than CHUNK_SERIAL runs, pairwise over the lanes.
+//
+// Both schedules hold back on shared memory: it comes out of the L1, and each
+// gather in flight holds a line there.  (4M-row Zipf matrix, 7.7 entries a row,
+// 32-byte gathers at 266-280 G/s at best, 117 us: the plain product took 229 and
+// 215 us for A x and A'y with both schedules' stages in one kernel, 183 and 163
+// with the chunked one's alone, 159 and 146 with its loads pipelined.)
 //
 // Summation order depends only on the matrix, never on timing, so results
 // are bit-reproducible.
 #pragma once
 #include <climits>
+#include <type_traits>
 
 #include "pgb.cuh"
 
@@ -34,6 +42,7 @@ namespace pgb {
 
 constexpr int SPMV_WARPS = BS / 32;  // warps per CTA
 constexpr int CHUNK_UNROLL = 4;      // chunked schedule: (index, value) pairs and gathers in flight per lane
+constexpr int CHUNK_SERIAL = 3;      // chunked schedule: most runs of a row added by its lane alone
 constexpr int CHUNK_TILE_COST = 4;   // chunked schedule: fixed cost of a tile, in units of 32 entries
 
 // One warp's shared-memory stage of the staged schedule: the block's
@@ -172,6 +181,17 @@ __device__ __forceinline__ double2 spmv_mac(double2 v, double2 x, double2 acc)
 __device__ __forceinline__ float spmv_add(float a, float b) { return a + b; }
 __device__ __forceinline__ double spmv_add(double a, double b) { return a + b; }
 __device__ __forceinline__ double2 spmv_add(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+
+__device__ __forceinline__ float spmv_shfl_down(float a, int o) { return __shfl_down_sync(0xffffffffu, a, o); }
+__device__ __forceinline__ double spmv_shfl_down(double a, int o) { return __shfl_down_sync(0xffffffffu, a, o); }
+__device__ __forceinline__ double2 spmv_shfl_down(double2 a, int o)
+{
+    return make_double2(spmv_shfl_down(a.x, o), spmv_shfl_down(a.y, o));
+}
+
+// FP32 sums stay in lane order: an FP32 addition by one lane costs little
+template <typename AT>
+__host__ __device__ constexpr bool chunk_pairwise() { return !std::is_same<AT, float>::value; }
 
 template <typename AT>
 struct ChunkStage {
@@ -313,19 +333,172 @@ __device__ __forceinline__ void csr_rows_chunked(const int *__restrict__ ptr, co
 #pragma unroll
             for (int u = 0; u < UNROLL; u++) step(v[u], xv[u]);
         }
+        // two at a time: one by one, the rest of a tile costs two dependent
+        // round trips an entry (4M-row Zipf matrix, run kernel: 218 -> 211 us)
+        for (; i + 1 < C; i += 2) {
+            const int c0 = ci[32 * i], c1 = ci[32 * i + 32];
+            const VT v0 = cv[32 * i], v1 = cv[32 * i + 32];
+            const AT x0 = (AT)xload(c0), x1 = (AT)xload(c1);
+            step(v0, x0);
+            step(v1, x1);
+        }
         for (; i < C; i++) step(cv[32 * i], (AT)xload(ci[32 * i]));
+        // row `lane`: its runs ls .. le, in lane order: the tails of the runs
+        // it is left open by, then its entries in the run where it ends
+        const int ls = lo / C, le = lo < hi ? (hi - 1) / C : ls;
+        const int span = (int)__reduce_max_sync(0xffffffffu, (unsigned)(le - ls));
+        const bool pairwise = chunk_pairwise<AT>() && span > CHUNK_SERIAL;
+        if (pairwise) {
+            // a row over many runs: the tails of each row are added pairwise
+            // over the lanes (a serial sum by the row's lane costs the FP64
+            // pipe a full warp instruction per run: complex 1M-row Zipf
+            // matrix, A v 153 -> 139 us, real 4M rows 226 -> 218)
+            for (int o = 1; o < span; o <<= 1) {
+                const AT a2 = spmv_shfl_down(acc, o);
+                const int q2 = __shfl_down_sync(0xffffffffu, q, o);
+                if (lane + o < 32 && q2 == q) acc = spmv_add(acc, a2);
+            }
+        }
         cs.tail[lane] = acc;
         __syncwarp();
-        // row `lane`: its runs ls .. le, added in lane order
         AT tot = spmv_zero<AT>();
         if (lo < hi) {
-            const int ls = lo / C, le = (hi - 1) / C;
-            if (ls == le) {
-                tot = cs.part[lane];
-            } else {
-                tot = cs.tail[ls];
-                for (int l2 = ls + 1; l2 < le; l2++) tot = spmv_add(tot, cs.tail[l2]);
-                tot = spmv_add(tot, cs.part[lane]);
+            tot = cs.part[lane];
+            if (ls != le) {
+                AT t = cs.tail[ls];
+                if (!pairwise)
+                    for (int l2 = ls + 1; l2 < le; l2++) t = spmv_add(t, cs.tail[l2]);
+                tot = spmv_add(t, tot);
+            }
+        }
+        if (r < nrows) epi(r, tot, pre);
+        __syncwarp();
+    }
+}
+
+// The same rows and sums for a kernel whose epilogue leaves it the registers.
+// The entries of a warp's tiles follow each other in memory, so it walks them
+// in groups of up to UNROLL units (a group ends with its tile): while a
+// group's gathers are under way the (index, value) pairs of the next one are
+// loaded, whichever tile it belongs to.  The product is bound by the latency
+// of those two dependent loads (counters, unpipelined: FP64 pipe and LSU 50 %
+// busy, DRAM 27 %, 63 % of the stalls on a load).  In the Lanczos run kernel
+// the registers of the next group spill and the product gets slower
+// (191 and 211 us become 266 and 306).
+// tb0 < 0: the warp's tiles are found here (chunk_warp_tiles)
+template <typename VT, typename AT, int UNROLL = CHUNK_UNROLL, typename XF, typename PF, typename EPI>
+__device__ __forceinline__ void csr_rows_piped(const int *__restrict__ ptr, const int *__restrict__ tbase,
+                                                 const int *__restrict__ cidx, const VT *__restrict__ cval,
+                                                 int nrows, XF xload, PF pre_load, EPI epi, ChunkStage<AT> *stages,
+                                                 int tb0 = -1, int tb1 = -1)
+{
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    ChunkStage<AT> &cs = stages[threadIdx.x >> 5];
+    if (tb0 < 0) chunk_warp_tiles(tbase, nrows, tb0, tb1);
+    if (tb0 >= tb1) return;
+    // a tile's bounds: lane l's row start (rows past the end are empty) and
+    // lane 31 also the tile's end; those of the next tile are loaded while
+    // the current one runs, its units' bounds one tile earlier still
+    int lo_c = 0, end_c = 0;
+    auto fetch = [&](int tile, int &lo_raw, int &end31) {
+        const int rr = tile * 32 + lane;
+        lo_raw = ptr[min(rr, nrows)];
+        end31 = lane == 31 ? ptr[min(rr + 1, nrows)] : 0;
+    };
+    fetch(tb0, lo_c, end_c);
+    int u0 = tbase[tb0], u1 = tbase[tb0 + 1], u2 = tb0 + 1 < tb1 ? tbase[tb0 + 2] : u1;
+    int c[UNROLL];
+    VT v[UNROLL];
+    auto load = [&](int unit, int cnt) {
+        const int *ci = cidx + (size_t)unit * 32 + lane;
+        const VT *cv = cval + (size_t)unit * 32 + lane;
+#pragma unroll
+        for (int u = 0; u < UNROLL; u++)
+            if (u < cnt) { c[u] = ci[32 * u]; v[u] = cv[32 * u]; }
+    };
+    load(u0, min(UNROLL, u1 - u0));
+    for (int tile = tb0; tile < tb1; tile++) {
+        const int r = tile * 32 + lane;
+        int lo_n = 0, end_n = 0, u3 = u2;
+        if (tile + 1 < tb1) fetch(tile + 1, lo_n, end_n);
+        if (tile + 2 < tb1) u3 = tbase[tile + 3];
+        const int eb = __shfl_sync(FULL, lo_c, 0);
+        const int hi_raw = __shfl_down_sync(FULL, lo_c, 1);
+        const int lo = lo_c - eb;
+        const int hi = (lane == 31 ? end_c : hi_raw) - eb;
+        const int C = u1 - u0;  // C >= 1
+        lo_c = lo_n;
+        end_c = end_n;
+        using PT = decltype(pre_load(0));
+        const PT pre = r < nrows ? pre_load(r) : PT{};
+        cs.bnd[lane] = lo;
+        if (lane == 31) cs.bnd[32] = hi;
+        cs.part[lane] = spmv_zero<AT>();
+        __syncwarp();
+        // the row holding the run's first entry p0: the last q with
+        // bnd[q] <= p0 (a non-empty row), or 32 when p0 is past the entries
+        const int p0 = lane * C;
+        int q = 0;
+#pragma unroll
+        for (int st = 16; st > 0; st >>= 1)
+            if (cs.bnd[q + st] <= p0) q += st;
+        if (cs.bnd[32] <= p0) q = 32;
+        int nend = q < 32 ? cs.bnd[q + 1] : INT_MAX;
+        int p = p0;
+        AT acc = spmv_zero<AT>();
+        // one entry of the run; closes row q when it ends at this entry
+        auto step = [&](VT vv, AT xv) {
+            acc = spmv_mac((AT)vv, xv, acc);
+            if (++p == nend) {
+                cs.part[q] = acc;
+                acc = spmv_zero<AT>();
+                do { ++q; } while (q < 32 && cs.bnd[q + 1] == p);
+                nend = q < 32 ? cs.bnd[q + 1] : INT_MAX;
+            }
+        };
+        for (int i = 0; i < C; i += UNROLL) {
+            const int cnt = min(UNROLL, C - i);
+            AT xv[UNROLL];
+            VT vc[UNROLL];
+#pragma unroll
+            for (int u = 0; u < UNROLL; u++) {
+                vc[u] = v[u];
+                if (u < cnt) xv[u] = (AT)xload(c[u]);
+            }
+            load(u0 + i + cnt, min(UNROLL, i + UNROLL < C ? C - i - UNROLL : u2 - u1));
+#pragma unroll
+            for (int u = 0; u < UNROLL; u++)
+                if (u < cnt) step(vc[u], xv[u]);
+        }
+        u0 = u1;
+        u1 = u2;
+        u2 = u3;
+        // row `lane`: its runs ls .. le, in lane order: the tails of the runs
+        // it is left open by, then its entries in the run where it ends
+        const int ls = lo / C, le = lo < hi ? (hi - 1) / C : ls;
+        const int span = (int)__reduce_max_sync(FULL, (unsigned)(le - ls));
+        const bool pairwise = chunk_pairwise<AT>() && span > CHUNK_SERIAL;
+        if (pairwise) {
+            // a row over many runs: the tails of each row are added pairwise
+            // over the lanes (a serial sum by the row's lane costs the FP64
+            // pipe a full warp instruction per run)
+            for (int o = 1; o < span; o <<= 1) {
+                const AT a2 = spmv_shfl_down(acc, o);
+                const int q2 = __shfl_down_sync(FULL, q, o);
+                if (lane + o < 32 && q2 == q) acc = spmv_add(acc, a2);
+            }
+        }
+        cs.tail[lane] = acc;
+        __syncwarp();
+        AT tot = spmv_zero<AT>();
+        if (lo < hi) {
+            tot = cs.part[lane];
+            if (ls != le) {
+                AT t = cs.tail[ls];
+                if (!pairwise)
+                    for (int l2 = ls + 1; l2 < le; l2++) t = spmv_add(t, cs.tail[l2]);
+                tot = spmv_add(t, tot);
             }
         }
         if (r < nrows) epi(r, tot, pre);
@@ -381,16 +554,6 @@ __device__ __forceinline__ void thin_phase(const Csr &Th, const T *x, const doub
             }
         }
     }
-}
-
-// the schedule chosen for the matrix
-template <typename VT, typename AT, typename XF, typename PF, typename EPI>
-__device__ __forceinline__ void csr_spmv(const Csr &A, const VT *__restrict__ val, XF xload, PF pre_load, EPI epi,
-                                         SpmvStage<VT, AT> *stages, ChunkStage<AT> *cstages)
-{
-    if (A.short_rows)
-        csr_rows_chunked<VT, AT>(A.ptr, A.tbase, A.cidx, chunk_vals<VT>(A), A.rows, xload, pre_load, epi, cstages);
-    else csr_rows_staged<VT, AT>(A.ptr, A.idx, val, A.blk, A.nblk, xload, pre_load, epi, stages);
 }
 
 }  // namespace pgb

@@ -1,0 +1,72 @@
+"""The chunked sparse product at the edges of its tiles: units past a multiple
+of the unrolling, rows over many runs, empty rows and tiles, a last partial
+tile, tiles shorter than a group; A x and A'y, real and complex, alone and
+inside a solve.
+
+Tolerance: a sum of k products in any order is off by at most
+(k + 2) eps sum |a x| (complex: 4 (k + 2) eps).
+"""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+import propack_gb300 as pg
+
+pytestmark = pytest.mark.gpu
+
+EPS = 2.0 ** -53
+
+
+def _rows(kind, m, rng):
+    if kind.startswith("const"):
+        return np.full(m, int(kind[5:]))
+    if kind == "empty":
+        return np.where(rng.random(m) < 0.7, 0, rng.integers(1, 9, m))
+    if kind == "tiles":  # every third tile empty
+        return np.where((np.arange(m) // 32) % 3 == 0, 0, rng.integers(1, 6, m))
+    if kind == "long":   # a few rows over all runs of their tile
+        cnt = rng.integers(0, 4, m)
+        cnt[rng.integers(0, m, 1 + m // 40)] = rng.integers(50, 900, 1 + m // 40)
+        return cnt
+    return np.minimum(1 + (0.6 / rng.random(m)).astype(int), 1500)  # Zipf
+
+
+def _matrix(kind, m, n, cplx, seed):
+    rng = np.random.default_rng(seed)
+    cnt = _rows(kind, m, rng)
+    nnz = int(cnt.sum())
+    val = rng.standard_normal(nnz) + (1j * rng.standard_normal(nnz) if cplx else 0.0)
+    ptr = np.concatenate([[0], np.cumsum(cnt)])
+    return sp.csr_array((val, rng.integers(0, n, nnz).astype(np.int32), ptr), shape=(m, n)), rng
+
+
+def _vec(n, cplx, rng):
+    return rng.standard_normal(n) + (1j * rng.standard_normal(n) if cplx else 0.0)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("m", [1, 31, 33, 4097])
+@pytest.mark.parametrize("kind", ["const1", "const2", "const3", "const5", "const7", "const9", "empty", "tiles", "long",
+                                  "zipf"])
+def test_products(kind, m, cplx):
+    n = 700
+    A, rng = _matrix(kind, m, n, cplx, 7 * m + len(kind))
+    op = pg.CsrOperator(A)
+    # (abs(A) would add repeated entries first; the bound is on all of them)
+    B = sp.csr_array((abs(A.data), A.indices.copy(), A.indptr.copy()), shape=A.shape)
+    for y, x, M, P in ((op.matvec, _vec(n, cplx, rng), A, B), (op.rmatvec, _vec(m, cplx, rng), A.conj().T, B.T)):
+        k = (np.diff(A.indptr) if P is B else np.bincount(A.indices, minlength=n)).max(initial=0)
+        lim = (4 if cplx else 1) * (k + 2) * EPS * (P @ abs(x))
+        # (the reference sum has the same bound)
+        assert np.all(abs(np.asarray(y(x)) - M @ x) <= 2 * lim)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("kind", ["const3", "empty", "long", "zipf"])
+def test_solve(kind, cplx):
+    A, _ = _matrix(kind, 3000, 2500, cplx, 5)
+    u, s, vt, _ = pg.svdp(pg.CsrOperator(A), 4, kmax=40, tol=1e-12, delta=0.0, rng=np.random.default_rng(0))
+    lim = (1e-12 + 64 * 3000 * 2 * EPS) * s[0]
+    v = vt.conj().T
+    assert np.max(np.linalg.norm(A @ v - u * s, axis=0)) <= lim
+    assert np.max(np.linalg.norm(A.conj().T @ u - v * s, axis=0)) <= lim
