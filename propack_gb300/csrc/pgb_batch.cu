@@ -965,7 +965,10 @@ __global__ void __launch_bounds__(BT, 2) k_batch_cycle(BProb *probs, const int *
 // columns on both sides, with the candidate row split g and projection tile
 // dc.  The operands are the problem's own basis arrays and planes, zeroed
 // beforehand: U(:,0) -> V(:,0) -> U(:,1), and column ncols of each side
-// against the ncols before it.
+// against the ncols before it.  Of a long side the first PROBE_ROWS rows stand
+// for all (a class is timed by its costliest problem: with all rows the tuning
+// of 192 problems of up to 40000 rows took 370 ms, five times their solve).
+constexpr int PROBE_ROWS = 2048;
 template <bool PL>
 __global__ void __launch_bounds__(BT) k_batch_probe(const BProb *probs, const int *sample, int ns, int g, int dc,
                                                     int ncols)
@@ -974,18 +977,19 @@ __global__ void __launch_bounds__(BT) k_batch_probe(const BProb *probs, const in
     cl_init(S);
     for (int q = blockIdx.x; q < ns; q += gridDim.x) {
         const BProb &P = probs[sample[q]];
+        const int m = min(P.m, PROBE_ROWS), n = min(P.n, PROBE_ROWS);
         if (PL) {
-            cta_spmv_pl(P.tptr, P.tidx, P.tval, P.n, P.Up, P.V, g, S);
-            cta_spmv_pl(P.ptr, P.idx, P.val, P.m, P.Vp, P.U + P.m, g, S);
-            cta_proj_pl_dc(P.Up, P.m, ncols, P.Up + (size_t)ncols * P.m, P.m, 1.0, S, dc);
+            cta_spmv_pl(P.tptr, P.tidx, P.tval, n, P.Up, P.V, g, S);
+            cta_spmv_pl(P.ptr, P.idx, P.val, m, P.Vp, P.U + P.m, g, S);
+            cta_proj_pl_dc(P.Up, P.m, ncols, P.Up + (size_t)ncols * P.m, m, 1.0, S, dc);
             __syncthreads();
-            cta_proj_pl_dc(P.Vp, P.n, ncols, P.Vp + (size_t)ncols * P.n, P.n, 1.0, S, dc);
+            cta_proj_pl_dc(P.Vp, P.n, ncols, P.Vp + (size_t)ncols * P.n, n, 1.0, S, dc);
         } else {
-            cta_spmv(P.tptr, P.tidx, P.tval, P.n, P.U, P.V, g, S);
-            cta_spmv(P.ptr, P.idx, P.val, P.m, P.V, P.U + P.m, g, S);
-            cta_proj_dc(P.U, P.m, ncols, P.U + (size_t)ncols * P.m, P.m, S, dc);
+            cta_spmv(P.tptr, P.tidx, P.tval, n, P.U, P.V, g, S);
+            cta_spmv(P.ptr, P.idx, P.val, m, P.V, P.U + P.m, g, S);
+            cta_proj_dc(P.U, P.m, ncols, P.U + (size_t)ncols * P.m, m, S, dc);
             __syncthreads();
-            cta_proj_dc(P.V, P.n, ncols, P.V + (size_t)ncols * P.n, P.n, S, dc);
+            cta_proj_dc(P.V, P.n, ncols, P.V + (size_t)ncols * P.n, n, S, dc);
         }
         __syncthreads();
     }
@@ -1124,15 +1128,15 @@ static int batch_cluster(const Batch &B)
     return cs;
 }
 
-// Time every candidate (row split g, projection tile dc) on a sample of each
+// Time the candidates (row split g, projection tile dc) on a sample of each
 // size class and keep the fastest; the defaults (1, 1) stay unless a
 // candidate is more than 3 % faster, so that near-ties do not flip the
 // choice (and with it the SpMV's summation order) between batches.
 template <bool PL>
 static void batch_tune(Batch *B, BProb *dprob, int grid, int dim, cudaStream_t s)
 {
-    static const int gs[] = {1, 4, 8, 32};
-    static const int dcs[] = {1, 2, 4};
+    static const int gs[] = {4, 8, 32};
+    static const int dcs[] = {2, 4};
     const int np = B->nprob, ncols = std::max(1, dim / 2);
     int *dsample = nullptr;
     PGB_CUDA(cudaMalloc(&dsample, sizeof(int) * std::max(1, np)));
@@ -1150,27 +1154,32 @@ static void batch_tune(Batch *B, BProb *dprob, int grid, int dim, cudaStream_t s
         for (int q = 0; q < ns; q++) sample[q] = B->order[p0 + (int)((int64_t)q * (p1 - p0) / ns)];
         PGB_CUDA(cudaMemcpyAsync(dsample, sample.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, s));
         float best = 0.f, def = 0.f;
-        for (int g : gs)
-            for (int dc : dcs) {
+        // the split changes the products alone and the tile the projections
+        // alone: first the splits with the default tile, then the tiles
+        auto time_of = [&](int g, int dc) {
+            k_batch_probe<PL><<<ns, BT, 0, s>>>(dprob, dsample, ns, g, dc, ncols);
+            PGB_LAUNCHED();
+            PGB_CUDA(cudaEventRecord(e0, s));
+            for (int r = 0; r < 2; r++) {
                 k_batch_probe<PL><<<ns, BT, 0, s>>>(dprob, dsample, ns, g, dc, ncols);
                 PGB_LAUNCHED();
-                PGB_CUDA(cudaEventRecord(e0, s));
-                for (int r = 0; r < 2; r++) {
-                    k_batch_probe<PL><<<ns, BT, 0, s>>>(dprob, dsample, ns, g, dc, ncols);
-                    PGB_LAUNCHED();
-                }
-                PGB_CUDA(cudaEventRecord(e1, s));
-                PGB_CUDA(cudaEventSynchronize(e1));
-                float ms = 0.f;
-                PGB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-                ms *= 0.5f;
-                if (g == 1 && dc == 1) def = ms;
-                if (best == 0.f || ms < best) {
-                    best = ms;
-                    B->g[c] = g;
-                    B->dc[c] = dc;
-                }
             }
+            PGB_CUDA(cudaEventRecord(e1, s));
+            PGB_CUDA(cudaEventSynchronize(e1));
+            float ms = 0.f;
+            PGB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
+            ms *= 0.5f;
+            if (best == 0.f || ms < best) {
+                best = ms;
+                B->g[c] = g;
+                B->dc[c] = dc;
+            }
+            return ms;
+        };
+        def = time_of(1, 1);
+        for (int g : gs) time_of(g, 1);
+        const int gb = B->g[c];
+        for (int dc : dcs) time_of(gb, dc);
         if (!(best < 0.97f * def)) {
             B->g[c] = 1;
             B->dc[c] = 1;
