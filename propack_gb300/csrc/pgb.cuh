@@ -491,7 +491,9 @@ cudaMemPool_t lib_pool();
 void release_host_kits();       // idle streams, events and pinned words of the drivers
 void release_bounce_buffers();  // the idle pinned bounce buffers of pageable result copies
 // host -> device copy on s; pageable sources go through the bounce buffers
-void h2d_bytes(void *dst, const void *src, size_t bytes, cudaStream_t s);
+// pieces: at least so many (of 4 MB and more), so that the first copies to the
+// device start early; the host's side of one piece costs some 50 us
+void h2d_bytes(void *dst, const void *src, size_t bytes, cudaStream_t s, int pieces = 1);
 // device -> host copy on s, the same way; pageable destinations are complete on return
 void d2h_bytes(void *dst, const void *src, size_t bytes, cudaStream_t s);
 void *pool_alloc(size_t bytes, cudaStream_t s);  // zero bytes allowed; never returns null

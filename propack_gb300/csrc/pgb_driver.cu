@@ -1253,7 +1253,7 @@ void d2h_bytes(void *dst, const void *src, size_t bytes, cudaStream_t s)
 // copied into a half by the host pool while the other half's copy to the
 // device runs.  Returns when the buffer is free again (its last copies
 // done); the device copies are ordered on s.
-void h2d_bytes(void *dst, const void *src, size_t bytes, cudaStream_t s)
+void h2d_bytes(void *dst, const void *src, size_t bytes, cudaStream_t s, int pieces)
 {
     if (bytes == 0) return;
     if (bytes < ((size_t)4 << 20) || host_pinned(src)) {
@@ -1263,15 +1263,13 @@ void h2d_bytes(void *dst, const void *src, size_t bytes, cudaStream_t s)
     BounceLease lease;
     Bounce &b = lease.b;
     HostPool &pool = HostPool::get();
-    // eight pieces at least (of 4 MB and more), so that the first copies to
-    // the device start early
-    const size_t piece = std::min(BOUNCE_BYTES, std::max((size_t)4 << 20, (bytes / 8 + 4095) / 4096 * 4096));
+    const size_t piece = std::min(BOUNCE_BYTES, std::max((size_t)4 << 20, (bytes / pieces + 4095) / 4096 * 4096));
     const size_t np = (bytes + piece - 1) / piece;
     for (size_t i = 0; i < np; i++) {
         const size_t off = i * piece, len = std::min(piece, bytes - off);
         char *half = b.buf + (i & 1) * BOUNCE_BYTES;
         if (i >= 2) PGB_CUDA(cudaEventSynchronize(b.ev[i & 1]));  // piece i-2 has left this half
-        const int parts = (int)std::min<size_t>((size_t)pool.threads() * 2, std::max<size_t>(1, len >> 20));
+        const int parts = (int)std::min<size_t>((size_t)pool.threads() * 2, std::max<size_t>(1, len >> 18));
         const size_t step = (len + parts - 1) / parts;
         const char *from = (const char *)src + off;
         pool.run(parts, [&](int q) {

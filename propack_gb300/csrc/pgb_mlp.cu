@@ -992,7 +992,7 @@ static void mlp_backward(Mlp &M, int m, int k)
 // features and the forward pass run; M.s waits for it
 static void mlp_upload(Mlp &M, const double *U, int ldu, int m, int k)
 {
-    if (ldu == m) h2d_bytes(M.U, U, sizeof(double) * (size_t)m * k, M.s2);
+    if (ldu == m) h2d_bytes(M.U, U, sizeof(double) * (size_t)m * k, M.s2, 8);
     else
         PGB_CUDA(cudaMemcpy2DAsync(M.U, sizeof(double) * m, U, sizeof(double) * ldu, sizeof(double) * m, k,
                                    cudaMemcpyHostToDevice, M.s2));
