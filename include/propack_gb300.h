@@ -356,7 +356,8 @@ int propack_mlp_set_impl(int impl);
  * nprob independent CSR matrices with FP32 values, solved by dlansvd_irl
  * (double/dlansvd_irl.F) with full reorthogonalisation (iterated classical
  * Gram-Schmidt on every step), FP64 vectors, p = dim - neig exact shifts,
- * one persistent kernel (a CTA per problem, work queue by decreasing size)
+ * one persistent kernel (a cluster of 1 to 8 CTAs per problem, work queue by
+ * decreasing size)
  * whose restart cycles are replayed as a CUDA graph.
  * Problem p: m[p] x n[p]; its m[p]+1 row pointers (0-based, its own
  * nonzeros) follow those of problem p-1 in `rowptr`; its column indices

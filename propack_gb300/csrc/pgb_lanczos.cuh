@@ -1078,7 +1078,7 @@ __device__ __forceinline__ void upd_f3(const LbArgs &a, int j, int L, double *dy
 // Each lane reads back only the vectors it wrote itself.  A group's sums
 // are reduced over the warp as compensated FP32 pairs (no FP64 operation
 // per group), then added over the warps in a fixed order, then over the
-// CTAs by the last CTA.  The grid is one wave at the kernel's occupancy (<= nb CTAs).
+// CTAs by CTA 0 or the grid (reduce_cols).  The grid is one wave at the kernel's occupancy (<= nb CTAs).
 constexpr int PL_WARPS = BS / 32;
 constexpr size_t PL_SMEM_MAX = 200 * 1024;  // bounds the dimension of the plane form (lb_planes_fit)
 constexpr int PL_SPLIT_UNROLL = 4;          // FP64 loads in flight per lane when a column is split
