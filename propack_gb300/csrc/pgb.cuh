@@ -481,6 +481,9 @@ struct Dev {
     int nb = 0;            // CTAs for the streaming kernels
 };
 const Dev &device_info();
+// lets fn take all the dynamic shared memory a CTA can have: the same value
+// from every thread, so that no call lowers the limit under another's launch
+void allow_dynamic_smem(const void *fn);
 
 // The library's own stream-ordered device memory pool (one per device).  It
 // keeps memory that is freed for the next allocation instead of returning

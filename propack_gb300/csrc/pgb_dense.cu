@@ -846,7 +846,7 @@ static int smem_for(const void *fn, size_t bytes)
         cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     }
     if (bytes + 1024 > (size_t)max_optin) return 0;
-    if (bytes > 48 * 1024) PGB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    if (bytes > 48 * 1024) allow_dynamic_smem(fn);
     return 1;
 }
 void launch_analyse_qr(const AnaArgs &a, cudaStream_t s)

@@ -1047,11 +1047,7 @@ static void oz_gemm_launch(int impl, int mr, int nc, int kk, const double *A, in
     oz_scratch(sc, (size_t)OZ_S * ncp * Kp, ncp);
     PGB_CUDA(cudaStreamWaitEvent(s, sc.used, 0));
     const size_t smem = sizeof(unsigned short) * OZ_S * OZ_BN * (size_t)(Kp + 8);
-    static thread_local size_t smem_set = 0;
-    if (smem > 48 * 1024 && smem_set < smem) {
-        PGB_CUDA(cudaFuncSetAttribute(k_oz_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        smem_set = smem;
-    }
+    if (smem > 48 * 1024) allow_dynamic_smem((const void *)k_oz_gemm);
     PGB_PROF(PK_GEMM, s, {
         k_oz_bdigits<<<(ncp + 127) / 128, 128, 0, s>>>(kk, nc, B, ldb, tb ? 1 : 0, Kp, ncp, sc.bd, sc.fe);
         PGB_LAUNCHED();

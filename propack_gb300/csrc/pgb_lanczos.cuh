@@ -26,6 +26,7 @@
 // row by row, writes the scaled value back.
 #pragma once
 #include <algorithm>
+#include <mutex>
 #include <type_traits>
 
 #include "pgb.cuh"
@@ -1679,6 +1680,7 @@ __device__ __forceinline__ void zupd_pl(const LbArgs &a, int j, int L, double *d
 enum { GO_NEXT = 0, GO_ELR = 1, GO_CGS = 2, GO_STOP = 3 };
 enum { GS_PL = 0, GS_F64 = 1, GS_F3 = 2 };  // Gram-Schmidt arithmetic of the instance
 constexpr unsigned RUN_SPIN_LIMIT = 1u << 24;
+constexpr size_t RUN_SMEM_L1 = 15 * 1024;  // a CTA's shared memory, so that four (and 1 KB each) fit in 64 KB
 constexpr int RUN_SMEM_KMAX = 300;  // recurrences in shared memory up to this dimension (17 KB of it)
 
 __device__ __forceinline__ unsigned ld_relaxed(const unsigned *p)
@@ -1763,7 +1765,8 @@ template <typename T, int SHORT>
 struct RunShared {
     union {
         SpmvShared<T, SHORT> spmv;
-        double buf[3 * BS];  // partial sums of the closing reductions
+        // partial sums of the closing reductions (three with complex products)
+        double buf[(SHORT == 1 && !std::is_same<T, double2>::value ? 2 : 3) * BS];
     };
     Tail t;  // CTA 0
     unsigned word;
@@ -1977,17 +1980,35 @@ static void launch_run(LbArgs a, RunArgs R, int want, cudaStream_t s)
     const bool wp = GS == GS_PL || std::is_same<T, float>::value;
     size_t sm = std::max(upd_smem(K), wp ? (cplx ? zpl_smem(K) : pl_smem(K)) : (size_t)0);
     sm = (sm + 15) / 16 * 16;
+    const Dev &d = device_info();
+    const size_t tail = sizeof(double) * 6 * (size_t)(K + 2) + sizeof(int) * (2 * (size_t)K + 8);
+    // A grid that fills the chip keeps the recurrences in global memory where
+    // they would take the CTAs past RUN_SMEM_L1: one scalar tail a half step is
+    // a microsecond longer, but the L1 that holds the gathers grows (4M rows,
+    // dimension 150, product and adjoint: 211 and 190 us with 100 KB of shared
+    // memory per SM, 207 and 184 with 64 KB, 233 and 214 with 132 KB).
+    const bool fills = want >= run_minb<T, SHORT>() * d.sms;
     R.smem_tail = 0;
-    if (K <= RUN_SMEM_KMAX) {
+    if (K <= RUN_SMEM_KMAX &&
+        !(SHORT == 1 && fills && sizeof(RunShared<T, SHORT>) + sm + tail > RUN_SMEM_L1)) {
         R.smem_tail = (int)(sm / sizeof(double));
-        sm += sizeof(double) * 6 * (size_t)(K + 2) + sizeof(int) * (2 * (size_t)K + 8);
+        sm += tail;
     }
     const void *fn = (const void *)k_lb_run<T, SHORT, GS, BLOCK>;
     static thread_local int per = 0, dev = -1;
     static thread_local size_t smem = 0;
-    const Dev &d = device_info();
     if (per == 0 || dev != d.device || smem != sm) {
-        PGB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        static std::mutex mu;
+        std::lock_guard<std::mutex> lk(mu);  // the hint and the question that depends on it
+        // the smallest carve-out for this size, left to L1 what it leaves (the
+        // runtime's own choice is larger: 64 KB asked for, 4M rows, dimension
+        // 150: 195 and 217 us with its choice, 188 and 211 with this one)
+        const size_t need = run_minb<T, SHORT>() * (sm + sizeof(RunShared<T, SHORT>) + 1024);
+        int kb = 228;
+        for (int c : {196, 164, 132, 100, 64, 32})
+            if (need <= (size_t)c * 1024) kb = c;
+        allow_dynamic_smem(fn);
+        PGB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, (kb * 100 + 227) / 228));
         PGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, BS, sm));
         dev = d.device;
         smem = sm;

@@ -105,6 +105,16 @@ const Dev &device_info()
     return d;
 }
 
+void allow_dynamic_smem(const void *fn)
+{
+    int dev = 0, most = 0;
+    cudaFuncAttributes at;
+    PGB_CUDA(cudaGetDevice(&dev));
+    PGB_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    PGB_CUDA(cudaFuncGetAttributes(&at, fn));
+    PGB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)at.sharedSizeBytes));
+}
+
 // ------------------------------------------------------ memory pool
 cudaMemPool_t lib_pool()
 {

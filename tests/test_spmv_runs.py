@@ -6,6 +6,8 @@ inside a solve.
 Tolerance: a sum of k products in any order is off by at most
 (k + 2) eps sum |a x| (complex: 4 (k + 2) eps).
 """
+from concurrent.futures import ThreadPoolExecutor
+
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -70,3 +72,31 @@ def test_solve(kind, cplx):
     v = vt.conj().T
     assert np.max(np.linalg.norm(A @ v - u * s, axis=0)) <= lim
     assert np.max(np.linalg.norm(A.conj().T @ u - v * s, axis=0)) <= lim
+
+
+@pytest.mark.parametrize("kmax", [30, 150])
+def test_solve_with_a_full_grid(kmax):
+    # enough rows to fill the chip: recurrences in shared (30) and in global memory (150)
+    m = 80011
+    A, _ = _matrix("zipf", m, m, False, 11)
+    u, s, vt, _ = pg.svdp(pg.CsrOperator(A), 4, kmax=kmax, tol=1e-12, delta=0.0, rng=np.random.default_rng(0))
+    lim = (1e-12 + 64 * m * 2 * EPS) * s[0]
+    assert np.max(np.linalg.norm(A @ vt.T - u * s, axis=0)) <= lim
+    assert np.max(np.linalg.norm(A.T @ u - vt.T * s, axis=0)) <= lim
+
+
+def test_dimensions_of_two_threads():
+    # a kernel's shared-memory limit belongs to the process: a small dimension
+    # on one thread must not lower it under another thread's larger one
+    A, _ = _matrix("zipf", 3000, 2500, False, 5)
+    op = pg.CsrOperator(A)
+
+    def values(kmax):
+        return pg.svdp(op, 4, kmax=kmax, tol=1e-12, delta=0.0, rng=np.random.default_rng(0))[1]
+
+    with ThreadPoolExecutor(1) as a, ThreadPoolExecutor(1) as b:
+        first = a.submit(values, 290).result()
+        for kmax in (12, 290, 30):
+            small, again = b.submit(values, kmax), a.submit(values, 290)
+            assert np.max(abs(small.result() - first)) <= (2e-12 + 128 * 3000 * EPS) * first[0]
+            assert np.array_equal(again.result(), first)
