@@ -50,6 +50,7 @@ constexpr double FUDGE = 1.01;                      // dlanbpro.F:117
 constexpr int NTRY = 5;                             // dreorth.F:64
 constexpr int BS = 256;                             // threads per CTA of the vector kernels
 constexpr int NNZ_PB = 2048;                        // nnz per CTA segment of the low-rank prepass
+constexpr int THIN_MIN = 256, THIN_CAP = 16;          // its warps' segments: at least so long; at most so many per NNZ_PB
 constexpr int NNZ_W = 256;                          // nnz staged per warp in the SpMV (multiple of 32)
 constexpr int ROWS_W = 32;                          // rows per SpMV row block (<= 32)
 
@@ -88,7 +89,7 @@ struct Operator {
     Csr fwd, adj, thin_r, thin_l;
     double *w = nullptr;
     double *zbuf = nullptr;      // r: the low-rank coefficients of the current product
-    double *zpart = nullptr;     // 4 * r * segs partials
+    double *zpart = nullptr;     // THIN_CAP * r * segs partials
     unsigned int *zticket = nullptr;  // r counters
     int64_t id = 0;
     int device = 0;

@@ -1543,7 +1543,7 @@ static void setup_operator(Ctx &c, propack_aprod_t aprod, double *dparm, int *ip
         c.run_ctas = std::max(c.run_ctas, c.nb);
         if (op->r > 0) {
             c.zb = c.dalloc<double>(op->r);
-            c.zpart = (double *)c.dbytes_raw(sizeof(double) * 4 * (size_t)op->r *
+            c.zpart = (double *)c.dbytes_raw(sizeof(double) * THIN_CAP * (size_t)op->r *
                                              std::max(op->thin_r.segs, op->thin_l.segs));
             c.ztick = c.dalloc<unsigned>(op->r);
         }

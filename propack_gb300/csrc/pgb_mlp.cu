@@ -893,7 +893,7 @@ static void mlp_features(Mlp &M, const Operator &op, unsigned long long seed)
     if (op.r > 0) {
         const int64_t mx = (int64_t)op.thin_r.segs * NNZ_PB;  // bounds the longest row
         int64_t seg = (mx * op.thin_r.rows / (8 * (int64_t)full) + 31) / 32 * 32;
-        seg = std::max<int64_t>(64, std::min<int64_t>(THIN_SEG, seg));
+        seg = std::max<int64_t>(64, std::min<int64_t>(512, seg));
         const int nseg = (int)((mx + seg - 1) / seg), nt = op.thin_r.rows * nseg;
         Z = (double *)pool_alloc(sizeof(double) * MLP_SK * (size_t)op.r, M.s);
         zpart = (double *)pool_alloc(sizeof(double) * MLP_SK * (size_t)nt, M.s);

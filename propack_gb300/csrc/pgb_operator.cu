@@ -768,7 +768,7 @@ void op_thin(const Operator &op, bool trans, const T *x, cudaStream_t s)
 {
     if (op.r <= 0) return;
     const Csr &Th = trans ? op.thin_l : op.thin_r;
-    const int nt = std::max(1, (Th.rows * Th.segs * 4 + SPMV_WARPS - 1) / SPMV_WARPS);
+    const int nt = (int)std::max<int64_t>(1, ((int64_t)Th.rows * Th.segs * (NNZ_PB / THIN_MIN) + SPMV_WARPS - 1) / SPMV_WARPS);
     k_thin<T><<<std::min(nt, device_info().nb), BS, 0, s>>>(Th, x, op.w, op.zpart, op.zbuf, op.zticket);
     PGB_LAUNCHED();
 }
@@ -1046,7 +1046,7 @@ static int create_operator(int m, int n, const int64_t *sp, const int32_t *si, c
         }
         const int segs = std::max(op->thin_r.segs, op->thin_l.segs);
         PGB_CUDA(cudaMalloc(&op->zbuf, sizeof(double) * r));
-        PGB_CUDA(cudaMalloc(&op->zpart, sizeof(double) * 4 * (size_t)r * segs));
+        PGB_CUDA(cudaMalloc(&op->zpart, sizeof(double) * THIN_CAP * (size_t)r * segs));
         PGB_CUDA(cudaMemset(op->zbuf, 0, sizeof(double) * r));
     }
     PGB_CUDA(cudaMalloc(&op->zticket, sizeof(unsigned int) * std::max(r, 1)));

@@ -507,26 +507,30 @@ __device__ __forceinline__ void csr_rows_piped(const int *__restrict__ ptr, cons
 }
 
 // The low-rank prepass z = w .* (Th x) of a thin matrix Th (few rows, each
-// up to the length of x): a warp per segment of THIN_SEG entries, eight
-// entries of a lane in flight; the warp that completes a row (its ticket)
-// adds the row's partials in order.  zpart: rows * 4 * segs doubles, tick:
-// rows zeroed counters, left zeroed.
-constexpr int THIN_SEG = NNZ_PB / 4;
+// up to the length of x): a row is cut into as many segments as the grid has
+// warps for it, of THIN_MIN entries at least, so that every warp takes one
+// (cut into 512 entries each, 32 rows of 200000 left the last of three rounds
+// half empty and 64 rows of 12500 two warps of three idle: 22.6 -> 18.3 us a
+// prepass on 200000 x 50000 with 32 dense factors, 14.7 -> 13.3 on 1000003 x
+// 250007 with 64 sparse ones); eight entries of a lane in flight.  The warp
+// that completes a row (its ticket) adds the row's partials in order.  zpart:
+// rows * THIN_CAP * segs doubles, tick: rows zeroed counters, left zeroed.
 template <typename T>
 __device__ __forceinline__ void thin_phase(const Csr &Th, const T *x, const double *w, double *zpart, double *z,
                                            unsigned int *tick)
 {
     const unsigned F = 0xffffffffu;
     const int lane = threadIdx.x & 31, nwarps = gridDim.x * SPMV_WARPS;
-    const int nseg = 4 * Th.segs;
+    const int nseg = min(THIN_CAP * Th.segs, max(1, nwarps / Th.rows));
     for (int t = blockIdx.x * SPMV_WARPS + (threadIdx.x >> 5); t < Th.rows * nseg; t += nwarps) {
         const int c = t / nseg, sg = t % nseg;
         const int p0 = Th.ptr[c], p1 = Th.ptr[c + 1];
-        const int used = max(1, (p1 - p0 + THIN_SEG - 1) / THIN_SEG);
+        const int seg = max(THIN_MIN, ((p1 - p0 + nseg - 1) / nseg + 31) / 32 * 32);
+        const int used = max(1, (p1 - p0 + seg - 1) / seg);
         if (sg >= used) continue;
-        const int b = min(p1, p0 + (sg + 1) * THIN_SEG);
+        const int b = min(p1, p0 + (sg + 1) * seg);
         double acc = 0.0;
-        int e = p0 + sg * THIN_SEG + lane;
+        int e = p0 + sg * seg + lane;
         for (; e + 32 * 7 < b; e += 32 * 8) {
             int ci[8];
             double v[8];

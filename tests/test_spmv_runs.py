@@ -100,3 +100,17 @@ def test_dimensions_of_two_threads():
             small, again = b.submit(values, kmax), a.submit(values, 290)
             assert np.max(abs(small.result() - first)) <= (2e-12 + 128 * 3000 * EPS) * first[0]
             assert np.array_equal(again.result(), first)
+
+
+@pytest.mark.parametrize("r", [1, 5, 33])
+@pytest.mark.parametrize("m,n", [(40, 255), (300, 257), (40000, 5000)])
+def test_low_rank_prepass(m, n, r):
+    # rows of the thin factors shorter than a segment, at its edges, and cut over the grid
+    S, rng = _matrix("const3", m, n, False, m + r)
+    L, R, w = rng.standard_normal((m, r)), rng.standard_normal((n, r)), rng.standard_normal(r)
+    op = pg.CsrOperator(S, sp.csr_array(L), sp.csr_array(R), w)
+    B = sp.csr_array((abs(S.data), S.indices.copy(), S.indptr.copy()), shape=S.shape)
+    for y, x, M, P, F, G in ((op.matvec, _vec(n, False, rng), S, B, L, R), (op.rmatvec, _vec(m, False, rng), S.T, B.T, R, L)):
+        ref = M @ x + F @ (w * (G.T @ x))
+        lim = (len(x) + r + 8) * EPS * (P @ abs(x) + abs(F) @ (abs(w) * (abs(G).T @ abs(x))))
+        assert np.all(abs(np.asarray(y(x)) - ref) <= 2 * lim)
