@@ -26,6 +26,7 @@
 // row by row, writes the scaled value back.
 #pragma once
 #include <algorithm>
+#include <map>
 #include <mutex>
 #include <type_traits>
 
@@ -1994,28 +1995,40 @@ static void launch_run(LbArgs a, RunArgs R, int want, cudaStream_t s)
         R.smem_tail = (int)(sm / sizeof(double));
         sm += tail;
     }
+    // the smallest carve-out for this size, left to L1 what it leaves (the
+    // runtime's own choice is larger: 64 KB asked for, 4M rows, dimension
+    // 150: 195 and 217 us with its choice, 188 and 211 with this one)
+    const size_t need = run_minb<T, SHORT>() * (sm + sizeof(RunShared<T, SHORT>) + 1024);
+    int kb = 228;
+    for (int c : {196, 164, 132, 100, 64, 32})
+        if (need <= (size_t)c * 1024) kb = c;
     const void *fn = (const void *)k_lb_run<T, SHORT, GS, BLOCK>;
-    static thread_local int per = 0, dev = -1;
-    static thread_local size_t smem = 0;
-    if (per == 0 || dev != d.device || smem != sm) {
-        static std::mutex mu;
-        std::lock_guard<std::mutex> lk(mu);  // the hint and the question that depends on it
-        // the smallest carve-out for this size, left to L1 what it leaves (the
-        // runtime's own choice is larger: 64 KB asked for, 4M rows, dimension
-        // 150: 195 and 217 us with its choice, 188 and 211 with this one)
-        const size_t need = run_minb<T, SHORT>() * (sm + sizeof(RunShared<T, SHORT>) + 1024);
-        int kb = 228;
-        for (int c : {196, 164, 132, 100, 64, 32})
-            if (need <= (size_t)c * 1024) kb = c;
-        allow_dynamic_smem(fn);
-        PGB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, (kb * 100 + 227) / 228));
-        PGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, BS, sm));
-        dev = d.device;
-        smem = sm;
-    }
-    const int g = std::max(1, std::min(want, std::min(d.nb, std::max(1, per) * d.sms)));
-    a.nb = g;
     PGB_CUDA(cudaMemsetAsync(R.sync, 0, 3 * sizeof(unsigned), s));
+    // The carve-out belongs to the kernel, not to the caller's thread, and a
+    // cooperative launch may not exceed the occupancy under it: hint, occupancy
+    // and launch are one critical section, and a call finds the hint of
+    // whichever thread launched last.
+    struct Hint {
+        int kb = 0, per = 0;
+        size_t smem = 0;
+    };
+    static std::mutex mu;
+    static std::map<int, Hint> hints;  // by device
+    std::lock_guard<std::mutex> lk(mu);
+    Hint &h = hints[d.device];
+    if (h.kb != kb || h.smem != sm) {
+        if (h.kb == 0) allow_dynamic_smem(fn);
+        if (h.kb != kb)
+            PGB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, (kb * 100 + 227) / 228));
+        h = Hint();  // a failed question leaves nothing behind
+        int per = 0;
+        PGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, BS, sm));
+        h.kb = kb;
+        h.per = per;
+        h.smem = sm;
+    }
+    const int g = std::max(1, std::min(want, std::min(d.nb, std::max(1, h.per) * d.sms)));
+    a.nb = g;
     void *args[] = {&a, &R};
     PGB_CUDA(cudaLaunchCooperativeKernel(fn, dim3(g), dim3(BS), args, sm, s));
     PGB_LAUNCHED();
