@@ -162,47 +162,55 @@ __global__ void __launch_bounds__(256) k_mlp_thin(Csr Th, const double *om, cons
 // products by one column each it read A sixteen times behind 48 launches (830
 // us at 200,000 x 50,000 with 14 entries per row, 500 us at a quarter of it).
 // Bound by the FP64 pipe: one FMA per entry and column.
-// Rows longer than SK_LONG wait in a list for the whole CTA (its half warps
-// take every 16th entry), so that no half warp walks one alone; rows are dealt
-// round-robin, so that few long rows reach all CTAs.
-constexpr int SK_LONG = 256, SK_LIST = 64;
-__global__ void __launch_bounds__(256) k_mlp_sketch(Csr A, const double *om, const double *Z, double *Y,
+// Rows longer than SK_LONG are left to the whole CTA (its half warps take every
+// 16th entry), so that no half warp walks one alone; the CTA takes its long
+// rows in the order of their index, so that Y and the sums of squares are the
+// same bits on every call.  Rows are dealt round-robin, so that few long rows
+// reach all CTAs.
+constexpr int SK_LONG = 256;
+__global__ void __launch_bounds__(256, 8) k_mlp_sketch(Csr A, const double *om, const double *Z, double *Y,
                                                     double *part)
 {
     __shared__ double buf[256];
-    __shared__ int list[SK_LIST], nlist;
-    const int c = threadIdx.x & 15, hw = threadIdx.x >> 4;
-    if (threadIdx.x == 0) nlist = 0;
-    __syncthreads();
+    __shared__ unsigned longs[8];
+    const int c = threadIdx.x & 15, hw = threadIdx.x >> 4, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     double sq = 0.0;
+    int seen = 0;
     for (long long rr = blockIdx.x + (long long)gridDim.x * hw; rr < A.rows; rr += (long long)gridDim.x * 16) {
         const int r = (int)rr, e0 = A.ptr[r], e1 = A.ptr[r + 1];
         if (e1 - e0 > SK_LONG) {
-            int at = 0;
-            if (c == 0) at = atomicAdd(&nlist, 1);
-            at = __shfl_sync(0xffffu << (threadIdx.x & 16), at, 0, 16);
-            if (at < SK_LIST) {
-                if (c == 0) list[at] = r;
-                continue;
-            }
+            seen = 1;
+            continue;
         }
         const double y = sketch_sum(A.idx, A.val, e0, e1, 1, A.ncol0, om, Z, c);
         Y[(size_t)r * MLP_SK + c] = y;
         sq = fma(y, y, sq);
     }
-    __syncthreads();
-    const int nl = min(nlist, SK_LIST);
-    for (int q = 0; q < nl; q++) {
-        const int r = list[q];
-        buf[threadIdx.x] = sketch_sum(A.idx, A.val, A.ptr[r] + hw, A.ptr[r + 1], 16, A.ncol0, om, Z, c);
-        __syncthreads();
-        if (hw == 0) {
-            double y = 0.0;
-            for (int i = 0; i < 16; i++) y += buf[16 * i + c];
-            Y[(size_t)r * MLP_SK + c] = y;
-            sq = fma(y, y, sq);
+    if (__syncthreads_or(seen)) {
+        // the CTA's rows, 256 at a time: bit l of longs[w] marks the long ones
+        for (long long base = blockIdx.x; base < A.rows; base += (long long)gridDim.x * 256) {
+            const long long rr = base + (long long)gridDim.x * threadIdx.x;
+            const bool lg = rr < A.rows && A.ptr[rr + 1] - A.ptr[rr] > SK_LONG;
+            const unsigned bits = __ballot_sync(0xffffffffu, lg);
+            if (lane == 0) longs[w] = bits;
+            __syncthreads();
+            for (int q = 0; q < 8; q++)
+                for (unsigned mask = longs[q]; mask; mask &= mask - 1) {
+                    const int r = (int)(base + (long long)gridDim.x * (32 * q + __ffs(mask) - 1));
+                    double y = sketch_sum(A.idx, A.val, A.ptr[r] + hw, A.ptr[r + 1], 16, A.ncol0, om, Z, c);
+                    y += __shfl_xor_sync(0xffffffffu, y, 16);
+                    if (lane < 16) buf[16 * w + c] = y;
+                    __syncthreads();
+                    if (hw == 0) {
+                        y = buf[c];
+                        for (int i = 1; i < 8; i++) y += buf[16 * i + c];
+                        Y[(size_t)r * MLP_SK + c] = y;
+                        sq = fma(y, y, sq);
+                    }
+                    __syncthreads();
+                }
+            __syncthreads();
         }
-        __syncthreads();
     }
     block_sums<256, 1>({sq}, buf, {part + blockIdx.x});
 }
