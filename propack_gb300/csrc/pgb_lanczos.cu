@@ -6,12 +6,11 @@ namespace pgb {
 // Gram-Schmidt arithmetic of the FP64 form (propack_set_cgs_arith)
 thread_local int g_cgs_arith = CGS_PLANES;
 
-// the planes are used when the driver allocated them (FP64 form, kmax up to
-// some 2800; complex vectors 1500)
-bool lb_planes_fit(int kmax, bool cplx)
-{
-    return (size_t)((cplx ? 2 : 1) * sizeof(double) * PL_WARPS + 2 * sizeof(int)) * (kmax + 1) <= PL_SMEM_MAX;
-}
+// The planes are used when the driver allocated them: FP64 form up to dimension
+// 2843, complex vectors 1504.  They take the memory of a second basis on each
+// side; beyond these dimensions the bases go without (a solve whose bases fill
+// the device still fits) and Gram-Schmidt runs on FP64 FMAs.
+bool lb_planes_fit(int kmax, bool cplx) { return kmax <= (cplx ? 1504 : 2843); }
 
 // device words of the barrier, the published scalars
 size_t lb_run_scratch() { return 64 + sizeof(LbPub); }

@@ -736,6 +736,16 @@ constexpr int DOT_COLS = 4;
 // columns whose per-slice partials lie in shared memory at a time: what a CTA
 // takes of it comes out of the L1 that holds the SpMV's gathers in flight
 constexpr int WPART_COLS = 64;
+// Selections of more columns (BIG instances: dimensions past GS_COLS) have their
+// indices and, in an update, their coefficients in shared memory GS_COLS at a
+// time.  x goes through memory once more per GS_COLS columns (1/256 of the pass),
+// but no dimension takes more than 7 KB (complex 11) out of the L1 or is refused
+// for its size: with all columns there (1000003 rows of 8 entries, kmax 2000, 989
+// steps) product and adjoint took 153 and 137 us, projections 1166, updates 820,
+// by blocks 79, 70, 937 and 689.  The smaller dimensions keep instances without
+// the loop over blocks: with it the compiler gives the product's loads fewer
+// registers (FP32, 500001 rows: 66 -> 80 us).
+constexpr int GS_COLS = 512;
 template <int SIDE>
 __device__ __forceinline__ void dots_f64(const LbArgs &a, int j, int L)
 {
@@ -808,12 +818,10 @@ __device__ __forceinline__ int dot_slices(int chunk)
 
 // projections of the FP32 form: compensated sums, the work layout of dots_pl
 // below (slices of 4-element vectors, groups of DOT_COLS columns)
-template <int SIDE>
+template <int SIDE, bool BIG>
 __device__ __forceinline__ void dots_f32(const LbArgs &a, int j, int L, double *wpart)
 {
     int *ssel = reinterpret_cast<int *>(wpart + BS / 32 * WPART_COLS);
-    for (int c = threadIdx.x; c < L; c += BS) ssel[c] = a.sel[c];
-    __syncthreads();
     const int len = SIDE == 0 ? a.adj.rows : a.fwd.rows;
     const size_t ldq = (size_t)(SIDE == 0 ? a.ldv : a.ldu) / 4;
     const float *W = (const float *)(SIDE == 0 ? a.V : a.U);
@@ -829,68 +837,71 @@ __device__ __forceinline__ void dots_f32(const LbArgs &a, int j, int L, double *
     const int v0 = min(cb1, cb0 + ws * sl), v1 = min(cb1, v0 + sl);
     // the rows past the last whole vector: the last slice's warps of the last CTA
     const int r0 = blockIdx.x == gridDim.x - 1 && ws == rs - 1 ? nvec * 4 + lane : len;
-    for (int b0 = 0; b0 < L; b0 += WPART_COLS) {
-        const int b1 = min(L, b0 + WPART_COLS);
-        for (int cb = b0 + wg * DOT_COLS; cb < b1; cb += cgs * DOT_COLS) {
-            const int nc = min(DOT_COLS, b1 - cb);
-            const float4 *Wq[DOT_COLS];
+    int s0 = 0;
+    do {
+        const int s1 = BIG ? min(L, s0 + GS_COLS) : L;
+        for (int c = threadIdx.x; c < s1 - s0; c += BS) ssel[c] = a.sel[s0 + c];
+        __syncthreads();
+        for (int b0 = s0; b0 < s1; b0 += WPART_COLS) {
+            const int b1 = min(s1, b0 + WPART_COLS);
+            for (int cb = b0 + wg * DOT_COLS; cb < b1; cb += cgs * DOT_COLS) {
+                const int nc = min(DOT_COLS, b1 - cb);
+                const int *scol = ssel + (cb - s0);
+                const float4 *Wq[DOT_COLS];
 #pragma unroll
-            for (int u = 0; u < DOT_COLS; u++) Wq[u] = Wv + (size_t)ssel[cb + (u < nc ? u : 0)] * ldq;
-            Acc<float> acc[DOT_COLS];
-            int v = v0 + lane;
+                for (int u = 0; u < DOT_COLS; u++) Wq[u] = Wv + (size_t)scol[u < nc ? u : 0] * ldq;
+                Acc<float> acc[DOT_COLS];
+                int v = v0 + lane;
 #pragma unroll 1
-            for (; v < v1; v += 32) {  // one vector of each column in flight: see dots_pl
-                float4 w0[DOT_COLS];
+                for (; v < v1; v += 32) {  // one vector of each column in flight: see dots_pl
+                    float4 w0[DOT_COLS];
 #pragma unroll
-                for (int u = 0; u < DOT_COLS; u++) w0[u] = __ldcs(Wq[u] + v);
-                const float4 x0 = xv[v];
+                    for (int u = 0; u < DOT_COLS; u++) w0[u] = __ldcs(Wq[u] + v);
+                    const float4 x0 = xv[v];
 #pragma unroll
-                for (int u = 0; u < DOT_COLS; u++)
+                    for (int u = 0; u < DOT_COLS; u++)
 #pragma unroll
-                    for (int q = 0; q < 4; q++) acc[u].add_prod(Vec16<float>::get(w0[u], q), Vec16<float>::get(x0, q));
+                        for (int q = 0; q < 4; q++) acc[u].add_prod(Vec16<float>::get(w0[u], q), Vec16<float>::get(x0, q));
+                }
+                if (r0 < len) {
+                    const float xr = x[r0];
+#pragma unroll
+                    for (int u = 0; u < DOT_COLS; u++)
+                        if (u < nc) acc[u].add_prod(W[(size_t)scol[u] * (4 * ldq) + r0], xr);
+                }
+                PlAcc p[DOT_COLS];
+#pragma unroll
+                for (int u = 0; u < DOT_COLS; u++) {
+                    p[u].s = acc[u].s;
+                    p[u].c = acc[u].c;
+                }
+                const PlAcc tot = pl_warp_sum4(p);
+                if ((lane & 7) == 0 && (lane >> 3) < nc) wpart[ws * WPART_COLS + cb - b0 + (lane >> 3)] = tot.value();
             }
-            if (r0 < len) {
-                const float xr = x[r0];
-#pragma unroll
-                for (int u = 0; u < DOT_COLS; u++)
-                    if (u < nc) acc[u].add_prod(W[(size_t)ssel[cb + u] * (4 * ldq) + r0], xr);
+            __syncthreads();
+            for (int c = threadIdx.x; c < b1 - b0; c += BS) {
+                double sum = 0.0;
+                for (int ww = 0; ww < rs; ww++) sum += wpart[ww * WPART_COLS + c];
+                a.part_cols[(size_t)(b0 + c) * a.nb + blockIdx.x] = sum;
             }
-            PlAcc p[DOT_COLS];
-#pragma unroll
-            for (int u = 0; u < DOT_COLS; u++) {
-                p[u].s = acc[u].s;
-                p[u].c = acc[u].c;
-            }
-            const PlAcc tot = pl_warp_sum4(p);
-            if ((lane & 7) == 0 && (lane >> 3) < nc) wpart[ws * WPART_COLS + cb - b0 + (lane >> 3)] = tot.value();
+            __syncthreads();
         }
-        __syncthreads();
-        for (int c = threadIdx.x; c < b1 - b0; c += BS) {
-            double sum = 0.0;
-            for (int ww = 0; ww < rs; ww++) sum += wpart[ww * WPART_COLS + c];
-            a.part_cols[(size_t)(b0 + c) * a.nb + blockIdx.x] = sum;
-        }
-        __syncthreads();
-    }
+        s0 += GS_COLS;
+    } while (BIG && s0 < L);
 }
 
 // x -= W(:,sel) h (dreorth.F:85-95, the dgemv('N') of dcgs) and ||x||^2:
 // one 16-byte row vector per thread and step, the selected columns streamed
 // with CGS_UNROLL loads in flight; h and the selection sit in shared memory.
 constexpr int CGS_UNROLL = 8;
-template <int SIDE, typename T>
+template <int SIDE, typename T, bool BIG>
 __device__ __forceinline__ void upd_full(const LbArgs &a, int j, int L, double *dyn, double *buf)
 {
     using VT = Vec16<T>;
     using V = typename VT::V;
-    // dyn: h[L] (as T, one double slot each) | sel[L]
+    // dyn: h (as T, one double slot each) | sel, of the block's columns
     T *hs = reinterpret_cast<T *>(dyn);
-    int *ssel = reinterpret_cast<int *>(dyn + L);
-    for (int c = threadIdx.x; c < L; c += BS) {
-        hs[c] = (T)a.h[c];
-        ssel[c] = a.sel[c];
-    }
-    __syncthreads();
+    int *ssel = reinterpret_cast<int *>(dyn + (BIG ? min(L, GS_COLS) : L));
     const int len = SIDE == 0 ? a.adj.rows : a.fwd.rows;
     const size_t ld = SIDE == 0 ? a.ldv : a.ldu;
     const T *W = (const T *)(SIDE == 0 ? a.V : a.U);
@@ -898,29 +909,43 @@ __device__ __forceinline__ void upd_full(const LbArgs &a, int j, int L, double *
     V *xv = reinterpret_cast<V *>(x);
     const int nvec = len / VT::W;
     Acc<T> sq;
-    for (int v = blockIdx.x * BS + threadIdx.x; v < nvec; v += gridDim.x * BS) {
-        V acc = xv[v];
-        int c = 0;
-        for (; c + CGS_UNROLL <= L; c += CGS_UNROLL) {
-            V wv[CGS_UNROLL];
-#pragma unroll
-            for (int u = 0; u < CGS_UNROLL; u++) wv[u] = reinterpret_cast<const V *>(W + (size_t)ssel[c + u] * ld)[v];
-#pragma unroll
-            for (int u = 0; u < CGS_UNROLL; u++) VT::fms(acc, wv[u], hs[c + u]);
+    int b0 = 0;
+    do {
+        const int nb = BIG ? min(GS_COLS, L - b0) : L;
+        const bool last = !BIG || b0 + nb >= L;
+        if (BIG && b0 > 0) __syncthreads();
+        for (int c = threadIdx.x; c < nb; c += BS) {
+            hs[c] = (T)a.h[b0 + c];
+            ssel[c] = a.sel[b0 + c];
         }
-        for (; c < L; c++) VT::fms(acc, reinterpret_cast<const V *>(W + (size_t)ssel[c] * ld)[v], hs[c]);
-        xv[v] = acc;
+        __syncthreads();
+        for (int v = blockIdx.x * BS + threadIdx.x; v < nvec; v += gridDim.x * BS) {
+            V acc = xv[v];
+            int c = 0;
+            for (; c + CGS_UNROLL <= nb; c += CGS_UNROLL) {
+                V wv[CGS_UNROLL];
 #pragma unroll
-        for (int q = 0; q < VT::W; q++) sq.add_prod(VT::get(acc, q), VT::get(acc, q));
-    }
-    if (blockIdx.x == gridDim.x - 1) {
-        for (int r = nvec * VT::W + threadIdx.x; r < len; r += BS) {
-            T y = x[r];
-            for (int c = 0; c < L; c++) y = fma(-W[(size_t)ssel[c] * ld + r], hs[c], y);
-            x[r] = y;
-            sq.add_prod(y, y);
+                for (int u = 0; u < CGS_UNROLL; u++)
+                    wv[u] = reinterpret_cast<const V *>(W + (size_t)ssel[c + u] * ld)[v];
+#pragma unroll
+                for (int u = 0; u < CGS_UNROLL; u++) VT::fms(acc, wv[u], hs[c + u]);
+            }
+            for (; c < nb; c++) VT::fms(acc, reinterpret_cast<const V *>(W + (size_t)ssel[c] * ld)[v], hs[c]);
+            xv[v] = acc;
+            if (last)
+#pragma unroll
+                for (int q = 0; q < VT::W; q++) sq.add_prod(VT::get(acc, q), VT::get(acc, q));
         }
-    }
+        if (blockIdx.x == gridDim.x - 1) {
+            for (int r = nvec * VT::W + threadIdx.x; r < len; r += BS) {
+                T y = x[r];
+                for (int c = 0; c < nb; c++) y = fma(-W[(size_t)ssel[c] * ld + r], hs[c], y);
+                x[r] = y;
+                if (last) sq.add_prod(y, y);
+            }
+        }
+        b0 += GS_COLS;
+    } while (BIG && b0 < L);
     block_sums<BS, 1>({sq.value()}, buf, {a.part_sq + blockIdx.x});
 }
 
@@ -987,14 +1012,14 @@ __device__ __forceinline__ void dots_f3(const LbArgs &a, int j, int L)
 // The FP64 form's update on the FP32 pipe: sum_c W(i, c) h_c at three
 // levels per row (h scaled by the power of two of its largest entry),
 // then one FP64 FMA per row applies it to x.
-template <int SIDE>
+template <int SIDE, bool BIG>
 __device__ __forceinline__ void upd_f3(const LbArgs &a, int j, int L, double *dyn, double *buf)
 {
     using V = double2;
-    // dyn: h[L] as F3 (one double2 slot each) | sel[L]
+    // dyn: h as F3 (one double2 slot each) | sel, of the block's columns
     __shared__ int hsh;
     F3 *h3 = reinterpret_cast<F3 *>(dyn);
-    int *ssel = reinterpret_cast<int *>(dyn + 2 * (size_t)L);
+    int *ssel = reinterpret_cast<int *>(dyn + 2 * (size_t)(BIG ? min(L, GS_COLS) : L));
     if (threadIdx.x == 0) hsh = 0;
     __syncthreads();
     int he = 0;
@@ -1002,11 +1027,6 @@ __device__ __forceinline__ void upd_f3(const LbArgs &a, int j, int L, double *dy
     if (he) atomicMax(&hsh, he);
     __syncthreads();
     const int hs = hsh == 0 ? 0 : hsh - 1023;  // |h 2^-hs| < 2
-    for (int c = threadIdx.x; c < L; c += BS) {
-        h3[c] = f3_split(a.h[c], hs);
-        ssel[c] = a.sel[c];
-    }
-    __syncthreads();
     const double back = f3_pow2(hs);
     const int len = SIDE == 0 ? a.adj.rows : a.fwd.rows;
     const size_t ld = SIDE == 0 ? a.ldv : a.ldu;
@@ -1015,41 +1035,56 @@ __device__ __forceinline__ void upd_f3(const LbArgs &a, int j, int L, double *dy
     V *xv = reinterpret_cast<V *>(x);
     const int nvec = len / 2;
     Acc<double> sq;
-    for (int v = blockIdx.x * BS + threadIdx.x; v < nvec; v += gridDim.x * BS) {
-        F3Acc s0, s1;
-        int c = 0;
-        for (; c + CGS_UNROLL <= L; c += CGS_UNROLL) {
-            V wv[CGS_UNROLL];
+    int b0 = 0;
+    do {
+        const int nb = BIG ? min(GS_COLS, L - b0) : L;
+        const bool last = !BIG || b0 + nb >= L;
+        if (BIG && b0 > 0) __syncthreads();
+        for (int c = threadIdx.x; c < nb; c += BS) {
+            h3[c] = f3_split(a.h[b0 + c], hs);
+            ssel[c] = a.sel[b0 + c];
+        }
+        __syncthreads();
+        for (int v = blockIdx.x * BS + threadIdx.x; v < nvec; v += gridDim.x * BS) {
+            F3Acc s0, s1;
+            int c = 0;
+            for (; c + CGS_UNROLL <= nb; c += CGS_UNROLL) {
+                V wv[CGS_UNROLL];
 #pragma unroll
-            for (int u = 0; u < CGS_UNROLL; u++) wv[u] = reinterpret_cast<const V *>(W + (size_t)ssel[c + u] * ld)[v];
+                for (int u = 0; u < CGS_UNROLL; u++)
+                    wv[u] = reinterpret_cast<const V *>(W + (size_t)ssel[c + u] * ld)[v];
 #pragma unroll
-            for (int u = 0; u < CGS_UNROLL; u++) {
-                const F3 hc = h3[c + u];
-                s0.add(f3_split(wv[u].x, 0), hc);
-                s1.add(f3_split(wv[u].y, 0), hc);
+                for (int u = 0; u < CGS_UNROLL; u++) {
+                    const F3 hc = h3[c + u];
+                    s0.add(f3_split(wv[u].x, 0), hc);
+                    s1.add(f3_split(wv[u].y, 0), hc);
+                }
+            }
+            for (; c < nb; c++) {
+                const V wc = reinterpret_cast<const V *>(W + (size_t)ssel[c] * ld)[v];
+                s0.add(f3_split(wc.x, 0), h3[c]);
+                s1.add(f3_split(wc.y, 0), h3[c]);
+            }
+            V acc = xv[v];
+            acc.x = fma(-s0.value(), back, acc.x);
+            acc.y = fma(-s1.value(), back, acc.y);
+            xv[v] = acc;
+            if (last) {
+                sq.add_prod(acc.x, acc.x);
+                sq.add_prod(acc.y, acc.y);
             }
         }
-        for (; c < L; c++) {
-            const V wc = reinterpret_cast<const V *>(W + (size_t)ssel[c] * ld)[v];
-            s0.add(f3_split(wc.x, 0), h3[c]);
-            s1.add(f3_split(wc.y, 0), h3[c]);
+        if (blockIdx.x == gridDim.x - 1) {
+            for (int r = nvec * 2 + threadIdx.x; r < len; r += BS) {
+                F3Acc sr;
+                for (int c = 0; c < nb; c++) sr.add(f3_split(W[(size_t)ssel[c] * ld + r], 0), h3[c]);
+                const double y = fma(-sr.value(), back, x[r]);
+                x[r] = y;
+                if (last) sq.add_prod(y, y);
+            }
         }
-        V acc = xv[v];
-        acc.x = fma(-s0.value(), back, acc.x);
-        acc.y = fma(-s1.value(), back, acc.y);
-        xv[v] = acc;
-        sq.add_prod(acc.x, acc.x);
-        sq.add_prod(acc.y, acc.y);
-    }
-    if (blockIdx.x == gridDim.x - 1) {
-        for (int r = nvec * 2 + threadIdx.x; r < len; r += BS) {
-            F3Acc sr;
-            for (int c = 0; c < L; c++) sr.add(f3_split(W[(size_t)ssel[c] * ld + r], 0), h3[c]);
-            const double y = fma(-sr.value(), back, x[r]);
-            x[r] = y;
-            sq.add_prod(y, y);
-        }
-    }
+        b0 += GS_COLS;
+    } while (BIG && b0 < L);
     block_sums<BS, 1>({sq.value()}, buf, {a.part_sq + blockIdx.x});
 }
 
@@ -1082,21 +1117,15 @@ __device__ __forceinline__ void upd_f3(const LbArgs &a, int j, int L, double *dy
 // per group), then added over the warps in a fixed order, then over the
 // CTAs by CTA 0 or the grid (reduce_cols).  The grid is one wave at the kernel's occupancy (<= nb CTAs).
 constexpr int PL_WARPS = BS / 32;
-constexpr size_t PL_SMEM_MAX = 200 * 1024;  // bounds the dimension of the plane form (lb_planes_fit)
 constexpr int PL_SPLIT_UNROLL = 4;          // FP64 loads in flight per lane when a column is split
-template <int SIDE>
+static_assert(GS_COLS % WPART_COLS == 0 && WPART_COLS % PL_WARPS == 0, "column groups stay with their warps");
+template <int SIDE, bool BIG>
 __device__ __forceinline__ void dots_pl(const LbArgs &a, int j, int L, double *wpart)
 {
-    // wpart: [PL_WARPS][WPART_COLS] per-slice partial projections | sel[kmax + 1] | fresh[kmax + 1]
+    // wpart: [PL_WARPS][WPART_COLS] per-slice partial projections | sel of GS_COLS columns and their stale flags
     int *ssel = reinterpret_cast<int *>(wpart + PL_WARPS * WPART_COLS);
-    int *sfresh = ssel + a.kmax + 1;
-    int *ok = SIDE == 0 ? a.okV : a.okU;
-    for (int c = threadIdx.x; c < L; c += BS) {
-        const int col = a.sel[c];
-        ssel[c] = col;
-        sfresh[c] = ok[col] == 0;
-    }
-    __syncthreads();
+    unsigned char *sstale = reinterpret_cast<unsigned char *>(ssel + min(a.kmax + 1, GS_COLS));
+    const int *ok = SIDE == 0 ? a.okV : a.okU;
     const int len = SIDE == 0 ? a.adj.rows : a.fwd.rows;
     const size_t ld = SIDE == 0 ? a.ldv : a.ldu;
     const size_t ldq = ld / 2;  // leading dimension in float4 (two elements)
@@ -1131,72 +1160,83 @@ __device__ __forceinline__ void dots_pl(const LbArgs &a, int j, int L, double *w
     }
     float2 xr = make_float2(0.f, 0.f);
     if (tail_row) xr = pl_xsplit(x[len - 1], xs);
-    // planes of the stale selected columns, on this lane's rows
-    for (int c = 0; c < L; c++) {
-        if (!sfresh[c] || (c / DOT_COLS) % cgs != wg) continue;
-        const int col = ssel[c];
-        float4 *Wq = reinterpret_cast<float4 *>(Wp) + (size_t)col * ldq;
-        const double2 *Wd = reinterpret_cast<const double2 *>(W + (size_t)col * ld);
-        int v = v0 + lane;
-        for (; v + 32 * (PL_SPLIT_UNROLL - 1) < v1; v += 32 * PL_SPLIT_UNROLL) {
-            double2 d[PL_SPLIT_UNROLL];
-#pragma unroll
-            for (int u = 0; u < PL_SPLIT_UNROLL; u++) d[u] = Wd[v + 32 * u];
-#pragma unroll
-            for (int u = 0; u < PL_SPLIT_UNROLL; u++) Wq[v + 32 * u] = pl_split2(d[u]);
+    int s0 = 0;
+    do {
+        const int s1 = BIG ? min(L, s0 + GS_COLS) : L;
+        for (int c = threadIdx.x; c < s1 - s0; c += BS) {
+            const int col = a.sel[s0 + c];
+            ssel[c] = col;
+            sstale[c] = ok[col] == 0;
         }
-        for (; v < v1; v += 32) Wq[v] = pl_split2(Wd[v]);
-        if (tail_row) Wp[(size_t)col * ld + len - 1] = pl_split(W[(size_t)col * ld + len - 1]);
-    }
-    for (int b0 = 0; b0 < L; b0 += WPART_COLS) {
-        const int b1 = min(L, b0 + WPART_COLS);
-        for (int cb = b0 + wg * DOT_COLS; cb < b1; cb += cgs * DOT_COLS) {
-            const int nc = min(DOT_COLS, b1 - cb);
-            const float4 *Wq[DOT_COLS];
-#pragma unroll
-            for (int u = 0; u < DOT_COLS; u++)
-                Wq[u] = reinterpret_cast<const float4 *>(Wp) + (size_t)ssel[cb + (u < nc ? u : 0)] * ldq;
-            PlAcc acc[DOT_COLS];
+        __syncthreads();
+        // planes of the stale columns, on this lane's rows
+        for (int c = 0; c < s1 - s0; c++) {
+            if (!sstale[c] || (c / DOT_COLS) % cgs != wg) continue;
+            const int col = ssel[c];
+            float4 *Wq = reinterpret_cast<float4 *>(Wp) + (size_t)col * ldq;
+            const double2 *Wd = reinterpret_cast<const double2 *>(W + (size_t)col * ld);
             int v = v0 + lane;
-            // The planes stream through once (evict-first), so that the x
-            // planes, read again by every group, stay in L2.  One vector of each
-            // column in flight per lane: a second one lets the warps' streams
-            // thrash each other (1000003 x 250007, 120 columns: 141 us a pass
-            // with two, 106 with one; 4M rows, 75 columns: 548 and 506), and
-            // eight columns at a time or slices interleaved over the CTA's warps do
-            // the same (146 and 151; 626 and 606).
+            for (; v + 32 * (PL_SPLIT_UNROLL - 1) < v1; v += 32 * PL_SPLIT_UNROLL) {
+                double2 d[PL_SPLIT_UNROLL];
+#pragma unroll
+                for (int u = 0; u < PL_SPLIT_UNROLL; u++) d[u] = Wd[v + 32 * u];
+#pragma unroll
+                for (int u = 0; u < PL_SPLIT_UNROLL; u++) Wq[v + 32 * u] = pl_split2(d[u]);
+            }
+            for (; v < v1; v += 32) Wq[v] = pl_split2(Wd[v]);
+            if (tail_row) Wp[(size_t)col * ld + len - 1] = pl_split(W[(size_t)col * ld + len - 1]);
+        }
+        for (int b0 = s0; b0 < s1; b0 += WPART_COLS) {
+            const int b1 = min(s1, b0 + WPART_COLS);
+            for (int cb = b0 + wg * DOT_COLS; cb < b1; cb += cgs * DOT_COLS) {
+                const int nc = min(DOT_COLS, b1 - cb);
+                const float4 *Wq[DOT_COLS];
+#pragma unroll
+                for (int u = 0; u < DOT_COLS; u++)
+                    Wq[u] = reinterpret_cast<const float4 *>(Wp) + (size_t)ssel[cb - s0 + (u < nc ? u : 0)] * ldq;
+                PlAcc acc[DOT_COLS];
+                int v = v0 + lane;
+                // The planes stream through once (evict-first), so that the x
+                // planes, read again by every group, stay in L2.  One vector of each
+                // column in flight per lane: a second one lets the warps' streams
+                // thrash each other (1000003 x 250007, 120 columns: 141 us a pass
+                // with two, 106 with one; 4M rows, 75 columns: 548 and 506), and
+                // eight columns at a time or slices interleaved over the CTA's warps do
+                // the same (146 and 151; 626 and 606).
 #pragma unroll 1
-            for (; v < v1; v += 32) {
-                float4 w0[DOT_COLS];
+                for (; v < v1; v += 32) {
+                    float4 w0[DOT_COLS];
 #pragma unroll
-                for (int u = 0; u < DOT_COLS; u++) w0[u] = __ldcs(Wq[u] + v);
-                const float4 x0 = xq[v];
+                    for (int u = 0; u < DOT_COLS; u++) w0[u] = __ldcs(Wq[u] + v);
+                    const float4 x0 = xq[v];
 #pragma unroll
-                for (int u = 0; u < DOT_COLS; u++) {
-                    acc[u].add(w0[u].x, w0[u].y, x0.x, x0.y);
-                    acc[u].add(w0[u].z, w0[u].w, x0.z, x0.w);
+                    for (int u = 0; u < DOT_COLS; u++) {
+                        acc[u].add(w0[u].x, w0[u].y, x0.x, x0.y);
+                        acc[u].add(w0[u].z, w0[u].w, x0.z, x0.w);
+                    }
                 }
-            }
-            if (tail_row) {
+                if (tail_row) {
 #pragma unroll
-                for (int u = 0; u < DOT_COLS; u++) {
-                    if (u >= nc) break;
-                    const float2 wr = Wp[(size_t)ssel[cb + u] * ld + len - 1];
-                    acc[u].add(wr.x, wr.y, xr.x, xr.y);
+                    for (int u = 0; u < DOT_COLS; u++) {
+                        if (u >= nc) break;
+                        const float2 wr = Wp[(size_t)ssel[cb - s0 + u] * ld + len - 1];
+                        acc[u].add(wr.x, wr.y, xr.x, xr.y);
+                    }
                 }
+                static_assert(DOT_COLS == 4, "pl_warp_sum4 sums four columns");
+                const PlAcc tot = pl_warp_sum4(acc);
+                if ((lane & 7) == 0 && (lane >> 3) < nc) wpart[ws * WPART_COLS + cb - b0 + (lane >> 3)] = tot.value() * back;
             }
-            static_assert(DOT_COLS == 4, "pl_warp_sum4 sums four columns");
-            const PlAcc tot = pl_warp_sum4(acc);
-            if ((lane & 7) == 0 && (lane >> 3) < nc) wpart[ws * WPART_COLS + cb - b0 + (lane >> 3)] = tot.value() * back;
+            __syncthreads();
+            for (int c = threadIdx.x; c < b1 - b0; c += BS) {
+                double s = 0.0;
+                for (int ww = 0; ww < rs; ww++) s += wpart[ww * WPART_COLS + c];
+                a.part_cols[(size_t)(b0 + c) * a.nb + blockIdx.x] = s;
+            }
+            __syncthreads();
         }
-        __syncthreads();
-        for (int c = threadIdx.x; c < b1 - b0; c += BS) {
-            double s = 0.0;
-            for (int ww = 0; ww < rs; ww++) s += wpart[ww * WPART_COLS + c];
-            a.part_cols[(size_t)(b0 + c) * a.nb + blockIdx.x] = s;
-        }
-        __syncthreads();
-    }
+        s0 += GS_COLS;
+    } while (BIG && s0 < L);
 }
 
 // x -= W(:,sel) h from the planes, and ||x||^2: one 2-element row vector
@@ -1204,13 +1244,13 @@ __device__ __forceinline__ void dots_pl(const LbArgs &a, int j, int L, double *w
 // 16-byte loads in flight.  h (scaled by the power of two of its largest
 // entry) sits in shared memory as (hi, lo) planes; each row's sum of
 // products is formed on the FP32 pipe and applied with one FP64 FMA.
-template <int SIDE>
+template <int SIDE, bool BIG>
 __device__ __forceinline__ void upd_pl(const LbArgs &a, int j, int L, double *dyn, double *buf)
 {
-    // dyn: h[L] as float2 planes (one double slot each) | sel[L]
+    // dyn: h as float2 planes (one double slot each) | sel, of the block's columns
     __shared__ int hsh;
     float2 *hp = reinterpret_cast<float2 *>(dyn);
-    int *ssel = reinterpret_cast<int *>(dyn + L);
+    int *ssel = reinterpret_cast<int *>(dyn + (BIG ? min(L, GS_COLS) : L));
     if (threadIdx.x == 0) hsh = 0;
     __syncthreads();
     int he = 0;
@@ -1219,11 +1259,6 @@ __device__ __forceinline__ void upd_pl(const LbArgs &a, int j, int L, double *dy
     __syncthreads();
     const int hs = hsh == 0 ? 0 : hsh - 1023;  // |h 2^-hs| < 2
     const double hscale = f3_pow2(-hs), back = f3_pow2(hs);
-    for (int c = threadIdx.x; c < L; c += BS) {
-        hp[c] = pl_split(a.h[c] * hscale);
-        ssel[c] = a.sel[c];
-    }
-    __syncthreads();
     const int len = SIDE == 0 ? a.adj.rows : a.fwd.rows;
     const size_t ld = SIDE == 0 ? a.ldv : a.ldu;
     const size_t ldq = ld / 2;
@@ -1233,45 +1268,59 @@ __device__ __forceinline__ void upd_pl(const LbArgs &a, int j, int L, double *dy
     double2 *xv = reinterpret_cast<double2 *>(x);
     const int nvec = len / 2;
     double sq = 0.0;
-    for (int v = blockIdx.x * BS + threadIdx.x; v < nvec; v += gridDim.x * BS) {
-        const double2 x0 = xv[v];
-        PlAcc s0, s1;
-        int c = 0;
-        for (; c + CGS_UNROLL <= L; c += CGS_UNROLL) {
-            float4 wv[CGS_UNROLL];
+    int b0 = 0;
+    do {
+        const int nb = BIG ? min(GS_COLS, L - b0) : L;
+        const bool last = !BIG || b0 + nb >= L;
+        if (BIG && b0 > 0) __syncthreads();
+        for (int c = threadIdx.x; c < nb; c += BS) {
+            hp[c] = pl_split(a.h[b0 + c] * hscale);
+            ssel[c] = a.sel[b0 + c];
+        }
+        __syncthreads();
+        for (int v = blockIdx.x * BS + threadIdx.x; v < nvec; v += gridDim.x * BS) {
+            const double2 x0 = xv[v];
+            PlAcc s0, s1;
+            int c = 0;
+            for (; c + CGS_UNROLL <= nb; c += CGS_UNROLL) {
+                float4 wv[CGS_UNROLL];
 #pragma unroll
-            for (int u = 0; u < CGS_UNROLL; u++) wv[u] = Wq[(size_t)ssel[c + u] * ldq + v];
+                for (int u = 0; u < CGS_UNROLL; u++) wv[u] = Wq[(size_t)ssel[c + u] * ldq + v];
 #pragma unroll
-            for (int u = 0; u < CGS_UNROLL; u++) {
-                const float2 hc = hp[c + u];
-                s0.add(wv[u].x, wv[u].y, hc.x, hc.y);
-                s1.add(wv[u].z, wv[u].w, hc.x, hc.y);
+                for (int u = 0; u < CGS_UNROLL; u++) {
+                    const float2 hc = hp[c + u];
+                    s0.add(wv[u].x, wv[u].y, hc.x, hc.y);
+                    s1.add(wv[u].z, wv[u].w, hc.x, hc.y);
+                }
+            }
+            for (; c < nb; c++) {
+                const float4 wc = Wq[(size_t)ssel[c] * ldq + v];
+                const float2 hc = hp[c];
+                s0.add(wc.x, wc.y, hc.x, hc.y);
+                s1.add(wc.z, wc.w, hc.x, hc.y);
+            }
+            double2 y;
+            y.x = fma(-pl_f2d(s0.c), back, fma(-pl_f2d(s0.s), back, x0.x));
+            y.y = fma(-pl_f2d(s1.c), back, fma(-pl_f2d(s1.s), back, x0.y));
+            xv[v] = y;
+            if (last) {
+                sq = fma(y.x, y.x, sq);
+                sq = fma(y.y, y.y, sq);
             }
         }
-        for (; c < L; c++) {
-            const float4 wc = Wq[(size_t)ssel[c] * ldq + v];
-            const float2 hc = hp[c];
-            s0.add(wc.x, wc.y, hc.x, hc.y);
-            s1.add(wc.z, wc.w, hc.x, hc.y);
+        if (blockIdx.x == gridDim.x - 1 && (len & 1) && threadIdx.x == 0) {
+            const int r = len - 1;
+            PlAcc sr;
+            for (int c = 0; c < nb; c++) {
+                const float2 wc = Wp[(size_t)ssel[c] * ld + r];
+                sr.add(wc.x, wc.y, hp[c].x, hp[c].y);
+            }
+            const double y = fma(-sr.value(), back, x[r]);
+            x[r] = y;
+            if (last) sq = fma(y, y, sq);
         }
-        double2 y;
-        y.x = fma(-pl_f2d(s0.c), back, fma(-pl_f2d(s0.s), back, x0.x));
-        y.y = fma(-pl_f2d(s1.c), back, fma(-pl_f2d(s1.s), back, x0.y));
-        xv[v] = y;
-        sq = fma(y.x, y.x, sq);
-        sq = fma(y.y, y.y, sq);
-    }
-    if (blockIdx.x == gridDim.x - 1 && (len & 1) && threadIdx.x == 0) {
-        const int r = len - 1;
-        PlAcc sr;
-        for (int c = 0; c < L; c++) {
-            const float2 wc = Wp[(size_t)ssel[c] * ld + r];
-            sr.add(wc.x, wc.y, hp[c].x, hp[c].y);
-        }
-        const double y = fma(-sr.value(), back, x[r]);
-        x[r] = y;
-        sq = fma(y, y, sq);
-    }
+        b0 += GS_COLS;
+    } while (BIG && b0 < L);
     block_sums<BS, 1>({sq}, buf, {a.part_sq + blockIdx.x});
 }
 
@@ -1445,37 +1494,46 @@ __device__ __forceinline__ void zdots_f64(const LbArgs &a, int j, int L)
 
 // x -= W(:,sel) h (the zgemv('N') of zcgs) and ||x||^2, one complex element
 // per thread and step; h (as double2) and the selection in shared memory
-template <int SIDE>
+template <int SIDE, bool BIG>
 __device__ __forceinline__ void zupd_f64(const LbArgs &a, int j, int L, double *dyn, double *buf)
 {
-    // dyn: h[L] as (re, im) | sel[L]
+    // dyn: h as (re, im) | sel, of the block's columns
     double2 *hs = reinterpret_cast<double2 *>(dyn);
-    int *ssel = reinterpret_cast<int *>(dyn + 2 * (size_t)L);
-    for (int c = threadIdx.x; c < L; c += BS) {
-        hs[c] = make_double2(a.h[2 * c], a.h[2 * c + 1]);
-        ssel[c] = a.sel[c];
-    }
-    __syncthreads();
+    int *ssel = reinterpret_cast<int *>(dyn + 2 * (size_t)(BIG ? min(L, GS_COLS) : L));
     const int len = (SIDE == 0 ? a.adj.rows : a.fwd.rows) / 2;
     const size_t ld = (size_t)(SIDE == 0 ? a.ldv : a.ldu) / 2;
     const double2 *W = reinterpret_cast<const double2 *>(SIDE == 0 ? a.V : a.U);
     double2 *x = reinterpret_cast<double2 *>(SIDE == 0 ? vcol<double>(a, j - 1) : ucol<double>(a, j));
     double sq = 0.0;
-    for (int v = blockIdx.x * BS + threadIdx.x; v < len; v += gridDim.x * BS) {
-        double2 acc = x[v];
-        int c = 0;
-        for (; c + CGS_UNROLL <= L; c += CGS_UNROLL) {
-            double2 wv[CGS_UNROLL];
-#pragma unroll
-            for (int u = 0; u < CGS_UNROLL; u++) wv[u] = W[(size_t)ssel[c + u] * ld + v];
-#pragma unroll
-            for (int u = 0; u < CGS_UNROLL; u++) zfms(acc, wv[u], hs[c + u]);
+    int b0 = 0;
+    do {
+        const int nb = BIG ? min(GS_COLS, L - b0) : L;
+        const bool last = !BIG || b0 + nb >= L;
+        if (BIG && b0 > 0) __syncthreads();
+        for (int c = threadIdx.x; c < nb; c += BS) {
+            hs[c] = make_double2(a.h[2 * (b0 + c)], a.h[2 * (b0 + c) + 1]);
+            ssel[c] = a.sel[b0 + c];
         }
-        for (; c < L; c++) zfms(acc, W[(size_t)ssel[c] * ld + v], hs[c]);
-        x[v] = acc;
-        sq = fma(acc.x, acc.x, sq);
-        sq = fma(acc.y, acc.y, sq);
-    }
+        __syncthreads();
+        for (int v = blockIdx.x * BS + threadIdx.x; v < len; v += gridDim.x * BS) {
+            double2 acc = x[v];
+            int c = 0;
+            for (; c + CGS_UNROLL <= nb; c += CGS_UNROLL) {
+                double2 wv[CGS_UNROLL];
+#pragma unroll
+                for (int u = 0; u < CGS_UNROLL; u++) wv[u] = W[(size_t)ssel[c + u] * ld + v];
+#pragma unroll
+                for (int u = 0; u < CGS_UNROLL; u++) zfms(acc, wv[u], hs[c + u]);
+            }
+            for (; c < nb; c++) zfms(acc, W[(size_t)ssel[c] * ld + v], hs[c]);
+            x[v] = acc;
+            if (last) {
+                sq = fma(acc.x, acc.x, sq);
+                sq = fma(acc.y, acc.y, sq);
+            }
+        }
+        b0 += GS_COLS;
+    } while (BIG && b0 < L);
     block_sums<BS, 1>({sq}, buf, {a.part_sq + blockIdx.x});
 }
 
@@ -1495,19 +1553,13 @@ __device__ __forceinline__ void zupd_f64(const LbArgs &a, int j, int L, double *
 // column c go to part_cols rows 2c (re) and 2c+1 (im), h comes out as
 // (re, im) pairs
 constexpr int ZPL_COLS = 2;
-template <int SIDE>
+template <int SIDE, bool BIG>
 __device__ __forceinline__ void zdots_pl(const LbArgs &a, int j, int L, double *wpart)
 {
-    // wpart: [PL_WARPS][2 WPART_COLS] per-slice partials | sel[kmax + 1] | fresh[kmax + 1]
+    // wpart: [PL_WARPS][2 WPART_COLS] per-slice partials | sel of GS_COLS columns and their stale flags
     int *ssel = reinterpret_cast<int *>(wpart + PL_WARPS * 2 * WPART_COLS);
-    int *sfresh = ssel + a.kmax + 1;
-    int *ok = SIDE == 0 ? a.okV : a.okU;
-    for (int c = threadIdx.x; c < L; c += BS) {
-        const int col = a.sel[c];
-        ssel[c] = col;
-        sfresh[c] = ok[col] == 0;
-    }
-    __syncthreads();
+    unsigned char *sstale = reinterpret_cast<unsigned char *>(ssel + min(a.kmax + 1, GS_COLS));
+    const int *ok = SIDE == 0 ? a.okV : a.okU;
     const int len = SIDE == 0 ? a.adj.rows : a.fwd.rows;  // real scalars: twice the complex length
     const size_t ld = SIDE == 0 ? a.ldv : a.ldu;
     const size_t ldq = ld / 2;  // leading dimension in float4 (one complex element)
@@ -1536,21 +1588,6 @@ __device__ __forceinline__ void zdots_pl(const LbArgs &a, int j, int L, double *
         const float2 p = pl_xsplit(xx.x, xs), q = pl_xsplit(xx.y, xs);
         xq[v] = make_float4(p.x, p.y, q.x, q.y);
     }
-    for (int c = 0; c < L; c++) {
-        if (!sfresh[c] || (c / ZPL_COLS) % cgs != wg) continue;
-        const int col = ssel[c];
-        float4 *Wq = reinterpret_cast<float4 *>(Wp) + (size_t)col * ldq;
-        const double2 *Wd = reinterpret_cast<const double2 *>(W + (size_t)col * ld);
-        int v = v0 + lane;
-        for (; v + 32 * (PL_SPLIT_UNROLL - 1) < v1; v += 32 * PL_SPLIT_UNROLL) {
-            double2 d[PL_SPLIT_UNROLL];
-#pragma unroll
-            for (int u = 0; u < PL_SPLIT_UNROLL; u++) d[u] = Wd[v + 32 * u];
-#pragma unroll
-            for (int u = 0; u < PL_SPLIT_UNROLL; u++) Wq[v + 32 * u] = pl_split2(d[u]);
-        }
-        for (; v < v1; v += 32) Wq[v] = pl_split2(Wd[v]);
-    }
     // conj(w) x into (re, im): w = (w.x + w.y, w.z + w.w), x likewise
     auto zacc = [](PlAcc &re, PlAcc &im, const float4 &wv, const float4 &xq4) {
         re.add(wv.x, wv.y, xq4.x, xq4.y);
@@ -1558,48 +1595,75 @@ __device__ __forceinline__ void zdots_pl(const LbArgs &a, int j, int L, double *
         im.add(wv.x, wv.y, xq4.z, xq4.w);
         im.add(wv.z, wv.w, -xq4.x, -xq4.y);
     };
-    for (int b0 = 0; b0 < L; b0 += WPART_COLS) {
-        const int b1 = min(L, b0 + WPART_COLS);
-        for (int cb = b0 + wg * ZPL_COLS; cb < b1; cb += cgs * ZPL_COLS) {
-            const int nc = min(ZPL_COLS, b1 - cb);
-            const float4 *Wq[ZPL_COLS];
-#pragma unroll
-            for (int u = 0; u < ZPL_COLS; u++)
-                Wq[u] = reinterpret_cast<const float4 *>(Wp) + (size_t)ssel[cb + (u < nc ? u : 0)] * ldq;
-            PlAcc acc[2 * ZPL_COLS];  // re, im of column cb, then of column cb + 1
+    int s0 = 0;
+    do {
+        const int s1 = BIG ? min(L, s0 + GS_COLS) : L;
+        for (int c = threadIdx.x; c < s1 - s0; c += BS) {
+            const int col = a.sel[s0 + c];
+            ssel[c] = col;
+            sstale[c] = ok[col] == 0;
+        }
+        __syncthreads();
+        // planes of the stale columns, on this lane's rows
+        for (int c = 0; c < s1 - s0; c++) {
+            if (!sstale[c] || (c / ZPL_COLS) % cgs != wg) continue;
+            const int col = ssel[c];
+            float4 *Wq = reinterpret_cast<float4 *>(Wp) + (size_t)col * ldq;
+            const double2 *Wd = reinterpret_cast<const double2 *>(W + (size_t)col * ld);
             int v = v0 + lane;
-            for (; v + 32 < v1; v += 64) {
-                float4 w0[ZPL_COLS], w1[ZPL_COLS];
+            for (; v + 32 * (PL_SPLIT_UNROLL - 1) < v1; v += 32 * PL_SPLIT_UNROLL) {
+                double2 d[PL_SPLIT_UNROLL];
 #pragma unroll
-                for (int u = 0; u < ZPL_COLS; u++) {
-                    w0[u] = __ldcs(Wq[u] + v);
-                    w1[u] = __ldcs(Wq[u] + v + 32);
-                }
-                const float4 x0 = xq[v], x1 = xq[v + 32];
+                for (int u = 0; u < PL_SPLIT_UNROLL; u++) d[u] = Wd[v + 32 * u];
 #pragma unroll
-                for (int u = 0; u < ZPL_COLS; u++) {
-                    zacc(acc[2 * u], acc[2 * u + 1], w0[u], x0);
-                    zacc(acc[2 * u], acc[2 * u + 1], w1[u], x1);
-                }
+                for (int u = 0; u < PL_SPLIT_UNROLL; u++) Wq[v + 32 * u] = pl_split2(d[u]);
             }
-            if (v < v1) {
-                const float4 x0 = xq[v];
+            for (; v < v1; v += 32) Wq[v] = pl_split2(Wd[v]);
+        }
+        for (int b0 = s0; b0 < s1; b0 += WPART_COLS) {
+            const int b1 = min(s1, b0 + WPART_COLS);
+            for (int cb = b0 + wg * ZPL_COLS; cb < b1; cb += cgs * ZPL_COLS) {
+                const int nc = min(ZPL_COLS, b1 - cb);
+                const float4 *Wq[ZPL_COLS];
 #pragma unroll
-                for (int u = 0; u < ZPL_COLS; u++) zacc(acc[2 * u], acc[2 * u + 1], __ldcs(Wq[u] + v), x0);
+                for (int u = 0; u < ZPL_COLS; u++)
+                    Wq[u] = reinterpret_cast<const float4 *>(Wp) + (size_t)ssel[cb - s0 + (u < nc ? u : 0)] * ldq;
+                PlAcc acc[2 * ZPL_COLS];  // re, im of column cb, then of column cb + 1
+                int v = v0 + lane;
+                for (; v + 32 < v1; v += 64) {
+                    float4 w0[ZPL_COLS], w1[ZPL_COLS];
+#pragma unroll
+                    for (int u = 0; u < ZPL_COLS; u++) {
+                        w0[u] = __ldcs(Wq[u] + v);
+                        w1[u] = __ldcs(Wq[u] + v + 32);
+                    }
+                    const float4 x0 = xq[v], x1 = xq[v + 32];
+#pragma unroll
+                    for (int u = 0; u < ZPL_COLS; u++) {
+                        zacc(acc[2 * u], acc[2 * u + 1], w0[u], x0);
+                        zacc(acc[2 * u], acc[2 * u + 1], w1[u], x1);
+                    }
+                }
+                if (v < v1) {
+                    const float4 x0 = xq[v];
+#pragma unroll
+                    for (int u = 0; u < ZPL_COLS; u++) zacc(acc[2 * u], acc[2 * u + 1], __ldcs(Wq[u] + v), x0);
+                }
+                static_assert(2 * ZPL_COLS == 4, "pl_warp_sum4 sums four accumulators");
+                const PlAcc tot = pl_warp_sum4(acc);
+                const int q = lane >> 3;  // accumulator q: column cb + q / 2, part q % 2
+                if ((lane & 7) == 0 && (q >> 1) < nc) wpart[(ws * WPART_COLS + cb - b0) * 2 + q] = tot.value() * back;
             }
-            static_assert(2 * ZPL_COLS == 4, "pl_warp_sum4 sums four accumulators");
-            const PlAcc tot = pl_warp_sum4(acc);
-            const int q = lane >> 3;  // accumulator q: column cb + q / 2, part q % 2
-            if ((lane & 7) == 0 && (q >> 1) < nc) wpart[(ws * WPART_COLS + cb - b0) * 2 + q] = tot.value() * back;
+            __syncthreads();
+            for (int c = threadIdx.x; c < 2 * (b1 - b0); c += BS) {
+                double s = 0.0;
+                for (int ww = 0; ww < rs; ww++) s += wpart[ww * 2 * WPART_COLS + c];
+                a.part_cols[(size_t)(2 * b0 + c) * a.nb + blockIdx.x] = s;
+            }
+            __syncthreads();
         }
-        __syncthreads();
-        for (int c = threadIdx.x; c < 2 * (b1 - b0); c += BS) {
-            double s = 0.0;
-            for (int ww = 0; ww < rs; ww++) s += wpart[ww * 2 * WPART_COLS + c];
-            a.part_cols[(size_t)(2 * b0 + c) * a.nb + blockIdx.x] = s;
-        }
-        __syncthreads();
-    }
+        s0 += GS_COLS;
+    } while (BIG && s0 < L);
 }
 
 // x -= W(:,sel) h (zgemv 'N' of zcgs) from the planes, and ||x||^2: one
@@ -1607,13 +1671,13 @@ __device__ __forceinline__ void zdots_pl(const LbArgs &a, int j, int L, double *
 // largest part) in shared memory as float4 planes (re hi, re lo, im hi,
 // im lo); Re and Im of each row's sum formed on the FP32 pipe and applied
 // with FP64 FMAs
-template <int SIDE>
+template <int SIDE, bool BIG>
 __device__ __forceinline__ void zupd_pl(const LbArgs &a, int j, int L, double *dyn, double *buf)
 {
-    // dyn: h[L] as float4 planes (two double slots each) | sel[L]
+    // dyn: h as float4 planes (two double slots each) | sel, of the block's columns
     __shared__ int hsh;
     float4 *hp = reinterpret_cast<float4 *>(dyn);
-    int *ssel = reinterpret_cast<int *>(dyn + 2 * (size_t)L);
+    int *ssel = reinterpret_cast<int *>(dyn + 2 * (size_t)(BIG ? min(L, GS_COLS) : L));
     if (threadIdx.x == 0) hsh = 0;
     __syncthreads();
     int he = 0;
@@ -1622,12 +1686,6 @@ __device__ __forceinline__ void zupd_pl(const LbArgs &a, int j, int L, double *d
     __syncthreads();
     const int hs = hsh == 0 ? 0 : hsh - 1023;  // |h 2^-hs| < 2
     const double hscale = f3_pow2(-hs), back = f3_pow2(hs);
-    for (int c = threadIdx.x; c < L; c += BS) {
-        const float2 hr = pl_split(a.h[2 * c] * hscale), hi = pl_split(a.h[2 * c + 1] * hscale);
-        hp[c] = make_float4(hr.x, hr.y, hi.x, hi.y);
-        ssel[c] = a.sel[c];
-    }
-    __syncthreads();
     const int len = SIDE == 0 ? a.adj.rows : a.fwd.rows;
     const size_t ldq = (size_t)(SIDE == 0 ? a.ldv : a.ldu) / 2;
     const float4 *Wq = reinterpret_cast<const float4 *>(SIDE == 0 ? a.Vp : a.Up);
@@ -1641,25 +1699,40 @@ __device__ __forceinline__ void zupd_pl(const LbArgs &a, int j, int L, double *d
         im.add(wv.z, wv.w, h.x, h.y);
     };
     double sq = 0.0;
-    for (int v = blockIdx.x * BS + threadIdx.x; v < nvec; v += gridDim.x * BS) {
-        const double2 x0 = xv[v];
-        PlAcc sr, si;
-        int c = 0;
-        for (; c + CGS_UNROLL <= L; c += CGS_UNROLL) {
-            float4 wv[CGS_UNROLL];
-#pragma unroll
-            for (int u = 0; u < CGS_UNROLL; u++) wv[u] = Wq[(size_t)ssel[c + u] * ldq + v];
-#pragma unroll
-            for (int u = 0; u < CGS_UNROLL; u++) zmul(sr, si, wv[u], hp[c + u]);
+    int b0 = 0;
+    do {
+        const int nb = BIG ? min(GS_COLS, L - b0) : L;
+        const bool last = !BIG || b0 + nb >= L;
+        if (BIG && b0 > 0) __syncthreads();
+        for (int c = threadIdx.x; c < nb; c += BS) {
+            const float2 hr = pl_split(a.h[2 * (b0 + c)] * hscale), hi = pl_split(a.h[2 * (b0 + c) + 1] * hscale);
+            hp[c] = make_float4(hr.x, hr.y, hi.x, hi.y);
+            ssel[c] = a.sel[b0 + c];
         }
-        for (; c < L; c++) zmul(sr, si, Wq[(size_t)ssel[c] * ldq + v], hp[c]);
-        double2 y;
-        y.x = fma(-pl_f2d(sr.c), back, fma(-pl_f2d(sr.s), back, x0.x));
-        y.y = fma(-pl_f2d(si.c), back, fma(-pl_f2d(si.s), back, x0.y));
-        xv[v] = y;
-        sq = fma(y.x, y.x, sq);
-        sq = fma(y.y, y.y, sq);
-    }
+        __syncthreads();
+        for (int v = blockIdx.x * BS + threadIdx.x; v < nvec; v += gridDim.x * BS) {
+            const double2 x0 = xv[v];
+            PlAcc sr, si;
+            int c = 0;
+            for (; c + CGS_UNROLL <= nb; c += CGS_UNROLL) {
+                float4 wv[CGS_UNROLL];
+#pragma unroll
+                for (int u = 0; u < CGS_UNROLL; u++) wv[u] = Wq[(size_t)ssel[c + u] * ldq + v];
+#pragma unroll
+                for (int u = 0; u < CGS_UNROLL; u++) zmul(sr, si, wv[u], hp[c + u]);
+            }
+            for (; c < nb; c++) zmul(sr, si, Wq[(size_t)ssel[c] * ldq + v], hp[c]);
+            double2 y;
+            y.x = fma(-pl_f2d(sr.c), back, fma(-pl_f2d(sr.s), back, x0.x));
+            y.y = fma(-pl_f2d(si.c), back, fma(-pl_f2d(si.s), back, x0.y));
+            xv[v] = y;
+            if (last) {
+                sq = fma(y.x, y.x, sq);
+                sq = fma(y.y, y.y, sq);
+            }
+        }
+        b0 += GS_COLS;
+    } while (BIG && b0 < L);
     block_sums<BS, 1>({sq}, buf, {a.part_sq + blockIdx.x});
 }
 
@@ -1777,7 +1850,7 @@ struct RunShared {
 // The phases of one half step; returns true when the run stops.
 // T double2: a native complex operator (or a host product); BLOCK: complex
 // vectors with the real 2x2-block operator (T double).
-template <int SIDE, typename T, int SHORT, int GS, bool BLOCK>
+template <int SIDE, typename T, int SHORT, int GS, bool BLOCK, bool BIG>
 __device__ __forceinline__ bool run_half(const LbArgs &a, const RunArgs &R, RunShared<T, SHORT> &sh, double *dyn,
                                          Run &rn, int j, unsigned long long &mark)
 {
@@ -1842,10 +1915,10 @@ __device__ __forceinline__ bool run_half(const LbArgs &a, const RunArgs &R, RunS
     }
     while (go == GO_CGS) {
         const int L = pub->nsel, ncols = CPLX ? 2 * L : L;
-        if constexpr (CPLX && GS == GS_PL) zdots_pl<SIDE>(a, j, L, dyn);
+        if constexpr (CPLX && GS == GS_PL) zdots_pl<SIDE, BIG>(a, j, L, dyn);
         else if constexpr (CPLX) zdots_f64<SIDE>(a, j, L);
-        else if constexpr (std::is_same<T, float>::value) dots_f32<SIDE>(a, j, L, dyn);
-        else if constexpr (GS == GS_PL) dots_pl<SIDE>(a, j, L, dyn);
+        else if constexpr (std::is_same<T, float>::value) dots_f32<SIDE, BIG>(a, j, L, dyn);
+        else if constexpr (GS == GS_PL) dots_pl<SIDE, BIG>(a, j, L, dyn);
         else if constexpr (GS == GS_F3) dots_f3<SIDE>(a, j, L);
         else dots_f64<SIDE>(a, j, L);
         // the CTAs' partials: few by CTA 0, many by one warp of the grid per
@@ -1866,11 +1939,11 @@ __device__ __forceinline__ bool run_half(const LbArgs &a, const RunArgs &R, RunS
             reduce_cols(a, ncols, gridDim.x, blockIdx.x * (BS / 32) + w, gridDim.x * (BS / 32));
             if (grid_step(R, rn, [&]() { return tail_end(R, t, 3, mark); }) == GO_STOP) return true;
         }
-        if constexpr (CPLX && GS == GS_PL) zupd_pl<SIDE>(a, j, L, dyn, sh.buf);
-        else if constexpr (CPLX) zupd_f64<SIDE>(a, j, L, dyn, sh.buf);
-        else if constexpr (std::is_same<T, double>::value && GS == GS_PL) upd_pl<SIDE>(a, j, L, dyn, sh.buf);
-        else if constexpr (std::is_same<T, double>::value && GS == GS_F3) upd_f3<SIDE>(a, j, L, dyn, sh.buf);
-        else upd_full<SIDE, T>(a, j, L, dyn, sh.buf);
+        if constexpr (CPLX && GS == GS_PL) zupd_pl<SIDE, BIG>(a, j, L, dyn, sh.buf);
+        else if constexpr (CPLX) zupd_f64<SIDE, BIG>(a, j, L, dyn, sh.buf);
+        else if constexpr (std::is_same<T, double>::value && GS == GS_PL) upd_pl<SIDE, BIG>(a, j, L, dyn, sh.buf);
+        else if constexpr (std::is_same<T, double>::value && GS == GS_F3) upd_f3<SIDE, BIG>(a, j, L, dyn, sh.buf);
+        else upd_full<SIDE, T, BIG>(a, j, L, dyn, sh.buf);
         go = grid_step(R, rn, [&]() {
             sum_parts<1>({a.part_sq}, gridDim.x, sh.buf, t);
             after_cgs<SIDE>(t, a, j);
@@ -1886,7 +1959,7 @@ __device__ __forceinline__ bool run_half(const LbArgs &a, const RunArgs &R, RunS
 template <typename T, int SHORT>
 constexpr int run_minb() { return SHORT == 1 && !std::is_same<T, double2>::value ? 4 : 3; }
 
-template <typename T, int SHORT, int GS, bool BLOCK>
+template <typename T, int SHORT, int GS, bool BLOCK, bool BIG>
 __global__ void __launch_bounds__(BS, run_minb<T, SHORT>()) k_lb_run(const __grid_constant__ LbArgs a,
                                                                      const __grid_constant__ RunArgs R)
 {
@@ -1941,9 +2014,9 @@ __global__ void __launch_bounds__(BS, run_minb<T, SHORT>()) k_lb_run(const __gri
     });
     for (int j = R.j0; j <= R.j1; j++) {
         if (j > R.j0 || R.side0 == 0)
-            if (run_half<0, T, SHORT, GS, BLOCK>(a, R, sh, dyn, rn, j, mark)) break;
+            if (run_half<0, T, SHORT, GS, BLOCK, BIG>(a, R, sh, dyn, rn, j, mark)) break;
         if (j < R.j1 || R.side1 == 1)
-            if (run_half<1, T, SHORT, GS, BLOCK>(a, R, sh, dyn, rn, j, mark)) break;
+            if (run_half<1, T, SHORT, GS, BLOCK, BIG>(a, R, sh, dyn, rn, j, mark)) break;
     }
     if (blockIdx.x == 0) {
         Tail &t = sh.t;
@@ -1963,23 +2036,26 @@ __global__ void __launch_bounds__(BS, run_minb<T, SHORT>()) k_lb_run(const __gri
 }
 
 // ------------------------------------------------------------ host side
-inline size_t pl_smem(int kmax)
+// shared memory of the projections (with planes, or of the FP32 form): the
+// slices' partials (complex: re, im), the selection and its stale flags
+inline size_t dots_smem(int kmax, bool cplx)
 {
-    return sizeof(double) * PL_WARPS * WPART_COLS + 2 * sizeof(int) * (size_t)(kmax + 1);
+    return sizeof(double) * PL_WARPS * (cplx ? 2 : 1) * WPART_COLS + (sizeof(int) + 1) * (size_t)std::min(kmax + 1, GS_COLS);
 }
-// the complex projections keep (re, im) partials per warp
-inline size_t zpl_smem(int kmax) { return pl_smem(kmax) + sizeof(double) * PL_WARPS * WPART_COLS; }
-// h (as two double slots per column at most) and the selection
-inline size_t upd_smem(int kmax) { return (2 * sizeof(double) + sizeof(int)) * (size_t)(kmax + 1) + 16; }
+// of the update: h (wide: two double slots per column) and the selection
+inline size_t upd_smem(int kmax, bool wide)
+{
+    return ((wide ? 2 : 1) * sizeof(double) + sizeof(int)) * (size_t)std::min(kmax + 1, GS_COLS) + 16;
+}
 
-template <typename T, int SHORT, int GS, bool BLOCK>
-static void launch_run(LbArgs a, RunArgs R, int want, cudaStream_t s)
+template <typename T, int SHORT, int GS, bool BLOCK, bool BIG>
+static void launch_run_as(LbArgs a, RunArgs R, int want, cudaStream_t s)
 {
     // dynamic shared memory: the Gram-Schmidt phases', then (CTA 0) the recurrences
     const int K = a.kmax;
     constexpr bool cplx = BLOCK || std::is_same<T, double2>::value;
     const bool wp = GS == GS_PL || std::is_same<T, float>::value;
-    size_t sm = std::max(upd_smem(K), wp ? (cplx ? zpl_smem(K) : pl_smem(K)) : (size_t)0);
+    size_t sm = std::max(upd_smem(K, cplx || GS == GS_F3), wp ? dots_smem(K, cplx) : (size_t)0);
     sm = (sm + 15) / 16 * 16;
     const Dev &d = device_info();
     const size_t tail = sizeof(double) * 6 * (size_t)(K + 2) + sizeof(int) * (2 * (size_t)K + 8);
@@ -2002,7 +2078,7 @@ static void launch_run(LbArgs a, RunArgs R, int want, cudaStream_t s)
     int kb = 228;
     for (int c : {196, 164, 132, 100, 64, 32})
         if (need <= (size_t)c * 1024) kb = c;
-    const void *fn = (const void *)k_lb_run<T, SHORT, GS, BLOCK>;
+    const void *fn = (const void *)k_lb_run<T, SHORT, GS, BLOCK, BIG>;
     PGB_CUDA(cudaMemsetAsync(R.sync, 0, 3 * sizeof(unsigned), s));
     // The carve-out belongs to the kernel, not to the caller's thread, and a
     // cooperative launch may not exceed the occupancy under it: hint, occupancy
@@ -2032,6 +2108,12 @@ static void launch_run(LbArgs a, RunArgs R, int want, cudaStream_t s)
     void *args[] = {&a, &R};
     PGB_CUDA(cudaLaunchCooperativeKernel(fn, dim3(g), dim3(BS), args, sm, s));
     PGB_LAUNCHED();
+}
+template <typename T, int SHORT, int GS, bool BLOCK>
+static void launch_run(const LbArgs &a, const RunArgs &R, int want, cudaStream_t s)
+{
+    if (a.kmax + 1 > GS_COLS) launch_run_as<T, SHORT, GS, BLOCK, true>(a, R, want, s);
+    else launch_run_as<T, SHORT, GS, BLOCK, false>(a, R, want, s);
 }
 
 }  // namespace pgb
