@@ -13,6 +13,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
+#include <cstddef>
 #include <cstring>
 #include <condition_variable>
 #include <functional>
@@ -737,11 +738,6 @@ struct LbResult {
     int ierr;
 };
 
-static void clear_prof(LbCtl &h)
-{
-    for (int i = 0; i < 6; i++) { h.prof_ns[i] = 0; h.prof_n[i] = 0; }
-}
-
 // Half steps (j0, side0) .. (j1, side1) on the device (one launch), then the
 // control block on the host.
 template <typename T>
@@ -759,6 +755,11 @@ static void run_steps(Ctx &c, int j0, int side0, int j1, int side1, bool host_pr
         R.w = c.op->w;
         R.z = c.zb; R.zpart = c.zpart; R.ztick = c.ztick;
     }
+    // every launch counts from zero (the device's block keeps the last one's)
+    if (g_prof_on) {
+        PGB_CUDA(cudaMemsetAsync((char *)c.ctl + offsetof(LbCtl, prof_ns), 0, sizeof(c.hctl->prof_ns), c.s));
+        PGB_CUDA(cudaMemsetAsync((char *)c.ctl + offsetof(LbCtl, prof_n), 0, sizeof(c.hctl->prof_n), c.s));
+    }
     lb_run<T>(c.args(), R, c.op && c.op->cplx == 1, c.run_ctas, c.s);
     PGB_CUDA(cudaMemcpyAsync(c.hstat, R.sync + 2, sizeof(int), cudaMemcpyDeviceToHost, c.s));
     c.get_ctl();
@@ -771,7 +772,6 @@ static void run_steps(Ctx &c, int j0, int side0, int j1, int side1, bool host_pr
         static const int kinds32[6] = {PK_SPMV_ADJ32, PK_SPMV_FWD32, PK_ELR, PK_CGS_DOTS32, PK_CGS_UPD32, PK_THIN};
         for (int i = 0; i < 6; i++)
             prof_add((sizeof(T) == 4 ? kinds32 : kinds)[i], 1e-6 * (double)c.hctl->prof_ns[i], c.hctl->prof_n[i]);
-        clear_prof(*c.hctl);
     }
 }
 
@@ -807,7 +807,6 @@ static void dev_lanbpro(Ctx &c, int k0, int *kp, double *rnorm, double *doption,
     h.elr_active = 0;
     h.reorth_active = 0;
     h.collapsed = 0;
-    clear_prof(h);
     double anorm;
     double *ba = c.hB, *bb = c.hB + c.kmax + 2;
     if (doption[2] > 0) {
