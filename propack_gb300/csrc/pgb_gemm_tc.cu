@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(OZ_WARPS * 32) k_oz_gemm(int mr, int nc, int k
                                                           const int *__restrict__ Fe, int Kp, int ncp,
                                                           double *__restrict__ C, int ldc)
 {
-    extern __shared__ unsigned short Bs[];
+    extern __shared__ __align__(16) unsigned short Bs[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int gid = lane >> 2, tig = lane & 3;
     // the column tiles of one row block are neighbours in the launch order,

@@ -1964,7 +1964,7 @@ __global__ void __launch_bounds__(BS, run_minb<T, SHORT>()) k_lb_run(const __gri
                                                                      const __grid_constant__ RunArgs R)
 {
     constexpr bool ZV = std::is_same<T, double2>::value;
-    extern __shared__ double dyn[];
+    extern __shared__ __align__(16) double dyn[];  // float4 and double2 in the complex updates
     __shared__ RunShared<T, SHORT> sh;
     Run rn;
     rn.word = &sh.word;

@@ -309,7 +309,7 @@ template <int MODE>
 __global__ void __launch_bounds__(256) k_mlp_mm(int m, const bf16 *X, const bf16 *Wt, const float *bias,
                                                const bf16 *mask, bf16 *Ob, float *Of)
 {
-    extern __shared__ unsigned short wsm[];  // 256 x W2S
+    extern __shared__ __align__(16) unsigned short wsm[];  // 256 x W2S
     for (int t = threadIdx.x; t < MLP_H * MLP_H / 2; t += blockDim.x) {
         const int n = t / (MLP_H / 2), k2 = t % (MLP_H / 2);
         reinterpret_cast<unsigned *>(wsm)[(n * W2S) / 2 + k2] = reinterpret_cast<const unsigned *>(Wt)[t];
