@@ -957,6 +957,7 @@ struct OzScratch {
     int *fe = nullptr;
     int *err = nullptr;
     int *herr = nullptr;
+    bool clear = true;  // err is to be cleared before the next product, on its stream
     size_t cap = 0, fecap = 0;
     int dev = -1;
     ~OzScratch()
@@ -991,7 +992,6 @@ static void oz_scratch(OzScratch &sc, size_t need, int nfe)
     }
     if (!sc.err) {
         PGB_CUDA(cudaMalloc(&sc.err, sizeof(int)));
-        PGB_CUDA(cudaMemset(sc.err, 0, sizeof(int)));
         PGB_CUDA(cudaMallocHost(&sc.herr, sizeof(int)));
         *sc.herr = 0;
         PGB_CUDA(cudaEventCreateWithFlags(&sc.used, cudaEventDisableTiming));
@@ -1002,7 +1002,7 @@ bool gemm_failed()
 {
     if (!t_oz.herr || *t_oz.herr == 0) return false;
     *t_oz.herr = 0;
-    cudaMemset(t_oz.err, 0, sizeof(int));
+    t_oz.clear = true;
     set_error("tensor-core GEMM: an mbarrier wait ran out");
     return true;
 }
@@ -1018,6 +1018,11 @@ static void oz_gemm_launch(int impl, int mr, int nc, int kk, const double *A, in
         const int nstage = (kk + UM_KC - 1) / UM_KC;
         oz_scratch(sc, (size_t)ntc * nstage * UM_BSTAGE / 2, ntc * UM_BN);
         PGB_CUDA(cudaStreamWaitEvent(s, sc.used, 0));
+        if (sc.clear) {
+            // (on s: a product on a non-blocking stream does not wait for a memset on the default one)
+            PGB_CUDA(cudaMemsetAsync(sc.err, 0, sizeof(int), s));
+            sc.clear = false;
+        }
         static thread_local int attr = -1;
         if (attr != 1) {
             PGB_CUDA(cudaFuncSetAttribute(k_oz_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, UM_SMEM));

@@ -947,7 +947,7 @@ static void mlp_check(Mlp &M)
     int e = 0;
     PGB_CUDA(cudaMemcpy(&e, M.err, sizeof(int), cudaMemcpyDeviceToHost));
     if (e) {
-        PGB_CUDA(cudaMemset(M.err, 0, sizeof(int)));
+        PGB_CUDA(cudaMemsetAsync(M.err, 0, sizeof(int), M.s));
         set_error("learned start: a tensor-core wait ran out");
         throw WaitFailure();
     }
@@ -1065,10 +1065,10 @@ extern "C" int propack_mlp_create(uint64_t seed, int64_t *handle)
         PGB_CUDA(cudaMalloc(&M->g, sizeof(float) * MLP_NP));
         PGB_CUDA(cudaMalloc(&M->m1, sizeof(float) * MLP_NP));
         PGB_CUDA(cudaMalloc(&M->m2, sizeof(float) * MLP_NP));
-        PGB_CUDA(cudaMemcpy(M->p, p.data(), sizeof(float) * MLP_NP, cudaMemcpyHostToDevice));
-        PGB_CUDA(cudaMemset(M->g, 0, sizeof(float) * MLP_NP));
-        PGB_CUDA(cudaMemset(M->m1, 0, sizeof(float) * MLP_NP));
-        PGB_CUDA(cudaMemset(M->m2, 0, sizeof(float) * MLP_NP));
+        PGB_CUDA(cudaMemcpyAsync(M->p, p.data(), sizeof(float) * MLP_NP, cudaMemcpyHostToDevice, M->s));
+        PGB_CUDA(cudaMemsetAsync(M->g, 0, sizeof(float) * MLP_NP, M->s));
+        PGB_CUDA(cudaMemsetAsync(M->m1, 0, sizeof(float) * MLP_NP, M->s));
+        PGB_CUDA(cudaMemsetAsync(M->m2, 0, sizeof(float) * MLP_NP, M->s));
         PGB_CUDA(cudaMalloc(&M->W1b, sizeof(bf16) * MLP_H * MLP_IN));
         PGB_CUDA(cudaMalloc(&M->W2b, sizeof(bf16) * MLP_H * MLP_H));
         PGB_CUDA(cudaMalloc(&M->W2Tb, sizeof(bf16) * MLP_H * MLP_H));
@@ -1084,7 +1084,7 @@ extern "C" int propack_mlp_create(uint64_t seed, int64_t *handle)
         PGB_CUDA(cudaFuncSetAttribute(k_mlp_mm_tc<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, TM_SMEM));
         PGB_CUDA(cudaFuncSetAttribute(k_mlp_mm_tc<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, TM_SMEM));
         PGB_CUDA(cudaMalloc(&M->err, sizeof(int)));
-        PGB_CUDA(cudaMemset(M->err, 0, sizeof(int)));
+        PGB_CUDA(cudaMemsetAsync(M->err, 0, sizeof(int), M->s));
         mlp_cast(*M);
         PGB_CUDA(cudaStreamSynchronize(M->s));
         std::lock_guard<std::mutex> lk(g_mlp_mu);

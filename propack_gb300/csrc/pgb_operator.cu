@@ -653,8 +653,8 @@ static void transpose_into(Csr &T, const int *ptr, const int *idx, const V *val,
         PGB_CUDA(cudaMalloc(&dl, sizeof(int) * hlong));
         PGB_CUDA(cudaMalloc(&doff, sizeof(int64_t) * (hlong + 1)));
         PGB_CUDA(cudaMalloc(&scr, sizeof(unsigned long long) * soff[hlong]));
-        PGB_CUDA(cudaMemcpy(dl, hl.data(), sizeof(int) * hlong, cudaMemcpyHostToDevice));
-        PGB_CUDA(cudaMemcpy(doff, soff.data(), sizeof(int64_t) * (hlong + 1), cudaMemcpyHostToDevice));
+        PGB_CUDA(cudaMemcpyAsync(dl, hl.data(), sizeof(int) * hlong, cudaMemcpyHostToDevice, s));
+        PGB_CUDA(cudaMemcpyAsync(doff, soff.data(), sizeof(int64_t) * (hlong + 1), cudaMemcpyHostToDevice, s));
         k_segsort_long<<<hlong, 1024, 0, s>>>(key, T.ptr, cnt, dl, doff, scr);
         PGB_LAUNCHED();
         PGB_CUDA(cudaStreamSynchronize(s));
@@ -1047,10 +1047,10 @@ static int create_operator(int m, int n, const int64_t *sp, const int32_t *si, c
         const int segs = std::max(op->thin_r.segs, op->thin_l.segs);
         PGB_CUDA(cudaMalloc(&op->zbuf, sizeof(double) * r));
         PGB_CUDA(cudaMalloc(&op->zpart, sizeof(double) * THIN_CAP * (size_t)r * segs));
-        PGB_CUDA(cudaMemset(op->zbuf, 0, sizeof(double) * r));
+        PGB_CUDA(cudaMemsetAsync(op->zbuf, 0, sizeof(double) * r, s));
     }
     PGB_CUDA(cudaMalloc(&op->zticket, sizeof(unsigned int) * std::max(r, 1)));
-    PGB_CUDA(cudaMemset(op->zticket, 0, sizeof(unsigned int) * std::max(r, 1)));
+    PGB_CUDA(cudaMemsetAsync(op->zticket, 0, sizeof(unsigned int) * std::max(r, 1), s));
     // FP32 copies of the values for the mixed-precision path
     for (Csr *A : {&op->fwd, &op->adj}) {
         A->valf = (float *)pool_alloc(sizeof(float) * std::max<int64_t>(A->nnz, 1), s);
@@ -1122,7 +1122,7 @@ static int create_zoperator(int m, int n, const int64_t *sp, const int32_t *si, 
         M->short_rows = 1;
     }
     PGB_CUDA(cudaMalloc(&op->zticket, sizeof(unsigned int)));
-    PGB_CUDA(cudaMemset(op->zticket, 0, sizeof(unsigned int)));
+    PGB_CUDA(cudaMemsetAsync(op->zticket, 0, sizeof(unsigned int), s));
     PGB_CUDA(cudaStreamSynchronize(s));
     PGB_CUDA(cudaStreamDestroy(s));
     {
