@@ -74,7 +74,8 @@ struct BCfg {
     double tol, min_relgap;
 };
 
-// per-CTA scratch (global memory): sizes for dimension dim
+// per-CTA scratch (global memory): sizes for dimension dim; maxrows: the most
+// rows (or columns) of a problem that one CTA owns
 struct BScrLayout {
     size_t P, Q, coef, tw, Xt, W, total;
 };
@@ -410,7 +411,7 @@ __device__ void cta_proj_pl(const float2 *Wp, int ld, int ncols, const float2 *x
         const int nc = min(DC, ncols - c0);
         PlAcc acc[DC];
         for (int i = o.a + lane; i < o.b; i += 32) {
-            const float2 xv = xq[i];
+            const float2 xv = xq[i - o.a];
 #pragma unroll
             for (int u = 0; u < DC; u++)
                 if (u < nc) {
@@ -433,7 +434,7 @@ __device__ void cta_proj_pl_dc(const float2 *Wp, int ld, int ncols, const float2
     else cta_proj_pl<1>(Wp, ld, ncols, xq, len, back, S);
 }
 
-// the CTA's own part of x as planes in xq, scaled by 2^-xs for its largest exponent
+// the CTA's own part of x as planes in xq (from its first row on), scaled by 2^-xs for its largest exponent
 // (|x 2^-xs| < 2); returns 2^xs
 __device__ double cta_xplanes(const double *x, int len, float2 *xq, BShared &S)
 {
@@ -445,13 +446,13 @@ __device__ double cta_xplanes(const double *x, int len, float2 *xq, BShared &S)
     if (e) atomicMax(&S.xe, e);
     __syncthreads();
     const int xs = S.xe == 0 ? 0 : S.xe - 1023;
-    for (int i = o.a + threadIdx.x; i < o.b; i += BT) xq[i] = pl_xsplit(x[i], xs);
+    for (int i = o.a + threadIdx.x; i < o.b; i += BT) xq[i - o.a] = pl_xsplit(x[i], xs);
     __syncthreads();
     return f3_pow2(xs);
 }
 
 // dreorth with iterated CGS on the planes of W (dreorth.F:106-210); the same
-// control flow as cta_reorth.  xq: len float2 of scratch
+// control flow as cta_reorth.  xq: float2 of scratch for the CTA's own rows
 __device__ void cta_reorth_pl(const float2 *Wp, int ld, int ncols, double *x, int len, double *nrm, BShared &S,
                               int &count, int dc, float2 *xq)
 {
@@ -833,14 +834,15 @@ __device__ void b_restart(BProb &P, const BCfg &c, BShared &S, double *scr, cons
         const double *B = side == 0 ? Pm : Qm;
         const int ldb = side == 0 ? dp1 : dim;
         const Own o = own_of(rows, S);
+        const size_t own = o.b - o.a;
         for (int i = o.a + threadIdx.x; i < o.b; i += BT)
             for (int cc = 0; cc < kout; cc++) {
                 double a = 0.0;
                 for (int l = 0; l < kin; l++) a = fma(A[(size_t)l * rows + i], B[(size_t)cc * ldb + l], a);
-                W[(size_t)cc * rows + i] = a;
+                W[cc * own + (i - o.a)] = a;
             }
         for (int cc = 0; cc < kout; cc++)
-            for (int i = o.a + threadIdx.x; i < o.b; i += BT) A[(size_t)cc * rows + i] = W[(size_t)cc * rows + i];
+            for (int i = o.a + threadIdx.x; i < o.b; i += BT) A[(size_t)cc * rows + i] = W[cc * own + (i - o.a)];
         __syncthreads();
     }
     if (threadIdx.x == 0 && S.rank == 0) {
@@ -886,15 +888,16 @@ __device__ bool b_ritz(BProb &P, const BCfg &c, BShared &S, double *scr, const B
         const int rows = side == 0 ? P.m : P.n, kin = side == 0 ? dp1 : dim;
         double *A = side == 0 ? P.U : P.V;
         const Own o = own_of(rows, S);
+        const size_t own = o.b - o.a;
         for (int i = o.a + threadIdx.x; i < o.b; i += BT)
             for (int q = 0; q < neig; q++) {
                 const double *b = side == 0 ? Xt + (size_t)q * dp1 : tw + (size_t)q * 4 * N;
                 double a = 0.0;
                 for (int l = 0; l < kin; l++) a = fma(A[(size_t)l * rows + i], b[l], a);
-                W[(size_t)q * rows + i] = a;
+                W[q * own + (i - o.a)] = a;
             }
         for (int q = 0; q < neig; q++)
-            for (int i = o.a + threadIdx.x; i < o.b; i += BT) A[(size_t)q * rows + i] = W[(size_t)q * rows + i];
+            for (int i = o.a + threadIdx.x; i < o.b; i += BT) A[(size_t)q * rows + i] = W[q * own + (i - o.a)];
         __syncthreads();
     }
     if (S.rank == 0)
@@ -1402,7 +1405,8 @@ extern "C" int propack_batch_solve(int64_t handle, int dim, int neig, int maxite
         }
         const int grid = cs * std::max(1, std::min(np, clusters));
         lc.gridDim = dim3((unsigned)grid);
-        const BScrLayout L = bscr_layout(dim, maxrows);
+        // (a cluster's CTAs share the products' rows, so their scratch is one CTA's)
+        const BScrLayout L = bscr_layout(dim, (maxrows + cs - 1) / cs);
         const size_t stride = (L.total + 31) / 32 * 32;
         alloc((void **)&scratch, sizeof(double) * stride * grid);
         // problem table
