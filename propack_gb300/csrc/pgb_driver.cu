@@ -1304,14 +1304,18 @@ static void copy_out(Ctx &c, double *U, int ldu, double *V, int ldv, int ncols, 
                             sizeof(float) * (size_t)ld, sizeof(float) * (size_t)rows, ncols, c.s);
                 continue;
             }
-            // widened on the device, all columns in one pass (the bases' pitch: one flat array)
-            const size_t len = (size_t)ld * (ncols - 1) + rows;
-            double *wide = (double *)pool_alloc(sizeof(double) * len, c.s);
-            c.allocs.push_back(wide);
-            k_widen<<<device_info().nb, 256, 0, c.s>>>(src, wide, len);
-            PGB_LAUNCHED();
-            d2h_columns((char *)(side == 0 ? U : V), sizeof(double) * (size_t)(side == 0 ? ldu : ldv),
-                        (const char *)wide, sizeof(double) * (size_t)ld, sizeof(double) * (size_t)rows, ncols, c.s);
+            // widened on the device (the bases' pitch: one flat array), as many columns
+            // at a time as the products' buffer holds: no memory beside the solve's
+            double *wide = (double *)c.gout;
+            const int fit = (int)std::max<size_t>(1, (size_t)std::max(c.ldu, c.ldv) * (c.kmax + 1) / 2 / (size_t)ld);
+            for (int c0 = 0; c0 < ncols; c0 += fit) {
+                const int nc = std::min(fit, ncols - c0);
+                k_widen<<<device_info().nb, 256, 0, c.s>>>(src + (size_t)c0 * ld, wide, (size_t)ld * (nc - 1) + rows);
+                PGB_LAUNCHED();
+                const size_t pitch = sizeof(double) * (size_t)(side == 0 ? ldu : ldv);
+                d2h_columns((char *)(side == 0 ? U : V) + pitch * c0, pitch, (const char *)wide,
+                            sizeof(double) * (size_t)ld, sizeof(double) * (size_t)rows, nc, c.s);
+            }
         }
         return;
     } else {
