@@ -53,10 +53,10 @@ struct Mlp {
     bf16 *W1b = nullptr, *W2b = nullptr, *W2Tb = nullptr, *w3b = nullptr;
     int64_t step = 0;
     int cap = 0;
-    int64_t ucap = 0, omcap = 0;
+    int64_t ucap = 0;
     float *F = nullptr, *out = nullptr, *gout = nullptr, *D1 = nullptr;
     bf16 *H1 = nullptr, *H2 = nullptr, *D2 = nullptr;
-    double *Y = nullptr, *om = nullptr, *U = nullptr, *red = nullptr, *coef = nullptr;
+    double *Y = nullptr, *U = nullptr, *red = nullptr, *coef = nullptr;
     float *part = nullptr;  // per-CTA partial sums of the reductions
     int *err = nullptr;     // set by the tensor-core kernel when a bounded wait runs out
     int device = 0;
@@ -886,15 +886,10 @@ static void mlp_features(Mlp &M, const Operator &op, unsigned long long seed)
     const int m = op.m, n = op.n;
     mlp_reserve(M, m, 1);
     const int64_t nom = (int64_t)std::max(n, 1) * MLP_SK;
-    if (nom > M.omcap) {
-        if (M.om) PGB_CUDA(cudaFree(M.om));
-        M.om = nullptr;
-        M.omcap = 0;
-        PGB_CUDA(cudaMalloc(&M.om, sizeof(double) * (size_t)nom));
-        M.omcap = nom;
-    }
+    // (16 numbers a column: the pool's, so that a wide operator's are not held beside its solve)
+    double *om = (double *)pool_alloc(sizeof(double) * (size_t)nom, M.s);
     const int full = 8 * device_info().sms;  // CTAs of 256 threads that fit at once
-    k_mlp_omega<<<std::min<int64_t>(full, (nom + 255) / 256), 256, 0, M.s>>>(n, seed, M.om);
+    k_mlp_omega<<<std::min<int64_t>(full, (nom + 255) / 256), 256, 0, M.s>>>(n, seed, om);
     PGB_LAUNCHED();
     double *Z = nullptr, *zpart = nullptr;
     unsigned *tick = nullptr;
@@ -907,16 +902,17 @@ static void mlp_features(Mlp &M, const Operator &op, unsigned long long seed)
         zpart = (double *)pool_alloc(sizeof(double) * MLP_SK * (size_t)nt, M.s);
         tick = (unsigned *)pool_alloc(sizeof(unsigned) * (size_t)op.r, M.s);
         PGB_CUDA(cudaMemsetAsync(tick, 0, sizeof(unsigned) * (size_t)op.r, M.s));
-        k_mlp_thin<<<std::max(1, std::min(full, (nt + 7) / 8)), 256, 0, M.s>>>(op.thin_r, M.om, op.w, (int)seg, nseg,
+        k_mlp_thin<<<std::max(1, std::min(full, (nt + 7) / 8)), 256, 0, M.s>>>(op.thin_r, om, op.w, (int)seg, nseg,
                                                                                          zpart, Z, tick);
         PGB_LAUNCHED();
     }
     const int64_t want = std::max<int64_t>((m + 15) / 16, std::min<int64_t>(m, op.fwd.nnz / 4096));
     const int g = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(full, MLP_RED_GRID), want));
-    k_mlp_sketch<<<g, 256, 0, M.s>>>(op.fwd, M.om, Z, M.Y, M.red);
+    k_mlp_sketch<<<g, 256, 0, M.s>>>(op.fwd, om, Z, M.Y, M.red);
     PGB_LAUNCHED();
     k_mlp_features<<<std::max(1, std::min(full, (m + 255) / 256)), 256, 0, M.s>>>(m, op.fwd.ptr, M.Y, M.red, g, M.F);
     PGB_LAUNCHED();
+    pool_free(om, M.s);
     pool_free(Z, M.s);
     pool_free(zpart, M.s);
     pool_free(tick, M.s);
@@ -1106,7 +1102,7 @@ extern "C" int propack_mlp_destroy(int64_t handle)
     cudaStreamSynchronize(M->s);
     for (void *q : {(void *)M->p, (void *)M->g, (void *)M->m1, (void *)M->m2, (void *)M->W1b, (void *)M->W2b,
                     (void *)M->W2Tb, (void *)M->w3b, (void *)M->F, (void *)M->out, (void *)M->gout, (void *)M->D1,
-                    (void *)M->H1, (void *)M->H2, (void *)M->D2, (void *)M->Y, (void *)M->om, (void *)M->U,
+                    (void *)M->H1, (void *)M->H2, (void *)M->D2, (void *)M->Y, (void *)M->U,
                     (void *)M->red, (void *)M->coef, (void *)M->part, (void *)M->err})
         if (q) cudaFree(q);
     cudaStreamDestroy(M->s);
