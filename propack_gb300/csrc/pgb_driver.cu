@@ -946,70 +946,68 @@ static void dev_lanbpro(Ctx &c, int k0, int *kp, double *rnorm, double *doption,
             set_error("device control block reports an unknown suspension");
             throw WaitFailure();
         }
-        if (h.susp_reason == 1) {
-            const int jj = h.susp_j;
-            h.status = 0;
-            if (h.susp_side == 0) {
-                // dlanbpro.F:372-405: new random v_j orthogonal to V(:,1:j-1)
-                // (u_j may still carry its deferred scale: apply it first)
+        const int jj = h.susp_j;
+        h.status = 0;
+        if (h.susp_side == 0) {
+            // dlanbpro.F:372-405: new random v_j orthogonal to V(:,1:j-1)
+            // (u_j may still carry its deferred scale: apply it first)
+            c.put_ctl();
+            apply_pend_col<T>(c, 0);
+            k_clear_pend<<<1, 1, 0, c.s>>>(c.ctl, 0);
+            PGB_LAUNCHED();
+            c.get_ctl();
+            double alpha = 0.0;
+            T *vj = c.Vcol<T>(jj - 1);
+            int e = dev_getu0<T>(c, true, jj - 1, 3, vj, &alpha, (T *)c.V, c.ldv, &anormest);
+            h.ierr = e;
+            if (alpha == 0.0) {
+                k = jj - 1;
+                h.ierr = -jj;
                 c.put_ctl();
-                apply_pend_col<T>(c, 0);
-                k_clear_pend<<<1, 1, 0, c.s>>>(c.ctl, 0);
-                PGB_LAUNCHED();
-                c.get_ctl();
-                double alpha = 0.0;
-                T *vj = c.Vcol<T>(jj - 1);
-                int e = dev_getu0<T>(c, true, jj - 1, 3, vj, &alpha, (T *)c.V, c.ldv, &anormest);
-                h.ierr = e;
-                if (alpha == 0.0) {
-                    k = jj - 1;
-                    h.ierr = -jj;
-                    c.put_ctl();
-                    finished = true;
-                    break;
-                }
-                dev_safescal<T>(c, vj, n, alpha);
-                h.alpha = 0.0;
-                h.force_reorth = 1;
-                if (h.delta > 0) h.full_reorth = 0;
-                const double z0 = 0.0;
-                PGB_CUDA(cudaMemcpyAsync(c.balpha + jj - 1, &z0, sizeof(double), cudaMemcpyHostToDevice, c.s));
-                h.pend_v.mode = 0;
-                h.pend_v_col = jj - 1;
-                c.put_ctl();
-                j = jj; side = 1;
-            } else {
-                // dlanbpro.F:503-535: new random u_{j+1} orthogonal to U(:,1:j)
-                c.put_ctl();
-                apply_pend_col<T>(c, 1);
-                k_clear_pend<<<1, 1, 0, c.s>>>(c.ctl, 1);
-                PGB_LAUNCHED();
-                c.get_ctl();
-                double beta = 0.0;
-                T *uj1 = c.Ucol<T>(jj);
-                int e = dev_getu0<T>(c, false, jj, 3, uj1, &beta, (T *)c.U, c.ldu, &anormest);
-                h.ierr = e;
-                if (beta == 0.0) {
-                    k = jj;
-                    h.ierr = -jj;
-                    c.put_ctl();
-                    finished = true;
-                    break;
-                }
-                dev_safescal<T>(c, uj1, m, beta);
-                h.beta = 0.0;
-                h.force_reorth = 1;
-                if (h.delta > 0) h.full_reorth = 0;
-                const double z0 = 0.0;
-                PGB_CUDA(cudaMemcpyAsync(c.bbeta + jj - 1, &z0, sizeof(double), cudaMemcpyHostToDevice, c.s));
-                h.pend_u.mode = 0;
-                h.pend_u_col = jj;
-                h.rnorm = 0.0;
-                c.put_ctl();
-                j = jj + 1; side = 0;
+                finished = true;
+                break;
             }
-            continue;
+            dev_safescal<T>(c, vj, n, alpha);
+            h.alpha = 0.0;
+            h.force_reorth = 1;
+            if (h.delta > 0) h.full_reorth = 0;
+            const double z0 = 0.0;
+            PGB_CUDA(cudaMemcpyAsync(c.balpha + jj - 1, &z0, sizeof(double), cudaMemcpyHostToDevice, c.s));
+            h.pend_v.mode = 0;
+            h.pend_v_col = jj - 1;
+            c.put_ctl();
+            j = jj; side = 1;
+        } else {
+            // dlanbpro.F:503-535: new random u_{j+1} orthogonal to U(:,1:j)
+            c.put_ctl();
+            apply_pend_col<T>(c, 1);
+            k_clear_pend<<<1, 1, 0, c.s>>>(c.ctl, 1);
+            PGB_LAUNCHED();
+            c.get_ctl();
+            double beta = 0.0;
+            T *uj1 = c.Ucol<T>(jj);
+            int e = dev_getu0<T>(c, false, jj, 3, uj1, &beta, (T *)c.U, c.ldu, &anormest);
+            h.ierr = e;
+            if (beta == 0.0) {
+                k = jj;
+                h.ierr = -jj;
+                c.put_ctl();
+                finished = true;
+                break;
+            }
+            dev_safescal<T>(c, uj1, m, beta);
+            h.beta = 0.0;
+            h.force_reorth = 1;
+            if (h.delta > 0) h.full_reorth = 0;
+            const double z0 = 0.0;
+            PGB_CUDA(cudaMemcpyAsync(c.bbeta + jj - 1, &z0, sizeof(double), cudaMemcpyHostToDevice, c.s));
+            h.pend_u.mode = 0;
+            h.pend_u_col = jj;
+            h.rnorm = 0.0;
+            c.put_ctl();
+            j = jj + 1; side = 0;
         }
+        continue;
     }
     // apply the deferred scaling of the newest columns (the kernel clears it)
     lb_enqueue_flush<T>(c.args(), c.s);

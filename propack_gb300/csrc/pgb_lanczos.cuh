@@ -37,9 +37,9 @@
 
 namespace pgb {
 
-// The scalar state of one tail: the control block, and the arrays of the
-// recurrences, in global memory (one kernel per phase) or in the shared
-// memory of the CTA that runs every tail (the run kernel below).
+// The scalar state of the tails: the control block, and the arrays of the
+// recurrences, in the shared memory of the CTA that runs every tail or
+// (launch_run decides) in global memory.
 constexpr int TAIL_WORDS = 128;  // bit words of the interval search: up to 4096 columns
 struct Tail {
     LbCtl c;
@@ -618,12 +618,12 @@ __device__ __forceinline__ LbPub publish(const LbCtl &c)
 
 // Shared memory of the SpMV.  SHORT 1: the matrix uses the chunked schedule
 // (compiled separately so that it carries neither the staged schedule's
-// shared memory nor its registers, and fits more CTAs per SM); 0: the staged
-// one; 2: either, by the matrix (Csr::short_rows).
+// shared memory nor its registers, and fits more CTAs per SM); 2: either
+// schedule, by the matrix (Csr::short_rows).
 template <typename T, int SHORT>
 struct SpmvShared {
     std::conditional_t<SHORT == 1, int, SpmvStage<T, T>[SPMV_WARPS]> st;
-    ChunkStage<T> cst[SHORT == 0 ? 1 : SPMV_WARPS];
+    ChunkStage<T> cst[SPMV_WARPS];
 };
 
 // The fused SpMV of one half step: the product (host_product: the caller's
